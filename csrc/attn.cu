@@ -516,6 +516,15 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
       }
     }
     const uint32_t kb = ks_a + buf * PF_BC * PF_ROW, vb = vs_a + buf * PF_BC * PF_ROW;
+    if constexpr (!FP8) {
+      if (kt == n_tiles - 1 && (n_keys & (KVB - 1)) != 0) {
+        // the last page's keys past the bound hold whatever the pool holds: their weights are 0, and 0 x V must be 0
+        const int r0 = n_keys - kt * PF_BC, r1 = (r0 + KVB - 1) / KVB * KVB;
+        for (int x = threadIdx.x; x < (r1 - r0) * PF_CHUNKS; x += blockDim.x)
+          asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(vb + pt_off(r0 + x / PF_CHUNKS, x % PF_CHUNKS)), "r"(0u) : "memory");
+        __syncthreads();
+      }
+    }
     if (have) {
     // ---- S = Q K^T for 32 keys: 4 n-tiles of 8 keys
     float sc[4][4];
