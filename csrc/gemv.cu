@@ -497,102 +497,190 @@ gemv_bf16_kernel(const bf16* x, int ldx, const bf16* __restrict__ w,
   }
 }
 
-// bf16 weights [N, K] for 3..16 activation rows on the tensor cores (mma.sync m16n8k16, fp32
-// accumulation): the weight matrix is streamed ONCE for all rows (the kernel above handles four rows
-// per pass).  A warp owns 16 weight rows; lane (g, t) = (lane / 4, lane % 4) loads 16 bytes (8
-// consecutive k) of rows g and g + 8 per 32-wide k step straight into A fragments.  A dot product
-// does not care in which order k is summed, so the 8 loaded values serve two MMAs under a fixed
-// permutation of k: fragment slots {2t, 2t+1, 2t+8, 2t+9} of the first MMA are elements 0..3 of the
-// lane's chunk, of the second elements 4..7; the B fragment (activation row g, staged as normalised
-// bf16 in shared memory) is the same 16-byte chunk of the activation row, split the same way.
-constexpr int BM_THREADS = 512, BM_PAD = 32;     // activation row stride K + 32 elements: 64 bytes off a bank cycle
-template <int NT, int EPI>                       // NT tiles of 8 activation rows
-__global__ void __launch_bounds__(BM_THREADS, 1)
-gemv_bf16_mma_kernel(const bf16* x, int ldx, const bf16* __restrict__ w, const float* __restrict__ norm_w, float eps,
-                     const bf16* residual, int ldr, void* yout, int ldy, int M, int N, int K) {
+// bf16 weights [N, K] for 1..16 activation rows on the tensor cores (mma.sync m16n8k16, fp32 accumulation): the weight
+// matrix is streamed once for all rows, which is what bounds the kernel.  KW of a block's 16 warps share the K of 16 weight
+// rows, K / KW each, so that a head of a few thousand rows (small vocabularies, tensor-parallel slices) fills every SM.  With
+// a warp per 16 whole rows, the split before this one, 15 520 rows were work for 61 of 148 SMs.  15 520 x 5120, launch included:
+// 1 / 8 / 16 rows 48 / 90 / 152 us before, 40 / 41 / 56 here (16 rows: the activation rows' shared-memory reads show);
+// 128 256 x 4096: 192 / 229 / 283 before, 184 / 185 / 192 here.
+// A warp needs its K range of the activation rows only: it loads, norms and keeps them as B fragments in its own part of shared
+// memory, 16 bytes a lane and step, and the rows' square sums are all the block exchanges.  The weights of the next steps are
+// in flight (registers, two sets) while those of this one are multiplied, across the block's reduction too.
+//
+// Lane (g, t) = (lane / 4, lane % 4) loads 16 bytes (8 consecutive k) of weight rows g and g + 8 per 32-wide step straight
+// into A fragments.  A dot product does not care in which order k is summed, so the 8 loaded values serve two MMAs under a
+// fixed permutation of k: fragment slots {2t, 2t+1, 2t+8, 2t+9} of the first MMA are elements 0..3 of the lane's chunk, of the
+// second elements 4..7; the B fragment is the same chunk of activation row g, split the same way.  The 16 partial sums of an
+// output are added in a fixed order.
+constexpr int BR_WARPS = 16, BR_THREADS = BR_WARPS * 32;
+template <int NT>
+struct BrCfg {                                   // NT tiles of 8 activation rows
+  static constexpr int RED_LD = NT * 128 + 1;    // floats of a warp's partial sums; odd: one bank apart from warp to warp
+  static constexpr size_t red_bytes(int nbuf) { return (size_t)nbuf * BR_WARPS * RED_LD * sizeof(float); }
+  static constexpr size_t x_bytes(int K, int kw) { return (size_t)BR_WARPS * ((K / 32 + kw - 1) / kw) * NT * 512; }
+};
+// BR_U: steps whose weight loads are in flight together (one set; 8 or 10 KB a warp with both)
+template <int NT, int KW, int BR_U, int EPI>
+__global__ void __launch_bounds__(BR_THREADS, 1)
+gemv_bf16_rows_kernel(const bf16* x, int ldx, const bf16* __restrict__ w, const float* __restrict__ norm_w, float eps,
+                      const bf16* residual, int ldr, void* yout, int ldy, int M, int N, int K, int nbuf, int aligned) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* xs = reinterpret_cast<bf16*>(smem_raw);                 // [NT * 8][K + BM_PAD]
-  __shared__ float red[32];
-  const int ldxs = K + BM_PAD;
+  __shared__ float ssp[BR_WARPS][NT * 8];
+  constexpr int RED_LD = BrCfg<NT>::RED_LD;
+  constexpr int RG = BR_WARPS / KW;              // groups of 16 rows a block works on at once
+  const int steps = K >> 5, per = (steps + KW - 1) / KW;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  uint4* xs = reinterpret_cast<uint4*>(smem_raw) + (size_t)warp * per * NT * 32 + lane;      // [per][NT][32]
+  float* red = reinterpret_cast<float*>(smem_raw + (size_t)BR_WARPS * per * NT * 512);        // [nbuf][warp][RED_LD]
+  const int j0 = min((warp % KW) * per, steps), nj = min(per, steps - j0), j1 = max(1, j0 + nj);
+  const int sub = (warp / KW) * 16;              // this warp's rows of a group
+  const int groups = (N + RG * 16 - 1) / (RG * 16), chunks = max(1, (nj + BR_U - 1) / BR_U);
   pdl_launch_dependents(6);
+
+  uint4 wa[2][BR_U], wb[2][BR_U];
+  // chunk c of group gr into register set `set` (compile-time after unrolling)
+  auto load = [&](uint4 (&a)[BR_U], uint4 (&b)[BR_U], int gr, int c) {
+    const bf16* pa = w + (size_t)min(gr * (RG * 16) + sub + g, N - 1) * K + (t << 3);
+    const bf16* pb = w + (size_t)min(gr * (RG * 16) + sub + g + 8, N - 1) * K + (t << 3);
+#pragma unroll
+    for (int u = 0; u < BR_U; ++u) {               // past the end: the last step again (its x is taken as zero below)
+      const int j = min(j0 + c * BR_U + u, j1 - 1) << 5;
+      a[u] = ldg_stream_16(pa + j), b[u] = ldg_stream_16(pb + j);
+    }
+  };
+  int gr = blockIdx.x, c = 0;
+  if (gr < groups) load(wa[0], wb[0], gr, 0);      // weights: constant, so before the wait for the predecessor
+
   pdl_wait();
-  for (int m = 0; m < NT * 8; ++m) {
-    bf16* dst = xs + (size_t)m * ldxs;
-    if (m >= M) {
-      for (int k = threadIdx.x; k < K; k += blockDim.x) dst[k] = __float2bfloat16(0.f);
-      continue;
-    }
-    const bf16* xr = x + (size_t)m * ldx;
-    float rstd = 1.f;
-    if (norm_w != nullptr) {
-      float ss = 0.f;
-      for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const float v = __bfloat162float(xr[k]);
-        ss += v * v;
-      }
-      ss = block_sum(ss, red);
-      rstd = rsqrtf(ss / (float)K + eps);
-    }
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-      float v = __bfloat162float(xr[k]);
-      if (norm_w != nullptr) v = v * rstd * norm_w[k];
-      dst[k] = __float2bfloat16(v);
-    }
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int warp = blockIdx.x * (BM_THREADS / 32) + (threadIdx.x >> 5);
-  const int nwarps = gridDim.x * (BM_THREADS / 32);
-  const int steps = K >> 5;                                    // 32 k per step
-  constexpr int U = NT == 1 ? 8 : 4;                           // steps whose weight loads are in flight together
-  for (int r0 = warp * 16; r0 < N; r0 += nwarps * 16) {
-    float acc[NT][4];
+  {
+    float ss[NT];
 #pragma unroll
-    for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    const bf16* wa = w + (size_t)min(r0 + g, N - 1) * K + (t << 3);
-    const bf16* wb = w + (size_t)min(r0 + g + 8, N - 1) * K + (t << 3);
-    const bf16* xb = xs + (size_t)g * ldxs + (t << 3);
-    for (int j0 = 0; j0 < steps; j0 += U) {
-      uint4 va[U], vb[U];
+    for (int i = 0; i < NT; ++i) ss[i] = 0.f;
+#pragma unroll 4
+    for (int j = 0; j < nj; ++j) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int j = min(j0 + u, steps - 1);
-        va[u] = ldg_stream_16(wa + ((size_t)j << 5));
-        vb[u] = ldg_stream_16(wb + ((size_t)j << 5));
-      }
+      for (int i = 0; i < NT; ++i) {
+        const int m = i * 8 + g;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (m < M) {
+          const bf16* xr = x + (size_t)m * ldx + ((size_t)(j0 + j) << 5) + (t << 3);
+          if (aligned) {
+            v = __ldcg(reinterpret_cast<const uint4*>(xr));
+          } else {
+            const unsigned short* h = reinterpret_cast<const unsigned short*>(xr);
+            uint32_t e[8];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (j0 + u < steps) {
-          const uint32_t a1[4] = {va[u].x, vb[u].x, va[u].y, vb[u].y};
-          const uint32_t a2[4] = {va[u].z, vb[u].z, va[u].w, vb[u].w};
-#pragma unroll
-          for (int i = 0; i < NT; ++i) {
-            const uint4 xv = *reinterpret_cast<const uint4*>(xb + (size_t)i * 8 * ldxs + ((j0 + u) << 5));
-            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                         : "+f"(acc[i][0]), "+f"(acc[i][1]), "+f"(acc[i][2]), "+f"(acc[i][3])
-                         : "r"(a1[0]), "r"(a1[1]), "r"(a1[2]), "r"(a1[3]), "r"(xv.x), "r"(xv.y));
-            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                         : "+f"(acc[i][0]), "+f"(acc[i][1]), "+f"(acc[i][2]), "+f"(acc[i][3])
-                         : "r"(a2[0]), "r"(a2[1]), "r"(a2[2]), "r"(a2[3]), "r"(xv.z), "r"(xv.w));
+            for (int k = 0; k < 8; ++k) e[k] = __ldcg(h + k);
+            v = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
           }
+        }
+        const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 f = bf162_bits_to_f2(q[k]);
+          ss[i] = fmaf(f.x, f.x, ss[i]), ss[i] = fmaf(f.y, f.y, ss[i]);
+        }
+        xs[(j * NT + i) * 32] = v;
+      }
+    }
+    if (norm_w != nullptr) {
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 1);
+        ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 2);
+        if (t == 0) ssp[warp][i * 8 + g] = ss[i];
+      }
+      __syncthreads();
+      float rstd[NT];
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < KW; ++k) v += ssp[(warp / KW) * KW + k][i * 8 + g];
+        rstd[i] = rsqrtf(v / (float)K + eps);
+      }
+#pragma unroll 2
+      for (int j = 0; j < nj; ++j) {
+        float nw[8];
+        const float* np = norm_w + ((size_t)(j0 + j) << 5) + (t << 3);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) nw[k] = np[k];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+          const uint4 v = xs[(j * NT + i) * 32];
+          const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+          uint32_t o[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float2 f = bf162_bits_to_f2(q[k]);
+            o[k] = f2_to_bf162_bits(f.x * rstd[i] * nw[2 * k], f.y * rstd[i] * nw[2 * k + 1]);
+          }
+          xs[(j * NT + i) * 32] = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
     }
-    // accumulator (row g | g + 8 of the warp's 16, activation rows 2t | 2t + 1 of tile i)
+  }
+
+  float acc[NT][4];
+#pragma unroll
+  for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+  int buf = 0;
+  // one chunk: start the loads of the following one, multiply this one, and at the end of a group add up the block's sums
+  auto chunk = [&](uint4 (&a)[BR_U], uint4 (&b)[BR_U], uint4 (&na)[BR_U], uint4 (&nb)[BR_U]) {
+    const int cc = c, cg = gr;
+    if (++c == chunks) c = 0, gr += gridDim.x;
+    if (gr < groups) load(na, nb, gr, c);
+#pragma unroll
+    for (int u = 0; u < BR_U; ++u) {
+      const int j = cc * BR_U + u;
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        uint4 xv = xs[(min(j, max(nj, 1) - 1) * NT + i) * 32];
+        if (j >= nj) xv = make_uint4(0u, 0u, 0u, 0u);
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(acc[i][0]), "+f"(acc[i][1]), "+f"(acc[i][2]), "+f"(acc[i][3])
+                     : "r"(a[u].x), "r"(b[u].x), "r"(a[u].y), "r"(b[u].y), "r"(xv.x), "r"(xv.y));
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(acc[i][0]), "+f"(acc[i][1]), "+f"(acc[i][2]), "+f"(acc[i][3])
+                     : "r"(a[u].z), "r"(b[u].z), "r"(a[u].w), "r"(b[u].w), "r"(xv.z), "r"(xv.w));
+      }
+    }
+    if (cc + 1 < chunks) return;
+    // accumulator of lane (g, t): weight rows g | g + 8, activation rows 2t | 2t + 1 of tile i
+    float* rb = red + (size_t)buf * BR_WARPS * RED_LD;
 #pragma unroll
     for (int i = 0; i < NT; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int n = r0 + g + (e >> 1) * 8, m = i * 8 + 2 * t + (e & 1);
-        if (n < N && m < M) {
-          float v = acc[i][e];
-          if (EPI == EPI_RESIDUAL) v += __bfloat162float(residual[(size_t)m * ldr + n]);
-          if (EPI == EPI_STORE_F32)
-            reinterpret_cast<float*>(yout)[(size_t)m * ldy + n] = v;
-          else
-            reinterpret_cast<bf16*>(yout)[(size_t)m * ldy + n] = __float2bfloat16(v);
-        }
+      for (int e = 0; e < 4; ++e) rb[warp * RED_LD + (i * 4 + e) * 32 + lane] = acc[i][e], acc[i][e] = 0.f;
+    __syncthreads();
+    constexpr int T = KW / (4 * NT) > 0 ? KW / (4 * NT) : 1;      // threads of an output
+    constexpr int OPT = RG * 128 * NT * T / BR_THREADS;           // outputs of a thread
+    static_assert(OPT >= 1 && OPT * BR_THREADS == RG * 128 * NT * T, "every partial sum is added once");
+#pragma unroll
+    for (int op = 0; op < OPT; ++op) {
+      const int o = (threadIdx.x + op * BR_THREADS) / T, q = threadIdx.x % T;
+      const int rg = o / (128 * NT), nl = o & 15, m = (o % (128 * NT)) >> 4, n = cg * (RG * 16) + rg * 16 + nl;
+      const float* src = rb + rg * KW * RED_LD + ((m >> 3) * 4 + ((nl >> 3) << 1) + (m & 1)) * 32 + ((nl & 7) << 2) + ((m & 7) >> 1);
+      float v = 0.f;
+#pragma unroll
+      for (int k = 0; k < KW; k += T) v += src[(k + q) * RED_LD];
+      if (T == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
+      if (T >= 2) v += __shfl_xor_sync(0xffffffffu, v, 1);
+      if (q == 0 && n < N && m < M) {
+        if (EPI == EPI_RESIDUAL) v += __bfloat162float(residual[(size_t)m * ldr + n]);
+        if (EPI == EPI_STORE_F32)
+          reinterpret_cast<float*>(yout)[(size_t)m * ldy + n] = v;
+        else
+          reinterpret_cast<bf16*>(yout)[(size_t)m * ldy + n] = __float2bfloat16(v);
       }
+    }
+    if (nbuf == 2) buf ^= 1;                       // the other buffer was last read before the barrier above
+    else __syncthreads();
+  };
+  while (gr < groups) {                            // every warp of the block runs through the same groups; those with fewer
+    chunk(wa[0], wb[0], wa[1], wb[1]);             // chunks than others (a short last range of K) only wait longer
+    if (gr >= groups) break;
+    chunk(wa[1], wb[1], wa[0], wb[0]);
   }
 }
 
@@ -713,33 +801,55 @@ TRL_API int trl_gemv_nvfp4(const void* x, int ldx, const void* wq, const void* w
   return 0;
 }
 
+// 1: trl_gemv_bf16 shares K between warps (up to 16 rows in one launch), 0: a warp for two whole rows, up to four a launch.
+// The activation rows (8 or 16, as MMA tiles go) and one reduction buffer have to fit shared memory: K up to 13 824 with
+// 8 rows, 6 656 with 16.
+constexpr size_t BR_SMEM = 226 * 1024 - 512;
+TRL_API int trl_gemv_bf16_one_pass(int M, int K) {
+  if (M < 1 || M > 16 || K % 32 != 0 || K < 32) return 0;
+  if (M == 1 && K < 2048) return 0;                // a short row for a warp of its own: 32 768 x 1024 22.6 us, 24.6 with K shared
+  return (M <= 8 ? BrCfg<1>::x_bytes(K, BR_WARPS) + BrCfg<1>::red_bytes(1) : BrCfg<2>::x_bytes(K, BR_WARPS) + BrCfg<2>::red_bytes(1)) <= BR_SMEM;
+}
+
 TRL_API int trl_gemv_bf16(const void* x, int ldx, const void* w, const void* norm_w, float eps,
                           const void* residual, int ldr, void* y, int ldy, int M, int N, int K, int epi,
                           void* stream) {
   if (K % 8 != 0 || N <= 0 || M <= 0) return (int)cudaErrorInvalidValue;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t ysz = (epi == EPI_STORE_F32) ? 4 : 2;
-  if (M > 2 && M <= 16 && K % 32 == 0 && (epi == EPI_STORE || epi == EPI_STORE_F32 || epi == EPI_RESIDUAL)) {
-    // 3..16 rows: one pass over the weights on the tensor cores, if the activation rows fit shared memory
-    // (measured on the 248 320 x 5120 head: 4 rows 762 us with the FMA kernel below, 8 rows 421 us here)
+  if (trl_gemv_bf16_one_pass(M, K) && (epi == EPI_STORE || epi == EPI_STORE_F32 || epi == EPI_RESIDUAL)) {
+    // up to 16 rows: one pass over the weights on the tensor cores
     const int nt = M <= 8 ? 1 : 2;
-    const size_t smem = (size_t)nt * 8 * (K + BM_PAD) * sizeof(bf16);
-    if (smem <= 200 * 1024) {
-      const int grid = min(num_sms(), (N + 16 * (BM_THREADS / 32) - 1) / (16 * (BM_THREADS / 32)));
-      cudaError_t e = cudaErrorInvalidValue;
-#define BM_CASE(NTT, EP)                                                                           \
-  if (nt == NTT && epi == EP) {                                                                    \
-    auto kern = gemv_bf16_mma_kernel<NTT, EP>;                                                     \
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);           \
-    e = trl_launch(kern, dim3(grid), dim3(BM_THREADS), smem, st, (const bf16*)x, ldx, (const bf16*)w, \
-                   (const float*)norm_w, eps, (const bf16*)residual, ldr, y, ldy, M, N, K);        \
+    // Warps that share K.  A barrier a group costs about as much as five steps of a warp, so K up to 5120 is shared by fewer
+    // than 16 (10 steps a warp at most) as long as there are two rounds of blocks; the
+    // activation rows are then kept once for each group of rows, which fits at these K.  The set of loads is 4 or 5 steps,
+    // whichever leaves less of the last one unused (128 256 x 4096, 16 rows: 192 us with 4, 235 with 5).
+    int kw = BR_WARPS;
+    while (kw > 4 && K / 32 <= 10 * (kw / 2) && (N + 15) / 16 >= 2 * num_sms() * (BR_WARPS / (kw / 2))) kw /= 2;
+    const size_t xb = nt == 1 ? BrCfg<1>::x_bytes(K, kw) : BrCfg<2>::x_bytes(K, kw);
+    int nbuf = 2;                                  // one reduction buffer (and a second barrier a group) where two do not fit
+    size_t smem = xb + (nt == 1 ? BrCfg<1>::red_bytes(2) : BrCfg<2>::red_bytes(2));
+    if (smem > BR_SMEM) nbuf = 1, smem = xb + (nt == 1 ? BrCfg<1>::red_bytes(1) : BrCfg<2>::red_bytes(1));
+    const int rows = 16 * (BR_WARPS / kw), grid = min(num_sms(), (N + rows - 1) / rows);
+    const int aligned = ldx % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    cudaError_t e = cudaErrorInvalidValue;
+    const int per = (K / 32 + kw - 1) / kw, u = (per + 3) / 4 * 4 < (per + 4) / 5 * 5 ? 4 : 5;
+#define BR_CASE(NTT, KWW, U, EP)                                                                          \
+  if (nt == NTT && kw == KWW && u == U && epi == EP) {                                                    \
+    auto kern = gemv_bf16_rows_kernel<NTT, KWW, U, EP>;                                                    \
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BR_SMEM);                \
+    e = trl_launch(kern, dim3(grid), dim3(BR_THREADS), smem, st, (const bf16*)x, ldx, (const bf16*)w,     \
+                   (const float*)norm_w, eps, (const bf16*)residual, ldr, y, ldy, M, N, K, nbuf, aligned); \
   }
-      BM_CASE(1, EPI_STORE) BM_CASE(1, EPI_STORE_F32) BM_CASE(1, EPI_RESIDUAL)
-      BM_CASE(2, EPI_STORE) BM_CASE(2, EPI_STORE_F32) BM_CASE(2, EPI_RESIDUAL)
-#undef BM_CASE
-      return (int)e;
-    }
+#define BR_CASES(NTT, KWW)                                                                                          \
+  BR_CASE(NTT, KWW, 4, EPI_STORE) BR_CASE(NTT, KWW, 4, EPI_STORE_F32) BR_CASE(NTT, KWW, 4, EPI_RESIDUAL)            \
+  BR_CASE(NTT, KWW, 5, EPI_STORE) BR_CASE(NTT, KWW, 5, EPI_STORE_F32) BR_CASE(NTT, KWW, 5, EPI_RESIDUAL)
+    BR_CASES(1, 4) BR_CASES(1, 8) BR_CASES(1, 16) BR_CASES(2, 4) BR_CASES(2, 8) BR_CASES(2, 16)
+#undef BR_CASES
+#undef BR_CASE
+    return (int)e;
   }
+  // one short row, rows too long for shared memory, K not a multiple of 32, more than 16 rows: fp32 FMA, up to four rows a pass
   int per = 4;
   while (per > 1 && (size_t)per * K * 4 > 190 * 1024) --per;
   for (int m0 = 0; m0 < M; m0 += per) {
@@ -747,7 +857,10 @@ TRL_API int trl_gemv_bf16(const void* x, int ldx, const void* w, const void* nor
     const bf16* xp = (const bf16*)x + (size_t)m0 * ldx;
     const bf16* rp = residual ? (const bf16*)residual + (size_t)m0 * ldr : nullptr;
     void* yp = (char*)y + (size_t)m0 * ldy * ysz;
-    const size_t smem = (size_t)mm * K * 4 + 32 * 4;
+    // at least half of an SM's shared memory: the blocks start while the kernel before them is still leaving (programmatic
+    // launch), and without it the SMs that empty first take three or four of them and the last ones none (32 768 x 1024 in a
+    // decode tick: 22.0 us after the last projection, 15.5 with one block an SM)
+    const size_t smem = max((size_t)mm * K * 4 + 32 * 4, (size_t)116 * 1024);
     const int grid = min(num_sms(), (N / 2 + GEMV_THREADS / 32 - 1) / (GEMV_THREADS / 32) + 1);
     cudaError_t e = cudaErrorInvalidValue;
 #define BF16_CASE(MM, EP)                                                                          \

@@ -222,7 +222,8 @@ class HybridModel:
         if rows is not None:
             xs = x[rows] if len(rows) else None
         else:
-            xs = x[batch.last_idx.long()] if last_only else x
+            # one token a sequence (decode ticks): every row is its sequence's last
+            xs = x[batch.last_idx.long()] if last_only and batch.n_tokens != batch.n_seqs else x
         head = P["embed"] if cfg.tie_embeddings else P["lm_head"]
         logits = None if xs is None else ops.lm_head(xs, P["final_norm"], head, eps)[..., :cfg.vocab]
         if aux_layers or return_hidden:

@@ -243,9 +243,8 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
                 x.data_ptr(), x.stride(0), w.data_ptr(), N.ptr(norm_w), eps, N.ptr(residual),
                 residual.stride(0) if residual is not None else 0, y.data_ptr(), y.stride(0),
                 m, n, k, epi, N.stream()), "gemv_bf16")
-            # 3..16 rows whose activations fit shared memory: one tensor-core pass over the weights
-            one_pass = 2 < m <= 16 and k % 32 == 0 and (8 if m <= 8 else 16) * (k + 32) * 2 <= 200 * 1024
-            N.count(1 if one_pass else (m + 3) // 4)
+            # up to 16 rows whose activations fit shared memory: one tensor-core pass over the weights
+            N.count(1 if self.lib.trl_gemv_bf16_one_pass(m, k) else (m + 3) // 4)
         elif isinstance(w, FP8BlockTensor):
             from . import gemm_fp8
             gemm_fp8.gemv(self, x, w, y, norm_w=norm_w, eps=eps, residual=residual, epi=epi)

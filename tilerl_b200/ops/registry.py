@@ -110,8 +110,8 @@ register("nvfp4", "sm100", {
 })
 register("bf16", "sm100", {
     "linear_bf16_gemv": Kernel("gemv_bf16_kernel", "csrc/gemv.cu", "trl_gemv_bf16"),
-    "linear_bf16_gemv_rows16": Kernel("gemv_bf16_mma_kernel", "csrc/gemv.cu", "trl_gemv_bf16",
-                                      note="3..16 rows (batched / verify lm_head): one mma.sync pass over the weights"),
+    "linear_bf16_gemv_rows16": Kernel("gemv_bf16_rows_kernel", "csrc/gemv.cu", "trl_gemv_bf16",
+                                      note="1..16 rows (lm_head): one mma.sync pass over the weights, K shared by a block's warps"),
     "linear_stream_rows": Kernel("linear_rows_kernel", "csrc/linear_rows.cu", "trl_linear_rows",
                                  note="few rows out of / into an fp32 stream: norm prologue, cp.async weight ring, mma.sync"),
     "linear_bf16_gemm": Kernel("torch.matmul (cuBLAS)", "tilerl_b200/ops/gemm.py", note="plain library GEMM"),
@@ -129,7 +129,8 @@ register("fp8", "sm100", {
     "attn_prep": Kernel("attn_prep_fp8_kernel", "csrc/attn_fp8.cu", "trl_attn_prep_fp8", note="e4m3 KV pool"),
     "paged_attention_decode_fused": Kernel("attn_decode_mma_kernel<true>", "csrc/attn.cu", "trl_attn_decode_fused",
                                            note="decode ticks, optional: prep + split-KV attention + split merge in one launch"),
-    "paged_attention_decode": Kernel("attn_split_fp8_kernel", "csrc/attn_fp8.cu", "trl_attn_paged_fp8"),
+    "paged_attention_decode": Kernel("attn_decode_fp8_kernel / attn_split_fp8_kernel", "csrc/attn_fp8.cu", "trl_attn_paged_fp8",
+                                     note="head dim 256 on mma.sync, 64 and 128 on FMAs"),
     "paged_attention_prefill": Kernel("attn_prefill_kernel<true>", "csrc/attn.cu", "trl_attn_prefill_fp8"),
 })
 register("any", "sm100", {
