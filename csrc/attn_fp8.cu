@@ -7,8 +7,9 @@
 //
 //   attn_prep_fp8  : q/k per-head RMSNorm + partial RoPE, normalised Q out in bf16, K / V rows
 //                    quantised and scattered with their scales (one warp per head).
-//   attn_split_fp8 : the split-KV kernel of attn.cu reading e4m3 rows (one 8-byte load per lane
-//                    at D = 256) and folding the row scales into the score and into p * V.
+//   attn_decode_fp8: head dim 256: split-KV on the tensor cores straight from the e4m3 rows (mma.sync, f16 operands, which
+//                    hold e4m3 exactly); the row scales go into the score and into the output weights.
+//   attn_split_fp8 : head dims 64 and 128: one key a warp, fp32 FMAs.
 //   attn_combine   : merge of the split partials + sigmoid gate (same maths as the bf16 path).
 //
 // Reference parity: kernels_mma.py:89-166,247-366 (fp8 write / attn_prep_fp8) and the `_fp8`
@@ -102,22 +103,13 @@ attn_prep_fp8_kernel(const bf16* qkv, int ld, const float* __restrict__ qw,
 
 template <int VEC>
 __device__ __forceinline__ void load_e4m3_row(const unsigned char* p, float (&f)[VEC]) {
-  if constexpr (VEC == 8) {
-    const uint2 w = *reinterpret_cast<const uint2*>(p);
-    const uint32_t u[2] = {w.x, w.y};
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float2 a = h2_to_f2(cvt_e4m3x2_to_h2((uint16_t)(u[i] & 0xFFFFu)));
-      const float2 b = h2_to_f2(cvt_e4m3x2_to_h2((uint16_t)(u[i] >> 16)));
-      f[4 * i] = a.x, f[4 * i + 1] = a.y, f[4 * i + 2] = b.x, f[4 * i + 3] = b.y;
-    }
-  } else if constexpr (VEC == 4) {
+  if constexpr (VEC == 4) {
     const uint32_t u = *reinterpret_cast<const uint32_t*>(p);
     const float2 a = h2_to_f2(cvt_e4m3x2_to_h2((uint16_t)(u & 0xFFFFu)));
     const float2 b = h2_to_f2(cvt_e4m3x2_to_h2((uint16_t)(u >> 16)));
     f[0] = a.x, f[1] = a.y, f[2] = b.x, f[3] = b.y;
   } else {
-    static_assert(VEC == 2, "head dim must be 64, 128 or 256");
+    static_assert(VEC == 2, "head dim must be 64 or 128");
     const float2 a = h2_to_f2(cvt_e4m3x2_to_h2(*reinterpret_cast<const uint16_t*>(p)));
     f[0] = a.x, f[1] = a.y;
   }
@@ -228,6 +220,254 @@ attn_split_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
   }
 }
 
+// ---- head dim 256 on the tensor cores ------------------------------------------------------------------
+// What bounds it is the pool's bytes, so a key's K and V are read once for the (up to 8) query heads of its kv head and go
+// from global memory to MMA fragments in registers, without a pass through shared memory.  Everything is transposed, so that
+// the few heads are the MMA's 8 columns and the accumulators stay small: S^T = K Q^T (16 keys of a page x heads), then
+// O^T += V^T P^T (16 dims x heads, 16 such tiles).  One warp works on one page at a time, its pages dealt round the block.
+// Lane (g, t) = (lane / 4, lane % 4):
+//   K   16 dims (16 bytes) of keys g and g + 8 a load: four MMAs under a fixed permutation of the dims, the query
+//       fragments (registers) permuted alike.
+//   V   16 bytes of keys 2t, 2t + 1, 2t + 8, 2t + 9 a load; byte i of two keys side by side is, converted, the A operand of
+//       dims g * 16 + i and 128 + g * 16 + i.  The next page's K is loaded when this one's scores are done, its V after the
+//       last product.
+//   P^T two f16 parts (value and rest: 22 bits), moved from accumulator to operand layout by movmatrix.  The weights that
+//       multiply V carry V's row scale and have a running maximum of their own, so that no scale leaves f16's range; the
+//       softmax's denominator is summed in fp32 from the unscaled weights.
+// Query rows are scaled by a power of two into f16's range (exact).  12 sequences of 3 000 to 6 000 keys, 4 kv heads x 6:
+// 620 us a layer with the one-key-a-warp kernel (products on the FMA pipe, a shuffle reduction for each score), 59 here with the
+// merge of the splits (the bytes: 17).
+constexpr int F8_WARPS = 4, F8_D = 256;
+
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t movmatrix_t(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+__device__ __forceinline__ uint32_t f2_to_h2_bits(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ float max_over_g(float v) {
+  v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 4));
+  v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 8));
+  return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 16));
+}
+
+__global__ void __launch_bounds__(F8_WARPS * 32)
+attn_decode_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld, const unsigned char* kcache,
+                       const unsigned char* vcache, const float* kscale, const float* vscale, const int* block_table,
+                       int max_blocks, const int* seq_ids, const int* positions, float* po, float* pm, float* pl, bf16* out,
+                       int n_q, int n_kv, int n_splits, float scale_log2e, int gated) {
+  __shared__ float s_m[F8_WARPS][MAXG], s_l[F8_WARPS][MAXG];
+  __shared__ __align__(16) float s_acc[F8_WARPS][MAXG][F8_D];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int split = blockIdx.x, kvh = blockIdx.y, tok = blockIdx.z;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int G = n_q / n_kv;
+  const int kv_len = positions[tok] + 1;
+  const int* table = block_table + (size_t)seq_ids[tok] * max_blocks;
+  const int pages = (kv_len + KVB - 1) / KVB;
+  // the launch's split count is fixed when a graph is captured, the context is not: a split gets 8 pages at least, blocks
+  // past the last one find an empty range and write a neutral partial
+  const int n_eff = max(1, min(n_splits, (pages + 7) / 8));
+  const int pps = (pages + n_eff - 1) / n_eff;
+  const int p_hi = min(pages, (split + 1) * pps);
+  int pg = split * pps + warp;
+
+  uint4 kr[2][4], vr[4][2];                        // keys g, g + 8 x 64-dim steps; keys 2t, 2t + 1, 2t + 8, 2t + 9 x halves
+  float ks[2], vs[2];
+  auto page_row = [&](int p) { return ((size_t)table[p] * n_kv + kvh) * KVB; };
+  auto load_k = [&](size_t row) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const unsigned char* src = kcache + (row + g + r * 8) * F8_D + t * 16;
+#pragma unroll
+      for (int st = 0; st < 4; ++st) kr[r][st] = __ldcg(reinterpret_cast<const uint4*>(src + st * 64));
+      ks[r] = __ldcg(kscale + row + g + r * 8);
+    }
+  };
+  auto load_v = [&](size_t row) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const unsigned char* src = vcache + (row + 2 * t + (r & 1) + (r >> 1) * 8) * F8_D + g * 16;
+      vr[r][0] = __ldcg(reinterpret_cast<const uint4*>(src)), vr[r][1] = __ldcg(reinterpret_cast<const uint4*>(src + 128));
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) vs[r] = __ldcg(vscale + row + g + r * 8);
+  };
+  size_t row = 0;
+  if (pg < p_hi) row = page_row(pg), load_k(row), load_v(row);
+
+  // query fragments: head g, dims 64 st + 16 t .. + 15; element pairs in the order of the K loads
+  uint32_t qf[4][8];
+  float qs0, qs1;                                  // score scale of heads 2t and 2t + 1
+  {
+    uint32_t raw[4][8];
+    float am = 0.f;
+#pragma unroll
+    for (int st = 0; st < 4; ++st) {
+      uint4 u0 = make_uint4(0u, 0u, 0u, 0u), u1 = u0;
+      if (g < G) {
+        const uint4* src = reinterpret_cast<const uint4*>(q + ((size_t)tok * n_q + kvh * G + g) * F8_D + st * 64 + t * 16);
+        u0 = __ldcg(src), u1 = __ldcg(src + 1);
+      }
+      const uint32_t w[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        raw[st][i] = w[i];
+        const float2 f = bf162_bits_to_f2(w[i]);
+        am = fmaxf(am, fmaxf(fabsf(f.x), fabsf(f.y)));
+      }
+    }
+    am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
+    am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
+    int e = (int)((__float_as_uint(am) >> 23) & 255u) - 127 - 10;      // the largest element to 2^10 .. 2^11
+    e = am > 0.f ? max(-116, min(126, e)) : 0;
+    const float down = __uint_as_float((uint32_t)(127 - e) << 23), up = __uint_as_float((uint32_t)(127 + e) << 23);
+#pragma unroll
+    for (int st = 0; st < 4; ++st)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 f = bf162_bits_to_f2(raw[st][i]);
+        qf[st][i] = f2_to_h2_bits(f.x * down, f.y * down);
+      }
+    qs0 = __shfl_sync(0xffffffffu, up, t * 8) * scale_log2e;
+    qs1 = __shfl_sync(0xffffffffu, up, t * 8 + 4) * scale_log2e;
+  }
+
+  float o[16][4];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  float m0 = -INFINITY, m1 = -INFINITY, n0 = -INFINITY, n1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+  while (pg < p_hi) {
+    const int left = kv_len - pg * KVB;            // keys of this page that exist
+    // ---- S^T = K Q^T
+    float sc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int st = 0; st < 4; ++st) {
+      const uint32_t ka[4] = {kr[0][st].x, kr[0][st].y, kr[0][st].z, kr[0][st].w};
+      const uint32_t kb[4] = {kr[1][st].x, kr[1][st].y, kr[1][st].z, kr[1][st].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t a[4] = {cvt_e4m3x2_to_h2((uint16_t)ka[i]), cvt_e4m3x2_to_h2((uint16_t)kb[i]),
+                               cvt_e4m3x2_to_h2((uint16_t)(ka[i] >> 16)), cvt_e4m3x2_to_h2((uint16_t)(kb[i] >> 16))};
+        mma_f16(sc, a, qf[st][2 * i], qf[st][2 * i + 1]);
+      }
+    }
+    const float k0 = ks[0], k1 = ks[1];
+    const int nxt = pg + F8_WARPS;
+    size_t nrow = 0;
+    if (nxt < p_hi) nrow = page_row(nxt), load_k(nrow);
+    // ---- scores (base 2), their running maximum, and that of the weights on V
+    const bool in0 = g < left, in1 = g + 8 < left;
+    const float lv0 = in0 ? log2f(vs[0]) : 0.f, lv1 = in1 ? log2f(vs[1]) : 0.f;
+    const float a0 = in0 ? sc[0] * (k0 * qs0) : -INFINITY, a1 = in0 ? sc[1] * (k0 * qs1) : -INFINITY;
+    const float a2 = in1 ? sc[2] * (k1 * qs0) : -INFINITY, a3 = in1 ? sc[3] * (k1 * qs1) : -INFINITY;
+    const float w0 = in0 ? a0 + lv0 : -INFINITY, w1 = in0 ? a1 + lv0 : -INFINITY;
+    const float w2 = in1 ? a2 + lv1 : -INFINITY, w3 = in1 ? a3 + lv1 : -INFINITY;
+    const float mm0 = fmaxf(m0, max_over_g(fmaxf(a0, a2))), mm1 = fmaxf(m1, max_over_g(fmaxf(a1, a3)));
+    const float nn0 = fmaxf(n0, max_over_g(fmaxf(w0, w2))), nn1 = fmaxf(n1, max_over_g(fmaxf(w1, w3)));
+    const float mb0 = mm0 == -INFINITY ? 0.f : mm0, mb1 = mm1 == -INFINITY ? 0.f : mm1;
+    const float nb0 = nn0 == -INFINITY ? 0.f : nn0, nb1 = nn1 == -INFINITY ? 0.f : nn1;
+    l0 = l0 * exp2f(m0 - mb0) + exp2f(a0 - mb0) + exp2f(a2 - mb0);      // this lane's keys; summed over g at the end
+    l1 = l1 * exp2f(m1 - mb1) + exp2f(a1 - mb1) + exp2f(a3 - mb1);
+    if (__any_sync(0xffffffffu, nn0 != n0 || nn1 != n1)) {
+      const float c0 = exp2f(n0 - nb0), c1 = exp2f(n1 - nb1);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) o[i][0] *= c0, o[i][1] *= c1, o[i][2] *= c0, o[i][3] *= c1;
+    }
+    m0 = mm0, m1 = mm1, n0 = nn0, n1 = nn1;
+    // ---- P^T: value and rest, transposed into the B operand
+    // (from the scores' distances to their own maximum: a + lv rounds at the size of a score, its maximum only sets a scale)
+    const float d0 = mb0 - nb0, d1 = mb1 - nb1;
+    const float p0 = exp2f((a0 - mb0) + (lv0 + d0)), p1 = exp2f((a1 - mb1) + (lv0 + d1));
+    const float p2 = exp2f((a2 - mb0) + (lv1 + d0)), p3 = exp2f((a3 - mb1) + (lv1 + d1));
+    const uint32_t h0 = f2_to_h2_bits(p0, p1), h1 = f2_to_h2_bits(p2, p3);
+    const float2 f0 = h2_to_f2(h0), f1 = h2_to_f2(h1);
+    const uint32_t bh0 = movmatrix_t(h0), bh1 = movmatrix_t(h1);
+    const uint32_t bl0 = movmatrix_t(f2_to_h2_bits(p0 - f0.x, p1 - f0.y)), bl1 = movmatrix_t(f2_to_h2_bits(p2 - f1.x, p3 - f1.y));
+    if (left < KVB) {
+      // the last page's keys past the sequence hold whatever the pool holds: their weights are 0, and 0 x V must be 0
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (2 * t + (r & 1) + (r >> 1) * 8 >= left) vr[r][0] = vr[r][1] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    // ---- O^T += V^T P^T
+#pragma unroll
+    for (int wi = 0; wi < 4; ++wi) {
+      uint32_t x[4][2];                            // [key][half] words wi: bytes 4 wi .. 4 wi + 3
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          x[r][h] = wi == 0 ? vr[r][h].x : wi == 1 ? vr[r][h].y : wi == 2 ? vr[r][h].z : vr[r][h].w;
+#pragma unroll
+      for (int b2 = 0; b2 < 2; ++b2) {             // two dims a byte permutation
+        const uint32_t sel = b2 == 0 ? 0x5140u : 0x7362u;
+        const uint32_t y0 = __byte_perm(x[0][0], x[1][0], sel), y1 = __byte_perm(x[0][1], x[1][1], sel);
+        const uint32_t y2 = __byte_perm(x[2][0], x[3][0], sel), y3 = __byte_perm(x[2][1], x[3][1], sel);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          const uint32_t a[4] = {cvt_e4m3x2_to_h2((uint16_t)(y0 >> (16 * b))), cvt_e4m3x2_to_h2((uint16_t)(y1 >> (16 * b))),
+                                 cvt_e4m3x2_to_h2((uint16_t)(y2 >> (16 * b))), cvt_e4m3x2_to_h2((uint16_t)(y3 >> (16 * b)))};
+          mma_f16(o[wi * 4 + b2 * 2 + b], a, bh0, bh1);
+          mma_f16(o[wi * 4 + b2 * 2 + b], a, bl0, bl1);
+        }
+      }
+    }
+    if (nxt < p_hi) load_v(nrow);
+    pg = nxt;
+  }
+#pragma unroll
+  for (int s = 4; s < 32; s <<= 1) l0 += __shfl_xor_sync(0xffffffffu, l0, s), l1 += __shfl_xor_sync(0xffffffffu, l1, s);
+
+  // ---- merge the warps: every accumulator relative to the warp's score maximum
+  {
+    const float c0 = m0 == -INFINITY ? 0.f : exp2f(n0 - m0), c1 = m1 == -INFINITY ? 0.f : exp2f(n1 - m1);
+    if (g == 0) s_m[warp][2 * t] = m0, s_m[warp][2 * t + 1] = m1, s_l[warp][2 * t] = l0, s_l[warp][2 * t + 1] = l1;
+#pragma unroll
+    for (int i = 0; i < 16; i += 4)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        *reinterpret_cast<float4*>(&s_acc[warp][2 * t][h * 128 + g * 16 + i]) =
+            make_float4(o[i][2 * h] * c0, o[i + 1][2 * h] * c0, o[i + 2][2 * h] * c0, o[i + 3][2 * h] * c0);
+        *reinterpret_cast<float4*>(&s_acc[warp][2 * t + 1][h * 128 + g * 16 + i]) =
+            make_float4(o[i][2 * h + 1] * c1, o[i + 1][2 * h + 1] * c1, o[i + 2][2 * h + 1] * c1, o[i + 3][2 * h + 1] * c1);
+      }
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < G * F8_D; idx += blockDim.x) {
+    const int gg = idx / F8_D, d = idx % F8_D;
+    float mm = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < F8_WARPS; ++w) mm = fmaxf(mm, s_m[w][gg]);
+    float ll = 0.f, a = 0.f;
+#pragma unroll
+    for (int w = 0; w < F8_WARPS; ++w) {
+      const float c = (s_m[w][gg] == -INFINITY) ? 0.f : exp2f(s_m[w][gg] - mm);
+      ll += s_l[w][gg] * c;
+      a += s_acc[w][gg][d] * c;
+    }
+    const int h = kvh * G + gg;
+    if (n_splits == 1) {
+      float v = ll > 0.f ? a / ll : 0.f;
+      if (gated) v *= sigmoid_f(__bfloat162float(gate_src[(size_t)tok * gate_ld + (size_t)h * 2 * F8_D + F8_D + d]));
+      out[((size_t)tok * n_q + h) * F8_D + d] = __float2bfloat16(v);
+    } else {
+      const size_t base = ((size_t)tok * n_q + h) * n_splits + split;
+      po[base * F8_D + d] = a;
+      if (d == 0) pm[base] = mm, pl[base] = ll;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256)
 attn_combine_fp8_kernel(const float* po, const float* pm,
                         const float* pl, const bf16* gate_src, int gate_ld,
@@ -291,7 +531,11 @@ TRL_API int trl_attn_paged_fp8(const void* q, const void* gate_src, int gate_ld,
                    (const int*)positions, (float*)po, (float*)pm, (float*)pl, (bf16*)out, n_q, n_kv,  \
                    n_splits, sl2, gated);                                                             \
   }
-  if (D == 256) SPLIT_CASE(8)
+  if (D == F8_D)
+    e = trl_launch(attn_decode_fp8_kernel, grid, dim3(F8_WARPS * 32), 0, st, (const bf16*)q, (const bf16*)gate_src, gate_ld,
+                   (const unsigned char*)kcache, (const unsigned char*)vcache, (const float*)kscale, (const float*)vscale,
+                   (const int*)block_table, max_blocks, (const int*)seq_ids, (const int*)positions, (float*)po, (float*)pm,
+                   (float*)pl, (bf16*)out, n_q, n_kv, n_splits, sl2, gated);
   else if (D == 128) SPLIT_CASE(4)
   else if (D == 64) SPLIT_CASE(2)
   else return (int)cudaErrorInvalidValue;

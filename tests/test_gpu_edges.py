@@ -44,3 +44,61 @@ def test_bf16_rows_for_every_split_of_k(ops, m, n, k, shift):
     ops.gemv_now(x, w, y, norm_w=nw, eps=1e-6, epi=3)
     h = ref.rmsnorm(x, nw, 1e-6).to(torch.bfloat16)
     assert _rel(y, h.double() @ w.double().t()) < 2e-4 + 2 ** -8 / k ** 0.5
+
+
+@pytest.mark.parametrize("g_heads,splits", [(1, 1), (6, 1), (6, 5), (8, 3)])
+@pytest.mark.parametrize("scale_v", [1.0, 1e-25, 1e12])
+def test_fp8_attention_on_tensor_cores(ops, g_heads, splits, scale_v):
+    """Contexts at the edges of pages and splits, bytes past the sequence's end that are NaN, V of any magnitude, query rows far
+    from one, against 64 bits.  The split's partial sums are fp32: weights in two f16 parts leave 2^-22 of each, sums over up
+    to 1 100 keys their fp32 rounding; the finished row is bf16."""
+    from tilerl_b200.ops import native as N
+    import math
+    n_kv, d = 2, 256
+    n_q = n_kv * g_heads
+    lens = [1, 2, 15, 16, 17, 127, 128, 129, 511, 1100]
+    g = torch.Generator(device=DEV).manual_seed(g_heads * 10 + splits)
+    t = len(lens)
+    mb = (max(lens) + 15) // 16
+    pages = t * mb + 1
+    e4 = lambda x: x.clamp(-448, 448).to(torch.float8_e4m3fn)
+    k8 = e4(torch.randn(pages, n_kv, 16, d, generator=g, device=DEV) * 40)
+    v8 = e4(torch.randn(pages, n_kv, 16, d, generator=g, device=DEV) * 100)
+    ks = torch.rand(pages, n_kv, 16, generator=g, device=DEV) * 0.02 + 0.01
+    vs = torch.exp(torch.randn(pages, n_kv, 16, generator=g, device=DEV)) * scale_v
+    table = (torch.randperm(pages - 1, generator=g, device=DEV)[:t * mb] + 1).int().view(t, mb)
+    kd, vd = k8.double() * ks.double().unsqueeze(-1), v8.double() * vs.double().unsqueeze(-1)
+    for i, n in enumerate(lens):                        # what lies past the sequence's end must not matter
+        if n % 16:
+            b = int(table[i, n // 16])
+            for s in (k8, v8):
+                s[b].view(torch.uint8)[:, n % 16:] = 0x7f
+            ks[b, :, n % 16:] = vs[b, :, n % 16:] = float("nan")
+    q = torch.randn(t, n_q, d, generator=g, device=DEV)
+    q[1] *= 2.0 ** 20
+    q[2] *= 2.0 ** -30
+    q[3] = 0
+    q = q.to(torch.bfloat16)
+    gate = torch.randn(t, n_q * 2 * d, generator=g, device=DEV).to(torch.bfloat16)
+    po = torch.full((t, n_q, splits, d), float("nan"), device=DEV)
+    pm, pl = (torch.full((t, n_q, splits), float("nan"), device=DEV) for _ in range(2))
+    out = torch.full((t, n_q * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV)
+    sid = torch.arange(t, dtype=torch.int32, device=DEV)
+    N.check(ops.lib.trl_attn_paged_fp8(q.data_ptr(), gate.data_ptr(), gate.stride(0), k8.data_ptr(), v8.data_ptr(), ks.data_ptr(),
+                                       vs.data_ptr(), table.data_ptr(), mb, sid.data_ptr(), pos.data_ptr(), po.data_ptr(),
+                                       pm.data_ptr(), pl.data_ptr(), out.data_ptr(), t, n_q, n_kv, d, splits, 1 / math.sqrt(d), 1,
+                                       N.stream()), "attn_paged_fp8")
+    for i, n in enumerate(lens):
+        b = table[i].long()
+        kk = kd[b].transpose(1, 2).reshape(-1, n_kv, d)[:n]
+        vv = vd[b].transpose(1, 2).reshape(-1, n_kv, d)[:n]
+        s = torch.einsum("hgd,nhd->hgn", q[i].double().view(n_kv, g_heads, d), kk) / math.sqrt(d)
+        want = torch.einsum("hgn,nhd->hgd", torch.softmax(s, -1), vv).reshape(n_q, d)
+        if splits > 1:
+            c = torch.exp2(pm[i].double() - pm[i].double().amax(-1, keepdim=True))
+            got = (po[i].double() * c.unsqueeze(-1)).sum(1) / (pl[i].double() * c).sum(1, keepdim=True)
+            tol = 2e-2 if i == 1 else 2e-5             # scores of 10^8: the last bit of an fp32 score is a factor in a weight
+            assert _rel(got, want) < tol, (n, _rel(got, want))
+        final = want * torch.sigmoid(gate[i].double().view(n_q, 2, d)[:, 1])
+        assert _rel(out[i].view(n_q, d), final) < (2e-2 if i == 1 else 2 ** -8), n

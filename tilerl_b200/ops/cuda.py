@@ -479,6 +479,10 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
             N.count(2)
             return out
         splits = self.attn_splits or self._pick_splits(batch, t, n_kv)
+        if d == 256:
+            # blocks of four warps, two to an SM, and contexts of unlike length: several splits a block slot even them out
+            # (the kernel gives a split eight pages at least)
+            splits = max(splits, min(64, -(-8 * self.sms // max(1, t * n_kv))))
         po = self.ws.get("attn_po", (t * n_q * splits * d,), torch.float32)
         pm = self.ws.get("attn_pm", (t * n_q * splits,), torch.float32)
         pl = self.ws.get("attn_pl", (t * n_q * splits,), torch.float32)
