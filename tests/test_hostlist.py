@@ -1,0 +1,77 @@
+"""Python lists into int32 staging memory (``csrc/hostlist.cu``): the same values as numpy's conversion, and everything that is
+not a plain list of integers left to it."""
+import numpy as np
+import pytest
+import torch
+
+from tilerl_b200.batch import Batch
+from tilerl_b200.graph import _Bucket, take_rows
+from tilerl_b200.ops import native
+
+needs_lib = pytest.mark.skipif(not native.loadable(), reason="the kernel library is not built")
+
+
+def _fill(b, mb, seqs, general):
+    bk = _Bucket(b, mb, torch.device("cpu"))
+    bk.np[:] = 7
+    keep = native.fill_decode
+    if general:
+        native.fill_decode = lambda *a: False
+    try:
+        bk.fill(seqs)
+    finally:
+        native.fill_decode = keep
+    return bk.np.copy(), bk.h2d_bytes
+
+
+@needs_lib
+@pytest.mark.parametrize("b,n,mb", [(1, 1, 1), (4, 3, 9), (8, 8, 130), (2, 0, 4)])
+def test_decode_inputs_equal_the_general_fill(b, n, mb):
+    rng = np.random.RandomState(b + mb)
+    seqs = []
+    for i in range(n):
+        nb = int(rng.randint(1, mb + 1))
+        seqs.append(dict(tokens=[int(rng.randint(1 << 17))], start=int(rng.randint(16 * nb)), slot=i + 1, keep=True,
+                         blocks=[int(v) for v in rng.randint(1, 1 << 20, nb)]))
+    if seqs:
+        assert native.fill_decode(seqs, np.empty(5 * b + b * mb, np.int32).ctypes.data, b, mb, 16)
+    got, want = _fill(b, mb, seqs, False), _fill(b, mb, seqs, True)
+    assert (got[0] == want[0]).all() and got[1] == want[1]
+
+
+@needs_lib
+def test_other_forms_go_the_general_way():
+    plain = dict(tokens=[3], start=20, blocks=[4, 5], slot=1)
+    room = np.empty(64, np.int32)
+    ok = lambda s: native.fill_decode(s, room.ctypes.data, 2, 4, 16)
+    assert ok([plain])
+    for change in (dict(tokens=torch.tensor([3])), dict(tokens=[3, 4]), dict(start=np.int64(20)), dict(start=-1), dict(start=32), dict(blocks=(4, "x")),
+                   dict(blocks=np.array([4, 5])), dict(blocks=[1] * 5), dict(blocks=[-1, 2]), dict(slot=None), dict(slot=True)):
+        assert not ok([dict(plain, **change)]), change
+    assert not ok([plain] * 3) and not ok((plain,)) and not ok([plain, 5])
+    # what the general way takes it still takes, and what it refuses it still refuses
+    a = _fill(2, 4, [dict(plain, blocks=np.array([4, 5]), start=np.int64(20))], False)[0]
+    assert (a == _fill(2, 4, [plain], True)[0]).all()
+    with pytest.raises(IndexError):
+        _fill(2, 4, [dict(plain, start=40)], False)
+
+
+@needs_lib
+def test_list_conversion_checks_type_range_and_room():
+    out = np.full(8, -7, np.int32)
+    conv = lambda x, cap=8, lo=-(1 << 31), hi=1 << 31: native.list_i32(x, out.ctypes.data, cap, lo, hi)
+    assert conv([5, -(1 << 31), (1 << 31) - 1]) == 3 and out[:4].tolist() == [5, -(1 << 31), (1 << 31) - 1, -7]
+    assert conv((9, 8)) == 2 and out[:2].tolist() == [9, 8] and conv([]) == 0
+    for bad in ([1.0], ["1"], [True], [1 << 31], [1 << 80], [None], np.arange(3), "12", {1: 2}):
+        assert conv(bad) == -1, bad
+    assert conv([1, 10], hi=10) == -1 and conv([-1], lo=0) == -1 and conv([1] * 9) == -2
+
+
+@pytest.mark.parametrize("rows", [[0], [3], [1, 2, 3], [0, 2], [2, 1], [1, 1], [-1], [-2, -1], []])
+def test_rows_that_are_a_range_equal_an_index(rows):
+    x = torch.arange(20.0).view(5, 4)
+    got = take_rows(x, rows)
+    assert torch.equal(got, x[torch.tensor(rows, dtype=torch.long)])
+    assert got.data_ptr() != x.data_ptr() or not len(rows)
+    r = Batch.row_range(rows)
+    assert r is None or list(range(5))[r] == rows

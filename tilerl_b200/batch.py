@@ -10,7 +10,6 @@ rows to a common width and masks with ``seq_q_lens`` -- here rows are ragged.
 """
 from __future__ import annotations
 
-import itertools
 import os
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence
@@ -43,6 +42,14 @@ class Batch:
     keep_rows: List[bool] = field(default_factory=list)   # per sequence: store per-token GDN states
     keep_flags: Optional[torch.Tensor] = None             # [B] int32 device copy of keep_rows
     h2d_bytes: int = 0
+
+    @staticmethod
+    def row_range(rows) -> Optional[slice]:
+        """The slice that a list of row numbers is, None when it is not a range (usual: every row, or the last one)."""
+        n = len(rows)
+        if n == 0 or rows[0] < 0 or rows[-1] - rows[0] + 1 != n or any(rows[i + 1] - rows[i] != 1 for i in range(n - 1)):
+            return None
+        return slice(rows[0], rows[-1] + 1)
 
     @staticmethod
     def build(seqs: Sequence[dict], device, max_blocks: Optional[int] = None,
@@ -124,8 +131,8 @@ def _fill_native(seqs, ql, keep, mb: int, flat: torch.Tensor) -> bool:
     nb = [len(s["blocks"]) for s in seqs]
     blk_off = np.zeros(n + 1, dtype=np.int32)
     np.cumsum(nb, out=blk_off[1:])
-    tokens = np.fromiter(itertools.chain.from_iterable(s["tokens"] for s in seqs), dtype=np.int32, count=int(tok_off[-1]))
-    blocks = np.fromiter(itertools.chain.from_iterable(s["blocks"] for s in seqs), dtype=np.int32, count=int(blk_off[-1]))
+    tokens = _joined([s["tokens"] for s in seqs], tok_off)
+    blocks = _joined([s["blocks"] for s in seqs], blk_off)
     starts = np.fromiter((int(s["start"]) for s in seqs), dtype=np.int32, count=n)
     slots = np.fromiter((int(s["slot"]) for s in seqs), dtype=np.int32, count=n)
     kp = np.fromiter((int(k) for k in keep), dtype=np.int32, count=n)
@@ -137,6 +144,17 @@ def _fill_native(seqs, ql, keep, mb: int, flat: torch.Tensor) -> bool:
     if wrote != flat.numel():
         raise RuntimeError(f"trl_batch_fill wrote {wrote} of {flat.numel()} values")
     return True
+
+
+def _joined(lists, off) -> np.ndarray:
+    """The integers of several lists back to back, int32."""
+    from .ops import native
+    out = np.empty(int(off[-1]), dtype=np.int32)
+    for i, x in enumerate(lists):
+        n = int(off[i + 1] - off[i])
+        if native.list_i32(x, out.ctypes.data + 4 * int(off[i]), n) != n:
+            out[off[i]:off[i + 1]] = np.fromiter(x, dtype=np.int32, count=n)
+    return out
 
 
 _RT = {"lib": None, "tried": False}

@@ -14,6 +14,7 @@ from __future__ import annotations
 import hashlib
 import os
 import subprocess
+import sysconfig
 import sys
 from concurrent.futures import ThreadPoolExecutor
 from typing import Optional
@@ -113,7 +114,7 @@ def build(force: bool = False, verbose: bool = False, extra_flags=(), trace: boo
         stamp = _stamp(sp)
         if not force and os.path.exists(op) and os.path.exists(st) and open(st).read() == stamp:
             continue
-        cmd = [nvcc, *NVCC_FLAGS, *extra_flags, "-x", "cu", "-c", sp, "-o", op]
+        cmd = [nvcc, *NVCC_FLAGS, *extra_flags, "-I", sysconfig.get_paths()["include"], "-x", "cu", "-c", sp, "-o", op]
         jobs.append((cmd, st, stamp))
 
     def run(job):

@@ -26,11 +26,13 @@ from collections import deque
 from dataclasses import dataclass, field
 from typing import Callable, Deque, Dict, List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
 from .batch import Batch
+from .graph import take_rows
 from .kv import GdnStatePool, NoPrefixStore, PagedKvPool, PoolExhausted
-from .ops import ref
+from .ops import native, ref
 from .ops.ref import KV_BLOCK
 
 
@@ -184,6 +186,7 @@ class Engine:
         self._running: List[_Req] = []
         self._reqs: Dict[int, _Req] = {}
         self._fed: Dict[str, _Req] = {}       # open requests of feed()
+        self._scratch_ids = np.empty(4096, dtype=np.int32)
         self._thread: Optional[threading.Thread] = None
         self._stop = threading.Event()
         self._wake = threading.Event()
@@ -415,7 +418,8 @@ class Engine:
                     raise ValueError(f"request {k!r} is not open")
             for key, tokens, want in entries:
                 n0 = len(self._fed[key].prompt) if key in self._fed else 0
-                if not len(tokens) or any(not 0 <= int(t) < self.model.cfg.vocab for t in tokens):
+                n = len(tokens)
+                if not n or (not self._plain_tokens(tokens) and any(not 0 <= int(t) < self.model.cfg.vocab for t in tokens)):
                     raise ValueError(f"request {key!r}: no tokens, or a token outside the vocabulary")
                 if any(not 0 <= int(w) < len(tokens) for w in want):
                     raise ValueError(f"request {key!r}: a wanted place outside its tokens")
@@ -428,7 +432,7 @@ class Engine:
                     r = _Req(self._next, [], SamplingParams(), state=PREFILL, slot=self.states.alloc_slot())
                     self._next += 1
                     self._fed[key] = r
-                start, toks = r.n_computed, [int(t) for t in tokens]
+                start, toks = r.n_computed, (list(tokens) if self._plain_tokens(tokens) else [int(t) for t in tokens])
                 if not self._grow(r, start + len(toks)):
                     raise PoolExhausted("KV pool has no free block for the fed tokens")
                 r.state = DECODE if start and len(toks) == 1 else PREFILL
@@ -449,6 +453,13 @@ class Engine:
             for k in end:
                 self._give_back(self._fed.pop(k))
             return logits
+
+    def _plain_tokens(self, tokens) -> bool:
+        """A list or tuple of plain integers inside the vocabulary (checked without an interpreter loop)."""
+        n = len(tokens)
+        if len(self._scratch_ids) < n:
+            self._scratch_ids = np.empty(max(n, 2 * len(self._scratch_ids)), dtype=np.int32)
+        return native.list_i32(tokens, self._scratch_ids.ctypes.data, n, 0, self.model.cfg.vocab) == n
 
     def _check_device_error(self) -> None:
         """A kernel's bounded wait that ran out (a TP peer that never pushed its partial rows, a
@@ -579,7 +590,7 @@ class Engine:
                 g = self.graph.run(seqs)
                 if g is not None:
                     self.counters["graph_ticks"] += 1
-                    out.logits, out.argmax = (g.logits, g.argmax) if rows is None else (g.logits[rows], None)
+                    out.logits, out.argmax = (g.logits, g.argmax) if rows is None else (take_rows(g.logits, rows), None)
                     return out
             if self.vgraph is not None and verify:
                 greedy = all(self._is_plain_greedy(r) for r, _, _ in plan)

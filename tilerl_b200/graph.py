@@ -22,6 +22,7 @@ import numpy as np
 import torch
 
 from .batch import Batch
+from .ops import native
 from .ops.ref import KV_BLOCK
 
 GRAPH_BUCKETS = (1, 2, 4, 8, 16, 24, 32, 48, 64, 96, 128)
@@ -32,6 +33,12 @@ def bucket_for(n: int, buckets: Sequence[int] = GRAPH_BUCKETS) -> Optional[int]:
         if n <= b:
             return b
     return None
+
+
+def take_rows(x: torch.Tensor, rows: Sequence[int]) -> torch.Tensor:
+    """``x[rows]`` (a new tensor), without an index tensor where the rows are a range."""
+    r = Batch.row_range(rows)
+    return x[rows] if r is None else x[r].clone()
 
 
 @dataclass
@@ -70,6 +77,9 @@ class _Bucket:
 
     def fill(self, seqs: Sequence[dict]) -> None:
         b, mb, a = self.b, self.max_blocks, self.np
+        self.h2d_bytes = a.nbytes
+        if native.fill_decode(seqs, a.ctypes.data, b, mb, KV_BLOCK):
+            return
         a[:] = 0  # pad rows: token 0, position 0, slot row 0 of page 0, state slot 0
         for r, s in enumerate(seqs):
             pos = int(s["start"])
@@ -80,7 +90,6 @@ class _Bucket:
             a[3 * b + r] = pos + 1
             a[4 * b + r] = s["slot"]
             a[5 * b + r * mb: 5 * b + r * mb + len(blocks)] = blocks
-        self.h2d_bytes = a.nbytes
 
 
 class DecodeGraphRunner:
@@ -326,7 +335,6 @@ class VerifyGraphRunner:
         self.d2h_bytes += (bk.tok_host.numel() if bk.out_pack is not None else t) * 4
         th = bk.tok_host.tolist()
         accept = th[t:t + len(seqs)] if bk.out_pack is not None else None
-        idx = torch.tensor(rows, dtype=torch.long, device=self.device) if (need_logits or bk.out_taps) else None
-        taps = {l: v[idx] for l, v in bk.out_taps.items()} if bk.out_taps else None
-        logits = bk.out_logits[idx] if need_logits else bk.out_logits
+        taps = {l: take_rows(v, rows) for l, v in bk.out_taps.items()} if bk.out_taps else None
+        logits = take_rows(bk.out_logits, rows) if need_logits else bk.out_logits
         return VerifyOut(logits, [th[r] for r in rows], taps, accept)

@@ -220,7 +220,8 @@ class HybridModel:
                 taps[i] = x.clone()  # the residual stream is updated in place
         settle()
         if rows is not None:
-            xs = x[rows] if len(rows) else None
+            span = batch.row_range(rows)
+            xs = x[rows if span is None else span] if len(rows) else None
         else:
             # one token a sequence (decode ticks): every row is its sequence's last
             xs = x[batch.last_idx.long()] if last_only and batch.n_tokens != batch.n_seqs else x

@@ -166,6 +166,36 @@ def lib() -> ctypes.CDLL:
     return _LIB
 
 
+_PYLIB = None        # the same library called with the interpreter locked: False when it has no such entry point
+
+
+def list_i32(seq, dst: int, cap: int, lo: int = -(1 << 31), hi: int = 1 << 31) -> int:
+    """The integers of a list or tuple into the int32 memory at ``dst`` (room for ``cap``); returns how many.  -1: not a list or
+    tuple of plain integers in ``[lo, hi)``, or a library without the entry point (callers then convert with numpy); -2: more
+    than ``cap``."""
+    lib_ = _pylib()
+    return lib_.trl_list_i32(seq, dst, cap, lo, hi) if lib_ else -1
+
+
+def fill_decode(seqs, dst: int, b: int, max_blocks: int, kv_block: int) -> bool:
+    """The inputs of a captured decode tick into its staging block (``csrc/hostlist.cu``); False: not of the plain form, or no
+    such entry point, and the caller fills the block itself."""
+    lib_ = _pylib()
+    return bool(lib_) and lib_.trl_fill_decode(seqs, dst, b, max_blocks, kv_block) == len(seqs)
+
+
+def _pylib():
+    global _PYLIB
+    if _PYLIB is None:
+        lib_ = ctypes.PyDLL(_PATH) if loadable() else None
+        _PYLIB = lib_ if lib_ is not None and hasattr(lib_, "trl_list_i32") else False
+        if _PYLIB:
+            _PYLIB.trl_list_i32.argtypes = [ctypes.py_object, P, L, L, L]
+            _PYLIB.trl_fill_decode.argtypes = [ctypes.py_object, P, L, L, L]
+            _PYLIB.trl_list_i32.restype = _PYLIB.trl_fill_decode.restype = L
+    return _PYLIB
+
+
 def register(name: str, sig) -> None:
     """Declare the signature of an entry point defined by another source file."""
     _SIGS[name] = sig
