@@ -92,32 +92,21 @@ gdn_prep_kernel(const bf16* inp, int ld, const float* __restrict__ conv_w,
       }
       val[e] = silu_f(acc);
     }
-  }
-  if (head < 2 * nk) {
-    float ss = 0.f;
+    if (head < 2 * nk) {
+      float ss = 0.f;
 #pragma unroll
-    for (int e = 0; e < 8; ++e) ss += val[e] * val[e];
-    for (int m = 1; m < tpt; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);   // the token's threads are lane-aligned
-    const float nrm = rsqrtf(ss + 1e-12f) * (head < nk ? rsqrtf((float)D) : 1.f);
-    if (t < T) {
-      float* dst = (head < nk ? qn + ((size_t)t * nk + head) * D : kn + ((size_t)t * nk + (head - nk)) * D) + d;
-      *reinterpret_cast<float4*>(dst) = make_float4(val[0] * nrm, val[1] * nrm, val[2] * nrm, val[3] * nrm);
-      *reinterpret_cast<float4*>(dst + 4) = make_float4(val[4] * nrm, val[5] * nrm, val[6] * nrm, val[7] * nrm);
-    }
-  } else if (t < T) {
-    float* dst = vc + ((size_t)t * nv + (head - 2 * nk)) * D + d;
-    *reinterpret_cast<float4*>(dst) = make_float4(val[0], val[1], val[2], val[3]);
-    *reinterpret_cast<float4*>(dst + 4) = make_float4(val[4], val[5], val[6], val[7]);
-  }
-  if (head == 0) {
-    const int tb = blockIdx.x * tpc;
-    for (int x = threadIdx.x; x < tpc * nv; x += blockDim.x) {
-      const int tt = tb + x / nv, h = x % nv;
-      if (tt >= T) break;
-      const bf16* ab = inp + (size_t)tt * ld + C + nv * D;
-      const float a = __bfloat162float(ab[h]), b = __bfloat162float(ab[nv + h]);
-      gout[(size_t)tt * nv + h] = -__expf(a_log[h]) * softplus_f(a + dt_bias[h]);
-      bout[(size_t)tt * nv + h] = sigmoid_f(b);
+      for (int e = 0; e < 8; ++e) ss += val[e] * val[e];
+      for (int m = 1; m < tpt; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);   // the token's threads are lane-aligned
+      const float nrm = rsqrtf(ss + 1e-12f) * (head < nk ? rsqrtf((float)D) : 1.f);
+      if (live) {
+        float* dst = (head < nk ? qn + ((size_t)t * nk + head) * D : kn + ((size_t)t * nk + (head - nk)) * D) + d;
+        *reinterpret_cast<float4*>(dst) = make_float4(val[0] * nrm, val[1] * nrm, val[2] * nrm, val[3] * nrm);
+        *reinterpret_cast<float4*>(dst + 4) = make_float4(val[4] * nrm, val[5] * nrm, val[6] * nrm, val[7] * nrm);
+      }
+    } else if (live) {
+      float* dst = vc + ((size_t)t * nv + (head - 2 * nk)) * D + d;
+      *reinterpret_cast<float4*>(dst) = make_float4(val[0], val[1], val[2], val[3]);
+      *reinterpret_cast<float4*>(dst + 4) = make_float4(val[4], val[5], val[6], val[7]);
     }
   }
 }
