@@ -28,10 +28,12 @@ namespace {
 
 constexpr int RING = 16;
 
-// grid = (ceil(tokens / TPC), 2*nk + nv), 128 threads: a thread owns 8 adjacent channels of one token
-// (D / 8 threads per token, TPC = 1024 / D tokens per CTA): four 16-byte row loads (the conv window), depthwise
-// causal conv + SiLU; q/k heads L2-normalise with shuffles inside the token's thread group; the head-0
-// CTA of a tile also emits the gates.  No shared memory, no block barrier.
+// grid = (ceil(tokens / (TPC * run)), 2*nk + nv + 1), 128 threads: a thread owns 8 adjacent channels of `run` consecutive
+// tokens (D / 8 threads per token, TPC = 1024 / D runs per CTA): it keeps its 32 taps and the last three rows in registers, so
+// a row is loaded once and not by each of the four tokens whose window it is in, and the taps once a run and not once a token
+// (128 bytes of taps for 16 bytes of row: with run = 1 a 2000-token layer took 155 us, 62 with 8).  Depthwise causal conv +
+// SiLU; q/k heads L2-normalise with shuffles inside the token's thread group; the last row of CTAs emits the gates.  No
+// shared memory, no block barrier.  Few tokens take run = 1: their CTAs are what fills the GPU.
 __global__ void __launch_bounds__(128)
 gdn_prep_kernel(const bf16* inp, int ld, const float* __restrict__ conv_w,
                 const float* __restrict__ dt_bias, const float* __restrict__ a_log,
@@ -39,56 +41,73 @@ gdn_prep_kernel(const bf16* inp, int ld, const float* __restrict__ conv_w,
                 const int* seq_ids, const int* q_start,
                 const int* state_slots, long ring_slot_stride,
                 float* qn, float* kn, float* vc,
-                float* gout, float* bout, int nk, int nv, int D, int KW, int T) {
+                float* gout, float* bout, int nk, int nv, int D, int KW, int T, int run) {
   pdl_launch_dependents(12);
-  pdl_wait();
   const int tpt = D >> 3;                       // threads per token
-  const int tpc = 128 / tpt;                    // tokens per CTA
-  const int t = blockIdx.x * tpc + threadIdx.x / tpt, head = blockIdx.y;
-  const int d = (threadIdx.x % tpt) * 8;
+  const int tpc = 128 / tpt;                    // runs per CTA
+  const int head = blockIdx.y;
   const int C = 2 * nk * D + nv * D;
-  const int c = head * D + d;
-  float val[8];
+  if (head == 2 * nk + nv) {                    // gates
+    pdl_wait();
+    const int tb = blockIdx.x * tpc * run, tn = min(tpc * run, T - tb);
+    for (int x = threadIdx.x; x < tn * nv; x += blockDim.x) {
+      const int tt = tb + x / nv, h = x % nv;
+      const bf16* ab = inp + (size_t)tt * ld + C + nv * D;
+      const float a = __bfloat162float(ab[h]), b = __bfloat162float(ab[nv + h]);
+      gout[(size_t)tt * nv + h] = -__expf(a_log[h]) * softplus_f(a + dt_bias[h]);
+      bout[(size_t)tt * nv + h] = sigmoid_f(b);
+    }
+    return;
+  }
+  const int t_first = (blockIdx.x * tpc + threadIdx.x / tpt) * run;
+  const int d = (threadIdx.x % tpt) * 8, c = head * D + d;
+  float wt[8][4];                               // tap of the row 3 - j back, oldest first
 #pragma unroll
-  for (int e = 0; e < 8; ++e) val[e] = 0.f;
-  if (t < T) {
-    const int pos = positions[t];
-    const int seq = seq_ids[t];
-    const int t0 = q_start[seq];
-    const bf16* rg = ring + (size_t)state_slots[seq] * ring_slot_stride;
-    uint4 rows[4];
+  for (int e = 0; e < 8; ++e) {
+    if (KW == 4) {
+      const float4 w4 = *reinterpret_cast<const float4*>(conv_w + (size_t)(c + e) * 4);
+      wt[e][0] = w4.x, wt[e][1] = w4.y, wt[e][2] = w4.z, wt[e][3] = w4.w;
+    } else {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {               // tap KW-1 multiplies the newest row
-      rows[j] = make_uint4(0u, 0u, 0u, 0u);
-      if (j < KW) {
-        const int back = KW - 1 - j;
-        const int pj = pos - back;
-        if (pj >= 0) {
-          const bf16* src = t - back >= t0 ? inp + (size_t)(t - back) * ld + c : rg + (size_t)(pj % RING) * C + c;
-          if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-            rows[j] = *reinterpret_cast<const uint4*>(src);
-          } else {                              // row width not a multiple of 8 (odd head counts of a TP shard): 4-byte pieces
-            const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src);
-            rows[j] = make_uint4(s32[0], s32[1], s32[2], s32[3]);
-          }
-        }
+      for (int j = 0; j < 4; ++j) wt[e][j] = j >= 4 - KW ? conv_w[(size_t)(c + e) * KW + j - (4 - KW)] : 0.f;
+    }
+  }
+  pdl_wait();
+  auto load8 = [&](const bf16* src) {
+    if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) return *reinterpret_cast<const uint4*>(src);
+    const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src);   // row width not a multiple of 8 (odd head counts of a TP
+    return make_uint4(s32[0], s32[1], s32[2], s32[3]);              // shard): 4-byte pieces
+  };
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  uint4 rows[4] = {zero, zero, zero, zero};
+  uint4 next = t_first < T ? load8(inp + (size_t)t_first * ld + c) : zero;
+  int next_seq = t_first < T ? seq_ids[t_first] : -1, seq = -1;
+#pragma unroll 1
+  for (int i = 0; i < run; ++i) {               // every lane of the warp goes round as often: the shuffles below want all of them
+    const int t = t_first + i;
+    const bool live = t < T;
+    float val[8];
+    const bool fresh = live && next_seq != seq;
+    seq = next_seq;
+    rows[0] = rows[1], rows[1] = rows[2], rows[2] = rows[3], rows[3] = next;
+    if (i + 1 < run && t + 1 < T) next = load8(inp + (size_t)(t + 1) * ld + c), next_seq = seq_ids[t + 1];
+    if (fresh) {                                // the run's or a sequence's first token: its window from the rows before it
+      const int pos = positions[t], t0 = q_start[seq];
+      const bf16* rg = ring + (size_t)state_slots[seq] * ring_slot_stride;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int back = 3 - j, pj = pos - back;
+        rows[j] = (back < KW && pj >= 0) ? load8(t - back >= t0 ? inp + (size_t)(t - back) * ld + c : rg + (size_t)(pj % RING) * C + c) : zero;
       }
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      float wt[4] = {0.f, 0.f, 0.f, 0.f};
-      if (KW == 4) {
-        const float4 w4 = *reinterpret_cast<const float4*>(conv_w + (size_t)(c + e) * 4);
-        wt[0] = w4.x, wt[1] = w4.y, wt[2] = w4.z, wt[3] = w4.w;
-      } else {
-        for (int j = 0; j < KW; ++j) wt[j] = conv_w[(size_t)(c + e) * KW + j];
-      }
       float acc = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const uint32_t wd = e < 2 ? rows[j].x : e < 4 ? rows[j].y : e < 6 ? rows[j].z : rows[j].w;
         const float2 f = bf162_bits_to_f2(wd);
-        acc = fmaf((e & 1) ? f.y : f.x, wt[j], acc);
+        acc = fmaf((e & 1) ? f.y : f.x, wt[e][j], acc);
       }
       val[e] = silu_f(acc);
     }
@@ -1241,6 +1260,231 @@ TRL_API void trl_gdn_set_wy(int on) { g_gdn_wy = on ? 1 : 0; }
 // Prefill scan on the tensor cores (gdn_chunk_mma_kernel): 1 on, 0 off (token-serial scan), -1 = the environment's choice.
 TRL_API void trl_gdn_set_mma(int on) { g_gdn_mma = on; }
 
+// The same step for many (sequence, value head) items, D = 128: one block an SM goes through its items with the 64 KB of
+// state in shared memory, three stages of bulk copies in and out, so that the copy engine always has the next states under way;
+// with a block per item the chain of a token (indices, convolution, two norms, the step) stood between a block's load and its
+// store, two blocks an SM.  Warps 0-7 compute (thread = column x half of the rows), 8-11 prepare the next item's token, 12 moves
+// states.  Bound by the state's bytes: 32 sequences x 48 heads, 201 MB: GDEC_BEFORE us before, GDEC_AFTER here; 8 sequences:
+// GDEC8_BEFORE, GDEC8_AFTER.
+struct GdSmem {
+  static constexpr int D = 128, STAGES = 3;
+  __align__(128) float st[STAGES][D][D];
+  __align__(16) float q[2][D], k[2][D];
+  float v[2][D], z[2][D];
+  float qk[2][4], gb[2][2];
+  float part[2][2][2][D];        // [half][rows of 32][k | q][column]
+  float ss[2][4], os[4];
+  unsigned long long full[STAGES], done[STAGES], prep_full[2], prep_empty[2];
+  int abort;
+};
+__global__ void __launch_bounds__(13 * 32, 1)
+gdn_decode_stream_kernel(const bf16* inp, int ld, const float* __restrict__ conv_w, const float* __restrict__ dt_bias,
+                         const float* __restrict__ a_log, const float* __restrict__ norm_w, float* states, const int* cur,
+                         bf16* ring, const int* positions, const int* q_start, const int* state_slots, long state_slot_stride,
+                         long plane_stride, long ring_slot_stride, float eps, bf16* out, int B, int nk, int nv, int KW) {
+  constexpr int D = GdSmem::D, NS = GdSmem::STAGES;
+  extern __shared__ __align__(128) unsigned char gd_raw[];
+  GdSmem& sm = *reinterpret_cast<GdSmem*>(gd_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int items = nv * B, n = (items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  volatile int* abort_flag = &sm.abort;
+  auto bar = [](unsigned long long* b) { return smem_u32(b); };
+  if (tid == 0) {
+    for (int i = 0; i < NS; ++i) mbar_init(bar(&sm.full[i]), 1), mbar_init(bar(&sm.done[i]), 256);
+    for (int i = 0; i < 2; ++i) mbar_init(bar(&sm.prep_full[i]), 128), mbar_init(bar(&sm.prep_empty[i]), 256);
+    sm.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  // true in every thread of the group when it is in every one of them; the group meets here whatever its waits returned
+  auto all_of = [](int id, int threads, bool ok) {
+    uint32_t r;
+    asm volatile(
+        "{ .reg .pred p, q;\n"
+        "  setp.ne.u32 q, %1, 0;\n"
+        "  bar.red.and.pred p, %2, %3, q;\n"
+        "  selp.u32 %0, 1, 0, p; }\n"
+        : "=r"(r) : "r"((uint32_t)ok), "r"(id), "r"(threads) : "memory");
+    return r != 0;
+  };
+
+  if (warp == 12) {
+    // ---------------- states: in, and out again ----------------
+    if (lane == 0) {
+      auto addr = [&](int i) {
+        const int item = (int)blockIdx.x + i * (int)gridDim.x, seq = item / nv, h = item % nv;
+        const int slot = state_slots[seq];
+        return states + (size_t)slot * state_slot_stride + (size_t)cur[slot] * plane_stride + (size_t)h * D * D;
+      };
+      auto load = [&](int i) {
+        const uint32_t b = bar(&sm.full[i % NS]);
+        mbar_expect_tx(b, D * D * 4);
+        bulk_load(smem_u32(&sm.st[i % NS][0][0]), addr(i), D * D * 4, b);
+      };
+      // slots and live planes are written by the host before a tick, the states by the previous tick: before the wait
+      for (int i = 0; i < min(n, NS); ++i) load(i);
+      pdl_launch_dependents(2);
+      pdl_wait();
+      for (int i = 0; i < n; ++i) {
+        if (!mbar_wait(bar(&sm.done[i % NS]), (uint32_t)(i / NS) & 1u, abort_flag)) break;
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                     ::"l"(addr(i)), "r"(smem_u32(&sm.st[i % NS][0][0])), "r"(D * D * 4) : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        if (i + NS < n) {
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          load(i + NS);
+        }
+      }
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+  } else if (warp >= 8) {
+    // ---------------- the token of each item ----------------
+    const int c = tid - 256, w = warp - 8;
+    pdl_launch_dependents(2);
+    pdl_wait();
+    const int C = 2 * nk * D + nv * D;
+    // Loads run ahead: the indices of the item after the next, the rows and taps of the next one, while this one is computed
+    // (in one chain they were 7 us an item, three times what its state takes to come in).
+    struct Idx { int h, slot, t, pos; };
+    struct Tok {
+      bf16 x[3][4], newest[3], z, a, b;
+      float wt[3][4], al, dt;
+    };
+    auto fetch_idx = [&](int i) {
+      Idx r{0, 0, 0, 0};
+      if (i < n) {
+        const int item = (int)blockIdx.x + i * (int)gridDim.x, seq = item / nv;
+        r.h = item % nv, r.slot = state_slots[seq], r.t = q_start[seq], r.pos = positions[r.t];
+      }
+      return r;
+    };
+    auto fetch_tok = [&](int i, const Idx& ix, Tok& k) {
+      if (i >= n) return;
+      const bf16* row = inp + (size_t)ix.t * ld;
+      const bf16* rg = ring + (size_t)ix.slot * ring_slot_stride;
+      const int kh = ix.h * nk / nv, ch[3] = {kh * D + c, nk * D + kh * D + c, 2 * nk * D + ix.h * D + c};
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        k.newest[e] = row[ch[e]];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {                  // tap KW-1 multiplies the newest row
+          const int back = KW - 1 - j, pj = ix.pos - back;
+          k.x[e][j] = (back > 0 && pj >= 0) ? rg[(size_t)(pj % RING) * C + ch[e]] : __float2bfloat16(0.f);
+          k.wt[e][j] = j < KW ? conv_w[(size_t)ch[e] * KW + j] : 0.f;
+        }
+      }
+      k.z = row[C + (size_t)ix.h * D + c];
+      k.a = row[C + nv * D + ix.h], k.b = row[C + nv * D + nv + ix.h], k.al = a_log[ix.h], k.dt = dt_bias[ix.h];
+    };
+    Idx ix = fetch_idx(0), ix1 = fetch_idx(1);
+    Tok tk, tk1;
+    fetch_tok(0, ix, tk);
+    for (int i = 0; i < n; ++i) {
+      const int h = ix.h, b = i & 1, kh = h * nk / nv;
+      const int ch[3] = {kh * D + c, nk * D + kh * D + c, 2 * nk * D + h * D + c};
+      fetch_tok(i + 1, ix1, tk1);
+      const Idx ix2 = fetch_idx(i + 2);
+      bf16* rg = ring + (size_t)ix.slot * ring_slot_stride;
+      float ga = 0.f, gbv = 0.f;
+      if (c == 0) {
+        ga = -__expf(tk.al) * softplus_f(__bfloat162float(tk.a) + tk.dt);
+        gbv = sigmoid_f(__bfloat162float(tk.b));
+      }
+      float val[3];
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc = fmaf(__bfloat162float(j == KW - 1 ? tk.newest[e] : tk.x[e][j]), tk.wt[e][j], acc);
+        val[e] = silu_f(acc);
+      }
+      // the compute warps are through with this buffer's last item
+      const bool ok = i < 2 || mbar_wait(bar(&sm.prep_empty[b]), (uint32_t)(i / 2 - 1) & 1u, abort_flag);
+      const float sq = warp_sum(val[0] * val[0]), sk = warp_sum(val[1] * val[1]);
+      if (lane == 0) sm.ss[0][w] = sq, sm.ss[1][w] = sk;
+      if (!all_of(3, 128, ok)) break;
+      const float qn = val[0] * (rsqrtf(((sm.ss[0][0] + sm.ss[0][1]) + sm.ss[0][2]) + sm.ss[0][3] + 1e-12f) * rsqrtf((float)D));
+      const float kn = val[1] * rsqrtf(((sm.ss[1][0] + sm.ss[1][1]) + sm.ss[1][2]) + sm.ss[1][3] + 1e-12f);
+      sm.q[b][c] = qn, sm.k[b][c] = kn, sm.v[b][c] = val[2], sm.z[b][c] = __bfloat162float(tk.z);
+      const float qk = warp_sum(qn * kn);
+      if (lane == 0) sm.qk[b][w] = qk;
+      if (c == 0) sm.gb[b][0] = ga, sm.gb[b][1] = gbv;
+      mbar_arrive(bar(&sm.prep_full[b]));
+      // ring refresh: the raw q / k rows by the first value head of each key head, the v row by every head
+      bf16* dst = rg + (size_t)(ix.pos % RING) * C;
+      if (h % (nv / nk) == 0) dst[ch[0]] = tk.newest[0], dst[ch[1]] = tk.newest[1];
+      dst[ch[2]] = tk.newest[2];
+      all_of(3, 128, true);                            // the square sums have been read: the next item may write them
+      ix = ix1, ix1 = ix2, tk = tk1;
+    }
+  } else {
+    // ---------------- the step ----------------
+    const int col = tid & 127, half = tid >> 7;
+    pdl_launch_dependents(2);
+    pdl_wait();
+    const float nw = norm_w[col];
+    for (int i = 0; i < n; ++i) {
+      const int item = (int)blockIdx.x + i * (int)gridDim.x, seq = item / nv, h = item % nv, b = i & 1, sg = i % NS;
+      bool ok = mbar_wait(bar(&sm.full[sg]), (uint32_t)(i / NS) & 1u, abort_flag);
+      ok = ok && mbar_wait(bar(&sm.prep_full[b]), (uint32_t)(i / 2) & 1u, abort_flag);
+      if (!all_of(1, 256, ok)) break;
+      float(*st)[D] = &sm.st[sg][half * 64];
+      const float4* k4 = reinterpret_cast<const float4*>(sm.k[b] + half * 64);
+      const float4* q4 = reinterpret_cast<const float4*>(sm.q[b] + half * 64);
+      // S <- e^g S;  d = beta (v - S^T k);  S <- S + k d^T;  o = S^T q; sums over 32 rows at a time
+      float S[64];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float ks = 0.f, qs = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 kk = k4[u * 8 + j], qq = q4[u * 8 + j];
+          const float kv[4] = {kk.x, kk.y, kk.z, kk.w}, qv[4] = {qq.x, qq.y, qq.z, qq.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float x = st[u * 32 + j * 4 + e][col];
+            S[u * 32 + j * 4 + e] = x;
+            ks = fmaf(kv[e], x, ks), qs = fmaf(qv[e], x, qs);
+          }
+        }
+        sm.part[half][u][0][col] = ks, sm.part[half][u][1][col] = qs;
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      const float eg = __expf(sm.gb[b][0]), beta = sm.gb[b][1];
+      const float ksum = (sm.part[0][0][0][col] + sm.part[0][1][0][col]) + (sm.part[1][0][0][col] + sm.part[1][1][0][col]);
+      const float qsum = (sm.part[0][0][1][col] + sm.part[0][1][1][col]) + (sm.part[1][0][1][col] + sm.part[1][1][1][col]);
+      const float d = beta * (sm.v[b][col] - eg * ksum);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float4 kk = k4[j];
+        st[4 * j][col] = fmaf(kk.x, d, eg * S[4 * j]), st[4 * j + 1][col] = fmaf(kk.y, d, eg * S[4 * j + 1]);
+        st[4 * j + 2][col] = fmaf(kk.z, d, eg * S[4 * j + 2]), st[4 * j + 3][col] = fmaf(kk.w, d, eg * S[4 * j + 3]);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the bulk store reads what was written here
+      mbar_arrive(bar(&sm.done[sg]));
+      float o = 0.f;
+      const float z = sm.z[b][col];
+      if (half == 0) {
+        o = fmaf(eg, qsum, ((sm.qk[b][0] + sm.qk[b][1]) + (sm.qk[b][2] + sm.qk[b][3])) * d);
+        const float w_ = warp_sum(o * o);
+        if (lane == 0) sm.os[warp] = w_;
+      }
+      mbar_arrive(bar(&sm.prep_empty[b]));
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // also: the partial sums have been read
+      if (half == 0) {
+        const float rstd = rsqrtf((((sm.os[0] + sm.os[1]) + sm.os[2]) + sm.os[3]) / (float)D + eps);
+        out[((size_t)q_start[seq] * nv + h) * D + col] = __float2bfloat16(o * rstd * nw * silu_f(z));
+      }
+    }
+  }
+  __syncthreads();
+  if (sm.abort) {                                      // copies may still be in flight towards this block's shared memory
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL) {
+    }
+  }
+}
+
 // Scratch (fp32): qn, kn [T*nk*D]; vc, o_scratch [T*nv*D]; g, beta [T*nv].
 TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_bias, const void* a_log,
                     const void* norm_w, void* states, void* cur, void* ring, const void* positions,
@@ -1253,10 +1497,13 @@ TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_
   if (KW > 4) return (int)cudaErrorInvalidValue;
   if ((D != 64 && D != 128) || (ld % 2) != 0) return (int)cudaErrorInvalidValue;
   const int prep_tpc = 1024 / D;
-  cudaError_t e = trl_launch(gdn_prep_kernel, dim3((T + prep_tpc - 1) / prep_tpc, 2 * nk + nv), dim3(128), 0, st,
+  int run = 8;
+  while (run > 1 && (long)(T + prep_tpc * run - 1) / (prep_tpc * run) * (2 * nk + nv) < 16 * 148) run >>= 1;
+  cudaError_t e = trl_launch(gdn_prep_kernel, dim3((T + prep_tpc * run - 1) / (prep_tpc * run), 2 * nk + nv + 1), dim3(128), 0, st,
                              (const bf16*)inp, ld, (const float*)conv_w, (const float*)dt_bias, (const float*)a_log,
                              (const bf16*)ring, (const int*)positions, (const int*)seq_ids,
                              (const int*)q_start, (const int*)state_slots, ring_slot_stride,
+  // runs as long as leaves about 16 CTAs of 128 threads for every SM
                              (float*)qn, (float*)kn, (float*)vc, (float*)g, (float*)beta, nk, nv, D, KW, T);
   if (e != cudaSuccess) return (int)e;
 #define RECUR(DD)                                                                                   \

@@ -102,3 +102,50 @@ def test_fp8_attention_on_tensor_cores(ops, g_heads, splits, scale_v):
             assert _rel(got, want) < tol, (n, _rel(got, want))
         final = want * torch.sigmoid(gate[i].double().view(n_q, 2, d)[:, 1])
         assert _rel(out[i].view(n_q, d), final) < (2e-2 if i == 1 else 2 ** -8), n
+
+
+@pytest.mark.parametrize("nk,nv,d,taps", [(2, 4, 128, 4), (1, 3, 128, 4), (2, 2, 64, 4), (2, 4, 128, 3)])
+def test_delta_rule_prep_over_runs_of_tokens(ops, nk, nv, d, taps):
+    """Convolution, norms and gates of tokens taken in runs of 8 (thousands of tokens), 4, 2 and 1: sequences that begin inside a
+    run, at position 0 and later (their window then comes from the ring), shorter than the window, and a last run that is not
+    full.  Scratch rows against 64 bits."""
+    from tilerl_b200.ops import native as N
+    c = (2 * nk + nv) * d
+    for lens in ([1], [3, 1, 2], [7, 40, 1, 9, 300], [1500, 2, 3, 1, 1700], [5000]):
+        g = torch.Generator().manual_seed(sum(lens) + d)
+        t, b = sum(lens), len(lens)
+        starts = [0 if i % 2 else 5 + 13 * i for i in range(b)]
+        inp = torch.randn(t, c + nv * d + 2 * nv, generator=g).to(DEV, torch.bfloat16)
+        conv = (torch.randn(c, taps, generator=g) * 0.3).to(DEV)
+        dt, al = torch.randn(nv, generator=g).to(DEV), torch.randn(nv, generator=g).to(DEV)
+        ring = torch.randn(b + 1, 16, c, generator=g).to(DEV, torch.bfloat16)
+        keep = ring.clone()
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+        q0 = [sum(lens[:i]) for i in range(b)]
+        pos = i32([s + j for s, n in zip(starts, lens) for j in range(n)])
+        seq = i32([i for i, n in enumerate(lens) for _ in range(n)])
+        states = torch.zeros(b + 1, 1, 1, nv, d, d, device=DEV)
+        f = lambda *s: torch.full(s, float("nan"), device=DEV)
+        qn, kn, vc, gg, bb, o = f(t, nk, d), f(t, nk, d), f(t, nv, d), f(t, nv), f(t, nv), f(t, nv, d)
+        out = torch.empty(t, nv * d, dtype=torch.bfloat16, device=DEV)
+        cur = torch.zeros(b + 1, dtype=torch.int32, device=DEV)
+        nw, qs, ql, slots = torch.ones(d, device=DEV), i32(q0), i32(lens), i32(list(range(1, b + 1)))
+        N.check(ops.lib.trl_gdn(inp.data_ptr(), inp.stride(0), conv.data_ptr(), dt.data_ptr(), al.data_ptr(), nw.data_ptr(),
+                                states.data_ptr(), cur.data_ptr(), ring.data_ptr(), pos.data_ptr(), seq.data_ptr(), qs.data_ptr(),
+                                ql.data_ptr(), slots.data_ptr(), None, states.stride(0), states.stride(2),
+                                ring.stride(0), qn.data_ptr(), kn.data_ptr(), vc.data_ptr(), gg.data_ptr(), bb.data_ptr(), o.data_ptr(),
+                                out.data_ptr(), t, b, nk, nv, d, taps, 1, 1e-6, N.stream()), "gdn")
+        x = inp.double()
+        want = []
+        for i, n in enumerate(lens):
+            halo = torch.stack([keep[i + 1, (starts[i] - taps + 1 + j) % 16].double() if starts[i] - taps + 1 + j >= 0 else
+                                torch.zeros(c, dtype=torch.float64, device=DEV) for j in range(taps - 1)])
+            rows = torch.cat([halo, x[q0[i]:q0[i] + n, :c]])
+            want.append(torch.nn.functional.silu(sum(rows[j:j + n] * conv[:, j].double() for j in range(taps))))
+        want = torch.cat(want)
+        unit = lambda a: a / torch.sqrt(a.pow(2).sum(-1, keepdim=True) + 1e-12)
+        assert _rel(qn, unit(want[:, :nk * d].view(t, nk, d)) / d ** 0.5) < 1e-5
+        assert _rel(kn, unit(want[:, nk * d:2 * nk * d].view(t, nk, d))) < 1e-5
+        assert _rel(vc, want[:, 2 * nk * d:].view(t, nv, d)) < 1e-5
+        assert _rel(bb, torch.sigmoid(x[:, c + nv * d + nv:])) < 1e-5
+        assert _rel(gg, -torch.exp(al.double()) * torch.nn.functional.softplus(x[:, c + nv * d:c + nv * d + nv] + dt.double())) < 1e-5
