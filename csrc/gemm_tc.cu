@@ -590,22 +590,149 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 // J NVFP4 residual terms per token.  column (tok*J + j): xq [cols, K/2], sf tiled (see
 // header), rs[col] fp32.
 //
-// Grid = (tokens, slices): every CTA first reduces the whole (L2-resident) row for the
-// norm statistics and the row maximum, then each thread owns one 16-element block and
-// runs all J terms in registers.  The row scale of term j is rs_0 / 4^j -- a bound, not a
-// reduction: one e2m1 term leaves a remainder of at most 1/4 of the block maximum it
-// encoded (worst gap 4..6 of 6 plus the e4m3 scale rounding) -- so no second pass over
-// the row is needed.
+// The row scale of term j is rs_0 / 4^j -- a bound, not a reduction: one e2m1 term leaves a remainder of at most 1/4 of the
+// block maximum it encoded (worst gap 4..6 of 6 plus the e4m3 scale rounding) -- so no second pass over the row is needed.
+
+// All J terms of one 16-element block (r: its values, replaced by the remainders), scales and e2m1 bytes out.
+struct QuantTerm { uint32_t lo, hi; uint32_t sf; };
+__device__ __forceinline__ QuantTerm quant_term(float (&r)[16], float rscale, bool more) {
+  QuantTerm o;
+  float bm = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) bm = fmaxf(bm, fabsf(r[i]));
+  const float s = fminf(__fdividef(bm, 6.f * rscale), 448.f);
+  uint16_t s16;
+  asm("{ .reg .b16 t; cvt.rn.satfinite.e4m3x2.f32 t, %1, %2; mov.b16 %0, t; }" : "=h"(s16) : "f"(0.f), "f"(s));
+  const float sfv = h2_to_f2(cvt_e4m3x2_to_h2(s16)).x;
+  const float denom = sfv * rscale;
+  const float inv = denom > 0.f ? __frcp_rn(denom) : 0.f;
+  uint32_t packed[2] = {0u, 0u};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {                           // byte i: elements 2i (low nibble), 2i + 1
+    uint16_t by;
+    asm("{ .reg .b8 t; cvt.rn.satfinite.e2m1x2.f32 t, %1, %2; cvt.u16.u8 %0, t; }" : "=h"(by) : "f"(r[2 * i + 1] * inv), "f"(r[2 * i] * inv));
+    packed[i >> 2] |= (uint32_t)(by & 0xff) << (8 * (i & 3));
+    if (more) {                                           // the next term encodes the remainder
+      uint32_t h;
+      asm("{ .reg .b8 t; cvt.u8.u16 t, %1; cvt.rn.f16x2.e2m1x2 %0, t; }" : "=r"(h) : "h"(by));
+      const float2 d = h2_to_f2(h);
+      r[2 * i] = fmaf(-d.x, denom, r[2 * i]);
+      r[2 * i + 1] = fmaf(-d.y, denom, r[2 * i + 1]);
+    }
+  }
+  o.lo = packed[0], o.hi = packed[1], o.sf = s16 & 0xff;
+  return o;
+}
+
+// Four scale bytes of four neighbouring lanes (blocks b .. b + 3 of a column are four bytes in a row) in the first of them.
+__device__ __forceinline__ uint32_t gather_sf4(uint32_t v) {
+  v |= __shfl_down_sync(0xffffffffu, v, 1) << 8;          // valid in even lanes
+  v = (v & 0xffffu) | (__shfl_down_sync(0xffffffffu, v, 2) << 16);
+  return v;
+}
+
+// One block per row, the row in registers: a thread owns NB whole 16-element blocks (b = thread + i * threads, so that loads,
+// e2m1 stores and groups of four scale bytes stay contiguous over a warp), reads them once, and the block's two reductions
+// (square sum, largest value) are the only exchanges.  Bound by the row's latency for a few rows (two reductions), by issue
+// for many.  2000 rows x 5120 with a norm: 27 us with the row in shared memory, 18 here; 17 408 wide: 64 -> 47; the four
+// launches of a layer, 8 rows: 31 -> 24 us.
+template <int NB>
+__global__ void __launch_bounds__(NB == 1 ? 640 : 576, 2)
+quant_act_rows_kernel(const bf16* x, int ldx, const float* __restrict__ norm_w, float eps, uint8_t* xq, uint8_t* sf,
+                      float* rs, int K, int J, int kt4, int swiglu_in) {
+  __shared__ float red[32];
+  const int tok = blockIdx.x, nt = blockDim.x, lane = threadIdx.x & 31;
+  pdl_launch_dependents();
+  pdl_wait();
+  const bf16* xr = x + (size_t)tok * ldx;
+  uint32_t pk[NB][8];                                     // the thread's values, bf16 pairs
+#pragma unroll
+  for (int i = 0; i < NB; ++i) {
+    const int k = ((int)threadIdx.x + i * nt) * 16;       // K % 16 == 0: a block is whole or padding
+    if (k >= K) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) pk[i][e] = 0u;
+    } else if (swiglu_in) {                               // interleaved (gate, up) pairs: K outputs from 2K inputs
+      uint4 u[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) u[e] = __ldcg(reinterpret_cast<const uint4*>(xr + 2 * k) + e);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 g0 = bf162_bits_to_f2(u[e].x), g1 = bf162_bits_to_f2(u[e].y), g2 = bf162_bits_to_f2(u[e].z), g3 = bf162_bits_to_f2(u[e].w);
+        pk[i][2 * e] = f2_to_bf162_bits(silu_f(g0.x) * g0.y, silu_f(g1.x) * g1.y);
+        pk[i][2 * e + 1] = f2_to_bf162_bits(silu_f(g2.x) * g2.y, silu_f(g3.x) * g3.y);
+      }
+    } else {
+      const uint4 u0 = __ldcg(reinterpret_cast<const uint4*>(xr + k)), u1 = __ldcg(reinterpret_cast<const uint4*>(xr + k) + 1);
+      pk[i][0] = u0.x, pk[i][1] = u0.y, pk[i][2] = u0.z, pk[i][3] = u0.w;
+      pk[i][4] = u1.x, pk[i][5] = u1.y, pk[i][6] = u1.z, pk[i][7] = u1.w;
+    }
+  }
+  if (norm_w != nullptr) {
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float2 f = bf162_bits_to_f2(pk[i][e]);
+        ss = fmaf(f.x, f.x, ss), ss = fmaf(f.y, f.y, ss);
+      }
+    ss = block_sum(ss, red);
+    const float rstd = rsqrtf(ss / (float)K + eps);
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int k = ((int)threadIdx.x + i * nt) * 16;
+      if (k < K) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float4 w = *reinterpret_cast<const float4*>(norm_w + k + 4 * e);
+          const float2 a = bf162_bits_to_f2(pk[i][2 * e]), c = bf162_bits_to_f2(pk[i][2 * e + 1]);
+          pk[i][2 * e] = f2_to_bf162_bits(a.x * rstd * w.x, a.y * rstd * w.y);
+          pk[i][2 * e + 1] = f2_to_bf162_bits(c.x * rstd * w.z, c.y * rstd * w.w);
+        }
+      }
+    }
+  }
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float2 f = bf162_bits_to_f2(pk[i][e]);
+      amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+    }
+  amax = block_max(amax, red);
+  const float rs0 = fmaxf(amax, 1e-30f) * (1.f / (6.f * 448.f));
+  if ((int)threadIdx.x < J) rs[tok * J + threadIdx.x] = rs0 * exp2f(-2.f * (float)threadIdx.x);
+#pragma unroll 1
+  for (int i = 0; i < NB; ++i) {                          // one block's values in fp32 at a time: two CTAs an SM
+    const int b = (int)threadIdx.x + i * nt, k = b * 16;
+    float r[16];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float2 f = bf162_bits_to_f2(pk[0][e]);
+      r[2 * e] = f.x, r[2 * e + 1] = f.y;
+      pk[0][e] = pk[NB - 1][e];
+    }
+    float rscale = rs0;
+    for (int j = 0; j < J; ++j, rscale *= 0.25f) {
+      const int col = tok * J + j;
+      const QuantTerm q = quant_term(r, rscale, j + 1 < J);
+      const uint32_t s4 = gather_sf4(k < K ? q.sf : 0u);
+      if (k < K) *reinterpret_cast<uint2*>(xq + (size_t)col * (K >> 1) + (size_t)b * 8) = make_uint2(q.lo, q.hi);
+      if ((lane & 3) == 0 && b < kt4 * 4)                 // whole groups of four: the padding of K is a multiple of four blocks
+        *reinterpret_cast<uint32_t*>(sf + ((size_t)(col >> 7) * kt4 + (b >> 2)) * SF_ATOM + (col & 31) * 16 + ((col & 127) >> 5) * 4) = s4;
+    }
+  }
+}
+
+// Rows that the kernel above does not take (over 18 432 values, or off a 16-byte boundary): grid = (tokens, slices), every
+// block reduces the whole (L2-resident) row, then a thread owns a quarter of a 16-element block per slice.
 __global__ void __launch_bounds__(256)
 quant_act_kernel(const bf16* x, int ldx, const float* __restrict__ norm_w, float eps,
                  uint8_t* xq, uint8_t* sf, float* rs, int K, int J,
                  int kt4, int swiglu_in) {
   __shared__ float red[32];
-  // one CTA per row (gridDim.y == 1): the pass that finds the row maximum leaves the (normalised) row in
-  // shared memory as bf16, and the quantising pass reads it from there -- read from L2 again, that pass
-  // is a chain of dependent loads, one per 1024 elements of the row
-  extern __shared__ __align__(16) uint2 qa_row[];
-  const bool staged = gridDim.y == 1;
   pdl_launch_dependents();
   pdl_wait();
   const int tok = blockIdx.x;
@@ -651,62 +778,10 @@ quant_act_kernel(const bf16* x, int ldx, const float* __restrict__ norm_w, float
       v[3] = __bfloat162float(__float2bfloat16(v[3] * rstd * w.w));
     }
     amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
-    if (staged) qa_row[k >> 2] = make_uint2(f2_to_bf162_bits(v[0], v[1]), f2_to_bf162_bits(v[2], v[3]));   // exact: v is bf16-valued
   }
   amax = block_max(amax, red);
   const float rs0 = fmaxf(amax, 1e-30f) * (1.f / (6.f * 448.f));
   if (blockIdx.y == 0 && threadIdx.x < J) rs[tok * J + threadIdx.x] = rs0 * exp2f(-2.f * (float)threadIdx.x);
-  if (staged) {
-    // one CTA per row: a thread takes whole 16-element blocks out of the staged row (the scale arithmetic
-    // is paid once per block, no shuffles; 8 bytes of e2m1 per term and block in one store).  Same
-    // arithmetic per element as the quarter-block form below, so the same bits.
-    const int n_blk = kt4 * 4;                            // 16-element blocks of the padded row
-    for (int b = threadIdx.x; b < n_blk; b += blockDim.x) {
-      const int k = b * 16;                               // K % 16 == 0: a block is whole or padding
-      float r[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) r[i] = 0.f;
-      if (k < K) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint2 u = qa_row[b * 4 + i];
-          const float2 a = bf162_bits_to_f2(u.x), b2 = bf162_bits_to_f2(u.y);
-          r[4 * i] = a.x, r[4 * i + 1] = a.y, r[4 * i + 2] = b2.x, r[4 * i + 3] = b2.y;
-        }
-      }
-      float rscale = rs0;
-      for (int j = 0; j < J; ++j, rscale *= 0.25f) {
-        const int col = tok * J + j;
-        float bm = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) bm = fmaxf(bm, fabsf(r[i]));
-        const float s = fminf(__fdividef(bm, 6.f * rscale), 448.f);
-        uint16_t s16;
-        asm("{ .reg .b16 t; cvt.rn.satfinite.e4m3x2.f32 t, %1, %2; mov.b16 %0, t; }" : "=h"(s16) : "f"(0.f), "f"(s));
-        const float sfv = h2_to_f2(cvt_e4m3x2_to_h2(s16)).x;
-        const float denom = sfv * rscale;
-        const float inv = denom > 0.f ? __frcp_rn(denom) : 0.f;
-        uint32_t packed[2] = {0u, 0u};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {                     // byte i: elements 2i (low nibble), 2i + 1
-          uint16_t by;
-          asm("{ .reg .b8 t; cvt.rn.satfinite.e2m1x2.f32 t, %1, %2; cvt.u16.u8 %0, t; }" : "=h"(by) : "f"(r[2 * i + 1] * inv), "f"(r[2 * i] * inv));
-          packed[i >> 2] |= (uint32_t)(by & 0xff) << (8 * (i & 3));
-          if (j + 1 < J) {                                // the next term encodes the remainder
-            uint32_t h;
-            asm("{ .reg .b8 t; cvt.u8.u16 t, %1; cvt.rn.f16x2.e2m1x2 %0, t; }" : "=r"(h) : "h"(by));
-            const float2 d = h2_to_f2(h);
-            r[2 * i] = fmaf(-d.x, denom, r[2 * i]);
-            r[2 * i + 1] = fmaf(-d.y, denom, r[2 * i + 1]);
-          }
-        }
-        if (k < K) *reinterpret_cast<uint2*>(xq + (size_t)col * (K >> 1) + (size_t)b * 8) = make_uint2(packed[0], packed[1]);
-        sf[((size_t)(col >> 7) * kt4 + (b >> 2)) * SF_ATOM + (col & 31) * 16 + ((col & 127) >> 5) * 4 + (b & 3)] =
-            (k < K) ? (uint8_t)(s16 & 0xff) : (uint8_t)0;
-      }
-    }
-    return;
-  }
   // this thread's quarter blocks: one per slice; gridDim.y slices run in parallel, the rest in
   // a loop (one CTA per row when there are enough rows to fill the GPU: the row is then read
   // from L2 by one CTA instead of by every slice's CTA)
@@ -812,17 +887,18 @@ TRL_API int trl_quant_act_nvfp4(const void* x, int ldx, const void* norm_w, floa
                                 void* rs, int tokens, int K, int J, int swiglu_in, void* stream) {
   if (K % 16 != 0 || J < 1 || J > 16) return (int)cudaErrorInvalidValue;
   const int nk = (K + KT_ELEMS - 1) / KT_ELEMS;
-  int slices = (nk * KT_ELEMS / 4 + 255) / 256;  // 4 elements per thread
-  if (tokens >= 128) slices = 1;                        // enough rows to fill the GPU: one CTA per row
-  const size_t smem = slices == 1 ? (size_t)((K + 3) / 4) * sizeof(uint2) : 0;      // the staged row, bf16
-  if (smem > 48 * 1024) {
-    static size_t configured = 0;
-    if (configured < smem) {
-      if (cudaFuncSetAttribute(quant_act_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 3;
-      configured = smem;
-    }
+  const bool aligned = ldx % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(norm_w) & 15) == 0;
+  const int blocks = nk * 16;                           // 16-element blocks of the padded row
+  if (aligned && blocks <= 2 * 576) {
+    // a thread a block up to 640 of them (the smaller rows, whole in flight at once), two above
+    const int nb = blocks <= 640 ? 1 : 2, threads = ((blocks + nb - 1) / nb + 31) / 32 * 32;
+    auto kern = nb == 1 ? quant_act_rows_kernel<1> : quant_act_rows_kernel<2>;
+    return (int)trl_launch(kern, dim3(tokens), dim3(threads), 0, (cudaStream_t)stream, (const bf16*)x, ldx,
+                           (const float*)norm_w, eps, (uint8_t*)xq, (uint8_t*)sf, (float*)rs, K, J, nk * 4, swiglu_in);
   }
-  return (int)trl_launch(quant_act_kernel, dim3(tokens, slices), dim3(256), smem, (cudaStream_t)stream, (const bf16*)x,
+  int slices = (nk * KT_ELEMS / 4 + 255) / 256;         // 4 elements per thread
+  if (tokens >= 128) slices = 1;                        // enough rows to fill the GPU: one block per row
+  return (int)trl_launch(quant_act_kernel, dim3(tokens, slices), dim3(256), 0, (cudaStream_t)stream, (const bf16*)x,
                          ldx, (const float*)norm_w, eps, (uint8_t*)xq, (uint8_t*)sf, (float*)rs, K, J, nk * 4,
                          swiglu_in);
 }

@@ -46,6 +46,38 @@ def test_bf16_rows_for_every_split_of_k(ops, m, n, k, shift):
     assert _rel(y, h.double() @ w.double().t()) < 2e-4 + 2 ** -8 / k ** 0.5
 
 
+@pytest.mark.parametrize("k", [32, 256, 288, 5120, 10240, 10496, 17408, 18432, 18464])
+@pytest.mark.parametrize("tokens,terms,swiglu", [(1, 4, False), (3, 2, True), (130, 2, False), (17, 1, False)])
+def test_activation_quantiser_row_kernel_gives_the_general_kernels_bits(ops, k, tokens, terms, swiglu):
+    """Rows on a 16-byte boundary up to 18 432 values take the kernel that keeps the row in registers, others the general one:
+    the same values in both alignments, the same bytes, zero scales in the padding of K (without a norm; with one, sums in
+    another order move the reciprocal root by its last bit, and single codes with it)."""
+    from tilerl_b200.ops.gemm_tc import quant_act
+    g = torch.Generator().manual_seed(k + tokens)
+    width = 2 * k if swiglu else k
+    x = (torch.randn(tokens, width, generator=g) * torch.exp(torch.randn(tokens, 1, generator=g))).to(DEV, torch.bfloat16)
+    x[0, :16] = 0
+    off = torch.zeros(tokens, width + 8, dtype=torch.bfloat16, device=DEV)[:, 4:4 + width]
+    off.copy_(x)
+    if swiglu:       # pairs are read 16 bytes at a time in both kernels
+        off = x
+    nk = (k + 255) // 256
+    cols = tokens * terms
+    xq, sf, rs = (a.clone() for a in quant_act(ops, x, k, terms, swiglu_in=swiglu))
+    yq, tf, ts = quant_act(ops, off, k, terms, swiglu_in=swiglu)
+    c = torch.arange(cols, device=DEV)
+    rows = lambda s: s.view(-1, nk * 4, 32, 4, 4).permute(0, 3, 2, 1, 4).reshape(-1, nk * 16)[c]
+    assert torch.equal(xq, yq) and torch.equal(rs, ts) and torch.equal(rows(sf), rows(tf))
+    assert int(rows(sf)[:, k // 16:].sum()) == 0
+    if swiglu:
+        return
+    nw = (1.0 + 0.1 * torch.randn(k, generator=g)).to(DEV)
+    xq, sf, rs = (a.clone() for a in quant_act(ops, x, k, terms, norm_w=nw, eps=1e-6))
+    yq, tf, ts = quant_act(ops, off, k, terms, norm_w=nw, eps=1e-6)
+    assert float((xq != yq).float().mean()) < 2e-3 and _rel(rs, ts) < 2 ** -7
+    assert float((rows(sf) != rows(tf)).float().mean()) < 2e-3
+
+
 @pytest.mark.parametrize("g_heads,splits", [(1, 1), (6, 1), (6, 5), (8, 3)])
 @pytest.mark.parametrize("scale_v", [1.0, 1e-25, 1e12])
 def test_fp8_attention_on_tensor_cores(ops, g_heads, splits, scale_v):
