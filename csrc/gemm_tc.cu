@@ -99,49 +99,66 @@ __device__ __forceinline__ void epi_store(const GemmParams& p, int tok, int n, i
   }
 }
 
-// Epilogue of one accumulator tile: TMEM -> registers in chunks of CH columns, J columns summed
-// per token with their activation scales, then either the final store (WHOLE) or this CTA's
-// split-K slot.  tok_first = first token of the tile; slot_row = slot + row.
-template <int BN, int J, int EPI, bool WHOLE>
-__device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t taddr0, const float* rs_s, float ts,
-                                              int tok_first, int n, int lane, float* slot_row) {
-  constexpr int CH = BN >= 32 ? 32 : 16;
-  constexpr int TPC = CH / J;
-#pragma unroll 1
-  for (int c = 0; c < BN / CH; ++c) {
-    uint32_t r[32];
-    if (CH == 32) tc_ld32(taddr0 + (uint32_t)(c * CH), r); else tc_ld16(taddr0 + (uint32_t)(c * CH), r);
-    const int tokc = tok_first + c * TPC;
-    float res[TPC];
+// The finished values of one row and up to 128 tokens, out.
+template <int V, int EPI>
+__device__ __forceinline__ void store_values(const GemmParams& p, const float (&v)[V], int tok, int n, int lane) {
+  constexpr int GRP = V < 16 ? V : 16;
 #pragma unroll
-    for (int t = 0; t < TPC; ++t)   // issued before the wait and before any store of this chunk
-      res[t] = (WHOLE && EPI == EPI_RESIDUAL && tokc + t < p.tokens && n < p.N)
-                   ? __bfloat162float(p.residual[(size_t)(tokc + t) * p.ldr + n]) : 0.f;
-    tc_wait_ld();
-    float v[TPC];
+  for (int c = 0; c < V; c += GRP) {
+    float res[GRP];
 #pragma unroll
-    for (int t = 0; t < TPC; ++t) {
-      float a = 0.f;
+    for (int t = 0; t < GRP; ++t)                // issued before any store of these tokens
+      res[t] = (EPI == EPI_RESIDUAL && tok + c + t < p.tokens && n < p.N)
+                   ? __bfloat162float(p.residual[(size_t)(tok + c + t) * p.ldr + n]) : 0.f;
 #pragma unroll
-      for (int j = 0; j < J; ++j) a = fmaf(__uint_as_float(r[t * J + j]), rs_s[c * CH + t * J + j], a);
-      v[t] = a * ts;
-    }
-#pragma unroll
-    for (int t = 0; t < TPC; ++t) {
-      if (WHOLE) epi_store<EPI>(p, tokc + t, n, lane, v[t], res[t]);
-      else slot_row[(size_t)(c * TPC + t) * TILE_N] = v[t];
-    }
+    for (int t = 0; t < GRP; ++t) epi_store<EPI>(p, tok + c + t, n, lane, v[c + t], res[t]);
   }
 }
 
+// Epilogue of one accumulator tile: TMEM -> registers (J columns summed per token with their activation scales, up to 128
+// tokens a thread), the accumulator given back, and only then the stores -- final values (whole) or this CTA's split-K slot --
+// which the next tile's MMAs run beside.  With the stores between the TMEM reads the tensor cores stood still for 5 (plain), 8
+// (SwiGLU) and 20 us (residual) a tile of 256 columns, against 14 for its 20 k-tiles.  tok_first = first token of the tile;
+// slot_row = slot + row.  2000 tokens, 34 816 x 5120 SwiGLU 677 -> 542 us;
+// 5120 x 6144 residual 189 -> 126.
 template <int BN, int J>
-__device__ __forceinline__ void epilogue_dispatch(const GemmParams& p, bool whole, uint32_t taddr0, const float* rs_s,
-                                                  float ts, int tok_first, int n, int lane, float* slot_row) {
-  if (!whole) epilogue_tile<BN, J, EPI_STORE, false>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
-  else if (p.epi == EPI_SWIGLU) epilogue_tile<BN, J, EPI_SWIGLU, true>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
-  else if (p.epi == EPI_RESIDUAL) epilogue_tile<BN, J, EPI_RESIDUAL, true>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
-  else if (p.epi == EPI_STORE_F32) epilogue_tile<BN, J, EPI_STORE_F32, true>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
-  else epilogue_tile<BN, J, EPI_STORE, true>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
+__device__ __forceinline__ void epilogue_tile(const GemmParams& p, bool whole, uint32_t taddr0, const float* rs_s, float ts,
+                                              int tok_first, int n, int lane, float* slot_row, uint32_t accum_empty) {
+  constexpr int CH = BN >= 32 ? 32 : 16, TPC = CH / J, V = BN / J < 128 ? BN / J : 128;
+#pragma unroll 1
+  for (int t0 = 0; t0 < BN / J; t0 += V) {
+    float v[V];
+#pragma unroll
+    for (int c = 0; c < V / TPC; ++c) {
+      uint32_t r[32];
+      const int col = t0 * J + c * CH;
+      if (CH == 32) tc_ld32(taddr0 + (uint32_t)col, r); else tc_ld16(taddr0 + (uint32_t)col, r);
+      tc_wait_ld();
+#pragma unroll
+      for (int t = 0; t < TPC; ++t) {
+        float a = 0.f;
+#pragma unroll
+        for (int j = 0; j < J; ++j) a = fmaf(__uint_as_float(r[t * J + j]), rs_s[col + t * J + j], a);
+        v[c * TPC + t] = a * ts;
+      }
+    }
+    if (t0 + V >= BN / J) {
+      tc_fence_before();
+      mbar_arrive(accum_empty);
+    }
+    if (!whole) {
+#pragma unroll
+      for (int t = 0; t < V; ++t) slot_row[(size_t)(t0 + t) * TILE_N] = v[t];
+    } else if (p.epi == EPI_SWIGLU) {
+      store_values<V, EPI_SWIGLU>(p, v, tok_first + t0, n, lane);
+    } else if (p.epi == EPI_RESIDUAL) {
+      store_values<V, EPI_RESIDUAL>(p, v, tok_first + t0, n, lane);
+    } else if (p.epi == EPI_STORE_F32) {
+      store_values<V, EPI_STORE_F32>(p, v, tok_first + t0, n, lane);
+    } else {
+      store_values<V, EPI_STORE>(p, v, tok_first + t0, n, lane);
+    }
+  }
 }
 
 template <int BN>
@@ -184,6 +201,113 @@ __device__ __forceinline__ void trace_stamp(int slot) {
 #else
   (void)slot;
 #endif
+}
+
+// Sums the per-segment slots of a split tile in segment order (bitwise reproducible) and finishes its values; the 128 epilogue
+// threads e = 0..127 of a block, `row` = this thread's row of the tile where one thread takes one row.
+__device__ __forceinline__ void finish_split_tile(const GemmParams& p, const float* tile_slots, int nseg, int ntok, int tok0,
+                                                  int nt, int row, int e) {
+  const int lane = e & 31, n = nt * TILE_N + row;
+  // finishing one (token, row) value of a split tile (run-time epilogue kind)
+  auto finish = [&](int tok, float v, float res) {
+    if (p.epi == EPI_SWIGLU) epi_store<EPI_SWIGLU>(p, tok, n, lane, v, res);
+    else if (p.epi == EPI_STORE_F32) epi_store<EPI_STORE_F32>(p, tok, n, lane, v, res);
+    else epi_store<EPI_STORE>(p, tok, n, lane, v, res);
+  };
+  auto load_res = [&](int tok) -> float {
+    return (p.epi == EPI_RESIDUAL && tok < p.tokens && n < p.N)
+               ? __bfloat162float(p.residual[(size_t)tok * p.ldr + n]) : 0.f;
+  };
+  const bool vec_ok = (p.N & 3) == 0 && (p.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 &&
+                      (p.epi != EPI_RESIDUAL ||
+                       ((p.ldr & 3) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 7) == 0));
+  if (vec_ok) {
+    // a thread owns 4 consecutive rows of 4 tokens per pass: 128-bit slot loads, one 64-bit
+    // (bf16) or 128-bit (fp32) store per token, a quarter of the memory instructions of the
+    // row-per-thread mapping; segments are summed in ascending order (bitwise reproducible)
+    constexpr int TQ = 4, SGB = 4;
+    const int rg = e & 31, tsub = e >> 5;
+    const int n4 = nt * TILE_N + rg * 4;
+    for (int g0 = 0; g0 < ntok; g0 += 4 * TQ) {
+      float4 acc[TQ];
+      uint2 res[TQ];
+#pragma unroll
+      for (int q = 0; q < TQ; ++q) {
+        const int g = g0 + q * 4 + tsub, tok = tok0 + g;
+        acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        res[q] = make_uint2(0u, 0u);
+        if (p.epi == EPI_RESIDUAL && g < ntok && tok < p.tokens && n4 < p.N)
+          res[q] = *reinterpret_cast<const uint2*>(p.residual + (size_t)tok * p.ldr + n4);
+      }
+      for (int sg0 = 0; sg0 < nseg; sg0 += SGB) {
+        float4 part[TQ][SGB];
+#pragma unroll
+        for (int q = 0; q < TQ; ++q)
+#pragma unroll
+          for (int sj = 0; sj < SGB; ++sj) {
+            const int g = g0 + q * 4 + tsub;
+            part[q][sj] = (sg0 + sj < nseg && g < ntok)
+                              ? __ldcg(reinterpret_cast<const float4*>(
+                                    tile_slots + ((size_t)(sg0 + sj) * ntok + g) * TILE_N + rg * 4))
+                              : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+#pragma unroll
+        for (int q = 0; q < TQ; ++q)
+#pragma unroll
+          for (int sj = 0; sj < SGB; ++sj) {
+            acc[q].x += part[q][sj].x, acc[q].y += part[q][sj].y;
+            acc[q].z += part[q][sj].z, acc[q].w += part[q][sj].w;
+          }
+      }
+#pragma unroll
+      for (int q = 0; q < TQ; ++q) {
+        const int g = g0 + q * 4 + tsub, tok = tok0 + g;
+        if (g >= ntok || tok >= p.tokens || n4 >= p.N) continue;
+        float4 a = acc[q];
+        if (p.epi == EPI_SWIGLU) {
+          const float y0 = __fdividef(a.x, 1.f + __expf(-a.x)) * a.y;
+          const float y1 = __fdividef(a.z, 1.f + __expf(-a.z)) * a.w;
+          *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(p.out) + (size_t)tok * p.ldo + (n4 >> 1)) =
+              f2_to_bf162_bits(y0, y1);
+        } else if (p.epi == EPI_STORE_F32) {
+          *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (size_t)tok * p.ldo + n4) = a;
+        } else {
+          const float2 r0 = bf162_bits_to_f2(res[q].x), r1 = bf162_bits_to_f2(res[q].y);
+          a.x += r0.x, a.y += r0.y, a.z += r1.x, a.w += r1.y;
+          *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(p.out) + (size_t)tok * p.ldo + n4) =
+              make_uint2(f2_to_bf162_bits(a.x, a.y), f2_to_bf162_bits(a.z, a.w));
+        }
+      }
+      if (g0 == 0 && e == 0) trace_stamp(11);
+    }
+  } else {
+  // row-per-thread fallback for outputs that do not allow vector stores
+  constexpr int GB = 16, SGB = 4;
+  for (int g0 = 0; g0 < ntok; g0 += GB) {
+    float acc[GB], res[GB];
+#pragma unroll
+    for (int gi = 0; gi < GB; ++gi) {
+      acc[gi] = 0.f;
+      res[gi] = g0 + gi < ntok ? load_res(tok0 + g0 + gi) : 0.f;
+    }
+    for (int sg0 = 0; sg0 < nseg; sg0 += SGB) {
+      float part[GB][SGB];
+#pragma unroll
+      for (int gi = 0; gi < GB; ++gi)
+#pragma unroll
+        for (int sj = 0; sj < SGB; ++sj)
+          part[gi][sj] = (sg0 + sj < nseg && g0 + gi < ntok)
+                             ? __ldcg(tile_slots + ((size_t)(sg0 + sj) * ntok + g0 + gi) * TILE_N + row) : 0.f;
+#pragma unroll
+      for (int gi = 0; gi < GB; ++gi)
+#pragma unroll
+        for (int sj = 0; sj < SGB; ++sj) acc[gi] += part[gi][sj];   // ascending segment order: bitwise reproducible
+    }
+#pragma unroll
+    for (int gi = 0; gi < GB; ++gi)
+      if (g0 + gi < ntok) finish(tok0 + g0 + gi, acc[gi], res[gi]);
+  }
+  }
 }
 
 template <int BN>
@@ -434,24 +558,12 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       if (!ok) break;
       tc_fence_after();
       if (seg == 0 && threadIdx.x == 64) trace_stamp(5);
-      // finishing one (token, row) value of a split tile (run-time epilogue kind)
-      auto finish = [&](int tok, float v, float res) {
-        if (p.epi == EPI_SWIGLU) epi_store<EPI_SWIGLU>(p, tok, n, lane, v, res);
-        else if (p.epi == EPI_STORE_F32) epi_store<EPI_STORE_F32>(p, tok, n, lane, v, res);
-        else epi_store<EPI_STORE>(p, tok, n, lane, v, res);
-      };
-      auto load_res = [&](int tok) -> float {
-        return (p.epi == EPI_RESIDUAL && tok < p.tokens && n < p.N)
-                   ? __bfloat162float(p.residual[(size_t)tok * p.ldr + n]) : 0.f;
-      };
       {
         const uint32_t taddr0 = tmem_base + ((uint32_t)(quad * 32) << 16);
-        if (J == 4) epilogue_dispatch<BN, 4>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row);
-        else if (J == 2) epilogue_dispatch<BN, 2>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row);
-        else epilogue_dispatch<BN, 1>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row);
+        if (J == 4) epilogue_tile<BN, 4>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
+        else if (J == 2) epilogue_tile<BN, 2>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
+        else epilogue_tile<BN, 1>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
       }
-      tc_fence_before();
-      mbar_arrive(accum_empty);
       if (threadIdx.x == 64) trace_stamp(6);
       if (!whole) {
         // split tile: the last CTA to arrive finishes it from the per-segment slots
@@ -468,98 +580,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         if (*last_flag) {
           __threadfence();
           if (threadIdx.x == 64) trace_stamp(10);
-          const int ntok = BN / J;
-          const bool vec_ok = (p.N & 3) == 0 && (p.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 &&
-                              (p.epi != EPI_RESIDUAL ||
-                               ((p.ldr & 3) == 0 && (reinterpret_cast<uintptr_t>(p.residual) & 7) == 0));
-          if (vec_ok) {
-            // a thread owns 4 consecutive rows of 4 tokens per pass: 128-bit slot loads, one 64-bit
-            // (bf16) or 128-bit (fp32) store per token, a quarter of the memory instructions of the
-            // row-per-thread mapping; segments are summed in ascending order (bitwise reproducible)
-            constexpr int TQ = 4, SGB = 4;
-            const int e = (int)threadIdx.x - 64;
-            const int rg = e & 31, tsub = e >> 5;
-            const int n4 = nt * TILE_N + rg * 4;
-            for (int g0 = 0; g0 < ntok; g0 += 4 * TQ) {
-              float4 acc[TQ];
-              uint2 res[TQ];
-#pragma unroll
-              for (int q = 0; q < TQ; ++q) {
-                const int g = g0 + q * 4 + tsub, tok = tok0 + g;
-                acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                res[q] = make_uint2(0u, 0u);
-                if (p.epi == EPI_RESIDUAL && g < ntok && tok < p.tokens && n4 < p.N)
-                  res[q] = *reinterpret_cast<const uint2*>(p.residual + (size_t)tok * p.ldr + n4);
-              }
-              for (int sg0 = 0; sg0 < nseg; sg0 += SGB) {
-                float4 part[TQ][SGB];
-#pragma unroll
-                for (int q = 0; q < TQ; ++q)
-#pragma unroll
-                  for (int sj = 0; sj < SGB; ++sj) {
-                    const int g = g0 + q * 4 + tsub;
-                    part[q][sj] = (sg0 + sj < nseg && g < ntok)
-                                      ? __ldcg(reinterpret_cast<const float4*>(
-                                            tile_slots + ((size_t)(sg0 + sj) * ntok + g) * TILE_N + rg * 4))
-                                      : make_float4(0.f, 0.f, 0.f, 0.f);
-                  }
-#pragma unroll
-                for (int q = 0; q < TQ; ++q)
-#pragma unroll
-                  for (int sj = 0; sj < SGB; ++sj) {
-                    acc[q].x += part[q][sj].x, acc[q].y += part[q][sj].y;
-                    acc[q].z += part[q][sj].z, acc[q].w += part[q][sj].w;
-                  }
-              }
-#pragma unroll
-              for (int q = 0; q < TQ; ++q) {
-                const int g = g0 + q * 4 + tsub, tok = tok0 + g;
-                if (g >= ntok || tok >= p.tokens || n4 >= p.N) continue;
-                float4 a = acc[q];
-                if (p.epi == EPI_SWIGLU) {
-                  const float y0 = __fdividef(a.x, 1.f + __expf(-a.x)) * a.y;
-                  const float y1 = __fdividef(a.z, 1.f + __expf(-a.z)) * a.w;
-                  *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(p.out) + (size_t)tok * p.ldo + (n4 >> 1)) =
-                      f2_to_bf162_bits(y0, y1);
-                } else if (p.epi == EPI_STORE_F32) {
-                  *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (size_t)tok * p.ldo + n4) = a;
-                } else {
-                  const float2 r0 = bf162_bits_to_f2(res[q].x), r1 = bf162_bits_to_f2(res[q].y);
-                  a.x += r0.x, a.y += r0.y, a.z += r1.x, a.w += r1.y;
-                  *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(p.out) + (size_t)tok * p.ldo + n4) =
-                      make_uint2(f2_to_bf162_bits(a.x, a.y), f2_to_bf162_bits(a.z, a.w));
-                }
-              }
-              if (g0 == 0 && threadIdx.x == 64) trace_stamp(11);
-            }
-          } else {
-          // row-per-thread fallback for outputs that do not allow vector stores
-          constexpr int GB = 16, SGB = 4;
-          for (int g0 = 0; g0 < ntok; g0 += GB) {
-            float acc[GB], res[GB];
-#pragma unroll
-            for (int gi = 0; gi < GB; ++gi) {
-              acc[gi] = 0.f;
-              res[gi] = g0 + gi < ntok ? load_res(tok0 + g0 + gi) : 0.f;
-            }
-            for (int sg0 = 0; sg0 < nseg; sg0 += SGB) {
-              float part[GB][SGB];
-#pragma unroll
-              for (int gi = 0; gi < GB; ++gi)
-#pragma unroll
-                for (int sj = 0; sj < SGB; ++sj)
-                  part[gi][sj] = (sg0 + sj < nseg && g0 + gi < ntok)
-                                     ? __ldcg(tile_slots + ((size_t)(sg0 + sj) * ntok + g0 + gi) * TILE_N + row) : 0.f;
-#pragma unroll
-              for (int gi = 0; gi < GB; ++gi)
-#pragma unroll
-                for (int sj = 0; sj < SGB; ++sj) acc[gi] += part[gi][sj];   // ascending segment order: bitwise reproducible
-            }
-#pragma unroll
-            for (int gi = 0; gi < GB; ++gi)
-              if (g0 + gi < ntok) finish(tok0 + g0 + gi, acc[gi], res[gi]);
-          }
-          }
+          finish_split_tile(p, tile_slots, nseg, BN / J, tok0, nt, quad * 32 + lane, (int)threadIdx.x - 64);
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
       }
@@ -903,6 +924,11 @@ TRL_API int trl_quant_act_nvfp4(const void* x, int ldx, const void* norm_w, floa
                          swiglu_in);
 }
 
+// How a product is laid out: columns a tile, CTAs, whole tiles or split ones.
+struct GemmPlan {
+  int BN, n_tiles, c_tiles, nk, grid, split, max_seg;
+};
+
 // Largest number of CTAs that share one output tile under the even stream-K split.
 static int max_segments(long long U, int G, int nk) {
   // a tile spans nk consecutive units; CTA ranges are ~U/G long
@@ -924,16 +950,31 @@ TRL_API int trl_gemm_trace_read(void* out, int n_ctas) {
   return (int)cudaMemcpyFromSymbol(out, g_gemm_trace, (size_t)n_ctas * TRACE_SLOTS * sizeof(unsigned long long));
 }
 
-TRL_API long trl_gemm_nvfp4_scratch_bytes(int tokens, int J, int N, int K, int max_ctas) {
-  const int cols = tokens * J, BN = pick_bn(cols);
-  const int n_tiles = (N + TILE_N - 1) / TILE_N, c_tiles = (cols + BN - 1) / BN, nk = (K + KT_ELEMS - 1) / KT_ELEMS;
+// split: 1 / 0 as the caller wants it, -1 by the rule below.  Tiles are split along K when the last round of whole tiles would
+// leave more of the GPU idle than adding up the partial tiles costs.  In units of one k-tile of one tile (0.55 us with up to
+// 128 columns, 0.7 us with 256) the addition costs about ten and 16: measured at 8, 32 and 37 rows 5.4 us, at 512 rows 11 us.
+// 8 rows x 16 480: whole 20 against 17.4 + 10, 23.6 us against 27.6; 512 rows x 5120 x 17 408: 136 against 73.5 + 16, 141 us
+// against 96.  The 5 %: not for every last round its scratch memory.
+static GemmPlan plan_gemm(int tokens, int J, int N, int K, int max_ctas, int split) {
+  GemmPlan g;
+  const int cols = tokens * J;
+  g.BN = pick_bn(cols);
+  g.n_tiles = (N + TILE_N - 1) / TILE_N, g.c_tiles = (cols + g.BN - 1) / g.BN, g.nk = (K + KT_ELEMS - 1) / KT_ELEMS;
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (max_ctas > 0) sms = min(sms, max_ctas);
-  const long long U = (long long)n_tiles * c_tiles * nk;
-  const int grid = (int)min((long long)sms, U);
-  return (long)n_tiles * c_tiles * max_segments(U, grid, nk) * (BN / J) * TILE_N * (long)sizeof(float);
+  const long long T = (long long)g.n_tiles * g.c_tiles, U = T * g.nk;
+  const double whole = (double)((T + sms - 1) / sms) * g.nk, even = (double)U / sms + (g.BN == 256 ? 16 : 10);
+  g.split = split >= 0 ? split : whole > 1.05 * even;
+  g.grid = (int)min((long long)sms, g.split ? U : T);
+  g.max_seg = g.split ? max_segments(U, g.grid, g.nk) : 1;
+  return g;
+}
+
+TRL_API long trl_gemm_nvfp4_scratch_bytes(int tokens, int J, int N, int K, int max_ctas, int split) {
+  const GemmPlan g = plan_gemm(tokens, J, N, K, max_ctas, split);
+  return g.split ? (long)g.n_tiles * g.c_tiles * g.max_seg * (g.BN / J) * TILE_N * (long)sizeof(float) : 0;
 }
 
 // out[tok, n] = epi(...).  wq [N, K/2] packed e2m1; sfw / sfx tiled scales; partial: fp32
@@ -945,37 +986,26 @@ TRL_API int trl_gemm_nvfp4(const void* wq, const void* sfw, const void* tscale, 
                            int split, int w_tiled, void* stream) {
   if (K % 32 != 0 || J < 1 || (32 % J) != 0 || J > 16) return (int)cudaErrorInvalidValue;
   const int cols = tokens * J;
-  const int BN = pick_bn(cols);
+  const GemmPlan g = plan_gemm(tokens, J, N, K, max_ctas, split);
   CUtensorMap mw, mx;
   {
-    const uint64_t nt = (N + TILE_N - 1) / TILE_N, nkk = (K + KT_ELEMS - 1) / KT_ELEMS;
+    const uint64_t nt = g.n_tiles, nkk = g.nk;
     const int rc = w_tiled ? make_map(&mw, wq, nt * nkk * TILE_N, KT_BYTES, TILE_N)
                            : make_map(&mw, wq, (uint64_t)N, (uint64_t)K / 2, TILE_N);
     if (rc) return (int)cudaErrorInvalidValue;
   }
-  if (make_map(&mx, xq, (uint64_t)cols, (uint64_t)K / 2, (uint32_t)BN)) return (int)cudaErrorInvalidValue;
+  if (make_map(&mx, xq, (uint64_t)cols, (uint64_t)K / 2, (uint32_t)g.BN)) return (int)cudaErrorInvalidValue;
   GemmParams p;
   p.sfw = (const uint8_t*)sfw, p.sfx = (const uint8_t*)sfx, p.tscale = (const float*)tscale, p.rs = (const float*)rs;
   p.residual = (const bf16*)residual, p.out = out, p.partial = (float*)partial, p.counters = (int*)counters;
   p.N = N, p.K = K, p.cols = cols, p.tokens = tokens, p.J = J, p.ldr = ldr, p.ldo = ldo;
-  p.n_tiles = (N + TILE_N - 1) / TILE_N;
-  p.c_tiles = (cols + BN - 1) / BN;
-  p.nk = (K + KT_ELEMS - 1) / KT_ELEMS;
-  p.kt4 = p.nk * 4;
-  p.epi = epi;
-  int sms = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (max_ctas > 0) sms = min(sms, max_ctas);
-  const long long U = (long long)p.n_tiles * p.c_tiles * p.nk;
-  p.split = split;
-  p.w_tiled = w_tiled;
-  const int grid = split ? (int)min((long long)sms, U) : min(sms, p.n_tiles * p.c_tiles);
-  p.max_seg = split ? max_segments(U, grid, p.nk) : 1;
-  if (split && (size_t)p.n_tiles * p.c_tiles * p.max_seg * (BN / J) * TILE_N * sizeof(float) > (size_t)partial_bytes)
+  p.n_tiles = g.n_tiles, p.c_tiles = g.c_tiles, p.nk = g.nk, p.kt4 = g.nk * 4;
+  p.epi = epi, p.split = g.split, p.w_tiled = w_tiled, p.max_seg = g.max_seg;
+  if (g.split && (size_t)g.n_tiles * g.c_tiles * g.max_seg * (g.BN / J) * TILE_N * sizeof(float) > (size_t)partial_bytes)
     return (int)cudaErrorMemoryAllocation;
   cudaStream_t st = (cudaStream_t)stream;
-  switch (BN) {
+  const int grid = g.grid;
+  switch (g.BN) {
     case 16: return launch<16>(mw, mx, p, grid, st);
     case 32: return launch<32>(mw, mx, p, grid, st);
     case 64: return launch<64>(mw, mx, p, grid, st);

@@ -136,6 +136,38 @@ def test_fp8_attention_on_tensor_cores(ops, g_heads, splits, scale_v):
         assert _rel(out[i].view(n_q, d), final) < (2e-2 if i == 1 else 2 ** -8), n
 
 
+@pytest.mark.parametrize("tokens,n,k", [(3, 20000, 512), (9, 700, 5120), (40, 19000, 288), (129, 128, 256), (130, 130, 288), (200, 384, 2048), (256, 1000, 5120), (257, 4130, 1056), (700, 640, 6144),
+                                        (1111, 5120, 1024), (2100, 5120, 256)])
+@pytest.mark.parametrize("split", [False, True, None])
+def test_gemm_tiles_whole_and_split_equal_one_cta_alone(ops, tokens, n, k, split):
+    """Tiles that several CTAs and one go through (their accumulator is given back before the values are stored), rows and K that
+    fill no tile, tiles whole and split, every epilogue, against the same kernel on one CTA.  The same products in
+    fp32, summed in another order where tiles are split."""
+    from tilerl_b200 import formats as F
+    from tilerl_b200.ops import native
+    from tilerl_b200.ops.gemm_tc import gemm_nvfp4
+    g = torch.Generator().manual_seed(tokens + n)
+    w = F.quantize_nvfp4(torch.randn(n, k, generator=g) * 0.02).to(DEV)
+    x = torch.randn(tokens, k, generator=g).to(DEV, torch.bfloat16)
+    got, want = (torch.full((tokens, n), float("nan"), device=DEV) for _ in range(2))
+    gemm_nvfp4(ops, x, w, want, terms=2, epi=3, max_ctas=1, split=False)
+    for _ in range(2):
+        gemm_nvfp4(ops, x, w, got, terms=2, epi=3, split=split)
+        assert _rel(got, want) < 1e-6
+    a = torch.full((tokens, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+    gemm_nvfp4(ops, x, w, a, terms=2, split=split)
+    assert _rel(a, want) < 2 ** -8
+    if n % 2 == 0:
+        h = torch.full((tokens, n // 2), float("nan"), dtype=torch.bfloat16, device=DEV)
+        gemm_nvfp4(ops, x, w, h, terms=2, epi=2, split=split)
+        assert _rel(h, torch.nn.functional.silu(want[:, 0::2].double()) * want[:, 1::2].double()) < 2 ** -8
+    r = torch.randn(tokens, n, generator=g).to(DEV, torch.bfloat16)
+    acc = r.clone()
+    gemm_nvfp4(ops, x, w, acc, terms=2, epi=1, residual=acc, split=split)
+    assert _rel(acc, want.double() + r.double()) < 2 ** -8
+    assert native.read_error()[0] == 0
+
+
 @pytest.mark.parametrize("nk,nv,d,taps", [(2, 4, 128, 4), (1, 3, 128, 4), (2, 2, 64, 4), (2, 4, 128, 3)])
 def test_delta_rule_prep_over_runs_of_tokens(ops, nk, nv, d, taps):
     """Convolution, norms and gates of tokens taken in runs of 8 (thousands of tokens), 4, 2 and 1: sequences that begin inside a

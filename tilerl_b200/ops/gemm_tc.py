@@ -20,7 +20,7 @@ from . import native as N
 N.register("trl_quant_act_nvfp4", [N.P, N.I, N.P, N.F, N.P, N.P, N.P, N.I, N.I, N.I, N.I, N.P])
 N.register("trl_gemm_nvfp4", [N.P, N.P, N.P, N.P, N.P, N.P, N.P, N.I, N.P, N.I, N.P, N.P, N.L,
                               N.I, N.I, N.I, N.I, N.I, N.I, N.I, N.I, N.P])
-N.register("trl_gemm_nvfp4_scratch_bytes", [N.I, N.I, N.I, N.I, N.I])
+N.register("trl_gemm_nvfp4_scratch_bytes", [N.I, N.I, N.I, N.I, N.I, N.I])
 N.register("trl_gemv_stream_bytes", [N.I, N.I])
 N.register("trl_gemv_stream_pack", [N.P, N.P, N.P, N.I, N.I, N.P])
 N.register("trl_gemv2_nvfp4", [N.P, N.I, N.P, N.P, N.P, N.F, N.P, N.I, N.P, N.I, N.I, N.I, N.I, N.I, N.P])
@@ -152,14 +152,11 @@ def _scratch(ops, nbytes: int, tiles: int):
     return buf, ops.ws.bufs["tc_counters"]
 
 
-def _want_split(ops, n: int, k: int, cols: int) -> bool:
-    """Split tiles along K only when whole tiles cannot occupy the SMs."""
+def _want_split() -> int:
+    """Split tiles along K: 1 / 0 forced by ``TRL_SPLITK``, -1: by the launcher's rule (``csrc/gemm_tc.cu::plan_gemm``)."""
     import os
     mode = os.environ.get("TRL_SPLITK", "auto")
-    if mode in ("0", "1"):
-        return mode == "1"
-    tiles = ((n + 127) // 128) * ((cols + 255) // 256 if cols > 256 else 1)
-    return tiles < ops.sms
+    return int(mode) if mode in ("0", "1") else -1
 
 
 def gemm_nvfp4(ops, x: torch.Tensor, w: NVFP4Tensor, y: torch.Tensor, *, terms: int = 1, norm_w=None,
@@ -175,14 +172,15 @@ def gemm_nvfp4(ops, x: torch.Tensor, w: NVFP4Tensor, y: torch.Tensor, *, terms: 
     c_tiles = (cols + bn - 1) // bn
     n_tiles = (n + 127) // 128
     ops.lib.trl_gemm_nvfp4_scratch_bytes.restype = __import__("ctypes").c_long
-    nbytes = ops.lib.trl_gemm_nvfp4_scratch_bytes(t, terms, n, k, max_ctas)
+    split = _want_split() if split is None else int(split)
+    nbytes = ops.lib.trl_gemm_nvfp4_scratch_bytes(t, terms, n, k, max_ctas, split)
     partial, counters = _scratch(ops, nbytes, n_tiles * c_tiles)
     tiled = getattr(ops, "tile_weights", True)
     N.check(ops.lib.trl_gemm_nvfp4(
         (wq_tiled(w) if tiled else w.wq).data_ptr(), sf_tiled(w).data_ptr(), w.tscale.data_ptr(), xq.data_ptr(), sfx.data_ptr(),
         rs.data_ptr(), N.ptr(residual), residual.stride(0) if residual is not None else 0,
         y.data_ptr(), y.stride(0), partial.data_ptr(), counters.data_ptr(), partial.numel() * 4, t, terms, n, k,
-        epi, max_ctas, int(_want_split(ops, n, k, cols) if split is None else split), int(tiled),
+        epi, max_ctas, split, int(tiled),
         N.stream()), "gemm_nvfp4")
     N.count()
 

@@ -146,7 +146,7 @@ def main():
             from tilerl_b200.ops.gemm_tc import _scratch
             import ctypes
             ops.lib.trl_gemm_nvfp4_scratch_bytes.restype = ctypes.c_long
-            nb = ops.lib.trl_gemm_nvfp4_scratch_bytes(args.m, args.terms, n, k, args.max_ctas)
+            nb = ops.lib.trl_gemm_nvfp4_scratch_bytes(args.m, args.terms, n, k, args.max_ctas, int(args.split))
             partial, counters = _scratch(ops, nb, 8192)
 
             def gemm_only(w):
