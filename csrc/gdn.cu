@@ -22,7 +22,10 @@
 // reference.py:1142-1277.
 #include <stdlib.h>
 
+#include <cuda.h>
+
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace {
 
@@ -790,17 +793,30 @@ gdn_scan_wy_kernel(const float* qn, const float* kn,
 // state scan, chunk output), here one kernel.
 constexpr int GC_C = 16, GC_D = 128, GC_ROW = GC_D * 2;     // chunk, head dim, bytes of a bf16 row over dk
 constexpr int GC_NS = 2, GC_DV = GC_D / GC_NS, GC_VROW = GC_DV * 2;   // value columns per CTA, bytes of such a row
-struct GcSmem {
-  float sq[2][GC_C][GC_D], sk[2][GC_C][GC_D];    // fp32 q, k of the current and the next chunk
-  float sv[2][GC_C][GC_DV];                      // fp32 v, this CTA's columns
-  float sg[2][GC_C], sb[2][GC_C];
-  __align__(128) unsigned char qraw[GC_C * GC_ROW], kraw[GC_C * GC_ROW], qe[GC_C * GC_ROW], kb[GC_C * GC_ROW],
-      ws[GC_C * GC_ROW];                                                 // bf16 [16][128 dk], 16-byte chunks XOR-swizzled
-  __align__(128) unsigned char vb[GC_C * GC_VROW], vn[GC_C * GC_VROW];   // bf16 [16][64 dv]
-  __align__(128) unsigned char sbf[GC_D * GC_VROW];                      // bf16 copy of the state [dk][64 dv], swizzled
-  __align__(16) unsigned char kdt[GC_D * 32];                            // (K e^{G_last - G})^T  bf16 [128][16]
-  __align__(16) unsigned char t_hi[GC_C * 32], t_lo[GC_C * 32], qkm[GC_C * 32];   // bf16 [16][16]
+constexpr int GC_SLOTS = 4, GC_GROUP = 256, GC_THREADS = 3 * GC_GROUP;
+struct GcPre {                                   // working memory of one group of preparing warps
+  float sq[GC_C][GC_D], sk[GC_C][GC_D];          // fp32 q, k of its chunk
+  float sv[GC_C][GC_DV];                         // fp32 v, this CTA's columns
+  float sg[2][GC_C], sb[2][GC_C];                // gates of its chunk and of its next one
+  __align__(128) unsigned char qraw[GC_C * GC_ROW], kraw[GC_C * GC_ROW], kb[GC_C * GC_ROW];   // bf16 [16][128 dk], 16-byte chunks XOR-swizzled
+  __align__(128) unsigned char vb[GC_C * GC_VROW];                       // bf16 [16][64 dv]
+  __align__(16) unsigned char t_hi[GC_C * 32], t_lo[GC_C * 32];          // bf16 [16][16]
   float a[GC_C][GC_C + 1];                       // fp32 A
+};
+struct GcSlot {                                  // what a chunk hands to the warps that hold the state
+  __align__(128) unsigned char qe[GC_C * GC_ROW], ws[GC_C * GC_ROW];     // Q e^G and W, as above
+  __align__(16) unsigned char kdt[GC_D * 32];                            // (K e^{G_last - G})^T  bf16 [128][16]
+  __align__(16) unsigned char qkm[GC_C * 32];                            // bf16 [16][16]
+  __align__(16) float4 u[GC_GROUP];                                      // U in accumulator fragments
+  float g_last;
+};
+struct GcSmem {
+  GcPre pre[2];
+  GcSlot slot[GC_SLOTS];
+  __align__(128) unsigned char vn[GC_C * GC_VROW];                       // bf16 [16][64 dv]
+  __align__(128) unsigned char sbf[GC_D * GC_VROW];                      // bf16 copy of the state [dk][64 dv], swizzled
+  unsigned long long full[GC_SLOTS], empty[GC_SLOTS];
+  int abort;
 };
 __device__ __forceinline__ void gc_cp4(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(gsrc) : "memory");
@@ -825,10 +841,13 @@ __device__ __forceinline__ void gc_mma(float (&c)[4], const uint32_t (&a)[4], ui
 }
 
 // grid (2 nv, B): CTA = (value head, half of its value columns, sequence).  The delta rule never mixes
-// value columns, so the two halves of a head are independent scans; what depends only on q, k and
-// the gates (KK, QK, T, W) is computed by both.  Raw outputs go to o_scratch (fp32); the gated
-// RMSNorm, which needs whole rows, is the small kernel below.
-__global__ void __launch_bounds__(256, 2)
+// value columns, so the two halves of a head are independent scans.  What depends only on q, k and the gates (KK, QK, T, W, and U
+// from v) does not wait for the state: two groups of eight warps prepare the chunks, one the even, one the odd ones, up to four
+// chunks ahead, and eight warps that hold the state take them over with two block-wide meetings a chunk.  In one sequence of
+// phases, as before, a chunk took 2.9 us (a 2000-token layer 360 us); here 2.0 us (251 us).  The chain of the chunks bounds it: products of
+// 16 rows, no unit is busy.  Raw outputs go to o_scratch (fp32); the gated RMSNorm, which needs whole rows, is the small
+// kernel below.
+__global__ void __launch_bounds__(GC_THREADS, 1)
 gdn_chunk_mma_kernel(const float* qn, const float* kn, const float* vc, const float* gin, const float* bin,
                      float* states, int* cur, bf16* ring, const bf16* inp, int ld, const int* q_start,
                      const int* q_len, const int* positions, const int* state_slots, long state_slot_stride,
@@ -839,272 +858,293 @@ gdn_chunk_mma_kernel(const float* qn, const float* kn, const float* vc, const fl
   pdl_launch_dependents(2);
   pdl_wait();
   const int h = blockIdx.x / GC_NS, c0 = (blockIdx.x % GC_NS) * DV, seq = blockIdx.y;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int group = threadIdx.x / GC_GROUP, tid = threadIdx.x % GC_GROUP, warp = tid >> 5, lane = tid & 31;
   const int T = q_len[seq], t0 = q_start[seq];
   if (T == 0) return;
+  const int chunks = (T + C - 1) / C;
   const int slot = state_slots[seq];
   const int kh = h * nk / nv;
-  const int live = cur[slot];
-  float* sp = states + (size_t)slot * state_slot_stride + (size_t)h * D * D + (size_t)live * plane_stride + c0;
   const int g8 = lane >> 2, t4 = lane & 3;
   const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8;      // ldmatrix row of this lane (both x4 layouts used here)
-
   auto u32 = [](const void* p) { return (uint32_t)__cvta_generic_to_shared(p); };
-  const uint32_t a_qraw = u32(sm.qraw), a_kraw = u32(sm.kraw), a_qe = u32(sm.qe), a_kb = u32(sm.kb), a_vb = u32(sm.vb),
-                 a_ws = u32(sm.ws), a_vn = u32(sm.vn), a_sbf = u32(sm.sbf), a_kdt = u32(sm.kdt), a_thi = u32(sm.t_hi),
-                 a_tlo = u32(sm.t_lo), a_qkm = u32(sm.qkm);
-
-  // state rows 16 warp .. 16 warp + 15, this CTA's 64 columns, as accumulator fragments
-  float S[DV / 8][4];
-#pragma unroll
-  for (int nt = 0; nt < DV / 8; ++nt) {
-    const float2 lo = *reinterpret_cast<const float2*>(sp + (size_t)(16 * warp + g8) * D + nt * 8 + t4 * 2);
-    const float2 hi = *reinterpret_cast<const float2*>(sp + (size_t)(16 * warp + g8 + 8) * D + nt * 8 + t4 * 2);
-    S[nt][0] = lo.x, S[nt][1] = lo.y, S[nt][2] = hi.x, S[nt][3] = hi.y;
+  volatile int* abort_flag = &sm.abort;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < GC_SLOTS; ++i) mbar_init(u32(&sm.full[i]), GC_GROUP), mbar_init(u32(&sm.empty[i]), GC_GROUP);
+    sm.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  auto store_sbf = [&]() {
-#pragma unroll
-    for (int nt = 0; nt < DV / 8; ++nt) {
-      *reinterpret_cast<uint32_t*>(sm.sbf + gc_offv(16 * warp + g8, nt) + t4 * 4) = f2_to_bf162_bits(S[nt][0], S[nt][1]);
-      *reinterpret_cast<uint32_t*>(sm.sbf + gc_offv(16 * warp + g8 + 8, nt) + t4 * 4) = f2_to_bf162_bits(S[nt][2], S[nt][3]);
-    }
-  };
-  store_sbf();
-
-  auto stage = [&](int i0, int b) {      // fp32 q, k, v rows and the gates of chunk i0 .. i0 + 15 (rows past T: zeros)
-    for (int x = tid; x < C * (D / 4); x += 256) {
-      const int tt = x / (D / 4), e = (x % (D / 4)) * 4;
-      if (i0 + tt < T) {
-        const size_t src = ((size_t)(t0 + i0 + tt) * nk + kh) * D + e;
-        cp_async16(&sm.sq[b][tt][e], qn + src);
-        cp_async16(&sm.sk[b][tt][e], kn + src);
-      } else {
-        *reinterpret_cast<float4*>(&sm.sq[b][tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
-        *reinterpret_cast<float4*>(&sm.sk[b][tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-    {
-      const int tt = tid >> 4, e = (tid & 15) * 4;
-      if (i0 + tt < T) cp_async16(&sm.sv[b][tt][e], vc + ((size_t)(t0 + i0 + tt) * nv + h) * D + c0 + e);
-      else *reinterpret_cast<float4*>(&sm.sv[b][tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    if (tid < C) {                       // gates: asynchronous too, nothing of the next chunk is waited for here
-      if (i0 + tid < T) {
-        gc_cp4(&sm.sg[b][tid], gin + (size_t)(t0 + i0 + tid) * nv + h);
-        gc_cp4(&sm.sb[b][tid], bin + (size_t)(t0 + i0 + tid) * nv + h);
-      } else {
-        sm.sg[b][tid] = 0.f, sm.sb[b][tid] = 0.f;                           // padding rows: no decay, no update
-      }
-    }
-    cp_async_commit();
+  __syncthreads();
+  // the group's threads meet; true when `ok` is in every one of them (a wait that ran out ends the whole group together)
+  auto meet = [&](bool ok) {
+    uint32_t r;
+    asm volatile(
+        "{ .reg .pred p, q;\n"
+        "  setp.ne.u32 q, %1, 0;\n"
+        "  bar.red.and.pred p, %2, %3, q;\n"
+        "  selp.u32 %0, 1, 0, p; }\n"
+        : "=r"(r) : "r"((uint32_t)ok), "r"(group + 1), "r"(GC_GROUP) : "memory");
+    return r != 0;
   };
 
-  stage(0, 0);
-  int b = 0;
-  for (int i0 = 0; i0 < T; i0 += C, b ^= 1) {
-    cp_async_wait<0>();
-    __syncthreads();                       // chunk b landed; the previous chunk's tiles are free
-    if (i0 + C < T) stage(i0 + C, b ^ 1);
-    // running sums of the log-decays, recomputed where they are needed (16 broadcast reads)
-    float g_last = 0.f;
-#pragma unroll
-    for (int j = 0; j < C; ++j) g_last += sm.sg[b][j];
-    // ---- operand tiles (bf16) from the staged fp32 rows: thread = (token, 8 columns)
-    {
-      const int tt = tid >> 4, ch = tid & 15, e = ch * 8;
-      float gi = 0.f;
-      for (int j = 0; j <= tt; ++j) gi += sm.sg[b][j];
-      const float eg = __expf(gi), beta = sm.sb[b][tt], kbs = beta * eg;
-      const float4 q0 = *reinterpret_cast<const float4*>(&sm.sq[b][tt][e]), q1 = *reinterpret_cast<const float4*>(&sm.sq[b][tt][e + 4]);
-      const float4 k0 = *reinterpret_cast<const float4*>(&sm.sk[b][tt][e]), k1 = *reinterpret_cast<const float4*>(&sm.sk[b][tt][e + 4]);
-      const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-      const float kv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
-      uint32_t oq[4], ok_[4], oqe[4], okb[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        oq[j] = f2_to_bf162_bits(qv[2 * j], qv[2 * j + 1]);
-        ok_[j] = f2_to_bf162_bits(kv[2 * j], kv[2 * j + 1]);
-        oqe[j] = f2_to_bf162_bits(qv[2 * j] * eg, qv[2 * j + 1] * eg);
-        okb[j] = f2_to_bf162_bits(kv[2 * j] * kbs, kv[2 * j + 1] * kbs);
+  if (group > 0) {
+    // ---------------- preparing groups ----------------
+    const int first = group - 1;
+    GcPre& w = sm.pre[first];
+    const uint32_t a_qraw = u32(w.qraw), a_kraw = u32(w.kraw), a_kb = u32(w.kb), a_vb = u32(w.vb), a_thi = u32(w.t_hi), a_tlo = u32(w.t_lo);
+    auto stage = [&](int i0, int b) {      // fp32 q, k, v rows and the gates of chunk i0 .. i0 + 15 (rows past T: zeros)
+      for (int x = tid; x < C * (D / 4); x += GC_GROUP) {
+        const int tt = x / (D / 4), e = (x % (D / 4)) * 4;
+        if (i0 + tt < T) {
+          const size_t src = ((size_t)(t0 + i0 + tt) * nk + kh) * D + e;
+          cp_async16(&w.sq[tt][e], qn + src);
+          cp_async16(&w.sk[tt][e], kn + src);
+        } else {
+          *reinterpret_cast<float4*>(&w.sq[tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
+          *reinterpret_cast<float4*>(&w.sk[tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
       }
-      const uint32_t off = gc_off(tt, ch);
-      *reinterpret_cast<uint4*>(sm.qraw + off) = make_uint4(oq[0], oq[1], oq[2], oq[3]);
-      *reinterpret_cast<uint4*>(sm.kraw + off) = make_uint4(ok_[0], ok_[1], ok_[2], ok_[3]);
-      *reinterpret_cast<uint4*>(sm.qe + off) = make_uint4(oqe[0], oqe[1], oqe[2], oqe[3]);
-      *reinterpret_cast<uint4*>(sm.kb + off) = make_uint4(okb[0], okb[1], okb[2], okb[3]);
-      if (ch < DV / 8) {
-        const float4 v0 = *reinterpret_cast<const float4*>(&sm.sv[b][tt][e]), v1 = *reinterpret_cast<const float4*>(&sm.sv[b][tt][e + 4]);
-        *reinterpret_cast<uint4*>(sm.vb + gc_offv(tt, ch)) =
-            make_uint4(f2_to_bf162_bits(v0.x * beta, v0.y * beta), f2_to_bf162_bits(v0.z * beta, v0.w * beta),
-                       f2_to_bf162_bits(v1.x * beta, v1.y * beta), f2_to_bf162_bits(v1.z * beta, v1.w * beta));
-      }
-    }
-    {
-      // transposed decayed keys [dk][token]: thread = (dk row, 8 tokens), one 16-byte store
-      const int r = tid & 127, half = tid >> 7;
-      float gi = 0.f;
-      for (int j = 0; j < half * 8; ++j) gi += sm.sg[b][j];
-      uint32_t o[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        gi += sm.sg[b][half * 8 + 2 * j];
-        const float x0 = sm.sk[b][half * 8 + 2 * j][r] * __expf(g_last - gi);
-        gi += sm.sg[b][half * 8 + 2 * j + 1];
-        const float x1 = sm.sk[b][half * 8 + 2 * j + 1][r] * __expf(g_last - gi);
-        o[j] = f2_to_bf162_bits(x0, x1);
-      }
-      *reinterpret_cast<uint4*>(sm.kdt + (size_t)r * 32 + half * 16) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
-    __syncthreads();
-    // ---- warp 0: KK -> A -> T = (I + A)^-1;  warp 1: QK';  warps 2..7 meanwhile start O = (Q e^G) S
-    float O[4] = {0.f, 0.f, 0.f, 0.f};     // this warp's 8 value columns
-    auto qs_product = [&]() {
-#pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) {
-        uint32_t af[4], bs[2];
-        gc_ldsm(af, a_qe + gc_off(lrow, kk * 2 + (lane >> 4)));
-        gc_ldsm2_t(bs, a_sbf + gc_offv(kk * 16 + lrow, warp));
-        gc_mma(O, af, bs[0], bs[1]);
-      }
-    };
-    if (warp < 2) {
-      float gc[C];                         // inclusive running sums
       {
-        float acc = 0.f;
-#pragma unroll
-        for (int j = 0; j < C; ++j) acc += sm.sg[b][j], gc[j] = acc;
+        const int tt = tid >> 4, e = (tid & 15) * 4;
+        if (i0 + tt < T) cp_async16(&w.sv[tt][e], vc + ((size_t)(t0 + i0 + tt) * nv + h) * D + c0 + e);
+        else *reinterpret_cast<float4*>(&w.sv[tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-      const uint32_t a_base = warp == 0 ? a_kraw : a_qraw;
-#pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) {
-        uint32_t af[4], bfr[4];
-        gc_ldsm(af, a_base + gc_off(lrow, kk * 2 + (lane >> 4)));
-        gc_ldsm(bfr, a_kraw + gc_off((lane & 7) + (lane >> 4) * 8, kk * 2 + ((lane >> 3) & 1)));
-        gc_mma(acc[0], af, bfr[0], bfr[1]);
-        gc_mma(acc[1], af, bfr[2], bfr[3]);
-      }
-#pragma unroll
-      for (int n8 = 0; n8 < 2; ++n8)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = g8 + (e >> 1) * 8, j = n8 * 8 + t4 * 2 + (e & 1);
-          float gi_ = 0.f, gj_ = 0.f;
-#pragma unroll
-          for (int q = 0; q < C; ++q) gi_ = q == i ? gc[q] : gi_, gj_ = q == j ? gc[q] : gj_;
-          const float dec = j <= i ? __expf(gi_ - gj_) : 0.f;
-          if (warp == 0) sm.a[i][j] = j < i ? sm.sb[b][i] * acc[n8][e] * dec : 0.f;
-          else *reinterpret_cast<bf16*>(sm.qkm + i * 32 + j * 2) = __float2bfloat16(acc[n8][e] * dec);
-        }
-      if (warp == 0) {
-        __syncwarp();
-        if (lane < C) {                    // lane j solves column j of T by forward substitution
-          float tcol[C];
-#pragma unroll
-          for (int i = 0; i < C; ++i) {
-            float v = i == lane ? 1.f : 0.f;
-#pragma unroll
-            for (int m = 0; m < i; ++m) v -= sm.a[i][m] * tcol[m];
-            tcol[i] = i < lane ? 0.f : v;
-          }
-#pragma unroll
-          for (int i = 0; i < C; ++i) {
-            const bf16 hi = __float2bfloat16(tcol[i]);
-            *reinterpret_cast<bf16*>(sm.t_hi + i * 32 + lane * 2) = hi;
-            *reinterpret_cast<bf16*>(sm.t_lo + i * 32 + lane * 2) = __float2bfloat16(tcol[i] - __bfloat162float(hi));
-          }
+      if (tid < C) {                       // gates: asynchronous too, nothing of the next chunk is waited for here
+        if (i0 + tid < T) {
+          gc_cp4(&w.sg[b][tid], gin + (size_t)(t0 + i0 + tid) * nv + h);
+          gc_cp4(&w.sb[b][tid], bin + (size_t)(t0 + i0 + tid) * nv + h);
+        } else {
+          w.sg[b][tid] = 0.f, w.sb[b][tid] = 0.f;                           // padding rows: no decay, no update
         }
       }
-    } else {
-      qs_product();
-    }
-    __syncthreads();
-    // ---- W = T (K beta e^G) over all of dk (16 columns per warp); U = T (V beta), this warp's 8 value columns
-    if (warp < 2) qs_product();
-    float U[4] = {0.f, 0.f, 0.f, 0.f};
-    {
-      float Wf[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-      uint32_t thi[4], tlo[4], bk[4], bv[2];
-      const uint32_t trow = (uint32_t)(lrow * 32 + (lane >> 4) * 16);
-      gc_ldsm(thi, a_thi + trow);
-      gc_ldsm(tlo, a_tlo + trow);
-      gc_ldsm_t(bk, a_kb + gc_off(lrow, 2 * warp + (lane >> 4)));
-      gc_ldsm2_t(bv, a_vb + gc_offv(lrow, warp));
-      gc_mma(Wf[0], thi, bk[0], bk[1]), gc_mma(Wf[1], thi, bk[2], bk[3]);
-      gc_mma(Wf[0], tlo, bk[0], bk[1]), gc_mma(Wf[1], tlo, bk[2], bk[3]);
-      gc_mma(U, thi, bv[0], bv[1]);
-      gc_mma(U, tlo, bv[0], bv[1]);
+      cp_async_commit();
+    };
+    if (first < chunks) stage(first * C, 0);
+    int b = 0;
+    for (int c = first; c < chunks; c += 2, b ^= 1) {
+      GcSlot& o = sm.slot[c % GC_SLOTS];
+      const bool ok = c < GC_SLOTS || mbar_wait(u32(&sm.empty[c % GC_SLOTS]), (uint32_t)(c / GC_SLOTS - 1) & 1u, abort_flag);
+      cp_async_wait<0>();
+      if (!meet(ok)) break;                // the chunk landed; this group's tiles and the slot are free
+      // running sums of the log-decays, recomputed where they are needed (16 broadcast reads)
+      float g_last = 0.f;
 #pragma unroll
-      for (int n8 = 0; n8 < 2; ++n8) {
-        *reinterpret_cast<uint32_t*>(sm.ws + gc_off(g8, 2 * warp + n8) + t4 * 4) = f2_to_bf162_bits(Wf[n8][0], Wf[n8][1]);
-        *reinterpret_cast<uint32_t*>(sm.ws + gc_off(g8 + 8, 2 * warp + n8) + t4 * 4) = f2_to_bf162_bits(Wf[n8][2], Wf[n8][3]);
+      for (int j = 0; j < C; ++j) g_last += w.sg[b][j];
+      if (tid == 0) o.g_last = g_last;
+      // ---- operand tiles (bf16) from the staged fp32 rows: thread = (token, 8 columns)
+      {
+        const int tt = tid >> 4, ch = tid & 15, e = ch * 8;
+        float gi = 0.f;
+        for (int j = 0; j <= tt; ++j) gi += w.sg[b][j];
+        const float eg = __expf(gi), beta = w.sb[b][tt], kbs = beta * eg;
+        const float4 q0 = *reinterpret_cast<const float4*>(&w.sq[tt][e]), q1 = *reinterpret_cast<const float4*>(&w.sq[tt][e + 4]);
+        const float4 k0 = *reinterpret_cast<const float4*>(&w.sk[tt][e]), k1 = *reinterpret_cast<const float4*>(&w.sk[tt][e + 4]);
+        const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+        const float kv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+        uint32_t oq[4], ok_[4], oqe[4], okb[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          oq[j] = f2_to_bf162_bits(qv[2 * j], qv[2 * j + 1]);
+          ok_[j] = f2_to_bf162_bits(kv[2 * j], kv[2 * j + 1]);
+          oqe[j] = f2_to_bf162_bits(qv[2 * j] * eg, qv[2 * j + 1] * eg);
+          okb[j] = f2_to_bf162_bits(kv[2 * j] * kbs, kv[2 * j + 1] * kbs);
+        }
+        const uint32_t off = gc_off(tt, ch);
+        *reinterpret_cast<uint4*>(w.qraw + off) = make_uint4(oq[0], oq[1], oq[2], oq[3]);
+        *reinterpret_cast<uint4*>(w.kraw + off) = make_uint4(ok_[0], ok_[1], ok_[2], ok_[3]);
+        *reinterpret_cast<uint4*>(o.qe + off) = make_uint4(oqe[0], oqe[1], oqe[2], oqe[3]);
+        *reinterpret_cast<uint4*>(w.kb + off) = make_uint4(okb[0], okb[1], okb[2], okb[3]);
+        if (ch < DV / 8) {
+          const float4 v0 = *reinterpret_cast<const float4*>(&w.sv[tt][e]), v1 = *reinterpret_cast<const float4*>(&w.sv[tt][e + 4]);
+          *reinterpret_cast<uint4*>(w.vb + gc_offv(tt, ch)) =
+              make_uint4(f2_to_bf162_bits(v0.x * beta, v0.y * beta), f2_to_bf162_bits(v0.z * beta, v0.w * beta),
+                         f2_to_bf162_bits(v1.x * beta, v1.y * beta), f2_to_bf162_bits(v1.z * beta, v1.w * beta));
+        }
       }
-    }
-    __syncthreads();
-    // ---- V' = U - W S (this warp's 8 columns), kept as the bf16 B operand of the next two products
-    {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      {
+        // transposed decayed keys [dk][token]: thread = (dk row, 8 tokens), one 16-byte store
+        const int r = tid & 127, half = tid >> 7;
+        float gi = 0.f;
+        for (int j = 0; j < half * 8; ++j) gi += w.sg[b][j];
+        uint32_t ov[4];
 #pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) {
-        uint32_t af[4], bs[2];
-        gc_ldsm(af, a_ws + gc_off(lrow, kk * 2 + (lane >> 4)));
-        gc_ldsm2_t(bs, a_sbf + gc_offv(kk * 16 + lrow, warp));
-        gc_mma(acc, af, bs[0], bs[1]);
+        for (int j = 0; j < 4; ++j) {
+          gi += w.sg[b][half * 8 + 2 * j];
+          const float x0 = w.sk[half * 8 + 2 * j][r] * __expf(g_last - gi);
+          gi += w.sg[b][half * 8 + 2 * j + 1];
+          const float x1 = w.sk[half * 8 + 2 * j + 1][r] * __expf(g_last - gi);
+          ov[j] = f2_to_bf162_bits(x0, x1);
+        }
+        *reinterpret_cast<uint4*>(o.kdt + (size_t)r * 32 + half * 16) = make_uint4(ov[0], ov[1], ov[2], ov[3]);
       }
-      *reinterpret_cast<uint32_t*>(sm.vn + gc_offv(g8, warp) + t4 * 4) = f2_to_bf162_bits(U[0] - acc[0], U[1] - acc[1]);
-      *reinterpret_cast<uint32_t*>(sm.vn + gc_offv(g8 + 8, warp) + t4 * 4) = f2_to_bf162_bits(U[2] - acc[2], U[3] - acc[3]);
-    }
-    __syncthreads();
-    // ---- O += QK' V' (this warp's 8 columns) -> raw rows; state rows of this warp: S <- e^{G_last} S + Kd^T V'
-    {
-      uint32_t aq[4], bvn[2];
-      gc_ldsm(aq, a_qkm + (uint32_t)(lrow * 32 + (lane >> 4) * 16));
-      gc_ldsm2_t(bvn, a_vn + gc_offv(lrow, warp));
-      gc_mma(O, aq, bvn[0], bvn[1]);
-      float* orow = o_scratch + ((size_t)(t0 + i0) * nv + h) * D + c0 + 8 * warp + t4 * 2;
-      if (i0 + g8 < T) *reinterpret_cast<float2*>(orow + (size_t)g8 * nv * D) = make_float2(O[0], O[1]);
-      if (i0 + g8 + 8 < T) *reinterpret_cast<float2*>(orow + (size_t)(g8 + 8) * nv * D) = make_float2(O[2], O[3]);
-      const float el = __expf(g_last);
-      uint32_t ak[4];
-      gc_ldsm(ak, a_kdt + (uint32_t)((16 * warp + lrow) * 32 + (lane >> 4) * 16));
+      meet(true);
+      if (c + 2 < chunks) stage((c + 2) * C, b ^ 1);       // the fp32 rows have been read
+      // ---- warp 0: KK -> A -> T = (I + A)^-1;  warp 1: QK'
+      if (warp < 2) {
+        float gc[C];                         // inclusive running sums
+        {
+          float acc = 0.f;
 #pragma unroll
-      for (int nt = 0; nt < DV / 8; nt += 2) {
-        uint32_t bvv[4];
-        gc_ldsm_t(bvv, a_vn + gc_offv(lrow, nt + (lane >> 4)));
+          for (int j = 0; j < C; ++j) acc += w.sg[b][j], gc[j] = acc;
+        }
+        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        const uint32_t a_base = warp == 0 ? a_kraw : a_qraw;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[nt][e] *= el, S[nt + 1][e] *= el;
-        gc_mma(S[nt], ak, bvv[0], bvv[1]);
-        gc_mma(S[nt + 1], ak, bvv[2], bvv[3]);
+        for (int kk = 0; kk < D / 16; ++kk) {
+          uint32_t af[4], bfr[4];
+          gc_ldsm(af, a_base + gc_off(lrow, kk * 2 + (lane >> 4)));
+          gc_ldsm(bfr, a_kraw + gc_off((lane & 7) + (lane >> 4) * 8, kk * 2 + ((lane >> 3) & 1)));
+          gc_mma(acc[0], af, bfr[0], bfr[1]);
+          gc_mma(acc[1], af, bfr[2], bfr[3]);
+        }
+#pragma unroll
+        for (int n8 = 0; n8 < 2; ++n8)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = g8 + (e >> 1) * 8, j = n8 * 8 + t4 * 2 + (e & 1);
+            float gi_ = 0.f, gj_ = 0.f;
+#pragma unroll
+            for (int q = 0; q < C; ++q) gi_ = q == i ? gc[q] : gi_, gj_ = q == j ? gc[q] : gj_;
+            const float dec = j <= i ? __expf(gi_ - gj_) : 0.f;
+            if (warp == 0) w.a[i][j] = j < i ? w.sb[b][i] * acc[n8][e] * dec : 0.f;
+            else *reinterpret_cast<bf16*>(o.qkm + i * 32 + j * 2) = __float2bfloat16(acc[n8][e] * dec);
+          }
+        if (warp == 0) {
+          __syncwarp();
+          if (lane < C) {                    // lane j solves column j of T by forward substitution
+            float tcol[C];
+#pragma unroll
+            for (int i = 0; i < C; ++i) {
+              float v = i == lane ? 1.f : 0.f;
+#pragma unroll
+              for (int m = 0; m < i; ++m) v -= w.a[i][m] * tcol[m];
+              tcol[i] = i < lane ? 0.f : v;
+            }
+#pragma unroll
+            for (int i = 0; i < C; ++i) {
+              const bf16 hi = __float2bfloat16(tcol[i]);
+              *reinterpret_cast<bf16*>(w.t_hi + i * 32 + lane * 2) = hi;
+              *reinterpret_cast<bf16*>(w.t_lo + i * 32 + lane * 2) = __float2bfloat16(tcol[i] - __bfloat162float(hi));
+            }
+          }
+        }
       }
-    }
-    __syncthreads();                       // every warp has read the old state copy
-    store_sbf();
-  }
-  // ---- state back to its plane; conv ring refresh for the last tokens (as the token-serial scan does)
+      meet(true);
+      // ---- W = T (K beta e^G) over all of dk (16 columns per warp); U = T (V beta), this warp's 8 value columns
+      {
+        float U[4] = {0.f, 0.f, 0.f, 0.f};
+        float Wf[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        uint32_t thi[4], tlo[4], bk[4], bv[2];
+        const uint32_t trow = (uint32_t)(lrow * 32 + (lane >> 4) * 16);
+        gc_ldsm(thi, a_thi + trow);
+        gc_ldsm(tlo, a_tlo + trow);
+        gc_ldsm_t(bk, a_kb + gc_off(lrow, 2 * warp + (lane >> 4)));
+        gc_ldsm2_t(bv, a_vb + gc_offv(lrow, warp));
+        gc_mma(Wf[0], thi, bk[0], bk[1]), gc_mma(Wf[1], thi, bk[2], bk[3]);
+        gc_mma(Wf[0], tlo, bk[0], bk[1]), gc_mma(Wf[1], tlo, bk[2], bk[3]);
+        gc_mma(U, thi, bv[0], bv[1]);
+        gc_mma(U, tlo, bv[0], bv[1]);
 #pragma unroll
-  for (int nt = 0; nt < DV / 8; ++nt) {
-    *reinterpret_cast<float2*>(sp + (size_t)(16 * warp + g8) * D + nt * 8 + t4 * 2) = make_float2(S[nt][0], S[nt][1]);
-    *reinterpret_cast<float2*>(sp + (size_t)(16 * warp + g8 + 8) * D + nt * 8 + t4 * 2) = make_float2(S[nt][2], S[nt][3]);
-  }
-  if (c0 == 0) {
-    const int cw = 2 * nk * D + nv * D;
-    bf16* rg = ring + (size_t)slot * ring_slot_stride;
-    const int first = max(0, T - RING);
-    const int rep = nv / nk;
-    for (int i = first; i < T; ++i) {
-      const int t = t0 + i;
-      const int rrow = positions[t] % RING;
-      const bf16* src = inp + (size_t)t * ld;
-      bf16* dst = rg + (size_t)rrow * cw;
-      if (h % rep == 0) {
-        for (int c = tid; c < 2 * D; c += 256) {
-          const int cc = (c < D) ? kh * D + c : nk * D + kh * D + (c - D);
+        for (int n8 = 0; n8 < 2; ++n8) {
+          *reinterpret_cast<uint32_t*>(o.ws + gc_off(g8, 2 * warp + n8) + t4 * 4) = f2_to_bf162_bits(Wf[n8][0], Wf[n8][1]);
+          *reinterpret_cast<uint32_t*>(o.ws + gc_off(g8 + 8, 2 * warp + n8) + t4 * 4) = f2_to_bf162_bits(Wf[n8][2], Wf[n8][3]);
+        }
+        o.u[tid] = make_float4(U[0], U[1], U[2], U[3]);
+      }
+      mbar_arrive(u32(&sm.full[c % GC_SLOTS]));
+    }
+    // ---- conv ring refresh for the last tokens (as the token-serial scan does)
+    if (group == 2 && c0 == 0) {
+      const int cw = 2 * nk * D + nv * D;
+      bf16* rg = ring + (size_t)slot * ring_slot_stride;
+      const int rep = nv / nk;
+      for (int i = max(0, T - RING); i < T; ++i) {
+        const int t = t0 + i;
+        const bf16* src = inp + (size_t)t * ld;
+        bf16* dst = rg + (size_t)(positions[t] % RING) * cw;
+        if (h % rep == 0) {
+          for (int c = tid; c < 2 * D; c += GC_GROUP) {
+            const int cc = (c < D) ? kh * D + c : nk * D + kh * D + (c - D);
+            dst[cc] = src[cc];
+          }
+        }
+        for (int c = tid; c < D; c += GC_GROUP) {
+          const int cc = 2 * nk * D + h * D + c;
           dst[cc] = src[cc];
         }
       }
-      for (int c = tid; c < D; c += 256) {
-        const int cc = 2 * nk * D + h * D + c;
-        dst[cc] = src[cc];
+    }
+  } else {
+    // ---------------- the state: rows 16 warp .. 16 warp + 15, this CTA's 64 columns, as accumulator fragments ----------------
+    float* sp = states + (size_t)slot * state_slot_stride + (size_t)h * D * D + (size_t)cur[slot] * plane_stride + c0;
+    const uint32_t a_vn = u32(sm.vn), a_sbf = u32(sm.sbf);
+    float S[DV / 8][4];
+#pragma unroll
+    for (int nt = 0; nt < DV / 8; ++nt) {
+      const float2 lo = *reinterpret_cast<const float2*>(sp + (size_t)(16 * warp + g8) * D + nt * 8 + t4 * 2);
+      const float2 hi = *reinterpret_cast<const float2*>(sp + (size_t)(16 * warp + g8 + 8) * D + nt * 8 + t4 * 2);
+      S[nt][0] = lo.x, S[nt][1] = lo.y, S[nt][2] = hi.x, S[nt][3] = hi.y;
+    }
+    auto store_sbf = [&]() {
+#pragma unroll
+      for (int nt = 0; nt < DV / 8; ++nt) {
+        *reinterpret_cast<uint32_t*>(sm.sbf + gc_offv(16 * warp + g8, nt) + t4 * 4) = f2_to_bf162_bits(S[nt][0], S[nt][1]);
+        *reinterpret_cast<uint32_t*>(sm.sbf + gc_offv(16 * warp + g8 + 8, nt) + t4 * 4) = f2_to_bf162_bits(S[nt][2], S[nt][3]);
+      }
+    };
+    store_sbf();
+    bool good = true;
+    for (int c = 0; c < chunks; ++c) {
+      const GcSlot& o = sm.slot[c % GC_SLOTS];
+      const uint32_t a_qe = u32(o.qe), a_ws = u32(o.ws), a_kdt = u32(o.kdt), a_qkm = u32(o.qkm);
+      good = meet(mbar_wait(u32(&sm.full[c % GC_SLOTS]), (uint32_t)(c / GC_SLOTS) & 1u, abort_flag));   // and: the state's copy is whole
+      if (!good) break;
+      // ---- O = (Q e^G) S and V' = U - W S, this warp's 8 value columns of both
+      float O[4] = {0.f, 0.f, 0.f, 0.f}, acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) {
+        uint32_t aw[4], aq[4], bs[2];
+        gc_ldsm(aw, a_ws + gc_off(lrow, kk * 2 + (lane >> 4)));
+        gc_ldsm(aq, a_qe + gc_off(lrow, kk * 2 + (lane >> 4)));
+        gc_ldsm2_t(bs, a_sbf + gc_offv(kk * 16 + lrow, warp));
+        gc_mma(acc, aw, bs[0], bs[1]);
+        gc_mma(O, aq, bs[0], bs[1]);
+      }
+      const float4 U = o.u[tid];
+      *reinterpret_cast<uint32_t*>(sm.vn + gc_offv(g8, warp) + t4 * 4) = f2_to_bf162_bits(U.x - acc[0], U.y - acc[1]);
+      *reinterpret_cast<uint32_t*>(sm.vn + gc_offv(g8 + 8, warp) + t4 * 4) = f2_to_bf162_bits(U.z - acc[2], U.w - acc[3]);
+      meet(true);                            // V' is whole, every warp has read the old state copy
+      // ---- O += QK' V' (this warp's 8 columns) -> raw rows; state rows of this warp: S <- e^{G_last} S + Kd^T V'
+      {
+        uint32_t aq[4], bvn[2];
+        gc_ldsm(aq, a_qkm + (uint32_t)(lrow * 32 + (lane >> 4) * 16));
+        gc_ldsm2_t(bvn, a_vn + gc_offv(lrow, warp));
+        const float el = __expf(o.g_last);
+        uint32_t ak[4];
+        gc_ldsm(ak, a_kdt + (uint32_t)((16 * warp + lrow) * 32 + (lane >> 4) * 16));
+#pragma unroll
+        for (int nt = 0; nt < DV / 8; nt += 2) {
+          uint32_t bvv[4];
+          gc_ldsm_t(bvv, a_vn + gc_offv(lrow, nt + (lane >> 4)));
+#pragma unroll
+          for (int e = 0; e < 4; ++e) S[nt][e] *= el, S[nt + 1][e] *= el;
+          gc_mma(S[nt], ak, bvv[0], bvv[1]);
+          gc_mma(S[nt + 1], ak, bvv[2], bvv[3]);
+        }
+        store_sbf();
+        gc_mma(O, aq, bvn[0], bvn[1]);
+        mbar_arrive(u32(&sm.empty[c % GC_SLOTS]));
+        const int i0 = c * C;
+        float* orow = o_scratch + ((size_t)(t0 + i0) * nv + h) * D + c0 + 8 * warp + t4 * 2;
+        if (i0 + g8 < T) *reinterpret_cast<float2*>(orow + (size_t)g8 * nv * D) = make_float2(O[0], O[1]);
+        if (i0 + g8 + 8 < T) *reinterpret_cast<float2*>(orow + (size_t)(g8 + 8) * nv * D) = make_float2(O[2], O[3]);
+      }
+    }
+    // ---- state back to its plane
+    if (good) {
+#pragma unroll
+      for (int nt = 0; nt < DV / 8; ++nt) {
+        *reinterpret_cast<float2*>(sp + (size_t)(16 * warp + g8) * D + nt * 8 + t4 * 2) = make_float2(S[nt][0], S[nt][1]);
+        *reinterpret_cast<float2*>(sp + (size_t)(16 * warp + g8 + 8) * D + nt * 8 + t4 * 2) = make_float2(S[nt][2], S[nt][3]);
       }
     }
   }
@@ -1122,7 +1162,9 @@ gdn_gated_norm_kernel(const float* o_scratch, const bf16* inp, int ld, const flo
   if (row >= rows) return;
   const int t = row / nv, h = row % nv;
   const float4 ov = __ldcg(reinterpret_cast<const float4*>(o_scratch + (size_t)row * D) + lane);
-  const uint2 zr = *reinterpret_cast<const uint2*>(inp + (size_t)t * ld + (2 * nk * D + nv * D) + (size_t)h * D + lane * 4);
+  // in 4-byte pieces: with an odd count of value heads a row of the projection starts on no wider boundary
+  const uint32_t* zp = reinterpret_cast<const uint32_t*>(inp + (size_t)t * ld + (2 * nk * D + nv * D) + (size_t)h * D + lane * 4);
+  const uint2 zr = make_uint2(zp[0], zp[1]);
   const float4 w = *reinterpret_cast<const float4*>(norm_w + lane * 4);
   const float ss = warp_sum(ov.x * ov.x + ov.y * ov.y + ov.z * ov.z + ov.w * ov.w);
   const float rstd = rsqrtf(ss / (float)D + eps);
@@ -1255,17 +1297,12 @@ gdn_decode_kernel(const bf16* inp, int ld, const float* __restrict__ conv_w,
   trl_trace_end();
 }
 
-// Turns the chunk-parallel prefill scan on or off at run time (tests compare the two paths).
-TRL_API void trl_gdn_set_wy(int on) { g_gdn_wy = on ? 1 : 0; }
-// Prefill scan on the tensor cores (gdn_chunk_mma_kernel): 1 on, 0 off (token-serial scan), -1 = the environment's choice.
-TRL_API void trl_gdn_set_mma(int on) { g_gdn_mma = on; }
-
 // The same step for many (sequence, value head) items, D = 128: one block an SM goes through its items with the 64 KB of
 // state in shared memory, three stages of bulk copies in and out, so that the copy engine always has the next states under way;
 // with a block per item the chain of a token (indices, convolution, two norms, the step) stood between a block's load and its
 // store, two blocks an SM.  Warps 0-7 compute (thread = column x half of the rows), 8-11 prepare the next item's token, 12 moves
-// states.  Bound by the state's bytes: 32 sequences x 48 heads, 201 MB: GDEC_BEFORE us before, GDEC_AFTER here; 8 sequences:
-// GDEC8_BEFORE, GDEC8_AFTER.
+// states.  Bound by the state's bytes: 32 sequences x 48 heads, 201 MB: 82 us before, 38 here; 8 sequences:
+// 20 before, 14 here.
 struct GdSmem {
   static constexpr int D = 128, STAGES = 3;
   __align__(128) float st[STAGES][D][D];
@@ -1485,6 +1522,11 @@ gdn_decode_stream_kernel(const bf16* inp, int ld, const float* __restrict__ conv
   }
 }
 
+// Turns the chunk-parallel prefill scan on or off at run time (tests compare the two paths).
+TRL_API void trl_gdn_set_wy(int on) { g_gdn_wy = on ? 1 : 0; }
+// Prefill scan on the tensor cores (gdn_chunk_mma_kernel): 1 on, 0 off (token-serial scan), -1 = the environment's choice.
+TRL_API void trl_gdn_set_mma(int on) { g_gdn_mma = on; }
+
 // Scratch (fp32): qn, kn [T*nk*D]; vc, o_scratch [T*nv*D]; g, beta [T*nv].
 TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_bias, const void* a_log,
                     const void* norm_w, void* states, void* cur, void* ring, const void* positions,
@@ -1496,6 +1538,7 @@ TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_
   cudaStream_t st = (cudaStream_t)stream;
   if (KW > 4) return (int)cudaErrorInvalidValue;
   if ((D != 64 && D != 128) || (ld % 2) != 0) return (int)cudaErrorInvalidValue;
+  // runs as long as leaves about 16 CTAs of 128 threads for every SM
   const int prep_tpc = 1024 / D;
   int run = 8;
   while (run > 1 && (long)(T + prep_tpc * run - 1) / (prep_tpc * run) * (2 * nk + nv) < 16 * 148) run >>= 1;
@@ -1503,8 +1546,7 @@ TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_
                              (const bf16*)inp, ld, (const float*)conv_w, (const float*)dt_bias, (const float*)a_log,
                              (const bf16*)ring, (const int*)positions, (const int*)seq_ids,
                              (const int*)q_start, (const int*)state_slots, ring_slot_stride,
-  // runs as long as leaves about 16 CTAs of 128 threads for every SM
-                             (float*)qn, (float*)kn, (float*)vc, (float*)g, (float*)beta, nk, nv, D, KW, T);
+                             (float*)qn, (float*)kn, (float*)vc, (float*)g, (float*)beta, nk, nv, D, KW, T, run);
   if (e != cudaSuccess) return (int)e;
 #define RECUR(DD)                                                                                   \
   e = trl_launch(gdn_recur_kernel<DD>, dim3(nv, B), dim3(DD * 4), 0, st, (const float*)qn,          \
@@ -1546,7 +1588,7 @@ TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_
         return 3;
       configured = true;
     }
-    e = trl_launch(gdn_chunk_mma_kernel, dim3(nv * GC_NS, B), dim3(256), sizeof(GcSmem), st, (const float*)qn,
+    e = trl_launch(gdn_chunk_mma_kernel, dim3(nv * GC_NS, B), dim3(GC_THREADS), sizeof(GcSmem), st, (const float*)qn,
                    (const float*)kn, (const float*)vc, (const float*)g, (const float*)beta, (float*)states, (int*)cur,
                    (bf16*)ring, (const bf16*)inp, ld, (const int*)q_start, (const int*)q_len, (const int*)positions,
                    (const int*)state_slots, state_slot_stride, plane_stride, ring_slot_stride, (float*)o_scratch, nk, nv);
@@ -1587,6 +1629,21 @@ TRL_API int trl_gdn_decode(const void* inp, int ld, const void* conv_w, const vo
                          (const float*)norm_w, (float*)states, (const int*)cur, (bf16*)ring,                \
                          (const int*)positions, (const int*)q_start, (const int*)state_slots,               \
                          state_slot_stride, plane_stride, ring_slot_stride, eps, (bf16*)out, nk, nv, KW)
+  // from as many heads as fill the SMs one and a half times over (below, a block an item finds an SM of its own at once)
+  if (D == 128 && KW <= 4 && nv * B >= 222) {
+    static bool configured = false;
+    if (!configured) {
+      if (cudaFuncSetAttribute(gdn_decode_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GdSmem)) != cudaSuccess) return 3;
+      configured = true;
+    }
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return (int)trl_launch(gdn_decode_stream_kernel, dim3(min(sms, nv * B)), dim3(13 * 32), sizeof(GdSmem), st, (const bf16*)inp, ld,
+                           (const float*)conv_w, (const float*)dt_bias, (const float*)a_log, (const float*)norm_w, (float*)states,
+                           (const int*)cur, (bf16*)ring, (const int*)positions, (const int*)q_start, (const int*)state_slots,
+                           state_slot_stride, plane_stride, ring_slot_stride, eps, (bf16*)out, B, nk, nv, KW);
+  }
   if (D == 128) DECODE(128);
   DECODE(64);
 #undef DECODE

@@ -213,3 +213,37 @@ def test_delta_rule_prep_over_runs_of_tokens(ops, nk, nv, d, taps):
         assert _rel(vc, want[:, 2 * nk * d:].view(t, nv, d)) < 1e-5
         assert _rel(bb, torch.sigmoid(x[:, c + nv * d + nv:])) < 1e-5
         assert _rel(gg, -torch.exp(al.double()) * torch.nn.functional.softplus(x[:, c + nv * d:c + nv * d + nv] + dt.double())) < 1e-5
+
+
+@pytest.mark.parametrize("nk,nv,b,taps", [(16, 48, 5, 4), (16, 48, 32, 4), (1, 3, 75, 4), (2, 6, 37, 3), (8, 8, 149, 4)])
+def test_decode_step_of_many_heads_equals_one_sequence_at_a_time(ops, nk, nv, b, taps):
+    """Items that the blocks share evenly and unevenly, as few as the kernel of many items takes, positions before the
+    convolution's window is full and past the ring's end, live planes other than the first.  The same arithmetic as the
+    kernel of one item a block (which a single sequence takes), except for the order of the sum q.k."""
+    from tilerl_b200.ops import native as N
+    d, planes = 128, 2
+    g = torch.Generator().manual_seed(b + nv)
+    c = (2 * nk + nv) * d
+    ld = c + nv * d + 2 * nv
+    inp = torch.randn(b, ld, generator=g).to(DEV, torch.bfloat16)
+    conv = (torch.randn(c, taps, generator=g) * 0.3).to(DEV)
+    dt, al, nw = torch.randn(nv, generator=g).to(DEV), torch.randn(nv, generator=g).to(DEV), torch.rand(d, generator=g).to(DEV)
+    ring = torch.randn(b + 1, 16, c, generator=g).to(DEV, torch.bfloat16)
+    states = torch.randn(b + 1, 1, planes, nv, d, d, device=DEV) * 0.05
+    cur = torch.randint(0, planes, (b + 1,), generator=g).to(DEV, torch.int32)
+    pos = torch.tensor([(0, 1, 2, 3, 15, 16, 17, 40)[i % 8] for i in range(b)], dtype=torch.int32, device=DEV)
+    qs = torch.arange(b, dtype=torch.int32, device=DEV)
+    slots = (torch.randperm(b, generator=g) + 1).to(DEV, torch.int32)
+
+    def step(s, r, o, rows):
+        for i, n in rows:
+            N.check(ops.lib.trl_gdn_decode(inp.data_ptr(), ld, conv.data_ptr(), dt.data_ptr(), al.data_ptr(), nw.data_ptr(), s.data_ptr(),
+                                           cur.data_ptr(), r.data_ptr(), pos.data_ptr(), qs[i:].data_ptr(), slots[i:].data_ptr(), s.stride(0),
+                                           s.stride(2), r.stride(0), o.data_ptr(), n, nk, nv, d, taps, 1e-6, N.stream()), "gdn_decode")
+    s1, r1, o1 = states.clone(), ring.clone(), torch.zeros(b, nv * d, dtype=torch.bfloat16, device=DEV)
+    s2, r2, o2 = states.clone(), ring.clone(), torch.zeros(b, nv * d, dtype=torch.bfloat16, device=DEV)
+    step(s1, r1, o1, [(0, b)])
+    step(s2, r2, o2, [(i, 1) for i in range(b)])
+    assert torch.equal(s1, s2) and torch.equal(r1, r2)
+    assert _rel(o1, o2) < 2e-4                        # a bf16 step where the sum's last bit tips a rounding over
+    assert not torch.equal(s1, states) and N.read_error()[0] == 0
