@@ -276,12 +276,16 @@ attn_combine_kernel(const float* po, const float* pm,
 
 // ---------------------------------------------------------------------------------------
 // Tiled prefill attention (legacy tensor-core path: mma.sync m16n8k16 bf16, fp32 accumulate).
-// One CTA = (16-token tile of one sequence, kv head); warp g of the CTA owns query head
-// kvh * G + g, so the G heads of a group share every K / V tile.  K and V tiles of 32 keys
-// (two 16-token pages) are gathered through the block table with cp.async into 128-bit-chunk
-// XOR-swizzled shared memory, double buffered; QK^T and PV run on mma.sync with the usual
-// register reuse of the score fragment as the A operand of PV; online softmax in the exp2
-// domain; causal by absolute position; sigmoid output gate fused.  D = 256.
+// One CTA = (16-token tile of one sequence, kv head); a pair of warps owns query head
+// kvh * G + pair, so the G heads of a group share every K / V tile of 64 keys (four pages, double
+// buffered).  The pair splits the tile's scores by keys (32 each) and the output by columns (128
+// each): the row maxima and the probabilities (as A fragments) cross through shared memory between
+// two barriers of the pair.  With a warp to a head, the output alone is 128 registers a thread, six
+// warps at 255 registers fill an SM, and the kernel waits on its own MMA and shared-memory latencies
+// (issue slots 23 % busy); a pair has 64 of them a thread, and twelve warps fit.  Online softmax in
+// the exp2 domain; causal by absolute position; sigmoid output gate fused.  D = 256.  The longest
+// tiles (most keys) come first in the grid, so that the last wave is made of short ones.
+// 2000 tokens x 24 heads: 491 us with a warp to a head and the short tiles first; 279 here.
 // The split-KV kernel above re-reads K / V for every query token; this one reads them once per
 // 16 tokens, which is what makes long prompts tractable.
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
@@ -301,11 +305,12 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-constexpr int PF_D = 256, PF_TQ = 16, PF_BC = 32, PF_ROW = PF_D * 2 /*bytes*/, PF_CHUNKS = PF_ROW / 16;
+constexpr int PF_D = 256, PF_TQ = 16, PF_BC = 64, PF_ROW = PF_D * 2 /*bytes*/, PF_CHUNKS = PF_ROW / 16;
+constexpr int PF_XCH = 32 * 32 + 2 * PF_TQ * 4;    // bytes one warp gives its partner: 8 registers of P a lane, row maxima, row sums
 
 // byte offset of 16-byte chunk `c` of row `r` in a swizzled [rows][512 B] tile
 __device__ __forceinline__ uint32_t pf_off(int r, int c) { return (uint32_t)(r * PF_ROW + ((c ^ (r & 7)) << 4)); }
-// bf16 pool: a K / V tile of 32 keys is two pages, each brought by one tiled copy as four slabs
+// bf16 pool: a K / V tile of 64 keys is four pages, each brought by one tiled copy as four slabs
 // [16 keys][128 B] under the tensor map's 128-byte swizzle (see attn_decode_mma_kernel below)
 __device__ __forceinline__ uint32_t pt_off(int r, int c) {
   return (uint32_t)((r >> 4) * (KVB * PF_ROW) + (c >> 3) * (KVB * 128) + (r & 15) * 128 + (((c & 7) ^ (r & 7)) << 4));
@@ -333,8 +338,9 @@ __device__ __forceinline__ void e4m3x16_to_bf16(const uint4& raw, float s, uint4
   o1 = make_uint4(r[4], r[5], r[6], r[7]);
 }
 
-template <bool FP8>
-__global__ void __launch_bounds__(256)
+// THREADS: 384 (up to six heads a group, 168 registers a thread) or 512
+template <bool FP8, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
                     const bf16* kcache, const bf16* vcache,
                     const float* kscale, const float* vscale,
@@ -350,20 +356,27 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
   unsigned char* pf_smem = pf_smem_raw + (((pf_raw_a + 1023u) & ~1023u) - pf_raw_a);    // swizzle atoms are 1024-byte aligned
   pdl_launch_dependents();
   pdl_wait();
-  const int tile = blockIdx.x, kvh = blockIdx.y, seq = blockIdx.z;
+  const int tile = (int)(gridDim.x - 1 - blockIdx.x), kvh = blockIdx.y, seq = blockIdx.z;
   const int G = n_q / n_kv;
   const int T = q_len[seq];
   if (tile * PF_TQ >= T) return;
   const int t0 = q_start[seq] + tile * PF_TQ;
   const int rows = min(PF_TQ, T - tile * PF_TQ);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int h = kvh * G + warp;
-  unsigned char* qs = pf_smem + (size_t)warp * PF_TQ * PF_ROW;                 // [G][16][512 B]
-  unsigned char* ks = pf_smem + (size_t)G * PF_TQ * PF_ROW;                    // [2][32][512 B] ([1] when FP8)
-  unsigned char* vs = ks + (FP8 ? 1 : 2) * PF_BC * PF_ROW;                     // [2][32][512 B] ([1] when FP8)
-  unsigned char* raw_k = vs + PF_BC * PF_ROW;                                  // FP8: [2][32][256 B] staged e4m3 rows
-  unsigned char* raw_v = raw_k + 2 * PF_BC * PF_D;                             // FP8: [2][32][256 B]
-  float* s_sc = reinterpret_cast<float*>(raw_v + 2 * PF_BC * PF_D);            // FP8: [2][K, V][32] row scales
+  const int pair = warp >> 1, half = warp & 1;     // half: which 32 keys of a tile, which 128 columns of the output
+  const int h = kvh * G + pair;
+  unsigned char* qs = pf_smem + (size_t)pair * PF_TQ * PF_ROW;                 // [G][16][512 B]
+  unsigned char* ks = pf_smem + (size_t)G * PF_TQ * PF_ROW;                    // [2][64][512 B] ([1] when FP8)
+  unsigned char* vs = ks + (FP8 ? 1 : 2) * PF_BC * PF_ROW;                     // [2][64][512 B] ([1] when FP8)
+  unsigned char* xch = vs + (FP8 ? 1 : 2) * PF_BC * PF_ROW;                    // [2 G][PF_XCH]
+  unsigned char* raw_k = xch + 2 * G * PF_XCH;                                 // FP8: [2][64][256 B] staged e4m3 rows
+  unsigned char* raw_v = raw_k + 2 * PF_BC * PF_D;                             // FP8: [2][64][256 B]
+  float* s_sc = reinterpret_cast<float*>(raw_v + 2 * PF_BC * PF_D);            // FP8: [2][K, V][64] row scales
+  uint4* x_mine = reinterpret_cast<uint4*>(xch + (size_t)warp * PF_XCH);       // P: [2][32 lanes] of 16 bytes; then max, sum [16]
+  const uint4* x_other = reinterpret_cast<const uint4*>(xch + (size_t)(warp ^ 1) * PF_XCH);
+  float* xm_mine = reinterpret_cast<float*>(x_mine + 64);
+  const float* xm_other = reinterpret_cast<const float*>(x_other + 64);
+  auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); };
   const uint32_t qs_a = (uint32_t)__cvta_generic_to_shared(qs);
   const uint32_t ks_a = (uint32_t)__cvta_generic_to_shared(ks), vs_a = (uint32_t)__cvta_generic_to_shared(vs);
   const int* table = block_table + (size_t)seq * max_blocks;
@@ -371,32 +384,14 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
   const int n_keys = positions[t0 + rows - 1] + 1;
   const int n_tiles = (n_keys + PF_BC - 1) / PF_BC;
 
-  // this warp's 16 query rows (zero rows past the end of the sequence)
-  for (int x = lane; x < PF_TQ * PF_CHUNKS; x += 32) {
+  // the pair's 16 query rows (zero rows past the end of the sequence)
+  for (int x = half * 32 + lane; x < PF_TQ * PF_CHUNKS; x += 64) {
     const int r = x / PF_CHUNKS, c = x % PF_CHUNKS;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (r < rows) v = *reinterpret_cast<const uint4*>(q + ((size_t)(t0 + r) * n_q + h) * PF_D + c * 8);
     *reinterpret_cast<uint4*>(qs + pf_off(r, c)) = v;
   }
-  auto load_kv = [&](int kt, int buf) {
-    const int j0 = kt * PF_BC;
-    for (int x = threadIdx.x; x < PF_BC * PF_CHUNKS; x += blockDim.x) {
-      const int r = x / PF_CHUNKS, c = x % PF_CHUNKS;
-      const int j = j0 + r;
-      const uint32_t dk = ks_a + buf * PF_BC * PF_ROW + pf_off(r, c);
-      const uint32_t dv = vs_a + buf * PF_BC * PF_ROW + pf_off(r, c);
-      if (j < n_keys) {
-        const size_t off = (((size_t)table[j / KVB] * n_kv + kvh) * KVB + (j % KVB)) * PF_D + c * 8;
-        cp16(dk, kcache + off);
-        cp16(dv, vcache + off);
-      } else {                      // rows past the bound: zeros (they are masked, but must not be NaN)
-        asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(dk), "r"(0u) : "memory");
-        asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(dv), "r"(0u) : "memory");
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // bf16 pool: thread 0 issues one tiled copy per K / V page of the tile (two pages), counted on full[buf]
+  // bf16 pool: thread 0 issues one tiled copy per K / V page of the tile (four pages), counted on full[buf]
   const uint32_t full_a = (uint32_t)__cvta_generic_to_shared(pf_full);
   auto load_kv_tma = [&](int kt, int buf) {
     const int j0 = kt * PF_BC;
@@ -463,14 +458,14 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
   const int r_lo = lane >> 2;                      // fragment rows r_lo and r_lo + 8
   const int pos_lo = r_lo < rows ? positions[t0 + r_lo] : -1;
   const int pos_hi = r_lo + 8 < rows ? positions[t0 + r_lo + 8] : -1;
-  float o[PF_D / 8][4];
+  float o[PF_D / 16][4];                           // 16 rows x this warp's 128 columns
 #pragma unroll
-  for (int i = 0; i < PF_D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  for (int i = 0; i < PF_D / 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;
 
   auto kv_off = [](int r, int c) { return FP8 ? pf_off(r, c) : pt_off(r, c); };
   if constexpr (!FP8) {
-    // barriers; the V buffers start as zeros (a tile whose second page lies past the bound is not copied
+    // barriers; the V buffers start as zeros (a tile whose last pages lie past the bound is not copied
     // there, and 0 x whatever shared memory held must be 0)
     if (threadIdx.x == 0) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full_a));
@@ -484,12 +479,10 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
     __syncthreads();
     if (threadIdx.x == 0) load_kv_tma(0, 0);
   } else {
-    (void)load_kv;
     stage_fp8(0, 0);
   }
   for (int kt = 0; kt < n_tiles; ++kt) {
     const int buf = FP8 ? 0 : (kt & 1);
-    bool have = true;
     if constexpr (FP8) {
       if (kt + 1 < n_tiles) {
         stage_fp8(kt + 1, (kt + 1) & 1);
@@ -508,8 +501,7 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
         for (uint32_t it = 1; !dm_try_wait(bar, parity); ++it) {
           if ((it & 63) == 0 && (!pf_ok || clock64() - t_begin > PF_WAIT_CYCLES)) {
             if (pf_ok) trl_set_error(TRL_ERR_MBAR_TIMEOUT, (int)blockIdx.x, 420 + buf, kt);
-            pf_ok = 0;
-            have = false;
+            pf_ok = 0;                               // the tile is still gone through: the pair meets twice in it
             break;
           }
         }
@@ -525,8 +517,7 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
         __syncthreads();
       }
     }
-    if (have) {
-    // ---- S = Q K^T for 32 keys: 4 n-tiles of 8 keys
+    // ---- S = Q K^T for this warp's 32 keys of the tile: 4 n-tiles of 8 keys
     float sc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
@@ -537,13 +528,13 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
 #pragma unroll
       for (int np = 0; np < 2; ++np) {             // two n-tiles per ldmatrix.x4
         uint32_t b[4];
-        ldsm_x4(b, kb + kv_off(np * 16 + (lane & 7) + (lane >> 4) * 8, kk * 2 + ((lane >> 3) & 1)));
+        ldsm_x4(b, kb + kv_off(half * 32 + np * 16 + (lane & 7) + (lane >> 4) * 8, kk * 2 + ((lane >> 3) & 1)));
         mma_bf16(sc[np * 2], a, b[0], b[1]);
         mma_bf16(sc[np * 2 + 1], a, b[2], b[3]);
       }
     }
     // ---- mask, scale, online softmax
-    const int j0 = kt * PF_BC;
+    const int j0 = kt * PF_BC + half * 32;
     float mx_lo = -INFINITY, mx_hi = -INFINITY;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
@@ -559,12 +550,14 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
     mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
     mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
     mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-    const float mn_lo = fmaxf(m_lo, mx_lo), mn_hi = fmaxf(m_hi, mx_hi);
+    if ((lane & 3) == 0) xm_mine[r_lo] = mx_lo, xm_mine[r_lo + 8] = mx_hi;
+    pair_sync();
+    const float mn_lo = fmaxf(m_lo, fmaxf(mx_lo, xm_other[r_lo])), mn_hi = fmaxf(m_hi, fmaxf(mx_hi, xm_other[r_lo + 8]));
     const float base_lo = mn_lo == -INFINITY ? 0.f : mn_lo, base_hi = mn_hi == -INFINITY ? 0.f : mn_hi;
     const float al_lo = exp2f(m_lo - base_lo), al_hi = exp2f(m_hi - base_hi);   // exp2(-inf) = 0 on the first tile
     m_lo = mn_lo, m_hi = mn_hi;
     float sum_lo = 0.f, sum_hi = 0.f;
-    uint32_t pa[2][4];                             // P as the A operand of PV: two k-steps of 16 keys
+    uint32_t pa[2][4];                             // P of these keys as the A operand of PV: two k-steps of 16 keys
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt) {
       const float p0 = exp2f(sc[nt][0] - base_lo), p1 = exp2f(sc[nt][1] - base_lo);
@@ -573,41 +566,53 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
       pa[nt >> 1][(nt & 1) * 2] = f2_to_bf162_bits(p0, p1);
       pa[nt >> 1][(nt & 1) * 2 + 1] = f2_to_bf162_bits(p2, p3);
     }
-    sum_lo += __shfl_xor_sync(0xffffffffu, sum_lo, 1);
-    sum_lo += __shfl_xor_sync(0xffffffffu, sum_lo, 2);
-    sum_hi += __shfl_xor_sync(0xffffffffu, sum_hi, 1);
-    sum_hi += __shfl_xor_sync(0xffffffffu, sum_hi, 2);
-    l_lo = l_lo * al_lo + sum_lo, l_hi = l_hi * al_hi + sum_hi;
+    x_mine[lane] = make_uint4(pa[0][0], pa[0][1], pa[0][2], pa[0][3]);
+    x_mine[32 + lane] = make_uint4(pa[1][0], pa[1][1], pa[1][2], pa[1][3]);
+    l_lo = l_lo * al_lo + sum_lo, l_hi = l_hi * al_hi + sum_hi;                 // of this lane's keys: summed after the last tile
 #pragma unroll
-    for (int i = 0; i < PF_D / 8; ++i) o[i][0] *= al_lo, o[i][1] *= al_lo, o[i][2] *= al_hi, o[i][3] *= al_hi;
-    // ---- O += P V
+    for (int i = 0; i < PF_D / 16; ++i) o[i][0] *= al_lo, o[i][1] *= al_lo, o[i][2] *= al_hi, o[i][3] *= al_hi;
+    // ---- O += P V: first this warp's keys, whose P it holds, then the partner's
+    auto pv = [&](const uint32_t (&a)[4], int row) {
+#pragma unroll
+      for (int nd = 0; nd < PF_D / 16; nd += 2) {
+        uint32_t b[4];
+        ldsm_x4_t(b, vb + kv_off(row + (lane & 7) + ((lane >> 3) & 1) * 8, half * (PF_D / 16) + nd + (lane >> 4)));
+        mma_bf16(o[nd], a, b[0], b[1]);
+        mma_bf16(o[nd + 1], a, b[2], b[3]);
+      }
+    };
+    pv(pa[0], half * 32), pv(pa[1], half * 32 + 16);
+    pair_sync();
 #pragma unroll
     for (int kk = 0; kk < 2; ++kk) {
-#pragma unroll
-      for (int nd = 0; nd < PF_D / 8; nd += 2) {
-        uint32_t b[4];
-        ldsm_x4_t(b, vb + kv_off(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, nd + (lane >> 4)));
-        mma_bf16(o[nd], pa[kk], b[0], b[1]);
-        mma_bf16(o[nd + 1], pa[kk], b[2], b[3]);
-      }
-    }
+      const uint4 w = x_other[kk * 32 + lane];
+      const uint32_t a[4] = {w.x, w.y, w.z, w.w};
+      pv(a, (half ^ 1) * 32 + kk * 16);
     }
     __syncthreads();                               // the other buffer may be overwritten next round
     if constexpr (!FP8) {
       if (!pf_ok) break;                           // a wait ran out (error word set): every thread leaves together
     }
   }
+  // row sums: over the four lanes of a row, then the partner's keys
+  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
+  l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
+  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
+  l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
+  if ((lane & 3) == 0) xm_mine[PF_TQ + r_lo] = l_lo, xm_mine[PF_TQ + r_lo + 8] = l_hi;
+  pair_sync();
+  l_lo += xm_other[PF_TQ + r_lo], l_hi += xm_other[PF_TQ + r_lo + 8];
   // ---- epilogue: normalise, gate, store
   const float inv_lo = l_lo > 0.f ? 1.f / l_lo : 0.f, inv_hi = l_hi > 0.f ? 1.f / l_hi : 0.f;
 #pragma unroll
-  for (int nd = 0; nd < PF_D / 8; ++nd) {
-    const int d = nd * 8 + (lane & 3) * 2;
+  for (int nd = 0; nd < PF_D / 16; ++nd) {
+    const int d = half * (PF_D / 2) + nd * 8 + (lane & 3) * 2;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int r = r_lo + half * 8;
+    for (int hi = 0; hi < 2; ++hi) {
+      const int r = r_lo + hi * 8;
       if (r >= rows) continue;
       const int t = t0 + r;
-      float v0 = o[nd][half * 2] * (half ? inv_hi : inv_lo), v1 = o[nd][half * 2 + 1] * (half ? inv_hi : inv_lo);
+      float v0 = o[nd][hi * 2] * (hi ? inv_hi : inv_lo), v1 = o[nd][hi * 2 + 1] * (hi ? inv_hi : inv_lo);
       if (gated) {
         const bf16* gp = gate_src + (size_t)t * gate_ld + (size_t)h * 2 * PF_D + PF_D + d;
         v0 *= sigmoid_f(__bfloat162float(gp[0])), v1 *= sigmoid_f(__bfloat162float(gp[1]));
@@ -1248,17 +1253,20 @@ TRL_API int trl_attn_prefill(const void* q, const void* gate_src, int gate_ld, c
   const int G = n_kv > 0 ? n_q / n_kv : 0;
   if (D != PF_D || G < 1 || G > 8 || n_q % n_kv != 0 || B <= 0 || max_q_len <= 0) return (int)cudaErrorInvalidValue;
   if (n_blocks <= 0 || ((uintptr_t)kcache & 15) || ((uintptr_t)vcache & 15)) return (int)cudaErrorInvalidValue;
-  const size_t smem = (size_t)G * PF_TQ * PF_ROW + (size_t)4 * PF_BC * PF_ROW + 1024;
+  constexpr int kv_bytes = 4 * PF_BC * PF_ROW + 1024;
+  constexpr int head_bytes = PF_TQ * PF_ROW + 2 * PF_XCH;
+  auto kernel = G <= 6 ? attn_prefill_kernel<false, 384> : attn_prefill_kernel<false, 512>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(attn_prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * PF_TQ * PF_ROW + 4 * PF_BC * PF_ROW + 1024) != cudaSuccess)
+    if (cudaFuncSetAttribute(attn_prefill_kernel<false, 384>, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * head_bytes + kv_bytes) != cudaSuccess ||
+        cudaFuncSetAttribute(attn_prefill_kernel<false, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * head_bytes + kv_bytes) != cudaSuccess)
       return 3;
     configured = true;
   }
   DmMaps maps;
   if (dm_get_maps(kcache, vcache, n_blocks, n_kv, &maps)) return (int)cudaErrorInvalidValue;
   const dim3 grid((max_q_len + PF_TQ - 1) / PF_TQ, n_kv, B);
-  return (int)trl_launch(attn_prefill_kernel<false>, grid, dim3(G * 32), smem, (cudaStream_t)stream, (const bf16*)q,
+  return (int)trl_launch(kernel, grid, dim3(G * 64), (size_t)G * head_bytes + kv_bytes, (cudaStream_t)stream, (const bf16*)q,
                          (const bf16*)gate_src, gate_ld, (const bf16*)kcache, (const bf16*)vcache,
                          (const float*)nullptr, (const float*)nullptr,
                          (const int*)block_table, max_blocks, (const int*)q_start, (const int*)q_len,
@@ -1275,17 +1283,18 @@ TRL_API int trl_attn_prefill_fp8(const void* q, const void* gate_src, int gate_l
                                  float scale, int gated, void* stream) {
   const int G = n_kv > 0 ? n_q / n_kv : 0;
   if (D != PF_D || G < 1 || G > 8 || n_q % n_kv != 0 || B <= 0 || max_q_len <= 0) return (int)cudaErrorInvalidValue;
-  constexpr size_t kv_bytes = (size_t)2 * PF_BC * PF_ROW + (size_t)4 * PF_BC * PF_D + (size_t)4 * PF_BC * sizeof(float) + 1024;
-  const size_t smem = (size_t)G * PF_TQ * PF_ROW + kv_bytes;
+  constexpr int kv_bytes = 2 * PF_BC * PF_ROW + 4 * PF_BC * PF_D + 4 * PF_BC * (int)sizeof(float) + 1024;
+  constexpr int head_bytes = PF_TQ * PF_ROW + 2 * PF_XCH;
+  auto kernel = G <= 6 ? attn_prefill_kernel<true, 384> : attn_prefill_kernel<true, 512>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(attn_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(8 * PF_TQ * PF_ROW + kv_bytes)) != cudaSuccess)
+    if (cudaFuncSetAttribute(attn_prefill_kernel<true, 384>, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * head_bytes + kv_bytes) != cudaSuccess ||
+        cudaFuncSetAttribute(attn_prefill_kernel<true, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * head_bytes + kv_bytes) != cudaSuccess)
       return 3;
     configured = true;
   }
   const dim3 grid((max_q_len + PF_TQ - 1) / PF_TQ, n_kv, B);
-  return (int)trl_launch(attn_prefill_kernel<true>, grid, dim3(G * 32), smem, (cudaStream_t)stream, (const bf16*)q,
+  return (int)trl_launch(kernel, grid, dim3(G * 64), (size_t)G * head_bytes + kv_bytes, (cudaStream_t)stream, (const bf16*)q,
                          (const bf16*)gate_src, gate_ld, (const bf16*)kcache, (const bf16*)vcache,
                          (const float*)kscale, (const float*)vscale,
                          (const int*)block_table, max_blocks, (const int*)q_start, (const int*)q_len,
