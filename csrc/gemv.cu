@@ -501,8 +501,8 @@ gemv_bf16_kernel(const bf16* x, int ldx, const bf16* __restrict__ w,
 // matrix is streamed once for all rows, which is what bounds the kernel.  KW of a block's 16 warps share the K of 16 weight
 // rows, K / KW each, so that a head of a few thousand rows (small vocabularies, tensor-parallel slices) fills every SM.  With
 // a warp per 16 whole rows, the split before this one, 15 520 rows were work for 61 of 148 SMs.  15 520 x 5120, launch included:
-// 1 / 8 / 16 rows 48 / 90 / 152 us before, 40 / 41 / 56 here (16 rows: the activation rows' shared-memory reads show);
-// 128 256 x 4096: 192 / 229 / 283 before, 184 / 185 / 192 here.
+// 1 / 8 / 16 rows 48 / 90 / 152 us before, 40 / 41 / 56 here (16 rows: the activation rows' shared-memory reads show), inside a
+// tick 40 / 69 / 194 before, 33 / 33 / 47 here; 128 256 x 4096: 192 / 229 / 283 before, 184 / 185 / 192 here.
 // A warp needs its K range of the activation rows only: it loads, norms and keeps them as B fragments in its own part of shared
 // memory, 16 bytes a lane and step, and the rows' square sums are all the block exchanges.  The weights of the next steps are
 // in flight (registers, two sets) while those of this one are multiplied, across the block's reduction too.
@@ -549,9 +549,9 @@ gemv_bf16_rows_kernel(const bf16* x, int ldx, const bf16* __restrict__ w, const 
     }
   };
   int gr = blockIdx.x, c = 0;
-  if (gr < groups) load(wa[0], wb[0], gr, 0);      // weights: constant, so before the wait for the predecessor
+  if (gr < groups) load(wa[0], wb[0], gr, 0);
 
-  pdl_wait();
+  pdl_wait();                                      // (at once where the launch is not a programmatic one)
   {
     float ss[NT];
 #pragma unroll
@@ -833,13 +833,24 @@ TRL_API int trl_gemv_bf16(const void* x, int ldx, const void* w, const void* nor
     const int rows = 16 * (BR_WARPS / kw), grid = min(num_sms(), (N + rows - 1) / rows);
     const int aligned = ldx % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
     cudaError_t e = cudaErrorInvalidValue;
+    // Logits (fp32) are not a programmatic launch: loads in flight to registers need L1, and a block that comes to an SM while the kernel before
+    // it leaves finds L1 as small as that kernel's shared memory made it.  In a decode tick, after projections with 228 KB of
+    // shared memory, most blocks took 8 us a round of rows instead of 4.5: 15 520 x 5120, 1 or 8 rows, 62 us after the last
+    // projection, 33 with the SMs empty first; 12 rows 45 to 68 from run to run (single slow SMs), 48 now; 16 rows 45.5, 47.5.
+    // bf16 projections follow kernels of their own kind, which leave L1 as it should be, and keep the overlap.
     const int per = (K / 32 + kw - 1) / kw, u = (per + 3) / 4 * 4 < (per + 4) / 5 * 5 ? 4 : 5;
 #define BR_CASE(NTT, KWW, U, EP)                                                                          \
   if (nt == NTT && kw == KWW && u == U && epi == EP) {                                                    \
     auto kern = gemv_bf16_rows_kernel<NTT, KWW, U, EP>;                                                    \
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BR_SMEM);                \
-    e = trl_launch(kern, dim3(grid), dim3(BR_THREADS), smem, st, (const bf16*)x, ldx, (const bf16*)w,     \
-                   (const float*)norm_w, eps, (const bf16*)residual, ldr, y, ldy, M, N, K, nbuf, aligned); \
+    if (EP == EPI_STORE_F32) {                                                                            \
+      kern<<<dim3(grid), dim3(BR_THREADS), smem, st>>>((const bf16*)x, ldx, (const bf16*)w,               \
+          (const float*)norm_w, eps, (const bf16*)residual, ldr, y, ldy, M, N, K, nbuf, aligned);         \
+      e = cudaGetLastError();                                                                             \
+    } else {                                                                                              \
+      e = trl_launch(kern, dim3(grid), dim3(BR_THREADS), smem, st, (const bf16*)x, ldx, (const bf16*)w,   \
+                     (const float*)norm_w, eps, (const bf16*)residual, ldr, y, ldy, M, N, K, nbuf, aligned); \
+    }                                                                                                     \
   }
 #define BR_CASES(NTT, KWW)                                                                                          \
   BR_CASE(NTT, KWW, 4, EPI_STORE) BR_CASE(NTT, KWW, 4, EPI_STORE_F32) BR_CASE(NTT, KWW, 4, EPI_RESIDUAL)            \
