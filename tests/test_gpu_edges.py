@@ -302,3 +302,47 @@ def test_prefill_attention_pairs_of_warps(ops, g_heads, fp8):
         want = torch.einsum("thgn,nhd->thgd", torch.softmax(s, -1), vv).reshape(n, n_q, d)
         want = (want * torch.sigmoid(gate[rows].double().view(n, n_q, 2, d)[:, :, 1])).reshape(n, -1)
         assert _rel(out[rows], want) < 2 ** -7, (n, h, _rel(out[rows], want))
+
+
+@pytest.mark.parametrize("nk,nv,d", [(2, 4, 128), (1, 3, 128), (2, 2, 64)])
+def test_delta_rule_scan_of_kept_states(ops, nk, nv, d):
+    """The state after every token, from states at even float addresses (the scan of two columns a lane) and at odd ones (the plain
+    recurrence), against the rule in 64 bits on the rows that the preparation left; fp32 sums over up to 17 tokens."""
+    from tilerl_b200.ops import native as N
+    lens, taps, planes = [8, 1, 17, 16], 4, 18
+    c, t, b = (2 * nk + nv) * d, sum(lens), len(lens)
+    g = torch.Generator().manual_seed(d + nv)
+    inp = torch.randn(t, c + nv * d + 2 * nv, generator=g).to(DEV, torch.bfloat16)
+    conv = (torch.randn(c, taps, generator=g) * 0.3).to(DEV)
+    dt, al, nw = torch.randn(nv, generator=g).to(DEV), torch.randn(nv, generator=g).to(DEV), torch.ones(d, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    q0 = [sum(lens[:i]) for i in range(b)]
+    pos, seq = i32([j for n in lens for j in range(n)]), i32([i for i, n in enumerate(lens) for _ in range(n)])
+    qs, ql, slots, keep = i32(q0), i32(lens), i32(list(range(1, b + 1))), i32([1] * b)
+    first = (torch.randn(b + 1, planes, nv, d, d, generator=g) * 0.05).to(DEV)
+    for odd in (0, 1):
+        states = torch.empty(first.numel() + 2, device=DEV)[odd:odd + first.numel()].view(first.shape)
+        states.copy_(first)
+        ring = torch.zeros(b + 1, 16, c, dtype=torch.bfloat16, device=DEV)
+        f = lambda *s: torch.full(s, float("nan"), device=DEV)
+        qn, kn, vc, gg, bb, o = f(t, nk, d), f(t, nk, d), f(t, nv, d), f(t, nv), f(t, nv), f(t, nv, d)
+        out = torch.empty(t, nv * d, dtype=torch.bfloat16, device=DEV)
+        cur = torch.full((b + 1,), planes - 1, dtype=torch.int32, device=DEV)
+        N.check(ops.lib.trl_gdn(inp.data_ptr(), inp.stride(0), conv.data_ptr(), dt.data_ptr(), al.data_ptr(), nw.data_ptr(),
+                                states.data_ptr(), cur.data_ptr(), ring.data_ptr(), pos.data_ptr(), seq.data_ptr(), qs.data_ptr(),
+                                ql.data_ptr(), slots.data_ptr(), keep.data_ptr(), states.stride(0), states.stride(1),
+                                ring.stride(0), qn.data_ptr(), kn.data_ptr(), vc.data_ptr(), gg.data_ptr(), bb.data_ptr(), o.data_ptr(),
+                                out.data_ptr(), t, b, nk, nv, d, taps, planes, 1e-6, N.stream()), "gdn")
+        rep = nv // nk
+        for i, n in enumerate(lens):
+            s = first[i + 1, planes - 1].double()
+            for j in range(n):
+                r = q0[i] + j
+                k, q, v = kn[r].double().repeat_interleave(rep, 0), qn[r].double().repeat_interleave(rep, 0), vc[r].double()
+                s = s * torch.exp(gg[r].double()).view(nv, 1, 1)
+                s = s + k.unsqueeze(2) * (bb[r].double().unsqueeze(1) * (v - torch.einsum("hd,hdc->hc", k, s))).unsqueeze(1)
+                assert _rel(states[i + 1, j], s) < 1e-5, (odd, n, j)
+                x = torch.einsum("hd,hdc->hc", q, s)
+                z = inp[r, c:c + nv * d].double().view(nv, d)
+                want = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * torch.nn.functional.silu(z)
+                assert _rel(out[r].view(nv, d), want) < 2 ** -7, (odd, n, j)
