@@ -950,11 +950,12 @@ TRL_API int trl_gemm_trace_read(void* out, int n_ctas) {
   return (int)cudaMemcpyFromSymbol(out, g_gemm_trace, (size_t)n_ctas * TRACE_SLOTS * sizeof(unsigned long long));
 }
 
-// split: 1 / 0 as the caller wants it, -1 by the rule below.  Tiles are split along K when the last round of whole tiles would
-// leave more of the GPU idle than adding up the partial tiles costs.  In units of one k-tile of one tile (0.55 us with up to
-// 128 columns, 0.7 us with 256) the addition costs about ten and 16: measured at 8, 32 and 37 rows 5.4 us, at 512 rows 11 us.
-// 8 rows x 16 480: whole 20 against 17.4 + 10, 23.6 us against 27.6; 512 rows x 5120 x 17 408: 136 against 73.5 + 16, 141 us
-// against 96.  The 5 %: not for every last round its scratch memory.
+// split: 1 / 0 as the caller wants it, -1 by the rule below.  Tiles are split along K when there are fewer than SMs, or when the
+// last round of whole tiles would leave more of the GPU idle than adding up the partial tiles costs.  In units of one k-tile of
+// one tile (0.55 us with up to 128 columns, 0.7 us with 256) the addition costs about ten and 16: measured at 8, 32 and 37 rows
+// 5.4 us, at 512 rows 11 us.  512 rows x 5120 x 17 408: 136 against 73.5 + 16, 141 us against 96.  The 5 %: not for every last
+// round its scratch memory.  Nearly as many tiles as SMs (8 rows x 16 480: 129) are faster whole when alone, 23.6 us against 27.6,
+// but not in a tick (8 sequences 590 us whole, 593 split; verify 2 x 8 rows 662 and 656): split, as fewer tiles are.
 static GemmPlan plan_gemm(int tokens, int J, int N, int K, int max_ctas, int split) {
   GemmPlan g;
   const int cols = tokens * J;
@@ -966,7 +967,7 @@ static GemmPlan plan_gemm(int tokens, int J, int N, int K, int max_ctas, int spl
   if (max_ctas > 0) sms = min(sms, max_ctas);
   const long long T = (long long)g.n_tiles * g.c_tiles, U = T * g.nk;
   const double whole = (double)((T + sms - 1) / sms) * g.nk, even = (double)U / sms + (g.BN == 256 ? 16 : 10);
-  g.split = split >= 0 ? split : whole > 1.05 * even;
+  g.split = split >= 0 ? split : (T < sms || whole > 1.05 * even);
   g.grid = (int)min((long long)sms, g.split ? U : T);
   g.max_seg = g.split ? max_segments(U, g.grid, g.nk) : 1;
   return g;
