@@ -75,3 +75,29 @@ def test_rows_that_are_a_range_equal_an_index(rows):
     assert got.data_ptr() != x.data_ptr() or not len(rows)
     r = Batch.row_range(rows)
     assert r is None or list(range(5))[r] == rows
+
+
+@pytest.mark.parametrize("rows", [[5], [4, 5], [0, 5], [7, 8], [-6], [-6, -5], [1, 9, 2]])
+def test_rows_that_are_not_there_are_refused(rows):
+    """As an index refuses them; a slice would return what there is of them."""
+    x = torch.arange(20.0).view(5, 4)
+    with pytest.raises(IndexError):
+        take_rows(x, rows)
+
+
+def _forward(lens, **kw):
+    from tilerl_b200.factory import build_model, make_ops
+    from tilerl_b200.kv import GdnStatePool, make_kv_pool
+    ops = make_ops("cpu")
+    model = build_model("tiny", "cpu", seed=0, ops=ops)
+    cfg = model.cfg
+    seqs = [dict(tokens=list(range(3 + i, 3 + i + n)), start=0, blocks=[i + 1], slot=i + 1) for i, n in enumerate(lens)]
+    pool = make_kv_pool(cfg, len(lens) + 1, torch.device("cpu"), torch.float32)
+    states = GdnStatePool(cfg, len(lens) + 1, "cpu", ring_dtype=torch.float32)
+    return model.forward(Batch.build(seqs, "cpu"), ops, pool, states, **kw)
+
+
+@pytest.mark.parametrize("rows", [[4], [3, 4], [-5]])
+def test_wanted_rows_that_are_not_there_are_refused(rows):
+    with pytest.raises(IndexError):
+        _forward([1, 3], rows=rows)

@@ -44,9 +44,12 @@ class Batch:
     h2d_bytes: int = 0
 
     @staticmethod
-    def row_range(rows) -> Optional[slice]:
-        """The slice that a list of row numbers is, None when it is not a range (usual: every row, or the last one)."""
+    def row_range(rows, of: Optional[int] = None) -> Optional[slice]:
+        """The slice that a list of row numbers is, None when it is not a range (usual: every row, or the last one).  A row
+        outside ``of`` rows (from the end: below zero) raises: a slice would come back short, an index fault on the device."""
         n = len(rows)
+        if of is not None and n and not (-of <= min(rows) and max(rows) < of):
+            raise IndexError(f"rows {min(rows)} to {max(rows)} of {of}")
         if n == 0 or rows[0] < 0 or rows[-1] - rows[0] + 1 != n or any(rows[i + 1] - rows[i] != 1 for i in range(n - 1)):
             return None
         return slice(rows[0], rows[-1] + 1)

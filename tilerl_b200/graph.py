@@ -37,7 +37,7 @@ def bucket_for(n: int, buckets: Sequence[int] = GRAPH_BUCKETS) -> Optional[int]:
 
 def take_rows(x: torch.Tensor, rows: Sequence[int]) -> torch.Tensor:
     """``x[rows]`` (a new tensor), without an index tensor where the rows are a range."""
-    r = Batch.row_range(rows)
+    r = Batch.row_range(rows, x.shape[0])
     return x[rows] if r is None else x[r].clone()
 
 

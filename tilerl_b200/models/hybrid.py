@@ -220,7 +220,7 @@ class HybridModel:
                 taps[i] = x.clone()  # the residual stream is updated in place
         settle()
         if rows is not None:
-            span = batch.row_range(rows)
+            span = batch.row_range(rows, x.shape[0])
             xs = x[rows if span is None else span] if len(rows) else None
         else:
             # one token a sequence (decode ticks): every row is its sequence's last
