@@ -97,6 +97,14 @@ def _forward(lens, **kw):
     return model.forward(Batch.build(seqs, "cpu"), ops, pool, states, **kw)
 
 
+@pytest.mark.parametrize("lens", [[2, 0], [1, 1], [0, 2, 1], [3]])
+def test_last_rows_are_each_sequences_last(lens):
+    """As many tokens as sequences is not one token each: a sequence may bring none."""
+    every = _forward(lens, last_only=False)
+    last = [sum(lens[:i + 1]) - 1 for i in range(len(lens))]
+    torch.testing.assert_close(_forward(lens), every[last], rtol=0, atol=1e-5)     # (the head of other row counts sums in another order)
+
+
 @pytest.mark.parametrize("rows", [[4], [3, 4], [-5]])
 def test_wanted_rows_that_are_not_there_are_refused(rows):
     with pytest.raises(IndexError):

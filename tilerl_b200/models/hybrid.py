@@ -224,7 +224,8 @@ class HybridModel:
             xs = x[rows if span is None else span] if len(rows) else None
         else:
             # one token a sequence (decode ticks): every row is its sequence's last
-            xs = x[batch.last_idx.long()] if last_only and batch.n_tokens != batch.n_seqs else x
+            single = batch.max_q_len == 1 and batch.n_tokens == batch.n_seqs
+            xs = x[batch.last_idx.long()] if last_only and not single else x
         head = P["embed"] if cfg.tie_embeddings else P["lm_head"]
         logits = None if xs is None else ops.lm_head(xs, P["final_norm"], head, eps)[..., :cfg.vocab]
         if aux_layers or return_hidden:
