@@ -109,3 +109,19 @@ def test_last_rows_are_each_sequences_last(lens):
 def test_wanted_rows_that_are_not_there_are_refused(rows):
     with pytest.raises(IndexError):
         _forward([1, 3], rows=rows)
+
+
+def test_library_of_another_interpreter_is_not_current(monkeypatch):
+    """The host sources read the interpreter's lists in place: its version and headers are part of what was built."""
+    import os
+    import sys
+    from tilerl_b200 import build
+    src = os.path.join(build.CSRC, "hostlist.cu")
+    here = build._stamp(src)
+    assert here == build._stamp(src)
+    with monkeypatch.context() as m:
+        m.setattr(sys, "version_info", (3, 99, 0, "final", 0))
+        assert build._stamp(src) != here
+    with monkeypatch.context() as m:
+        m.setattr(build, "_include", lambda: "/nowhere")
+        assert build._stamp(src) != here

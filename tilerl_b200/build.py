@@ -60,7 +60,18 @@ def _stamp(path: str) -> str:
             with open(os.path.join(CSRC, hdr), "rb") as f:
                 h.update(f.read())
     h.update(" ".join(NVCC_FLAGS).encode())
+    h.update(_interpreter().encode())
     return h.hexdigest()
+
+
+def _interpreter() -> str:
+    """The interpreter whose headers the host sources are compiled with: they read its lists and tuples in place, so an object
+    built for another version is not current."""
+    return f"{sysconfig.get_config_var('SOABI')} {sys.version_info[:3]} {os.path.exists(os.path.join(_include(), 'Python.h'))}"
+
+
+def _include() -> str:
+    return sysconfig.get_paths()["include"]
 
 
 def _digest(sources, flags) -> str:
@@ -114,7 +125,7 @@ def build(force: bool = False, verbose: bool = False, extra_flags=(), trace: boo
         stamp = _stamp(sp)
         if not force and os.path.exists(op) and os.path.exists(st) and open(st).read() == stamp:
             continue
-        cmd = [nvcc, *NVCC_FLAGS, *extra_flags, "-I", sysconfig.get_paths()["include"], "-x", "cu", "-c", sp, "-o", op]
+        cmd = [nvcc, *NVCC_FLAGS, *extra_flags, "-I", _include(), "-x", "cu", "-c", sp, "-o", op]
         jobs.append((cmd, st, stamp))
 
     def run(job):
