@@ -231,10 +231,15 @@ attn_split_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
 //   V   16 bytes of keys 2t, 2t + 1, 2t + 8, 2t + 9 a load; byte i of two keys side by side is, converted, the A operand of
 //       dims g * 16 + i and 128 + g * 16 + i.  The next page's K is loaded when this one's scores are done, its V after the
 //       last product.
-//   P^T two f16 parts (value and rest: 22 bits), moved from accumulator to operand layout by movmatrix.  The weights that
-//       multiply V carry V's row scale and have a running maximum of their own, so that no scale leaves f16's range; the
-//       softmax's denominator is summed in fp32 from the unscaled weights.
-// Query rows are scaled by a power of two into f16's range (exact).  12 sequences of 3 000 to 6 000 keys, 4 kv heads x 6:
+//   P^T two f16 parts (value and rest), moved from accumulator to operand layout by movmatrix.  The weights that multiply V
+//       carry V's row scale (one fp32 product) and a power of two that puts the largest of them between 2^14 and 2^15: what
+//       is above 2^-16 of the largest keeps 23 bits, and what is lost of a smaller one is below 2^-39 of the largest -- a
+//       flat tail of tens of thousands of keys under one large weight loses 2^-24 of that.  The softmax's denominator is
+//       summed in fp32 from the unscaled weights.
+// An MMA's sums are cut off, not rounded, and the cuts of a long chain add up (a running O through 250 pages was 1e-5 off), so
+// a chain is two products long and what it gives is added in fp32.
+// Query rows are scaled by a power of two into f16's range: exact for elements above 2^-27 of the row's largest, within
+// 2^-35 of the largest for those below.  12 sequences of 3 000 to 6 000 keys, 4 kv heads x 6:
 // 620 us a layer with the one-key-a-warp kernel (products on the FMA pipe, a shuffle reduction for each score), 59 here with the
 // merge of the splits (the bytes: 17).
 constexpr int F8_WARPS = 4, F8_D = 256;
@@ -259,6 +264,13 @@ __device__ __forceinline__ float max_over_g(float v) {
   return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 16));
 }
 
+// 2^e, e from -126 to 127 (beyond: the nearest of these)
+__device__ __forceinline__ float pow2i(int e) { return __uint_as_float((uint32_t)(max(-126, min(127, e)) + 127) << 23); }
+// The shift that puts the largest weight between 2^14 and 2^15; none known yet: as it is.
+__device__ __forceinline__ int weight_shift(float largest, int now) {
+  const int e = (int)((__float_as_uint(largest) >> 23) & 255u) - 127;
+  return largest > 0.f ? min(120, 14 - e) : now;
+}
 __global__ void __launch_bounds__(F8_WARPS * 32)
 attn_decode_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld, const unsigned char* kcache,
                        const unsigned char* vcache, const float* kscale, const float* vscale, const int* block_table,
@@ -345,11 +357,13 @@ attn_decode_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld, const u
   float o[16][4];
 #pragma unroll
   for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  float m0 = -INFINITY, m1 = -INFINITY, n0 = -INFINITY, n1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+  // of heads 2t and 2t + 1: largest score, largest weight (as of the last shift), shift, denominator
+  float m0 = -INFINITY, m1 = -INFINITY, n0 = 0.f, n1 = 0.f, l0 = 0.f, l1 = 0.f;
+  int s0 = 0, s1 = 0;
   while (pg < p_hi) {
     const int left = kv_len - pg * KVB;            // keys of this page that exist
     // ---- S^T = K Q^T
-    float sc[4] = {0.f, 0.f, 0.f, 0.f};
+    float sc[4], part[4];
 #pragma unroll
     for (int st = 0; st < 4; ++st) {
       const uint32_t ka[4] = {kr[0][st].x, kr[0][st].y, kr[0][st].z, kr[0][st].w};
@@ -358,37 +372,43 @@ attn_decode_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld, const u
       for (int i = 0; i < 4; ++i) {
         const uint32_t a[4] = {cvt_e4m3x2_to_h2((uint16_t)ka[i]), cvt_e4m3x2_to_h2((uint16_t)kb[i]),
                                cvt_e4m3x2_to_h2((uint16_t)(ka[i] >> 16)), cvt_e4m3x2_to_h2((uint16_t)(kb[i] >> 16))};
-        mma_f16(sc, a, qf[st][2 * i], qf[st][2 * i + 1]);
+        if (i % 2 == 0) part[0] = part[1] = part[2] = part[3] = 0.f;
+        mma_f16(part, a, qf[st][2 * i], qf[st][2 * i + 1]);
+        if (i % 2 == 1) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sc[e] = st == 0 && i == 1 ? part[e] : sc[e] + part[e];
+        }
       }
     }
     const float k0 = ks[0], k1 = ks[1];
     const int nxt = pg + F8_WARPS;
     size_t nrow = 0;
     if (nxt < p_hi) nrow = page_row(nxt), load_k(nrow);
-    // ---- scores (base 2), their running maximum, and that of the weights on V
+    // ---- scores (base 2) and their running maximum
     const bool in0 = g < left, in1 = g + 8 < left;
-    const float lv0 = in0 ? log2f(vs[0]) : 0.f, lv1 = in1 ? log2f(vs[1]) : 0.f;
+    const float v0 = in0 ? vs[0] : 0.f, v1 = in1 ? vs[1] : 0.f;
     const float a0 = in0 ? sc[0] * (k0 * qs0) : -INFINITY, a1 = in0 ? sc[1] * (k0 * qs1) : -INFINITY;
     const float a2 = in1 ? sc[2] * (k1 * qs0) : -INFINITY, a3 = in1 ? sc[3] * (k1 * qs1) : -INFINITY;
-    const float w0 = in0 ? a0 + lv0 : -INFINITY, w1 = in0 ? a1 + lv0 : -INFINITY;
-    const float w2 = in1 ? a2 + lv1 : -INFINITY, w3 = in1 ? a3 + lv1 : -INFINITY;
     const float mm0 = fmaxf(m0, max_over_g(fmaxf(a0, a2))), mm1 = fmaxf(m1, max_over_g(fmaxf(a1, a3)));
-    const float nn0 = fmaxf(n0, max_over_g(fmaxf(w0, w2))), nn1 = fmaxf(n1, max_over_g(fmaxf(w1, w3)));
     const float mb0 = mm0 == -INFINITY ? 0.f : mm0, mb1 = mm1 == -INFINITY ? 0.f : mm1;
-    const float nb0 = nn0 == -INFINITY ? 0.f : nn0, nb1 = nn1 == -INFINITY ? 0.f : nn1;
-    l0 = l0 * exp2f(m0 - mb0) + exp2f(a0 - mb0) + exp2f(a2 - mb0);      // this lane's keys; summed over g at the end
-    l1 = l1 * exp2f(m1 - mb1) + exp2f(a1 - mb1) + exp2f(a3 - mb1);
-    if (__any_sync(0xffffffffu, nn0 != n0 || nn1 != n1)) {
-      const float c0 = exp2f(n0 - nb0), c1 = exp2f(n1 - nb1);
+    const float e0 = exp2f(a0 - mb0), e1 = exp2f(a1 - mb1), e2 = exp2f(a2 - mb0), e3 = exp2f(a3 - mb1);
+    const float t0 = exp2f(m0 - mb0), t1 = exp2f(m1 - mb1);
+    l0 = fmaf(l0, t0, e0 + e2), l1 = fmaf(l1, t1, e1 + e3);             // this lane's keys; summed over g at the end
+    // ---- weights on V, and the power of two that they are held with
+    const float w0 = e0 * v0, w1 = e1 * v0, w2 = e2 * v1, w3 = e3 * v1;
+    const float x0 = fmaxf(fabsf(w0), fabsf(w2)), x1 = fmaxf(fabsf(w1), fabsf(w3));
+    if (__any_sync(0xffffffffu, mm0 != m0 || mm1 != m1 || x0 * pow2i(s0) > 32768.f || x1 * pow2i(s1) > 32768.f)) {
+      n0 = fmaxf(n0 * t0, max_over_g(x0)), n1 = fmaxf(n1 * t1, max_over_g(x1));
+      const int r0 = weight_shift(n0, s0), r1 = weight_shift(n1, s1);
+      const float c0 = t0 * pow2i(r0 - s0), c1 = t1 * pow2i(r1 - s1);
+      s0 = r0, s1 = r1;
 #pragma unroll
       for (int i = 0; i < 16; ++i) o[i][0] *= c0, o[i][1] *= c1, o[i][2] *= c0, o[i][3] *= c1;
     }
-    m0 = mm0, m1 = mm1, n0 = nn0, n1 = nn1;
+    m0 = mm0, m1 = mm1;
     // ---- P^T: value and rest, transposed into the B operand
-    // (from the scores' distances to their own maximum: a + lv rounds at the size of a score, its maximum only sets a scale)
-    const float d0 = mb0 - nb0, d1 = mb1 - nb1;
-    const float p0 = exp2f((a0 - mb0) + (lv0 + d0)), p1 = exp2f((a1 - mb1) + (lv0 + d1));
-    const float p2 = exp2f((a2 - mb0) + (lv1 + d0)), p3 = exp2f((a3 - mb1) + (lv1 + d1));
+    const float f_0 = pow2i(s0), f_1 = pow2i(s1);
+    const float p0 = w0 * f_0, p1 = w1 * f_1, p2 = w2 * f_0, p3 = w3 * f_1;
     const uint32_t h0 = f2_to_h2_bits(p0, p1), h1 = f2_to_h2_bits(p2, p3);
     const float2 f0 = h2_to_f2(h0), f1 = h2_to_f2(h1);
     const uint32_t bh0 = movmatrix_t(h0), bh1 = movmatrix_t(h1);
@@ -417,8 +437,11 @@ attn_decode_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld, const u
         for (int b = 0; b < 2; ++b) {
           const uint32_t a[4] = {cvt_e4m3x2_to_h2((uint16_t)(y0 >> (16 * b))), cvt_e4m3x2_to_h2((uint16_t)(y1 >> (16 * b))),
                                  cvt_e4m3x2_to_h2((uint16_t)(y2 >> (16 * b))), cvt_e4m3x2_to_h2((uint16_t)(y3 >> (16 * b)))};
-          mma_f16(o[wi * 4 + b2 * 2 + b], a, bh0, bh1);
-          mma_f16(o[wi * 4 + b2 * 2 + b], a, bl0, bl1);
+          float part[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_f16(part, a, bh0, bh1);
+          mma_f16(part, a, bl0, bl1);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) o[wi * 4 + b2 * 2 + b][i] += part[i];
         }
       }
     }
@@ -428,9 +451,9 @@ attn_decode_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld, const u
 #pragma unroll
   for (int s = 4; s < 32; s <<= 1) l0 += __shfl_xor_sync(0xffffffffu, l0, s), l1 += __shfl_xor_sync(0xffffffffu, l1, s);
 
-  // ---- merge the warps: every accumulator relative to the warp's score maximum
+  // ---- merge the warps: every accumulator relative to the warp's score maximum, without its shift
   {
-    const float c0 = m0 == -INFINITY ? 0.f : exp2f(n0 - m0), c1 = m1 == -INFINITY ? 0.f : exp2f(n1 - m1);
+    const float c0 = pow2i(-s0), c1 = pow2i(-s1);
     if (g == 0) s_m[warp][2 * t] = m0, s_m[warp][2 * t + 1] = m1, s_l[warp][2 * t] = l0, s_l[warp][2 * t + 1] = l1;
 #pragma unroll
     for (int i = 0; i < 16; i += 4)

@@ -346,3 +346,58 @@ def test_delta_rule_scan_of_kept_states(ops, nk, nv, d):
                 z = inp[r, c:c + nv * d].double().view(nv, d)
                 want = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * torch.nn.functional.silu(z)
                 assert _rel(out[r].view(nv, d), want) < 2 ** -7, (odd, n, j)
+
+
+def _fp8_decode(ops, q, k8, v8, ks, vs, table, ctx, splits, gate=None):
+    """(partial rows, maxima, sums, finished rows) of ``trl_attn_paged_fp8``: a row of ``q [t, heads, 256]`` a sequence."""
+    from tilerl_b200.ops import native as N
+    t, n_q, d = q.shape
+    po = torch.full((t, n_q, splits, d), float("nan"), device=DEV)
+    pm, pl = (torch.full((t, n_q, splits), float("nan"), device=DEV) for _ in range(2))
+    out = torch.full((t, n_q * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    pos, sid = i32([n - 1 for n in ctx]), i32(list(range(t)))
+    g = torch.zeros(t, n_q * 2 * d, dtype=torch.bfloat16, device=DEV) if gate is None else gate
+    N.check(ops.lib.trl_attn_paged_fp8(q.data_ptr(), g.data_ptr(), g.stride(0), k8.data_ptr(), v8.data_ptr(), ks.data_ptr(),
+                                       vs.data_ptr(), table.data_ptr(), table.shape[1], sid.data_ptr(), pos.data_ptr(), po.data_ptr(),
+                                       pm.data_ptr(), pl.data_ptr(), out.data_ptr(), t, n_q, k8.shape[1], d, splits, 1 / d ** 0.5,
+                                       int(gate is not None), N.stream()), "attn_paged_fp8")
+    return po, pm, pl, out
+
+
+@pytest.mark.parametrize("kind,splits,bound", [
+    ("typical", 9, 1e-6), ("long", 2, 1e-6), ("tail 14", 2, 1e-6), ("tail 20", 2, 1e-6), ("tail 20", 9, 1e-6), ("tail 25", 2, 2 ** -14)])
+def test_fp8_attention_keeps_its_sums_in_fp32(ops, kind, splits, bound):
+    """Partial sums against 64 bits, with contexts that a long chain of MMAs or weights cut to f16's range would show in: up to
+    32 000 keys, and a flat tail of 30 000 keys that each weigh 2^-14 to 2^-25 of the first key, seen in the columns where that
+    one's V is zero.  Scores of up to 20 are rounded to 2^-20 of a power of two in fp32, 7e-7 of a weight.  A weight of 2^-25
+    of the largest keeps what is above 2^-39 of that, 2^-14 of itself."""
+    d, n_kv, gh = 256, 2, 6
+    t, ctx = (3, 6000) if kind == "typical" else (1, 32000 if kind == "long" else 30000)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    mb = (ctx + 15) // 16
+    k, v = (torch.randn(t * mb + 1, n_kv, 16, d, generator=g, device=DEV) for _ in range(2))
+    v *= torch.exp(torch.randn(t * mb + 1, n_kv, 16, 1, generator=g, device=DEV))
+    table = (torch.randperm(t * mb, generator=g, device=DEV) + 1).int().view(t, mb)
+    q = torch.randn(t, n_kv * gh, d, generator=g, device=DEV)
+    cols = slice(None)
+    if kind.startswith("tail"):
+        cols = slice(1, None)
+        q.zero_()
+        q[..., 0], k[..., 0] = 16.0, 0.0
+        first = int(table[0, 0])
+        k[first, :, 0, 0] = int(kind.split()[1]) * 0.6931471805599453
+        v[..., 1:] += 1.0
+        v[first, :, 0], v[first, :, 0, 0] = 0.0, 3.0
+    q = q.to(torch.bfloat16)
+    ks, vs = k.abs().amax(-1).clamp_min(1e-8) / 448, v.abs().amax(-1).clamp_min(1e-8) / 448
+    k8, v8 = ((x / s.unsqueeze(-1)).clamp(-448, 448).to(torch.float8_e4m3fn) for x, s in ((k, ks), (v, vs)))
+    po, pm, pl, _ = _fp8_decode(ops, q, k8, v8, ks, vs, table, [ctx] * t, splits)
+    c = torch.exp2(pm.double() - pm.double().amax(-1, keepdim=True))
+    got = (po.double() * c.unsqueeze(-1)).sum(2) / (pl.double() * c).sum(-1, keepdim=True)
+    for i in range(t):
+        b = table[i].long()
+        kk, vv = ((x[b].double() * s[b].double().unsqueeze(-1)).transpose(1, 2).reshape(-1, n_kv, d)[:ctx] for x, s in ((k8, ks), (v8, vs)))
+        s = torch.einsum("hgd,nhd->hgn", q[i].double().view(n_kv, gh, d), kk) / d ** 0.5
+        want = torch.einsum("hgn,nhd->hgd", torch.softmax(s, -1), vv).reshape(n_kv * gh, d)
+        assert _rel(got[i][:, cols], want[:, cols]) < bound, _rel(got[i][:, cols], want[:, cols])
