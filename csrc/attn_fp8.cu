@@ -9,7 +9,7 @@
 //                    quantised and scattered with their scales (one warp per head).
 //   attn_decode_fp8: head dim 256: split-KV on the tensor cores straight from the e4m3 rows (mma.sync, f16 operands, which
 //                    hold e4m3 exactly); the row scales go into the score and into the output weights.
-//   attn_split_fp8 : head dims 64 and 128: one key a warp, fp32 FMAs.
+//   attn_split_fp8 : head dims 64 and 128, and rows off a 16-byte boundary: one key a warp, fp32 FMAs.
 //   attn_combine   : merge of the split partials + sigmoid gate (same maths as the bf16 path).
 //
 // Reference parity: kernels_mma.py:89-166,247-366 (fp8 write / attn_prep_fp8) and the `_fp8`
@@ -103,13 +103,22 @@ attn_prep_fp8_kernel(const bf16* qkv, int ld, const float* __restrict__ qw,
 
 template <int VEC>
 __device__ __forceinline__ void load_e4m3_row(const unsigned char* p, float (&f)[VEC]) {
-  if constexpr (VEC == 4) {
+  if constexpr (VEC == 8) {
+    const uint2 w = *reinterpret_cast<const uint2*>(p);
+    const uint32_t u[2] = {w.x, w.y};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float2 a = h2_to_f2(cvt_e4m3x2_to_h2((uint16_t)(u[i] & 0xFFFFu)));
+      const float2 b = h2_to_f2(cvt_e4m3x2_to_h2((uint16_t)(u[i] >> 16)));
+      f[4 * i] = a.x, f[4 * i + 1] = a.y, f[4 * i + 2] = b.x, f[4 * i + 3] = b.y;
+    }
+  } else if constexpr (VEC == 4) {
     const uint32_t u = *reinterpret_cast<const uint32_t*>(p);
     const float2 a = h2_to_f2(cvt_e4m3x2_to_h2((uint16_t)(u & 0xFFFFu)));
     const float2 b = h2_to_f2(cvt_e4m3x2_to_h2((uint16_t)(u >> 16)));
     f[0] = a.x, f[1] = a.y, f[2] = b.x, f[3] = b.y;
   } else {
-    static_assert(VEC == 2, "head dim must be 64 or 128");
+    static_assert(VEC == 2, "head dim must be 64, 128 or 256");
     const float2 a = h2_to_f2(cvt_e4m3x2_to_h2(*reinterpret_cast<const uint16_t*>(p)));
     f[0] = a.x, f[1] = a.y;
   }
@@ -554,11 +563,14 @@ TRL_API int trl_attn_paged_fp8(const void* q, const void* gate_src, int gate_ld,
                    (const int*)positions, (float*)po, (float*)pm, (float*)pl, (bf16*)out, n_q, n_kv,  \
                    n_splits, sl2, gated);                                                             \
   }
-  if (D == F8_D)
+  // the tensor-core kernel reads rows 16 bytes at a time, the other one 8 (K, V) and 2 (query)
+  const bool tc = D == F8_D && ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 15) == 0;
+  if (tc)
     e = trl_launch(attn_decode_fp8_kernel, grid, dim3(F8_WARPS * 32), 0, st, (const bf16*)q, (const bf16*)gate_src, gate_ld,
                    (const unsigned char*)kcache, (const unsigned char*)vcache, (const float*)kscale, (const float*)vscale,
                    (const int*)block_table, max_blocks, (const int*)seq_ids, (const int*)positions, (float*)po, (float*)pm,
                    (float*)pl, (bf16*)out, n_q, n_kv, n_splits, sl2, gated);
+  else if (D == F8_D) SPLIT_CASE(8)
   else if (D == 128) SPLIT_CASE(4)
   else if (D == 64) SPLIT_CASE(2)
   else return (int)cudaErrorInvalidValue;

@@ -401,3 +401,28 @@ def test_fp8_attention_keeps_its_sums_in_fp32(ops, kind, splits, bound):
         s = torch.einsum("hgd,nhd->hgn", q[i].double().view(n_kv, gh, d), kk) / d ** 0.5
         want = torch.einsum("hgn,nhd->hgd", torch.softmax(s, -1), vv).reshape(n_kv * gh, d)
         assert _rel(got[i][:, cols], want[:, cols]) < bound, _rel(got[i][:, cols], want[:, cols])
+
+
+@pytest.mark.parametrize("off_q,off_kv", [(1, 0), (0, 8), (4, 8)])
+def test_fp8_attention_takes_rows_off_a_16_byte_boundary(ops, off_q, off_kv):
+    """Queries on any element, K and V on any 8 bytes, as the kernel for one key a warp takes them, against the aligned call
+    (the same weights and sums in fp32, in another order)."""
+    d, n_kv, gh, t, ctx = 256, 2, 6, 3, 300
+    g = torch.Generator(device=DEV).manual_seed(off_q + off_kv)
+    mb = (ctx + 15) // 16
+    pages = t * mb + 1
+    k8, v8 = ((torch.randn(pages, n_kv, 16, d, generator=g, device=DEV) * 50).clamp(-448, 448).to(torch.float8_e4m3fn) for _ in range(2))
+    ks, vs = (torch.rand(pages, n_kv, 16, generator=g, device=DEV) * 0.02 + 0.01 for _ in range(2))
+    table = (torch.randperm(pages - 1, generator=g, device=DEV) + 1).int().view(t, mb)
+    q = torch.randn(t, n_kv * gh, d, generator=g, device=DEV).to(torch.bfloat16)
+
+    def moved(x, off):
+        room = torch.empty(x.numel() + 64, dtype=x.dtype, device=DEV)
+        y = room[off:off + x.numel()].view(x.shape)
+        y.copy_(x)
+        assert y.data_ptr() % 16 == off * x.element_size() % 16
+        return y
+    for splits in (1, 3):
+        a = _fp8_decode(ops, q, k8, v8, ks, vs, table, [ctx, 17, 128], splits)[3]
+        b = _fp8_decode(ops, moved(q, off_q), moved(k8, off_kv), moved(v8, off_kv), ks, vs, table, [ctx, 17, 128], splits)[3]
+        assert _rel(b, a) < 2e-4                       # a bf16 step where the sum's last bits tip a rounding over
