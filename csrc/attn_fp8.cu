@@ -280,6 +280,14 @@ __device__ __forceinline__ int weight_shift(float largest, int now) {
   const int e = (int)((__float_as_uint(largest) >> 23) & 255u) - 127;
   return largest > 0.f ? min(120, 14 - e) : now;
 }
+// Pages of a split and splits that have any: a split gets `least` pages, so that a context shorter than the launch's split
+// count was chosen for (a captured one is fixed) is not cut to pieces.  The splits after them are empty.
+__device__ __forceinline__ int split_pages(int pages, int n_splits, int least) {
+  const int n = max(1, min(n_splits, (pages + least - 1) / least));
+  return (pages + n - 1) / n;
+}
+constexpr int F8_LEAST = 8;
+
 __global__ void __launch_bounds__(F8_WARPS * 32)
 attn_decode_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld, const unsigned char* kcache,
                        const unsigned char* vcache, const float* kscale, const float* vscale, const int* block_table,
@@ -295,11 +303,16 @@ attn_decode_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld, const u
   const int kv_len = positions[tok] + 1;
   const int* table = block_table + (size_t)seq_ids[tok] * max_blocks;
   const int pages = (kv_len + KVB - 1) / KVB;
-  // the launch's split count is fixed when a graph is captured, the context is not: a split gets 8 pages at least, blocks
-  // past the last one find an empty range and write a neutral partial
-  const int n_eff = max(1, min(n_splits, (pages + 7) / 8));
-  const int pps = (pages + n_eff - 1) / n_eff;
+  const int pps = split_pages(pages, n_splits, F8_LEAST);
   const int p_hi = min(pages, (split + 1) * pps);
+  if (split * pps >= pages) {                      // an empty split: a neutral partial (which the merge does not read)
+    for (int idx = threadIdx.x; idx < G * (F8_D / 4); idx += blockDim.x) {
+      const size_t base = ((size_t)tok * n_q + kvh * G + idx / (F8_D / 4)) * n_splits + split;
+      reinterpret_cast<float4*>(po + base * F8_D)[idx % (F8_D / 4)] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (idx % (F8_D / 4) == 0) pm[base] = -INFINITY, pl[base] = 0.f;
+    }
+    return;
+  }
   int pg = split * pps + warp;
 
   uint4 kr[2][4], vr[4][2];                        // keys g, g + 8 x 64-dim steps; keys 2t, 2t + 1, 2t + 8, 2t + 9 x halves
@@ -502,17 +515,19 @@ attn_decode_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld, const u
 
 __global__ void __launch_bounds__(256)
 attn_combine_fp8_kernel(const float* po, const float* pm,
-                        const float* pl, const bf16* gate_src, int gate_ld,
-                        bf16* out, int n_q, int D, int n_splits, int gated) {
+                        const float* pl, const bf16* gate_src, int gate_ld, const int* positions,
+                        bf16* out, int n_q, int D, int n_splits, int least, int gated) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x, h = blockIdx.y;
   const size_t base = ((size_t)t * n_q + h) * n_splits;
+  const int pages = (positions[t] + KVB) / KVB, pps = split_pages(pages, n_splits, least);
+  const int used = (pages + pps - 1) / pps;        // the splits after these are empty
   float mm = -INFINITY;
-  for (int s = 0; s < n_splits; ++s) mm = fmaxf(mm, pm[base + s]);
+  for (int s = 0; s < used; ++s) mm = fmaxf(mm, pm[base + s]);
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     float ll = 0.f, a = 0.f;
-    for (int s = 0; s < n_splits; ++s) {
+    for (int s = 0; s < used; ++s) {
       const float ms = pm[base + s];
       const float c = (ms == -INFINITY) ? 0.f : exp2f(ms - mm);
       ll += pl[base + s] * c;
@@ -578,7 +593,7 @@ TRL_API int trl_attn_paged_fp8(const void* q, const void* gate_src, int gate_ld,
   if (e != cudaSuccess) return (int)e;
   if (n_splits > 1)
     e = trl_launch(attn_combine_fp8_kernel, dim3(T, n_q), dim3(min(D, 256)), 0, st, (const float*)po,
-                   (const float*)pm, (const float*)pl, (const bf16*)gate_src, gate_ld, (bf16*)out, n_q, D,
-                   n_splits, gated);
+                   (const float*)pm, (const float*)pl, (const bf16*)gate_src, gate_ld, (const int*)positions, (bf16*)out, n_q, D,
+                   n_splits, tc ? F8_LEAST : 1, gated);
   return (int)e;
 }

@@ -426,3 +426,47 @@ def test_fp8_attention_takes_rows_off_a_16_byte_boundary(ops, off_q, off_kv):
         a = _fp8_decode(ops, q, k8, v8, ks, vs, table, [ctx, 17, 128], splits)[3]
         b = _fp8_decode(ops, moved(q, off_q), moved(k8, off_kv), moved(v8, off_kv), ks, vs, table, [ctx, 17, 128], splits)[3]
         assert _rel(b, a) < 2e-4                       # a bf16 step where the sum's last bits tip a rounding over
+
+
+@pytest.mark.parametrize("ctx", [[5], [128, 129, 40], [1100, 16]])
+def test_fp8_attention_of_short_contexts_in_many_splits(ops, ctx):
+    """More splits than the contexts have groups of eight pages for: the empty ones are neutral partials, the merge gives what
+    one split gives (the same weights, sums in another order)."""
+    d, n_kv, gh, t = 256, 2, 6, len(ctx)
+    g = torch.Generator(device=DEV).manual_seed(sum(ctx))
+    mb = (max(ctx) + 15) // 16
+    k8, v8 = ((torch.randn(t * mb + 1, n_kv, 16, d, generator=g, device=DEV) * 50).clamp(-448, 448).to(torch.float8_e4m3fn) for _ in range(2))
+    ks, vs = (torch.rand(t * mb + 1, n_kv, 16, generator=g, device=DEV) * 0.02 + 0.01 for _ in range(2))
+    table = (torch.randperm(t * mb, generator=g, device=DEV) + 1).int().view(t, mb)
+    q = torch.randn(t, n_kv * gh, d, generator=g, device=DEV).to(torch.bfloat16)
+    gate = torch.randn(t, n_kv * gh * 2 * d, generator=g, device=DEV).to(torch.bfloat16)
+    one = _fp8_decode(ops, q, k8, v8, ks, vs, table, ctx, 1, gate)[3]
+    for splits in (2, 9, 64):
+        po, pm, pl, out = _fp8_decode(ops, q, k8, v8, ks, vs, table, ctx, splits, gate)
+        assert _rel(out, one) < 2e-4
+        for i, n in enumerate(ctx):
+            used = min(splits, ((n + 15) // 16 + 7) // 8)
+            assert bool((pm[i, :, used:] == -float("inf")).all()) and float(pl[i, :, used:].abs().sum() + po[i, :, used:].abs().sum()) == 0
+
+
+def test_explicit_split_count_is_taken_for_the_e4m3_pool(ops):
+    """``attn_splits`` as set: with one split the rows are finished in one launch, without a merge."""
+    from tilerl_b200.batch import Batch
+    from tilerl_b200.config import get_config
+    from tilerl_b200.kv import make_kv_pool
+    from tilerl_b200.ops import native
+    cfg = get_config("small-gpu")
+    pool = make_kv_pool(cfg, 40, torch.device(DEV), fp8=True)
+    batch = Batch.build([dict(tokens=[3], start=500, blocks=list(range(1, 36)), slot=1)], DEV)
+    qkv = torch.randn(1, 2 * cfg.n_q_heads * 256 + 2 * cfg.n_kv_heads * 256, device=DEV).to(torch.bfloat16)
+    lp = dict(q_norm=torch.ones(256, device=DEV), k_norm=torch.ones(256, device=DEV))
+    outs = {}
+    try:
+        for splits, launches in ((0, 3), (1, 2), (2, 3)):
+            ops.attn_splits = splits
+            before = native.launch_count
+            outs[splits] = ops.attention(qkv, lp, batch, pool, 0, cfg, cfg.n_q_heads, cfg.n_kv_heads).clone()
+            assert native.launch_count - before == launches, splits
+    finally:
+        ops.attn_splits = 0
+    assert _rel(outs[0], outs[1]) < 2e-4 and _rel(outs[2], outs[1]) < 2e-4

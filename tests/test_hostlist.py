@@ -125,3 +125,21 @@ def test_library_of_another_interpreter_is_not_current(monkeypatch):
     with monkeypatch.context() as m:
         m.setattr(build, "_include", lambda: "/nowhere")
         assert build._stamp(src) != here
+
+
+@pytest.mark.parametrize("rows,n_kv,pages,want", [(1, 4, 1, 1), (1, 4, 8, 1), (1, 4, 9, 2), (1, 4, 4000, 64), (12, 4, 400, 25), (12, 4, 24, 3), (32, 4, 400, 10),
+                                                  (500, 8, 400, 1), (0, 4, 400, 50)])
+def test_splits_of_attention_over_an_e4m3_pool(rows, n_kv, pages, want):
+    """Four splits a block slot, none of them under eight pages, 64 at most."""
+    from tilerl_b200.ops.cuda import fp8_splits
+    assert fp8_splits(148, rows, n_kv, pages) == want
+
+
+def test_captured_ticks_choose_their_splits_once():
+    """One rule for the runners: the e4m3 one for pools of head dim 256, the bf16 kernel's for others."""
+    from types import SimpleNamespace as NS
+    from tilerl_b200.graph import _splits
+    runner = lambda fp8, dim, mb: NS(ops=NS(sms=148), model=NS(dims=NS(n_kv=4), cfg=NS(head_dim=dim)), kv=NS(fp8=fp8), max_blocks=mb)
+    assert _splits(runner(False, 256, 400), 12, 64) == 3 and _splits(runner(True, 128, 400), 12, 64) == 3
+    assert _splits(runner(True, 256, 400), 12, 64) == 25 and _splits(runner(True, 256, 24), 12, 64) == 3
+    assert _splits(runner(False, 256, 400), 1, 32) == 32

@@ -41,6 +41,15 @@ def take_rows(x: torch.Tensor, rows: Sequence[int]) -> torch.Tensor:
     return x[rows] if r is None else x[r].clone()
 
 
+def _splits(runner, rows: int, most: int) -> int:
+    """Key splits that a captured tick's attention is launched with: contexts may grow up to ``max_blocks`` pages later."""
+    sms, n_kv = getattr(runner.ops, "sms", 148), runner.model.dims.n_kv
+    if getattr(runner.kv, "fp8", False) and runner.model.cfg.head_dim == 256:
+        from .ops.cuda import fp8_splits
+        return fp8_splits(sms, rows, n_kv, runner.max_blocks)
+    return max(1, min(most, sms // max(1, rows * n_kv)))
+
+
 @dataclass
 class TickOut:
     logits: Optional[torch.Tensor]
@@ -107,8 +116,7 @@ class DecodeGraphRunner:
         self.replays = 0
 
     def _splits_for(self, b: int) -> int:
-        sms = getattr(self.ops, "sms", 148)
-        return max(1, min(64, sms // max(1, b * self.model.dims.n_kv)))
+        return _splits(self, b, 64)
 
     def _forward(self, bk: _Bucket):
         self.ops.attn_splits = self._splits_for(bk.b)
@@ -278,8 +286,7 @@ class VerifyGraphRunner:
         self.h2d_bytes = self.d2h_bytes = self.replays = 0
 
     def _forward(self, bk: _VBucket):
-        sms = getattr(self.ops, "sms", 148)
-        self.ops.attn_splits = max(1, min(32, sms // max(1, bk.b * bk.w * self.model.dims.n_kv)))
+        self.ops.attn_splits = _splits(self, bk.b * bk.w, 32)
         res = self.model.forward(bk.batch, self.ops, self.kv, self.states, last_only=False, aux_layers=self.aux)
         self.ops.attn_splits = 0
         logits, taps = (res[0], res[2]) if self.aux else (res, None)

@@ -71,6 +71,13 @@ class Workspace:
         return t[:n].view(*shape)
 
 
+def fp8_splits(sms: int, rows: int, n_kv: int, pages: int) -> int:
+    """Splits of the keys for decode attention over an e4m3 pool (head dim 256) with contexts up to ``pages`` pages.  Blocks of
+    four warps, two to an SM, and contexts of unlike length: four splits a block slot even them out.  The kernel gives a split
+    eight pages at least, so there are no more of them than that."""
+    return max(1, min(64, -(-8 * sms // max(1, rows * n_kv)), -(-pages // 8)))
+
+
 class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
     name = "cuda"
 
@@ -478,11 +485,10 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
                 "attn_prefill_fp8")
             N.count(2)
             return out
-        splits = self.attn_splits or self._pick_splits(batch, t, n_kv)
-        if d == 256:
-            # blocks of four warps, two to an SM, and contexts of unlike length: several splits a block slot even them out
-            # (the kernel gives a split eight pages at least)
-            splits = max(splits, min(64, -(-8 * self.sms // max(1, t * n_kv))))
+        splits = self.attn_splits
+        if not splits:
+            longest = max(batch.host_kv_len) if batch.host_kv_len else 1
+            splits = fp8_splits(self.sms, t, n_kv, -(-longest // 16)) if d == 256 else self._pick_splits(batch, t, n_kv)
         po = self.ws.get("attn_po", (t * n_q * splits * d,), torch.float32)
         pm = self.ws.get("attn_pm", (t * n_q * splits,), torch.float32)
         pl = self.ws.get("attn_pl", (t * n_q * splits,), torch.float32)
