@@ -115,15 +115,47 @@ __device__ __forceinline__ void store_values(const GemmParams& p, const float (&
   }
 }
 
-// Epilogue of one accumulator tile: TMEM -> registers (J columns summed per token with their activation scales, up to 128
-// tokens a thread), the accumulator given back, and only then the stores -- final values (whole) or this CTA's split-K slot --
-// which the next tile's MMAs run beside.  With the stores between the TMEM reads the tensor cores stood still for 5 (plain), 8
-// (SwiGLU) and 20 us (residual) a tile of 256 columns, against 14 for its 20 k-tiles.  tok_first = first token of the tile;
-// slot_row = slot + row.  2000 tokens, 34 816 x 5120 SwiGLU 677 -> 542 us;
-// 5120 x 6144 residual 189 -> 126.
+// Epilogue of one accumulator tile: TMEM -> registers in chunks of CH columns, J columns summed per token with their activation
+// scales, then either the final store (WHOLE) or this CTA's split-K slot.  tok_first = first token of the tile; slot_row =
+// slot + row.
+template <int BN, int J, int EPI, bool WHOLE>
+__device__ __forceinline__ void epilogue_chunks(const GemmParams& p, uint32_t taddr0, const float* rs_s, float ts,
+                                                int tok_first, int n, int lane, float* slot_row) {
+  constexpr int CH = BN >= 32 ? 32 : 16, TPC = CH / J;
+#pragma unroll 1
+  for (int c = 0; c < BN / CH; ++c) {
+    uint32_t r[32];
+    if (CH == 32) tc_ld32(taddr0 + (uint32_t)(c * CH), r); else tc_ld16(taddr0 + (uint32_t)(c * CH), r);
+    const int tokc = tok_first + c * TPC;
+    float res[TPC];
+#pragma unroll
+    for (int t = 0; t < TPC; ++t)                // issued before the wait and before any store of this chunk
+      res[t] = (WHOLE && EPI == EPI_RESIDUAL && tokc + t < p.tokens && n < p.N)
+                   ? __bfloat162float(p.residual[(size_t)(tokc + t) * p.ldr + n]) : 0.f;
+    tc_wait_ld();
+    float v[TPC];
+#pragma unroll
+    for (int t = 0; t < TPC; ++t) {
+      float a = 0.f;
+#pragma unroll
+      for (int j = 0; j < J; ++j) a = fmaf(__uint_as_float(r[t * J + j]), rs_s[c * CH + t * J + j], a);
+      v[t] = a * ts;
+    }
+#pragma unroll
+    for (int t = 0; t < TPC; ++t) {
+      if (WHOLE) epi_store<EPI>(p, tokc + t, n, lane, v[t], res[t]);
+      else slot_row[(size_t)(c * TPC + t) * TILE_N] = v[t];
+    }
+  }
+}
+
+// The same for a whole tile that this CTA's next one follows: up to 128 tokens a thread into registers, the accumulator given
+// back, and only then the stores, which the next tile's MMAs run beside.  With the stores between the TMEM reads the tensor
+// cores stood still for 5 (plain), 8 (SwiGLU) and 20 us (residual) a tile of 256 columns, against 14 for its 20 k-tiles.
+// 2000 tokens, 34 816 x 5120 SwiGLU 677 -> 542 us; 5120 x 6144 residual 189 -> 126.
 template <int BN, int J>
-__device__ __forceinline__ void epilogue_tile(const GemmParams& p, bool whole, uint32_t taddr0, const float* rs_s, float ts,
-                                              int tok_first, int n, int lane, float* slot_row, uint32_t accum_empty) {
+__device__ __forceinline__ void epilogue_ahead(const GemmParams& p, uint32_t taddr0, const float* rs_s, float ts,
+                                               int tok_first, int n, int lane, uint32_t accum_empty) {
   constexpr int CH = BN >= 32 ? 32 : 16, TPC = CH / J, V = BN / J < 128 ? BN / J : 128;
 #pragma unroll 1
   for (int t0 = 0; t0 < BN / J; t0 += V) {
@@ -146,19 +178,81 @@ __device__ __forceinline__ void epilogue_tile(const GemmParams& p, bool whole, u
       tc_fence_before();
       mbar_arrive(accum_empty);
     }
-    if (!whole) {
-#pragma unroll
-      for (int t = 0; t < V; ++t) slot_row[(size_t)(t0 + t) * TILE_N] = v[t];
-    } else if (p.epi == EPI_SWIGLU) {
+    if (p.epi == EPI_SWIGLU) {
       store_values<V, EPI_SWIGLU>(p, v, tok_first + t0, n, lane);
     } else if (p.epi == EPI_RESIDUAL) {
       store_values<V, EPI_RESIDUAL>(p, v, tok_first + t0, n, lane);
-    } else if (p.epi == EPI_STORE_F32) {
-      store_values<V, EPI_STORE_F32>(p, v, tok_first + t0, n, lane);
     } else {
-      store_values<V, EPI_STORE>(p, v, tok_first + t0, n, lane);
+      store_values<V, EPI_STORE_F32>(p, v, tok_first + t0, n, lane);
     }
   }
+}
+
+// Plain bf16 results wait in registers as pairs: half as many.  2000 tokens, 20 000 x 2048: 171 us as fp32, 143 here.
+template <int BN, int J>
+__device__ __forceinline__ void epilogue_ahead_bf16(const GemmParams& p, uint32_t taddr0, const float* rs_s, float ts,
+                                                    int tok_first, int n, uint32_t accum_empty) {
+  constexpr int CH = BN >= 32 ? 32 : 16, TPC = CH / J, V = BN / J < 128 ? BN / J : 128;
+#pragma unroll 1
+  for (int t0 = 0; t0 < BN / J; t0 += V) {
+    uint32_t pk[V / 2];
+#pragma unroll
+    for (int c = 0; c < V / TPC; ++c) {
+      uint32_t r[32];
+      const int col = t0 * J + c * CH;
+      if (CH == 32) tc_ld32(taddr0 + (uint32_t)col, r); else tc_ld16(taddr0 + (uint32_t)col, r);
+      tc_wait_ld();
+#pragma unroll
+      for (int t = 0; t < TPC; t += 2) {
+        float a = 0.f, b = 0.f;
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          a = fmaf(__uint_as_float(r[t * J + j]), rs_s[col + t * J + j], a);
+          b = fmaf(__uint_as_float(r[(t + 1) * J + j]), rs_s[col + (t + 1) * J + j], b);
+        }
+        pk[(c * TPC + t) / 2] = f2_to_bf162_bits(a * ts + 0.f, b * ts + 0.f);      // (+ 0: no negative zero, as epi_store)
+      }
+    }
+    if (t0 + V >= BN / J) {
+      tc_fence_before();
+      mbar_arrive(accum_empty);
+    }
+    uint16_t* out = reinterpret_cast<uint16_t*>(p.out) + n;
+#pragma unroll
+    for (int t = 0; t < V; ++t) {
+      const int tok = tok_first + t0 + t;
+      if (tok < p.tokens && n < p.N) out[(size_t)tok * p.ldo] = (uint16_t)(t & 1 ? pk[t / 2] >> 16 : pk[t / 2]);
+    }
+  }
+}
+
+// How a kernel stores its tiles (the forms are kept apart: together they spill registers in one another's loops).  CHUNKS: a
+// CTA has a tile or parts of some.  AHEAD, AHEAD_BF16 (plain bf16 results): CTAs that go through whole tiles one after the
+// other.  `follows`: this CTA has another one.  The last tile's stores run beside nothing and go out chunk by chunk, but for
+// residuals, whose loads wait for one another there.
+enum { STORES_CHUNKS = 0, STORES_AHEAD = 1, STORES_AHEAD_BF16 = 2 };
+template <int BN, int J, int STORES>
+__device__ __forceinline__ void epilogue_tile(const GemmParams& p, bool whole, bool follows, uint32_t taddr0, const float* rs_s,
+                                              float ts, int tok_first, int n, int lane, float* slot_row, uint32_t accum_empty) {
+  if constexpr (STORES == STORES_AHEAD_BF16) {
+    if (whole && follows) {
+      epilogue_ahead_bf16<BN, J>(p, taddr0, rs_s, ts, tok_first, n, accum_empty);
+      return;
+    }
+  }
+  if constexpr (STORES == STORES_AHEAD) {
+    if (whole && (follows || p.epi == EPI_RESIDUAL)) {
+      epilogue_ahead<BN, J>(p, taddr0, rs_s, ts, tok_first, n, lane, accum_empty);
+      return;
+    }
+  }
+  if (!whole) epilogue_chunks<BN, J, EPI_STORE, false>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
+  else if (p.epi == EPI_SWIGLU) epilogue_chunks<BN, J, EPI_SWIGLU, true>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
+  else if (p.epi == EPI_RESIDUAL) epilogue_chunks<BN, J, EPI_RESIDUAL, true>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
+  else if (p.epi == EPI_STORE_F32) epilogue_chunks<BN, J, EPI_STORE_F32, true>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
+  else epilogue_chunks<BN, J, EPI_STORE, true>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
+  tc_fence_before();
+  mbar_arrive(accum_empty);
 }
 
 template <int BN>
@@ -310,7 +404,7 @@ __device__ __forceinline__ void finish_split_tile(const GemmParams& p, const flo
   }
 }
 
-template <int BN>
+template <int BN, int STORES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                   const GemmParams p) {
@@ -560,9 +654,10 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       if (seg == 0 && threadIdx.x == 64) trace_stamp(5);
       {
         const uint32_t taddr0 = tmem_base + ((uint32_t)(quad * 32) << 16);
-        if (J == 4) epilogue_tile<BN, 4>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
-        else if (J == 2) epilogue_tile<BN, 2>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
-        else epilogue_tile<BN, 1>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
+        const bool follows = u + len < u1;
+        if (J == 4) epilogue_tile<BN, 4, STORES>(p, whole, follows, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
+        else if (J == 2) epilogue_tile<BN, 2, STORES>(p, whole, follows, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
+        else epilogue_tile<BN, 1, STORES>(p, whole, follows, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
       }
       if (threadIdx.x == 64) trace_stamp(6);
       if (!whole) {
@@ -877,10 +972,10 @@ int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t row_bytes
   return r == CUDA_SUCCESS ? 0 : 2;
 }
 
-template <int BN>
+template <int BN, int STORES>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, GemmParams p, int grid, cudaStream_t st) {
   using C = Cfg<BN>;
-  auto kern = gemm_nvfp4_kernel<BN>;
+  auto kern = gemm_nvfp4_kernel<BN, STORES>;
   // default: equal rings (one barrier pair per stage); unequal rings are an experiment knob --
   // measured on the 27B shapes they did not pay for their second wait / commit per unit
   int sa = C::RING_BYTES / (C::A_STAGE + C::B_STAGE);
@@ -923,6 +1018,9 @@ TRL_API int trl_quant_act_nvfp4(const void* x, int ldx, const void* norm_w, floa
                          ldx, (const float*)norm_w, eps, (uint8_t*)xq, (uint8_t*)sf, (float*)rs, K, J, nk * 4,
                          swiglu_in);
 }
+
+// k-tiles from which the stores of a tile run beside the next one's MMAs: with fewer, the stores bound either way.
+constexpr int AHEAD_NK = 8;
 
 // How a product is laid out: columns a tile, CTAs, whole tiles or split ones.
 struct GemmPlan {
@@ -1006,11 +1104,22 @@ TRL_API int trl_gemm_nvfp4(const void* wq, const void* sfw, const void* tscale, 
     return (int)cudaErrorMemoryAllocation;
   cudaStream_t st = (cudaStream_t)stream;
   const int grid = g.grid;
+  const long long tiles = (long long)g.n_tiles * g.c_tiles;
+  // (SwiGLU of little more than a wide tile a CTA: 128 rows x 34 816, 272 tiles, 50.3 us ahead, 48.9 in chunks; residuals
+  // already with four k-tiles: 4096 rows x 1024 x 1024 30.7 us in chunks, 28.5 ahead)
+  const bool ahead = tiles > grid && g.nk >= (epi == EPI_RESIDUAL ? AHEAD_NK / 2 : AHEAD_NK) &&
+                     (epi != EPI_SWIGLU || g.BN < 256 || tiles >= 2 * grid);
+  const int stores = !ahead ? STORES_CHUNKS : epi == EPI_STORE ? STORES_AHEAD_BF16 : STORES_AHEAD;
+#define GEMM_CASE(B)                                                                     \
+  return stores == STORES_CHUNKS  ? launch<B, STORES_CHUNKS>(mw, mx, p, grid, st)        \
+         : stores == STORES_AHEAD ? launch<B, STORES_AHEAD>(mw, mx, p, grid, st)         \
+                                  : launch<B, STORES_AHEAD_BF16>(mw, mx, p, grid, st)
   switch (g.BN) {
-    case 16: return launch<16>(mw, mx, p, grid, st);
-    case 32: return launch<32>(mw, mx, p, grid, st);
-    case 64: return launch<64>(mw, mx, p, grid, st);
-    case 128: return launch<128>(mw, mx, p, grid, st);
-    default: return launch<256>(mw, mx, p, grid, st);
+    case 16: GEMM_CASE(16);
+    case 32: GEMM_CASE(32);
+    case 64: GEMM_CASE(64);
+    case 128: GEMM_CASE(128);
+    default: GEMM_CASE(256);
   }
+#undef GEMM_CASE
 }

@@ -470,3 +470,40 @@ def test_explicit_split_count_is_taken_for_the_e4m3_pool(ops):
     finally:
         ops.attn_splits = 0
     assert _rel(outs[0], outs[1]) < 2e-4 and _rel(outs[2], outs[1]) < 2e-4
+
+
+@pytest.mark.parametrize("tokens,n,k", [(3, 19001, 2080), (10, 19001, 2304), (20, 20000, 2048), (40, 19074, 2304), (128, 9999, 2080), (200, 19072, 2048),
+                                        (900, 5120, 2304), (600, 6000, 1056)])
+def test_gemm_stores_beside_the_next_tile(ops, tokens, n, k):
+    """More tiles than CTAs and K long enough that a tile's stores run beside the next one's MMAs, in every tile width, with rows
+    and columns that fill no tile: every epilogue, against the same kernel on one CTA per tile in chunks (split: one tile a
+    CTA at a time)."""
+    from tilerl_b200 import formats as F
+    from tilerl_b200.ops import native
+    from tilerl_b200.ops.gemm_tc import gemm_nvfp4
+    g = torch.Generator().manual_seed(tokens + n)
+    w = F.quantize_nvfp4(torch.randn(n, k, generator=g) * 0.02).to(DEV)
+    x = torch.randn(tokens, k, generator=g).to(DEV, torch.bfloat16)
+    want = torch.full((tokens, n), float("nan"), device=DEV)
+    for a in range(0, n, 2560):                       # at most 20 tiles of rows: the form for few tiles
+        part = F.NVFP4Tensor(w.wq[a:a + 2560].contiguous(), w.scale[a:a + 2560].contiguous(), w.tscale)
+        y = torch.empty(tokens, part.wq.shape[0], device=DEV)
+        gemm_nvfp4(ops, x[:60], part, y[:60], terms=2, epi=3, split=False)
+        for b in range(60, tokens, 60):
+            gemm_nvfp4(ops, x[b:b + 60], part, y[b:b + 60], terms=2, epi=3, split=False)
+        want[:, a:a + 2560] = y
+    for split in (False, True, None):
+        f32, bf16 = torch.full((tokens, n), float("nan"), device=DEV), torch.full((tokens, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+        gemm_nvfp4(ops, x, w, f32, terms=2, epi=3, split=split)
+        assert _rel(f32, want) < 1e-6
+        gemm_nvfp4(ops, x, w, bf16, terms=2, split=split)
+        assert _rel(bf16, want) < 2 ** -8
+        r = torch.randn(tokens, n, generator=g).to(DEV, torch.bfloat16)
+        acc = r.clone()
+        gemm_nvfp4(ops, x, w, acc, terms=2, epi=1, residual=acc, split=split)
+        assert _rel(acc, want.double() + r.double()) < 2 ** -8
+        if n % 2 == 0:
+            h = torch.full((tokens, n // 2), float("nan"), dtype=torch.bfloat16, device=DEV)
+            gemm_nvfp4(ops, x, w, h, terms=2, epi=2, split=split)
+            assert _rel(h, torch.nn.functional.silu(want[:, 0::2].double()) * want[:, 1::2].double()) < 2 ** -8
+    assert native.read_error()[0] == 0
