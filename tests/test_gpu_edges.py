@@ -507,3 +507,26 @@ def test_gemm_stores_beside_the_next_tile(ops, tokens, n, k):
             gemm_nvfp4(ops, x, w, h, terms=2, epi=2, split=split)
             assert _rel(h, torch.nn.functional.silu(want[:, 0::2].double()) * want[:, 1::2].double()) < 2 ** -8
     assert native.read_error()[0] == 0
+
+
+@pytest.mark.parametrize("k", [1040, 18464, 24576, 28672])
+@pytest.mark.parametrize("terms,swiglu", [(1, False), (2, False), (2, True), (4, False)])
+def test_activation_quantiser_with_the_row_staged(ops, k, terms, swiglu):
+    """Rows that the row kernel does not take: a block a row, the row staged in shared memory (128 rows and more), against blocks
+    of slices (fewer rows): the same values, the same bytes."""
+    from tilerl_b200.ops.gemm_tc import quant_act
+    g = torch.Generator().manual_seed(k)
+    width = 2 * k if swiglu else k
+    room = torch.zeros(130, width + 8, dtype=torch.bfloat16, device=DEV)
+    x = room[:, :width] if swiglu or k > 18432 else room[:, 4:4 + width]
+    x.copy_(torch.randn(130, width, generator=g) * torch.exp(torch.randn(130, 1, generator=g)))
+    nw = None if swiglu else (1.0 + 0.1 * torch.randn(k, generator=g)).to(DEV)
+    nk = (k + 255) // 256
+
+    def codes(rows):
+        xq, sf, rs = quant_act(ops, rows, k, terms, norm_w=nw, eps=1e-6, swiglu_in=swiglu)
+        c = torch.arange(rows.shape[0] * terms, device=DEV)
+        return xq.clone(), rs.clone(), sf.view(-1, nk * 4, 32, 4, 4).permute(0, 3, 2, 1, 4).reshape(-1, nk * 16)[c].clone()
+    many, few = codes(x), codes(x[:100])
+    assert all(torch.equal(a[:100 * terms], b) for a, b in zip(many, few))
+    assert int(many[2][:, k // 16:].sum()) == 0
