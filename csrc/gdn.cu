@@ -264,12 +264,13 @@ gdn_recur_kernel(const float* qn, const float* kn,
 
 // ---------------------------------------------------------------------------------------
 // Column-sliced scan.  The delta rule never mixes state columns, so one (sequence, value
-// head) is cut into D/32 CTAs of 32 columns each; a warp owns 8 columns, a lane two of them,
-// and the lanes split the dk rows in eight groups (lane = group * 4 + column pair), so a step needs
-// two 3-level shuffles and no block barrier.  With the state of every token kept (verify) the
-// planes' stores bound it: two columns a lane make them whole 32-byte sectors (one column a lane
-// wrote halves), and a k or q element read from shared memory serves both columns.  2 sequences x 8
-// tokens x 48 heads, 50 MB of planes: 38 us with one column a lane, 30 here.  q / k / v / gates of 16 tokens at a time are staged in
+// head) is cut into D/32 CTAs of 32 columns each; a lane owns COLS adjacent ones, and the lanes of
+// a warp split the dk rows in eight groups (lane = group * 4 + columns), so a step needs two 3-level
+// shuffles and no block barrier.  One column a lane (eight warps keep every scheduler busy while each
+// waits on its own dependent FMA chain) is the shorter step, and the form for a few heads and for
+// prompts.  With the state of every token kept (verify) and many heads the planes' stores bound it:
+// two columns a lane (four warps) make them whole 32-byte sectors instead of halves.
+// q / k / v / gates of 16 tokens at a time are staged in
 // shared memory with cp.async one chunk ahead, so no step waits on global memory.  The raw
 // outputs of a chunk go out coalesced; the last CTA of a head to finish (device counter)
 // runs the gated RMSNorm over the whole head.
@@ -284,8 +285,11 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <int D>
-__global__ void __launch_bounds__(128)
+template <int N> struct ScanCols;                 // N adjacent floats as they are loaded and stored
+template <> struct ScanCols<1> { typedef float type; };
+template <> struct ScanCols<2> { typedef float2 type; };
+template <int D, int COLS>
+__global__ void __launch_bounds__(256 / COLS)
 gdn_scan_kernel(const float* qn, const float* kn,
                 const float* vc, const float* gin,
                 const float* bin, const bf16* inp, int ld,
@@ -299,7 +303,8 @@ gdn_scan_kernel(const float* qn, const float* kn,
   constexpr int R = D / Q;        // state rows per thread
   constexpr int NS = D / 32;      // column slices (CTAs) per head
   constexpr int KP = R + 4;       // padded group stride: the eight groups hit different banks
-  constexpr int NT = 128, NW = NT / 32, CW = 32 / Q;   // threads, warps, column pairs per warp
+  constexpr int NT = 256 / COLS, NW = NT / 32, CW = 32 / Q;   // threads, warps, lanes of a row group
+  typedef typename ScanCols<COLS>::type vec;
   constexpr int TC = SCAN_TC;
   __shared__ __align__(16) float s_q[2][TC][Q * KP];
   __shared__ __align__(16) float s_k[2][TC][Q * KP];
@@ -311,7 +316,7 @@ gdn_scan_kernel(const float* qn, const float* kn,
   pdl_wait();
   const int h = blockIdx.x / NS, slice = blockIdx.x % NS, seq = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int r = lane / CW, cl = 2 * (warp * CW + lane % CW), col = slice * 32 + cl;
+  const int r = lane / CW, cl = COLS * (warp * CW + lane % CW), col = slice * 32 + cl;
   const int T = q_len[seq], t0 = q_start[seq];
   if (T == 0) return;
   const int slot = state_slots[seq];
@@ -320,9 +325,20 @@ gdn_scan_kernel(const float* qn, const float* kn,
   const int live = cur[slot];
   float* sbase = states + (size_t)slot * state_slot_stride + (size_t)h * D * D;
   const float* sin_ = sbase + (size_t)live * plane_stride;
-  float2 S[R];                    // columns col and col + 1
+  float S[R][COLS];
+  auto get = [](float (&x)[COLS], const float* src) {
+    const vec v = *reinterpret_cast<const vec*>(src);
 #pragma unroll
-  for (int j = 0; j < R; ++j) S[j] = *reinterpret_cast<const float2*>(sin_ + (size_t)(r * R + j) * D + col);
+    for (int c = 0; c < COLS; ++c) x[c] = reinterpret_cast<const float*>(&v)[c];
+  };
+  auto put = [](float* dst, const float (&x)[COLS]) {
+    vec v;
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) reinterpret_cast<float*>(&v)[c] = x[c];
+    *reinterpret_cast<vec*>(dst) = v;
+  };
+#pragma unroll
+  for (int j = 0; j < R; ++j) get(S[j], sin_ + (size_t)(r * R + j) * D + col);
 
   auto stage = [&](int i0, int b) {
     const int n = min(TC, T - i0);
@@ -369,35 +385,43 @@ gdn_scan_kernel(const float* qn, const float* kn,
     __syncthreads();                       // s_qk visible, s_o flushed
     for (int tt = 0; tt < n; ++tt) {
       const float eg = __expf(s_g[b][tt]), beta = s_b[b][tt], qk = s_qk[b][tt];
-      const float2 v = *reinterpret_cast<const float2*>(&s_v[b][tt][cl]);
+      float v[COLS], o[COLS], d[COLS];
+      get(v, &s_v[b][tt][cl]);
       const float4* k4 = reinterpret_cast<const float4*>(&s_k[b][tt][r * KP]);
       const float4* q4 = reinterpret_cast<const float4*>(&s_q[b][tt][r * KP]);
       float kreg[R];
-      float2 ks0 = {0.f, 0.f}, ks1 = ks0, qs0 = ks0, qs1 = ks0;
-      auto fma2 = [](float a, float2 x, float2& acc) { acc.x = fmaf(a, x.x, acc.x), acc.y = fmaf(a, x.y, acc.y); };
+      float ks[2][COLS], qs[2][COLS];      // even and odd rows
+#pragma unroll
+      for (int c = 0; c < COLS; ++c) ks[0][c] = ks[1][c] = qs[0][c] = qs[1][c] = 0.f;
 #pragma unroll
       for (int j = 0; j < R / 4; ++j) {
         const float4 kk = k4[j], qq = q4[j];
         kreg[4 * j] = kk.x, kreg[4 * j + 1] = kk.y, kreg[4 * j + 2] = kk.z, kreg[4 * j + 3] = kk.w;
-        fma2(kk.x, S[4 * j], ks0), fma2(kk.y, S[4 * j + 1], ks1);
-        fma2(kk.z, S[4 * j + 2], ks0), fma2(kk.w, S[4 * j + 3], ks1);
-        fma2(qq.x, S[4 * j], qs0), fma2(qq.y, S[4 * j + 1], qs1);
-        fma2(qq.z, S[4 * j + 2], qs0), fma2(qq.w, S[4 * j + 3], qs1);
-      }
-      float2 ks = {ks0.x + ks1.x, ks0.y + ks1.y}, qs = {qs0.x + qs1.x, qs0.y + qs1.y};
 #pragma unroll
-      for (int m = CW; m < 32; m <<= 1) {
-        ks.x += __shfl_xor_sync(0xffffffffu, ks.x, m), ks.y += __shfl_xor_sync(0xffffffffu, ks.y, m);
-        qs.x += __shfl_xor_sync(0xffffffffu, qs.x, m), qs.y += __shfl_xor_sync(0xffffffffu, qs.y, m);
+        for (int c = 0; c < COLS; ++c) {
+          ks[0][c] = fmaf(kk.x, S[4 * j][c], ks[0][c]), ks[1][c] = fmaf(kk.y, S[4 * j + 1][c], ks[1][c]);
+          ks[0][c] = fmaf(kk.z, S[4 * j + 2][c], ks[0][c]), ks[1][c] = fmaf(kk.w, S[4 * j + 3][c], ks[1][c]);
+          qs[0][c] = fmaf(qq.x, S[4 * j][c], qs[0][c]), qs[1][c] = fmaf(qq.y, S[4 * j + 1][c], qs[1][c]);
+          qs[0][c] = fmaf(qq.z, S[4 * j + 2][c], qs[0][c]), qs[1][c] = fmaf(qq.w, S[4 * j + 3][c], qs[1][c]);
+        }
       }
-      const float dx = beta * (v.x - eg * ks.x), dy = beta * (v.y - eg * ks.y);
 #pragma unroll
-      for (int j = 0; j < R; ++j) S[j].x = fmaf(kreg[j], dx, eg * S[j].x), S[j].y = fmaf(kreg[j], dy, eg * S[j].y);
-      if (r == 0) *reinterpret_cast<float2*>(&s_o[tt][cl]) = make_float2(fmaf(eg, qs.x, qk * dx), fmaf(eg, qs.y, qk * dy));
+      for (int c = 0; c < COLS; ++c) {
+        float k_ = ks[0][c] + ks[1][c], q_ = qs[0][c] + qs[1][c];
+#pragma unroll
+        for (int m = CW; m < 32; m <<= 1) k_ += __shfl_xor_sync(0xffffffffu, k_, m), q_ += __shfl_xor_sync(0xffffffffu, q_, m);
+        d[c] = beta * (v[c] - eg * k_);
+        o[c] = fmaf(eg, q_, qk * d[c]);
+      }
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) S[j][c] = fmaf(kreg[j], d[c], eg * S[j][c]);
+      if (r == 0) put(&s_o[tt][cl], o);
       if (keep && i0 + tt < planes) {
         float* sp = sbase + (size_t)(i0 + tt) * plane_stride;
 #pragma unroll
-        for (int j = 0; j < R; ++j) *reinterpret_cast<float2*>(sp + (size_t)(r * R + j) * D + col) = S[j];
+        for (int j = 0; j < R; ++j) put(sp + (size_t)(r * R + j) * D + col, S[j]);
       }
     }
   }
@@ -410,7 +434,7 @@ gdn_scan_kernel(const float* qn, const float* kn,
   if (!keep) {
     float* sp = sbase + (size_t)live * plane_stride;
 #pragma unroll
-    for (int j = 0; j < R; ++j) *reinterpret_cast<float2*>(sp + (size_t)(r * R + j) * D + col) = S[j];
+    for (int j = 0; j < R; ++j) put(sp + (size_t)(r * R + j) * D + col, S[j]);
   }
   const int C = 2 * nk * D + nv * D;
   if (slice == 0) {
@@ -472,8 +496,8 @@ gdn_scan_kernel(const float* qn, const float* kn,
 
 
 // ---------------------------------------------------------------------------------------
-// Chunk-parallel scan for prefill: the same column slicing as the scan above, one column a lane and
-// eight warps, but the 16 tokens of a chunk are not walked one after the other.  With the chunk's
+// Chunk-parallel scan for prefill: the same column slicing and thread mapping as the scan above with
+// one column a lane, but the 16 tokens of a chunk are not walked one after the other.  With the chunk's
 // cumulative log-decay G_i, the chunk-start state S0 and, per state column,
 //   p_i = k_i . S0,  r_i = q_i . S0                        (all tokens at once, no chain)
 //   M_ij = beta_i e^{G_i-G_j} (k_i . k_j)  (j < i),   N_ij = e^{G_i-G_j} (q_i . k_j)  (j <= i)
@@ -1181,6 +1205,13 @@ gdn_gated_norm_kernel(const float* o_scratch, const bf16* inp, int ld, const flo
 
 }  // namespace
 
+static int num_sms() {
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 static int g_gdn_wy = -1;   // -1: read TRL_GDN_WY at the first launch
 static int g_gdn_mma = -1;  // -1: on unless TRL_GDN_MMA=0 (read at the first launch)
 
@@ -1559,8 +1590,8 @@ TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_
                  (const int*)q_len, (const int*)positions, (const int*)state_slots,                 \
                  (const int*)keep_flags, state_slot_stride, plane_stride, ring_slot_stride,         \
                  (const float*)norm_w, eps, (float*)o_scratch, (bf16*)out, nk, nv, planes)
-#define SCAN(DD)                                                                                    \
-  e = trl_launch(gdn_scan_kernel<DD>, dim3(nv * (DD / 32), B), dim3(128), 0, st, (const float*)qn,  \
+#define SCAN(DD, COLS)                                                                              \
+  e = trl_launch(gdn_scan_kernel<DD, COLS>, dim3(nv * (DD / 32), B), dim3(256 / COLS), 0, st, (const float*)qn, \
                  (const float*)kn, (const float*)vc, (const float*)g, (const float*)beta,           \
                  (const bf16*)inp, ld, (float*)states, (int*)cur, (bf16*)ring, (const int*)q_start, \
                  (const int*)q_len, (const int*)positions, (const int*)state_slots,                 \
@@ -1607,12 +1638,17 @@ TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_
   // 512-token layer); it needs more row groups per column to pay off.
   if (g_gdn_wy < 0) g_gdn_wy = (getenv("TRL_GDN_WY") && atoi(getenv("TRL_GDN_WY")) != 0) ? 1 : 0;
   const bool wy_on = g_gdn_wy != 0;
-  // (the scans read the state in pairs; a state at an odd float goes through the plain recurrence)
-  const bool pairs = ((uintptr_t)states & 7) == 0 && ((state_slot_stride | plane_stride) & 1) == 0;
-  const bool scan = !legacy && pairs && (long)B * nv <= GDN_DONE_CAP;
+  const bool scan = !legacy && (long)B * nv <= GDN_DONE_CAP;
+  // two columns a lane, where the states can be read in pairs: with kept states from more CTAs than two an SM, for short heads
+  // always, without from more than four.  Layer with its preparation, kept states of 8 tokens: 72 heads x 128 35.8 us with one
+  // column, 40.0 with two; 96 heads 50.2 and 40.0; 384 heads 115.8 and 82.9.  Prompts of 300 tokens: 96 heads x 64 220 and 282,
+  // 192 heads 247 and 294, 384 heads 415 and 382.
+  const long ctas = (long)B * nv * (D / 32);
+  const bool pairs = ((uintptr_t)states & 7) == 0 && ((state_slot_stride | plane_stride) & 1) == 0 &&
+                     (keep_flags != nullptr ? D == 64 || ctas > 2 * num_sms() : ctas > 4 * num_sms());
   const bool wy = scan && wy_on && T > B && keep_flags == nullptr;
-  if (D == 128) { if (wy) SCANWY(128) else if (scan) SCAN(128); else RECUR(128); }
-  else if (D == 64) { if (wy) SCANWY(64) else if (scan) SCAN(64); else RECUR(64); }
+  if (D == 128) { if (wy) SCANWY(128) else if (scan && pairs) SCAN(128, 2); else if (scan) SCAN(128, 1); else RECUR(128); }
+  else if (D == 64) { if (wy) SCANWY(64) else if (scan && pairs) SCAN(64, 2); else if (scan) SCAN(64, 1); else RECUR(64); }
   else return (int)cudaErrorInvalidValue;
 #undef RECUR
 #undef SCAN

@@ -530,3 +530,45 @@ def test_activation_quantiser_with_the_row_staged(ops, k, terms, swiglu):
     many, few = codes(x), codes(x[:100])
     assert all(torch.equal(a[:100 * terms], b) for a, b in zip(many, few))
     assert int(many[2][:, k // 16:].sum()) == 0
+
+
+@pytest.mark.parametrize("nk,nv,d,lens,keep,odd", [
+    (8, 24, 128, [3, 1, 8, 17], True, 0), (8, 24, 128, [3, 1, 8, 17], True, 1), (2, 4, 64, [8, 1, 5], True, 0), (2, 4, 64, [8, 1, 5], True, 1),
+    (16, 48, 64, [40, 1, 17, 5, 16, 33, 2], False, 0), (16, 48, 64, [40, 1, 17, 5, 16, 33, 2], False, 1)])
+def test_delta_rule_scan_forms_equal_one_sequence_at_a_time(ops, nk, nv, d, lens, keep, odd):
+    """Two columns a lane (many heads, kept states of short ones) and one (few heads, states at odd float addresses) do the same
+    arithmetic on a column: the same states and rows as each sequence alone, bit for bit."""
+    from tilerl_b200.ops import native as N
+    c, t, b, planes = (2 * nk + nv) * d, sum(lens), len(lens), max(lens) + 1 if keep else 1
+    g = torch.Generator().manual_seed(d + nv + odd)
+    inp = torch.randn(t, c + nv * d + 2 * nv, generator=g).to(DEV, torch.bfloat16)
+    conv = (torch.randn(c, 4, generator=g) * 0.3).to(DEV)
+    dt, al, nw = torch.randn(nv, generator=g).to(DEV), torch.randn(nv, generator=g).to(DEV), torch.rand(d, generator=g).to(DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    q0 = [sum(lens[:i]) for i in range(b)]
+    first = torch.randn(b + 1, planes, nv, d, d, generator=torch.Generator(device=DEV).manual_seed(d), device=DEV) * 0.05
+
+    def run(groups):
+        states = torch.empty(first.numel() + 2, device=DEV)[odd:odd + first.numel()].view(first.shape)
+        states.copy_(first)
+        out = torch.zeros(t, nv * d, dtype=torch.bfloat16, device=DEV)
+        ring = torch.zeros(b + 1, 16, c, dtype=torch.bfloat16, device=DEV)
+        cur = torch.full((b + 1,), planes - 1, dtype=torch.int32, device=DEV)
+        for seqs in groups:
+            n = [lens[i] for i in seqs]
+            a, m = q0[seqs[0]], sum(n)
+            f = lambda *s: torch.full(s, float("nan"), device=DEV)
+            sc = [f(m, nk, d), f(m, nk, d), f(m, nv, d), f(m, nv), f(m, nv), f(m, nv, d)]
+            pos, seq = i32([j for x in n for j in range(x)]), i32([i for i, x in enumerate(n) for _ in range(x)])
+            qs, ql, slots, kp = i32([sum(n[:i]) for i in range(len(n))]), i32(n), i32([i + 1 for i in seqs]), i32([1] * len(n))
+            rows = inp[a:a + m]
+            N.check(ops.lib.trl_gdn(rows.data_ptr(), rows.stride(0), conv.data_ptr(), dt.data_ptr(), al.data_ptr(), nw.data_ptr(),
+                                    states.data_ptr(), cur.data_ptr(), ring.data_ptr(), pos.data_ptr(), seq.data_ptr(), qs.data_ptr(),
+                                    ql.data_ptr(), slots.data_ptr(), kp.data_ptr() if keep else None, states.stride(0), states.stride(1),
+                                    ring.stride(0), *(x.data_ptr() for x in sc), out[a:].data_ptr(), m, len(n), nk, nv, d, 4, planes,
+                                    1e-6, N.stream()), "gdn")
+        return states, out
+    s1, o1 = run([list(range(b))])
+    s2, o2 = run([[i] for i in range(b)])
+    assert torch.equal(s1, s2) and torch.equal(o1, o2)
+    assert not torch.equal(s1, first) and bool(torch.isfinite(o1.float()).all())
