@@ -92,7 +92,8 @@ gdn_prep_kernel(const bf16* inp, int ld, const float* __restrict__ conv_w,
     float val[8];
     const bool fresh = live && next_seq != seq;
     seq = next_seq;
-    rows[0] = rows[1], rows[1] = rows[2], rows[2] = rows[3], rows[3] = next;
+    // (rows older than a shorter window stay zero: their taps are, but 0 x infinity is not)
+    rows[0] = KW > 3 ? rows[1] : zero, rows[1] = KW > 2 ? rows[2] : zero, rows[2] = KW > 1 ? rows[3] : zero, rows[3] = next;
     if (i + 1 < run && t + 1 < T) next = load8(inp + (size_t)(t + 1) * ld + c), next_seq = seq_ids[t + 1];
     if (fresh) {                                // the run's or a sequence's first token: its window from the rows before it
       const int pos = positions[t], t0 = q_start[seq];

@@ -572,3 +572,34 @@ def test_delta_rule_scan_forms_equal_one_sequence_at_a_time(ops, nk, nv, d, lens
     s2, o2 = run([[i] for i in range(b)])
     assert torch.equal(s1, s2) and torch.equal(o1, o2)
     assert not torch.equal(s1, first) and bool(torch.isfinite(o1.float()).all())
+
+
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+def test_delta_rule_prep_does_not_read_past_a_short_window(ops, taps):
+    """A row that is not finite is seen by the ``taps`` tokens whose window it is in, and by none after them, where tokens are
+    taken in runs too."""
+    from tilerl_b200.ops import native as N
+    nk, nv, d, t = 2, 4, 128, 3000
+    c = (2 * nk + nv) * d
+    g = torch.Generator().manual_seed(taps)
+    inp = torch.randn(t, c + nv * d + 2 * nv, generator=g).to(DEV, torch.bfloat16)
+    bad = [0, 9, 1203, 2998]
+    for i, r in enumerate(bad):
+        inp[r, :c] = float("nan") if i % 2 else float("inf")
+    conv = torch.rand(c, taps, generator=g).to(DEV) + 0.1
+    dt, al, nw = torch.randn(nv, generator=g).to(DEV), torch.randn(nv, generator=g).to(DEV), torch.ones(d, device=DEV)
+    ring = torch.zeros(2, 16, c, dtype=torch.bfloat16, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pos, seq, qs, ql, slots, cur = i32(list(range(t))), i32([0] * t), i32([0]), i32([t]), i32([1]), i32([0, 0])
+    states = torch.zeros(2, 1, nv, d, d, device=DEV)
+    f = lambda *s: torch.zeros(s, device=DEV)
+    qn, kn, vc, gg, bb, o = f(t, nk, d), f(t, nk, d), f(t, nv, d), f(t, nv), f(t, nv), f(t, nv, d)
+    out = torch.empty(t, nv * d, dtype=torch.bfloat16, device=DEV)
+    N.check(ops.lib.trl_gdn(inp.data_ptr(), inp.stride(0), conv.data_ptr(), dt.data_ptr(), al.data_ptr(), nw.data_ptr(), states.data_ptr(),
+                            cur.data_ptr(), ring.data_ptr(), pos.data_ptr(), seq.data_ptr(), qs.data_ptr(), ql.data_ptr(), slots.data_ptr(),
+                            None, states.stride(0), states.stride(1), ring.stride(0), qn.data_ptr(), kn.data_ptr(), vc.data_ptr(), gg.data_ptr(),
+                            bb.data_ptr(), o.data_ptr(), out.data_ptr(), t, 1, nk, nv, d, taps, 1, 1e-6, N.stream()), "gdn")
+    seen = torch.zeros(t, dtype=torch.bool)
+    for r in bad:
+        seen[r:r + taps] = True
+    assert torch.equal(torch.isfinite(vc).all(-1).all(-1).cpu(), ~seen)
