@@ -1577,7 +1577,7 @@ TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_
   // runs as long as leaves about 16 CTAs of 128 threads for every SM
   const int prep_tpc = 1024 / D;
   int run = 8;
-  while (run > 1 && (long)(T + prep_tpc * run - 1) / (prep_tpc * run) * (2 * nk + nv) < 16 * 148) run >>= 1;
+  while (run > 1 && (long)(T + prep_tpc * run - 1) / (prep_tpc * run) * (2 * nk + nv) < 16 * num_sms()) run >>= 1;
   cudaError_t e = trl_launch(gdn_prep_kernel, dim3((T + prep_tpc * run - 1) / (prep_tpc * run), 2 * nk + nv + 1), dim3(128), 0, st,
                              (const bf16*)inp, ld, (const float*)conv_w, (const float*)dt_bias, (const float*)a_log,
                              (const bf16*)ring, (const int*)positions, (const int*)seq_ids,
@@ -1672,18 +1672,17 @@ TRL_API int trl_gdn_decode(const void* inp, int ld, const void* conv_w, const vo
                          (const float*)norm_w, (float*)states, (const int*)cur, (bf16*)ring,                \
                          (const int*)positions, (const int*)q_start, (const int*)state_slots,               \
                          state_slot_stride, plane_stride, ring_slot_stride, eps, (bf16*)out, nk, nv, KW)
-  // from as many heads as fill the SMs one and a half times over (below, a block an item finds an SM of its own at once)
+  // from as many heads as fill the SMs one and a half times over (below, a block an item finds an SM of its own at once: 216
+  // heads 22.6 us in either form, 224 22.6 and 16.4, 384 30.7 and 20.5)
   // and where bulk copies can take the states (16-byte addresses)
   const bool bulk = ((uintptr_t)states & 15) == 0 && ((state_slot_stride | plane_stride) & 3) == 0;
-  if (D == 128 && KW <= 4 && bulk && nv * B >= 222) {
+  const int sms = num_sms();
+  if (D == 128 && KW <= 4 && bulk && 2L * nv * B >= 3L * sms) {
     static bool configured = false;
     if (!configured) {
       if (cudaFuncSetAttribute(gdn_decode_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GdSmem)) != cudaSuccess) return 3;
       configured = true;
     }
-    int sms = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return (int)trl_launch(gdn_decode_stream_kernel, dim3(min(sms, nv * B)), dim3(13 * 32), sizeof(GdSmem), st, (const bf16*)inp, ld,
                            (const float*)conv_w, (const float*)dt_bias, (const float*)a_log, (const float*)norm_w, (float*)states,
                            (const int*)cur, (bf16*)ring, (const int*)positions, (const int*)q_start, (const int*)state_slots,
