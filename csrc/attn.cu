@@ -276,16 +276,17 @@ attn_combine_kernel(const float* po, const float* pm,
 
 // ---------------------------------------------------------------------------------------
 // Tiled prefill attention (legacy tensor-core path: mma.sync m16n8k16 bf16, fp32 accumulate).
-// One CTA = (16-token tile of one sequence, kv head); a pair of warps owns query head
-// kvh * G + pair, so the G heads of a group share every K / V tile of 64 keys (four pages, double
-// buffered).  The pair splits the tile's scores by keys (32 each) and the output by columns (128
-// each): the row maxima and the probabilities (as A fragments) cross through shared memory between
-// two barriers of the pair.  With a warp to a head, the output alone is 128 registers a thread, six
-// warps at 255 registers fill an SM, and the kernel waits on its own MMA and shared-memory latencies
-// (issue slots 23 % busy); a pair has 64 of them a thread, and twelve warps fit.  Online softmax in
-// the exp2 domain; causal by absolute position; sigmoid output gate fused.  D = 256.  The longest
-// tiles (most keys) come first in the grid, so that the last wave is made of short ones.
-// 2000 tokens x 24 heads: 491 us with a warp to a head and the short tiles first; 279 here.
+// One CTA = (16-token tile of one sequence, kv head); WPH warps own query head kvh * G + i, so the G heads of a group share
+// every K / V tile (double buffered, pages of 16 keys).  A pair of warps splits the tile's scores by keys (KPW each) and the
+// output by columns (128 each): the row maxima and the probabilities (as A fragments) cross through shared memory between
+// two barriers of the pair.  With a warp to a head, the output alone is 128 registers a thread, six warps at 255 registers
+// fill an SM, and the kernel waits on its own MMA and shared-memory latencies (issue slots 23 % busy); a pair has 64 of them a
+// thread, and twelve warps fit.  Online softmax in the exp2 domain; causal by absolute position; sigmoid output gate fused.
+// D = 256.  The grid's slowest dimension is the tile: first tile 0 (of a sequence that decodes it is the only one, and has
+// all its keys), then the others, the longest first, of all sequences and heads, so that the last wave is made of short ones.
+// 2000 tokens x 24 heads: 491 us with a warp to a head and the short tiles first; 293 with pairs; 4 x 512 tokens 295, 180 with
+// the longest tiles of one head and sequence after the other, 168 here.
+// Up to four heads a group leave shared memory and registers for two blocks an SM: see pf_pick.
 // The split-KV kernel above re-reads K / V for every query token; this one reads them once per
 // 16 tokens, which is what makes long prompts tractable.
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
@@ -305,8 +306,9 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-constexpr int PF_D = 256, PF_TQ = 16, PF_BC = 64, PF_ROW = PF_D * 2 /*bytes*/, PF_CHUNKS = PF_ROW / 16;
-constexpr int PF_XCH = 32 * 32 + 2 * PF_TQ * 4;    // bytes one warp gives its partner: 8 registers of P a lane, row maxima, row sums
+constexpr int PF_D = 256, PF_TQ = 16, PF_ROW = PF_D * 2 /*bytes*/, PF_CHUNKS = PF_ROW / 16;
+// bytes one warp gives its partner: its keys' P (KPW / 4 registers a lane), row maxima, row sums
+__host__ __device__ constexpr int pf_xch(int wph, int kpw) { return wph == 2 ? kpw * 32 + 2 * PF_TQ * 4 : 0; }
 
 // byte offset of 16-byte chunk `c` of row `r` in a swizzled [rows][512 B] tile
 __device__ __forceinline__ uint32_t pf_off(int r, int c) { return (uint32_t)(r * PF_ROW + ((c ^ (r & 7)) << 4)); }
@@ -338,9 +340,9 @@ __device__ __forceinline__ void e4m3x16_to_bf16(const uint4& raw, float s, uint4
   o1 = make_uint4(r[4], r[5], r[6], r[7]);
 }
 
-// THREADS: 384 (up to six heads a group, 168 registers a thread) or 512
-template <bool FP8, int THREADS>
-__global__ void __launch_bounds__(THREADS, 1)
+// WPH: warps of a head.  KPW: keys of a tile that a warp scores.  THREADS, BLOCKS: of a block at most, of an SM at least.
+template <bool FP8, int WPH, int KPW, int THREADS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS)
 attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
                     const bf16* kcache, const bf16* vcache,
                     const float* kscale, const float* vscale,
@@ -349,6 +351,8 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
                     int n_q, int n_kv, float scale_log2e, int gated,
                     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, int map3d,
                     int n_blocks) {
+  constexpr int PF_BC = WPH * KPW, PF_XCH = pf_xch(WPH, KPW), KS = KPW / 16;   // keys of a tile, k-steps of a warp's P
+  constexpr int NO = PF_D / 8 / WPH;               // n-tiles of a warp's output columns
   extern __shared__ unsigned char pf_smem_raw[];
   __shared__ uint64_t pf_full[2];
   __shared__ volatile int pf_ok;
@@ -356,27 +360,29 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
   unsigned char* pf_smem = pf_smem_raw + (((pf_raw_a + 1023u) & ~1023u) - pf_raw_a);    // swizzle atoms are 1024-byte aligned
   pdl_launch_dependents();
   pdl_wait();
-  const int tile = (int)(gridDim.x - 1 - blockIdx.x), kvh = blockIdx.y, seq = blockIdx.z;
+  const int tile = blockIdx.z == 0 ? 0 : (int)(gridDim.z - blockIdx.z), kvh = blockIdx.x, seq = blockIdx.y;
   const int G = n_q / n_kv;
   const int T = q_len[seq];
   if (tile * PF_TQ >= T) return;
   const int t0 = q_start[seq] + tile * PF_TQ;
   const int rows = min(PF_TQ, T - tile * PF_TQ);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int pair = warp >> 1, half = warp & 1;     // half: which 32 keys of a tile, which 128 columns of the output
+  const int pair = warp / WPH, half = warp % WPH;     // half: which keys of a tile, which 128 columns of the output
   const int h = kvh * G + pair;
   unsigned char* qs = pf_smem + (size_t)pair * PF_TQ * PF_ROW;                 // [G][16][512 B]
-  unsigned char* ks = pf_smem + (size_t)G * PF_TQ * PF_ROW;                    // [2][64][512 B] ([1] when FP8)
-  unsigned char* vs = ks + (FP8 ? 1 : 2) * PF_BC * PF_ROW;                     // [2][64][512 B] ([1] when FP8)
+  unsigned char* ks = pf_smem + (size_t)G * PF_TQ * PF_ROW;                    // [2][BC][512 B] ([1] when FP8)
+  unsigned char* vs = ks + (FP8 ? 1 : 2) * PF_BC * PF_ROW;                     // [2][BC][512 B] ([1] when FP8)
   unsigned char* xch = vs + (FP8 ? 1 : 2) * PF_BC * PF_ROW;                    // [2 G][PF_XCH]
-  unsigned char* raw_k = xch + 2 * G * PF_XCH;                                 // FP8: [2][64][256 B] staged e4m3 rows
-  unsigned char* raw_v = raw_k + 2 * PF_BC * PF_D;                             // FP8: [2][64][256 B]
-  float* s_sc = reinterpret_cast<float*>(raw_v + 2 * PF_BC * PF_D);            // FP8: [2][K, V][64] row scales
-  uint4* x_mine = reinterpret_cast<uint4*>(xch + (size_t)warp * PF_XCH);       // P: [2][32 lanes] of 16 bytes; then max, sum [16]
+  unsigned char* raw_k = xch + WPH * G * PF_XCH;                                 // FP8: [2][BC][256 B] staged e4m3 rows
+  unsigned char* raw_v = raw_k + 2 * PF_BC * PF_D;                             // FP8: [2][BC][256 B]
+  float* s_sc = reinterpret_cast<float*>(raw_v + 2 * PF_BC * PF_D);            // FP8: [2][K, V][BC] row scales
+  uint4* x_mine = reinterpret_cast<uint4*>(xch + (size_t)warp * PF_XCH);       // P: [KS][32 lanes] of 16 bytes; then max, sum [16]
   const uint4* x_other = reinterpret_cast<const uint4*>(xch + (size_t)(warp ^ 1) * PF_XCH);
-  float* xm_mine = reinterpret_cast<float*>(x_mine + 64);
-  const float* xm_other = reinterpret_cast<const float*>(x_other + 64);
-  auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory"); };
+  float* xm_mine = reinterpret_cast<float*>(x_mine + KS * 32);
+  const float* xm_other = reinterpret_cast<const float*>(x_other + KS * 32);
+  auto pair_sync = [&] {
+    if (WPH == 2) asm volatile("bar.sync %0, 64;" ::"r"(pair + 1) : "memory");
+  };
   const uint32_t qs_a = (uint32_t)__cvta_generic_to_shared(qs);
   const uint32_t ks_a = (uint32_t)__cvta_generic_to_shared(ks), vs_a = (uint32_t)__cvta_generic_to_shared(vs);
   const int* table = block_table + (size_t)seq * max_blocks;
@@ -385,13 +391,13 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
   const int n_tiles = (n_keys + PF_BC - 1) / PF_BC;
 
   // the pair's 16 query rows (zero rows past the end of the sequence)
-  for (int x = half * 32 + lane; x < PF_TQ * PF_CHUNKS; x += 64) {
+  for (int x = half * 32 + lane; x < PF_TQ * PF_CHUNKS; x += 32 * WPH) {
     const int r = x / PF_CHUNKS, c = x % PF_CHUNKS;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (r < rows) v = *reinterpret_cast<const uint4*>(q + ((size_t)(t0 + r) * n_q + h) * PF_D + c * 8);
     *reinterpret_cast<uint4*>(qs + pf_off(r, c)) = v;
   }
-  // bf16 pool: thread 0 issues one tiled copy per K / V page of the tile (four pages), counted on full[buf]
+  // bf16 pool: thread 0 issues one tiled copy per K / V page of the tile, counted on full[buf]
   const uint32_t full_a = (uint32_t)__cvta_generic_to_shared(pf_full);
   auto load_kv_tma = [&](int kt, int buf) {
     const int j0 = kt * PF_BC;
@@ -458,9 +464,9 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
   const int r_lo = lane >> 2;                      // fragment rows r_lo and r_lo + 8
   const int pos_lo = r_lo < rows ? positions[t0 + r_lo] : -1;
   const int pos_hi = r_lo + 8 < rows ? positions[t0 + r_lo + 8] : -1;
-  float o[PF_D / 16][4];                           // 16 rows x this warp's 128 columns
+  float o[NO][4];                           // 16 rows x this warp's 128 columns
 #pragma unroll
-  for (int i = 0; i < PF_D / 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  for (int i = 0; i < NO; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;
 
   auto kv_off = [](int r, int c) { return FP8 ? pf_off(r, c) : pt_off(r, c); };
@@ -517,27 +523,27 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
         __syncthreads();
       }
     }
-    // ---- S = Q K^T for this warp's 32 keys of the tile: 4 n-tiles of 8 keys
-    float sc[4][4];
+    // ---- S = Q K^T for this warp's keys of the tile: n-tiles of 8 keys
+    float sc[KPW / 8][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
+    for (int i = 0; i < KPW / 8; ++i) sc[i][0] = sc[i][1] = sc[i][2] = sc[i][3] = 0.f;
 #pragma unroll
     for (int kk = 0; kk < PF_D / 16; ++kk) {
       uint32_t a[4];
       ldsm_x4(a, qs_a + pf_off((lane & 7) + ((lane >> 3) & 1) * 8, kk * 2 + (lane >> 4)));
 #pragma unroll
-      for (int np = 0; np < 2; ++np) {             // two n-tiles per ldmatrix.x4
+      for (int np = 0; np < KS; ++np) {            // two n-tiles per ldmatrix.x4
         uint32_t b[4];
-        ldsm_x4(b, kb + kv_off(half * 32 + np * 16 + (lane & 7) + (lane >> 4) * 8, kk * 2 + ((lane >> 3) & 1)));
+        ldsm_x4(b, kb + kv_off(half * KPW + np * 16 + (lane & 7) + (lane >> 4) * 8, kk * 2 + ((lane >> 3) & 1)));
         mma_bf16(sc[np * 2], a, b[0], b[1]);
         mma_bf16(sc[np * 2 + 1], a, b[2], b[3]);
       }
     }
     // ---- mask, scale, online softmax
-    const int j0 = kt * PF_BC + half * 32;
+    const int j0 = kt * PF_BC + half * KPW;
     float mx_lo = -INFINITY, mx_hi = -INFINITY;
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
+    for (int nt = 0; nt < KPW / 8; ++nt) {
       const int j = j0 + nt * 8 + (lane & 3) * 2;
       sc[nt][0] = (j <= pos_lo) ? sc[nt][0] * scale_log2e : -INFINITY;
       sc[nt][1] = (j + 1 <= pos_lo) ? sc[nt][1] * scale_log2e : -INFINITY;
@@ -550,44 +556,48 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
     mx_lo = fmaxf(mx_lo, __shfl_xor_sync(0xffffffffu, mx_lo, 2));
     mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 1));
     mx_hi = fmaxf(mx_hi, __shfl_xor_sync(0xffffffffu, mx_hi, 2));
-    if ((lane & 3) == 0) xm_mine[r_lo] = mx_lo, xm_mine[r_lo + 8] = mx_hi;
-    pair_sync();
-    const float mn_lo = fmaxf(m_lo, fmaxf(mx_lo, xm_other[r_lo])), mn_hi = fmaxf(m_hi, fmaxf(mx_hi, xm_other[r_lo + 8]));
+    if constexpr (WPH == 2) {
+      if ((lane & 3) == 0) xm_mine[r_lo] = mx_lo, xm_mine[r_lo + 8] = mx_hi;
+      pair_sync();
+      mx_lo = fmaxf(mx_lo, xm_other[r_lo]), mx_hi = fmaxf(mx_hi, xm_other[r_lo + 8]);
+    }
+    const float mn_lo = fmaxf(m_lo, mx_lo), mn_hi = fmaxf(m_hi, mx_hi);
     const float base_lo = mn_lo == -INFINITY ? 0.f : mn_lo, base_hi = mn_hi == -INFINITY ? 0.f : mn_hi;
     const float al_lo = exp2f(m_lo - base_lo), al_hi = exp2f(m_hi - base_hi);   // exp2(-inf) = 0 on the first tile
     m_lo = mn_lo, m_hi = mn_hi;
     float sum_lo = 0.f, sum_hi = 0.f;
-    uint32_t pa[2][4];                             // P of these keys as the A operand of PV: two k-steps of 16 keys
+    uint32_t pa[KS][4];                            // P of these keys as the A operand of PV: k-steps of 16 keys
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
+    for (int nt = 0; nt < KPW / 8; ++nt) {
       const float p0 = exp2f(sc[nt][0] - base_lo), p1 = exp2f(sc[nt][1] - base_lo);
       const float p2 = exp2f(sc[nt][2] - base_hi), p3 = exp2f(sc[nt][3] - base_hi);
       sum_lo += p0 + p1, sum_hi += p2 + p3;
       pa[nt >> 1][(nt & 1) * 2] = f2_to_bf162_bits(p0, p1);
       pa[nt >> 1][(nt & 1) * 2 + 1] = f2_to_bf162_bits(p2, p3);
     }
-    x_mine[lane] = make_uint4(pa[0][0], pa[0][1], pa[0][2], pa[0][3]);
-    x_mine[32 + lane] = make_uint4(pa[1][0], pa[1][1], pa[1][2], pa[1][3]);
+#pragma unroll
+    for (int kk = 0; kk < KS && WPH == 2; ++kk) x_mine[kk * 32 + lane] = make_uint4(pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3]);
     l_lo = l_lo * al_lo + sum_lo, l_hi = l_hi * al_hi + sum_hi;                 // of this lane's keys: summed after the last tile
 #pragma unroll
-    for (int i = 0; i < PF_D / 16; ++i) o[i][0] *= al_lo, o[i][1] *= al_lo, o[i][2] *= al_hi, o[i][3] *= al_hi;
+    for (int i = 0; i < NO; ++i) o[i][0] *= al_lo, o[i][1] *= al_lo, o[i][2] *= al_hi, o[i][3] *= al_hi;
     // ---- O += P V: first this warp's keys, whose P it holds, then the partner's
     auto pv = [&](const uint32_t (&a)[4], int row) {
 #pragma unroll
-      for (int nd = 0; nd < PF_D / 16; nd += 2) {
+      for (int nd = 0; nd < NO; nd += 2) {
         uint32_t b[4];
-        ldsm_x4_t(b, vb + kv_off(row + (lane & 7) + ((lane >> 3) & 1) * 8, half * (PF_D / 16) + nd + (lane >> 4)));
+        ldsm_x4_t(b, vb + kv_off(row + (lane & 7) + ((lane >> 3) & 1) * 8, half * NO + nd + (lane >> 4)));
         mma_bf16(o[nd], a, b[0], b[1]);
         mma_bf16(o[nd + 1], a, b[2], b[3]);
       }
     };
-    pv(pa[0], half * 32), pv(pa[1], half * 32 + 16);
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk) pv(pa[kk], half * KPW + kk * 16);
     pair_sync();
 #pragma unroll
-    for (int kk = 0; kk < 2; ++kk) {
+    for (int kk = 0; kk < KS && WPH == 2; ++kk) {
       const uint4 w = x_other[kk * 32 + lane];
       const uint32_t a[4] = {w.x, w.y, w.z, w.w};
-      pv(a, (half ^ 1) * 32 + kk * 16);
+      pv(a, (half ^ 1) * KPW + kk * 16);
     }
     __syncthreads();                               // the other buffer may be overwritten next round
     if constexpr (!FP8) {
@@ -599,14 +609,16 @@ attn_prefill_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
   l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
   l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
   l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
-  if ((lane & 3) == 0) xm_mine[PF_TQ + r_lo] = l_lo, xm_mine[PF_TQ + r_lo + 8] = l_hi;
-  pair_sync();
-  l_lo += xm_other[PF_TQ + r_lo], l_hi += xm_other[PF_TQ + r_lo + 8];
+  if constexpr (WPH == 2) {
+    if ((lane & 3) == 0) xm_mine[PF_TQ + r_lo] = l_lo, xm_mine[PF_TQ + r_lo + 8] = l_hi;
+    pair_sync();
+    l_lo += xm_other[PF_TQ + r_lo], l_hi += xm_other[PF_TQ + r_lo + 8];
+  }
   // ---- epilogue: normalise, gate, store
   const float inv_lo = l_lo > 0.f ? 1.f / l_lo : 0.f, inv_hi = l_hi > 0.f ? 1.f / l_hi : 0.f;
 #pragma unroll
-  for (int nd = 0; nd < PF_D / 16; ++nd) {
-    const int d = half * (PF_D / 2) + nd * 8 + (lane & 3) * 2;
+  for (int nd = 0; nd < NO; ++nd) {
+    const int d = half * (PF_D / WPH) + nd * 8 + (lane & 3) * 2;
 #pragma unroll
     for (int hi = 0; hi < 2; ++hi) {
       const int r = r_lo + hi * 8;
@@ -1244,29 +1256,63 @@ TRL_API size_t trl_attn_static_scratch_needed(int T, int n_q, int D, int n_split
   return (size_t)T * n_q * n_splits * ((size_t)D + 2) * sizeof(float);
 }
 
+// Form of the prefill kernel for g heads a group: its shared memory, threads and the kernel, allowed that much.
+struct PfForm {
+  size_t smem;
+  int threads;
+  decltype(&attn_prefill_kernel<false, 2, 32, 512, 1>) kernel;
+};
+template <bool FP8, int WPH, int KPW, int THREADS, int BLOCKS>
+static bool pf_form(int g, PfForm* f) {
+  constexpr int BC = WPH * KPW, heads = THREADS / (32 * WPH);
+  constexpr int kv_bytes = (FP8 ? 2 * BC * PF_ROW + 4 * BC * PF_D + 4 * BC * (int)sizeof(float) : 4 * BC * PF_ROW) + 1024;
+  constexpr int head_bytes = PF_TQ * PF_ROW + WPH * pf_xch(WPH, KPW);
+  f->smem = (size_t)g * head_bytes + kv_bytes, f->threads = g * 32 * WPH;
+  f->kernel = attn_prefill_kernel<FP8, WPH, KPW, THREADS, BLOCKS>;
+  static bool configured = false;
+  if (!configured)
+    configured = cudaFuncSetAttribute(f->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, heads * head_bytes + kv_bytes) == cudaSuccess;
+  return configured;
+}
+// Forms for up to four heads a group.  0: pairs of warps, tiles of 64 keys, one block an SM: a block is through soonest, right
+// while the blocks are no more than the SMs, or few of them long.  Otherwise two blocks an SM get more done: 1: a warp a head,
+// tiles of 32 keys, the cheaper a key; 2: pairs, tiles of 32 keys, the cheaper a block, and for e4m3 pools, whose rows the block
+// has to convert first, always the better one.  us, forms 0 / 1 / 2: 8 kv heads x 4, 2000 tokens 483 / 411 / 381, 1000 after
+// 3000 696 / 519 / 612; 2 kv heads x 4, 2000 tokens 133 / 165 / 168.
+template <bool FP8>
+static bool pf_pick(int g, int form, PfForm* f) {
+  if (g > 6) return pf_form<FP8, 2, 32, 512, 1>(g, f);
+  if (g > 4 || form == 0) return pf_form<FP8, 2, 32, 384, 1>(g, f);
+  if constexpr (!FP8) {
+    if (form == 1) return pf_form<FP8, 1, 32, 128, 2>(g, f);
+  }
+  return pf_form<FP8, 2, 16, 256, 2>(g, f);
+}
+// By what a launch alone says (the tiles and keys there can be); callers that know the sequences say which form.
+static int pf_default(const dim3& grid, int max_blocks) {
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return (long)grid.x * grid.y * grid.z <= sms ? 0 : max_blocks * KVB <= 2048 ? 2 : 1;
+}
+
 // Tiled prefill attention over whole sequences of the batch (D = 256, G = n_q / n_kv <= 8):
 // q_start / q_len give each sequence's token range in the flat batch; `out` [T, n_q * D].
-TRL_API int trl_attn_prefill(const void* q, const void* gate_src, int gate_ld, const void* kcache, const void* vcache,
-                             const void* block_table, int max_blocks, int n_blocks, const void* q_start, const void* q_len,
-                             const void* positions, void* out, int B, int max_q_len, int n_q, int n_kv, int D,
-                             float scale, int gated, void* stream) {
+// form: 0 to 2 as above, -1: by the launch.
+TRL_API int trl_attn_prefill_form(const void* q, const void* gate_src, int gate_ld, const void* kcache, const void* vcache,
+                                  const void* block_table, int max_blocks, int n_blocks, const void* q_start,
+                                  const void* q_len, const void* positions, void* out, int B, int max_q_len, int n_q,
+                                  int n_kv, int D, float scale, int gated, int form, void* stream) {
   const int G = n_kv > 0 ? n_q / n_kv : 0;
   if (D != PF_D || G < 1 || G > 8 || n_q % n_kv != 0 || B <= 0 || max_q_len <= 0) return (int)cudaErrorInvalidValue;
   if (n_blocks <= 0 || ((uintptr_t)kcache & 15) || ((uintptr_t)vcache & 15)) return (int)cudaErrorInvalidValue;
-  constexpr int kv_bytes = 4 * PF_BC * PF_ROW + 1024;
-  constexpr int head_bytes = PF_TQ * PF_ROW + 2 * PF_XCH;
-  auto kernel = G <= 6 ? attn_prefill_kernel<false, 384> : attn_prefill_kernel<false, 512>;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attn_prefill_kernel<false, 384>, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * head_bytes + kv_bytes) != cudaSuccess ||
-        cudaFuncSetAttribute(attn_prefill_kernel<false, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * head_bytes + kv_bytes) != cudaSuccess)
-      return 3;
-    configured = true;
-  }
+  const dim3 grid(n_kv, B, (max_q_len + PF_TQ - 1) / PF_TQ);       // the tile is the slowest: longest ones of every sequence first
+  if (grid.z > 65535) return (int)cudaErrorInvalidValue;
+  PfForm f;
+  if (!pf_pick<false>(G, form < 0 ? pf_default(grid, max_blocks) : form, &f)) return 3;
   DmMaps maps;
   if (dm_get_maps(kcache, vcache, n_blocks, n_kv, &maps)) return (int)cudaErrorInvalidValue;
-  const dim3 grid((max_q_len + PF_TQ - 1) / PF_TQ, n_kv, B);
-  return (int)trl_launch(kernel, grid, dim3(G * 64), (size_t)G * head_bytes + kv_bytes, (cudaStream_t)stream, (const bf16*)q,
+  return (int)trl_launch(f.kernel, grid, dim3(f.threads), f.smem, (cudaStream_t)stream, (const bf16*)q,
                          (const bf16*)gate_src, gate_ld, (const bf16*)kcache, (const bf16*)vcache,
                          (const float*)nullptr, (const float*)nullptr,
                          (const int*)block_table, max_blocks, (const int*)q_start, (const int*)q_len,
@@ -1274,32 +1320,42 @@ TRL_API int trl_attn_prefill(const void* q, const void* gate_src, int gate_ld, c
                          maps.mode3d, n_blocks);
 }
 
+TRL_API int trl_attn_prefill(const void* q, const void* gate_src, int gate_ld, const void* kcache, const void* vcache,
+                             const void* block_table, int max_blocks, int n_blocks, const void* q_start, const void* q_len,
+                             const void* positions, void* out, int B, int max_q_len, int n_q, int n_kv, int D,
+                             float scale, int gated, void* stream) {
+  return trl_attn_prefill_form(q, gate_src, gate_ld, kcache, vcache, block_table, max_blocks, n_blocks, q_start, q_len, positions,
+                               out, B, max_q_len, n_q, n_kv, D, scale, gated, -1, stream);
+}
+
 // The same over an e4m3 pool: kcache / vcache are the e4m3 bytes of one layer, kscale / vscale its
 // fp32 row scales [blocks, hkv, 16].
-TRL_API int trl_attn_prefill_fp8(const void* q, const void* gate_src, int gate_ld, const void* kcache,
-                                 const void* vcache, const void* kscale, const void* vscale,
-                                 const void* block_table, int max_blocks, const void* q_start, const void* q_len,
-                                 const void* positions, void* out, int B, int max_q_len, int n_q, int n_kv, int D,
-                                 float scale, int gated, void* stream) {
+TRL_API int trl_attn_prefill_fp8_form(const void* q, const void* gate_src, int gate_ld, const void* kcache,
+                                      const void* vcache, const void* kscale, const void* vscale,
+                                      const void* block_table, int max_blocks, const void* q_start, const void* q_len,
+                                      const void* positions, void* out, int B, int max_q_len, int n_q, int n_kv, int D,
+                                      float scale, int gated, int form, void* stream) {
   const int G = n_kv > 0 ? n_q / n_kv : 0;
   if (D != PF_D || G < 1 || G > 8 || n_q % n_kv != 0 || B <= 0 || max_q_len <= 0) return (int)cudaErrorInvalidValue;
-  constexpr int kv_bytes = 2 * PF_BC * PF_ROW + 4 * PF_BC * PF_D + 4 * PF_BC * (int)sizeof(float) + 1024;
-  constexpr int head_bytes = PF_TQ * PF_ROW + 2 * PF_XCH;
-  auto kernel = G <= 6 ? attn_prefill_kernel<true, 384> : attn_prefill_kernel<true, 512>;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(attn_prefill_kernel<true, 384>, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * head_bytes + kv_bytes) != cudaSuccess ||
-        cudaFuncSetAttribute(attn_prefill_kernel<true, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * head_bytes + kv_bytes) != cudaSuccess)
-      return 3;
-    configured = true;
-  }
-  const dim3 grid((max_q_len + PF_TQ - 1) / PF_TQ, n_kv, B);
-  return (int)trl_launch(kernel, grid, dim3(G * 64), (size_t)G * head_bytes + kv_bytes, (cudaStream_t)stream, (const bf16*)q,
+  const dim3 grid(n_kv, B, (max_q_len + PF_TQ - 1) / PF_TQ);       // the tile is the slowest: longest ones of every sequence first
+  if (grid.z > 65535) return (int)cudaErrorInvalidValue;
+  PfForm f;
+  if (!pf_pick<true>(G, form < 0 ? pf_default(grid, max_blocks) : form, &f)) return 3;
+  return (int)trl_launch(f.kernel, grid, dim3(f.threads), f.smem, (cudaStream_t)stream, (const bf16*)q,
                          (const bf16*)gate_src, gate_ld, (const bf16*)kcache, (const bf16*)vcache,
                          (const float*)kscale, (const float*)vscale,
                          (const int*)block_table, max_blocks, (const int*)q_start, (const int*)q_len,
                          (const int*)positions, (bf16*)out, n_q, n_kv, scale * 1.4426950408889634f, gated, CUtensorMap{},
                          CUtensorMap{}, 0, 0);
+}
+
+TRL_API int trl_attn_prefill_fp8(const void* q, const void* gate_src, int gate_ld, const void* kcache,
+                                 const void* vcache, const void* kscale, const void* vscale,
+                                 const void* block_table, int max_blocks, const void* q_start, const void* q_len,
+                                 const void* positions, void* out, int B, int max_q_len, int n_q, int n_kv, int D,
+                                 float scale, int gated, void* stream) {
+  return trl_attn_prefill_fp8_form(q, gate_src, gate_ld, kcache, vcache, kscale, vscale, block_table, max_blocks, q_start, q_len,
+                                   positions, out, B, max_q_len, n_q, n_kv, D, scale, gated, -1, stream);
 }
 
 TRL_API int trl_attn_paged_static(const void* q, const void* gate_src, int gate_ld, const void* kcache,

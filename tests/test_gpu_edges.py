@@ -603,3 +603,60 @@ def test_delta_rule_prep_does_not_read_past_a_short_window(ops, taps):
     for r in bad:
         seen[r:r + taps] = True
     assert torch.equal(torch.isfinite(vc).all(-1).all(-1).cpu(), ~seen)
+
+
+@pytest.mark.parametrize("g_heads", [1, 3, 4])
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("form", [-1, 0, 1, 2])
+def test_prefill_attention_forms(ops, g_heads, fp8, form):
+    """The forms for up to four heads a group: queries and histories at the edges of 16-row tiles and of tiles of 32 and 64 keys,
+    sequences of one row (first in the grid) among longer ones, pool rows past a sequence's end that are NaN, against 64
+    bits.  Weights and the result are bf16: 2^-9 each of what they carry, in the rms over rows whose keys are independent."""
+    from tilerl_b200.ops import native as N
+    import math
+    n_kv, d = 2, 256
+    n_q = n_kv * g_heads
+    seqs = [(1, 0), (1, 700), (16, 0), (17, 15), (32, 0), (15, 49), (33, 31), (64, 1), (5, 123), (2, 127), (70, 500)]
+    g = torch.Generator(device=DEV).manual_seed(g_heads * 2 + fp8)
+    b, t = len(seqs), sum(n for n, _ in seqs)
+    mb = max((n + h + 15) // 16 for n, h in seqs)
+    pages = b * mb + 1
+    k, v = (torch.randn(pages, n_kv, 16, d, generator=g, device=DEV) for _ in range(2))
+    scales = [torch.ones(pages, n_kv, 16, device=DEV) for _ in range(2)]
+    if fp8:
+        scales = [torch.rand(pages, n_kv, 16, generator=g, device=DEV) * 0.02 + 0.01 for _ in range(2)]
+        k, v = ((x * 50).clamp(-448, 448).to(torch.float8_e4m3fn) for x in (k, v))
+    else:
+        k, v = k.to(torch.bfloat16), v.to(torch.bfloat16)
+    kd, vd = (x.double() * s.double().unsqueeze(-1) for x, s in zip((k, v), scales))
+    table = (torch.randperm(pages - 1, generator=g, device=DEV)[:b * mb] + 1).int().view(b, mb)
+    for i, (n, h) in enumerate(seqs):                   # what lies past the sequence's end must not matter
+        if (n + h) % 16:
+            pg, r = int(table[i, (n + h) // 16]), (n + h) % 16
+            for x in (k, v):
+                x[pg].view(torch.uint8 if fp8 else torch.int16)[:, r:] = 0x7f if fp8 else 0x7fc0
+            if fp8:
+                scales[0][pg, :, r:] = scales[1][pg, :, r:] = float("nan")
+    q = torch.randn(t, n_q, d, generator=g, device=DEV).to(torch.bfloat16)
+    gate = torch.randn(t, n_q * 2 * d, generator=g, device=DEV).to(torch.bfloat16)
+    out = torch.full((t, n_q * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    starts = [sum(n for n, _ in seqs[:i]) for i in range(b)]
+    qs, ql, pos = i32(starts), i32([n for n, _ in seqs]), i32([h + j for n, h in seqs for j in range(n)])
+    tail = (qs.data_ptr(), ql.data_ptr(), pos.data_ptr(), out.data_ptr(), b, max(n for n, _ in seqs), n_q, n_kv, d,
+            1 / math.sqrt(d), 1, form, N.stream())
+    head = (q.data_ptr(), gate.data_ptr(), gate.stride(0), k.data_ptr(), v.data_ptr())
+    if fp8:
+        N.check(ops.lib.trl_attn_prefill_fp8_form(*head, scales[0].data_ptr(), scales[1].data_ptr(), table.data_ptr(), mb, *tail), "prefill_fp8")
+    else:
+        N.check(ops.lib.trl_attn_prefill_form(*head, table.data_ptr(), mb, pages, *tail), "prefill")
+    for i, (n, h) in enumerate(seqs):
+        blocks = table[i].long()
+        kk, vv = (x[blocks].transpose(1, 2).reshape(-1, n_kv, d)[:n + h] for x in (kd, vd))
+        rows = slice(starts[i], starts[i] + n)
+        s = torch.einsum("thgd,nhd->thgn", q[rows].double().view(n, n_kv, g_heads, d), kk) / math.sqrt(d)
+        s.masked_fill_((torch.arange(n + h, device=DEV) > (h + torch.arange(n, device=DEV)).view(n, 1)).view(n, 1, 1, -1), -math.inf)
+        want = torch.einsum("thgn,nhd->thgd", torch.softmax(s, -1), vv).reshape(n, n_q, d)
+        want = (want * torch.sigmoid(gate[rows].double().view(n, n_q, 2, d)[:, :, 1])).reshape(n, -1)
+        assert _rel(out[rows], want) < 2 ** -7, (n, h, _rel(out[rows], want))
+    assert N.read_error()[0] == 0

@@ -143,3 +143,13 @@ def test_captured_ticks_choose_their_splits_once():
     assert _splits(runner(False, 256, 400), 12, 64) == 3 and _splits(runner(True, 128, 400), 12, 64) == 3
     assert _splits(runner(True, 256, 400), 12, 64) == 25 and _splits(runner(True, 256, 24), 12, 64) == 3
     assert _splits(runner(False, 256, 400), 1, 32) == 32
+
+
+@pytest.mark.parametrize("q,kv,n_kv,g,want", [
+    ([2000], [2000], 2, 4, 0), ([2000], [2000], 4, 4, 2), ([512], [512], 4, 3, 0), ([512], [512], 8, 4, 2), ([100] * 8, [100] * 8, 4, 1, 2),
+    ([2048], [8192], 2, 4, 1), ([1000], [4000], 2, 4, 0), ([1000], [4000], 4, 4, 1), ([300], [3300], 8, 2, 1), ([64], [8064], 8, 4, 0),
+    ([1] * 12 + [64], [4001] * 12 + [64], 8, 4, 0), ([2048], [8192], 4, 6, 0), ([1], [1], 1, 1, 0)])
+def test_form_of_prefill_attention(q, kv, n_kv, g, want):
+    """One block an SM while the blocks are through with the longest one; else two, by the length of the contexts."""
+    from tilerl_b200.ops.cuda import prefill_form
+    assert prefill_form(q, kv, n_kv, g, 148) == want

@@ -42,6 +42,7 @@ class Batch:
     keep_rows: List[bool] = field(default_factory=list)   # per sequence: store per-token GDN states
     keep_flags: Optional[torch.Tensor] = None             # [B] int32 device copy of keep_rows
     h2d_bytes: int = 0
+    prefill_forms: dict = field(default_factory=dict)     # by kv heads: form of the prefill attention kernel (the same in every layer)
 
     @staticmethod
     def row_range(rows, of: Optional[int] = None) -> Optional[slice]:

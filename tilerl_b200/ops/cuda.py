@@ -71,6 +71,23 @@ class Workspace:
         return t[:n].view(*shape)
 
 
+def prefill_form(q_lens, kv_lens, n_kv: int, g: int, sms: int) -> int:
+    """Form of the prefill attention kernel (``csrc/attn.cu::pf_pick``) for sequences of ``q_lens`` new tokens and ``kv_lens``
+    keys in all.  With a block an SM the blocks are through about when the longest is, if their keys (and 128 more that a block
+    costs) are no more than the SMs get done meanwhile and those over half as long find an SM each.  Otherwise two blocks an SM:
+    contexts up to 2048 keys in the form that is cheaper a block, others in the one that is cheaper a key."""
+    if g > 4:
+        return 0
+    longest, work, long = max(kv_lens), 0, 0
+    for n, kv in zip(q_lens, kv_lens):
+        start, tiles = kv - n, -(-n // 16)
+        work += tiles * (start + 128) + 8 * tiles * (tiles + 1)
+        long += max(0, tiles - max(0, (longest // 2 - start) // 16))
+    if work * n_kv <= sms * (longest + 128) and long * n_kv <= sms:
+        return 0
+    return 2 if longest <= 2048 else 1
+
+
 def fp8_splits(sms: int, rows: int, n_kv: int, pages: int) -> int:
     """Splits of the keys for decode attention over an e4m3 pool (head dim 256) with contexts up to ``pages`` pages.  Blocks of
     four warps, two to an SM, and contexts of unlike length: four splits a block slot even them out.  The kernel gives a split
@@ -428,11 +445,11 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
                 and n_q // n_kv <= 8 and not getattr(batch, "keep_steps", 0)):
             # prefill chunks (and whatever decode rows ride along): K / V tiles are read once per
             # 16 query tokens by the tiled tensor-core kernel
-            N.check(self.lib.trl_attn_prefill(
+            N.check(self.lib.trl_attn_prefill_form(
                 q.data_ptr(), qkv.data_ptr(), qkv.stride(0), kc.data_ptr(), vc.data_ptr(), table.data_ptr(),
                 table.stride(0), kc.shape[0], batch.q_start.data_ptr(), batch.q_len.data_ptr(), pos.data_ptr(),
                 out.data_ptr(), batch.n_seqs, batch.max_q_len, n_q, n_kv, d, 1.0 / math.sqrt(d), int(cfg.attn_gated),
-                st), "attn_prefill")
+                self._prefill_form(batch, n_kv, n_q // n_kv), st), "attn_prefill")
             N.count(2)
             return out
         if sparse_now:
@@ -477,12 +494,12 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
             int(cfg.attn_gated), st), "attn_prep_fp8")
         if (self.prefill_attn and batch.max_q_len >= 16 and d == 256 and n_q % n_kv == 0 and n_q // n_kv <= 8
                 and not getattr(batch, "keep_steps", 0)):
-            N.check(self.lib.trl_attn_prefill_fp8(
+            N.check(self.lib.trl_attn_prefill_fp8_form(
                 q.data_ptr(), qkv.data_ptr(), qkv.stride(0), kc.data_ptr(), vc.data_ptr(), ks.data_ptr(),
                 vs.data_ptr(), batch.block_table.data_ptr(), batch.block_table.stride(0),
                 batch.q_start.data_ptr(), batch.q_len.data_ptr(), batch.positions.data_ptr(), out.data_ptr(),
-                batch.n_seqs, batch.max_q_len, n_q, n_kv, d, 1.0 / math.sqrt(d), int(cfg.attn_gated), st),
-                "attn_prefill_fp8")
+                batch.n_seqs, batch.max_q_len, n_q, n_kv, d, 1.0 / math.sqrt(d), int(cfg.attn_gated),
+                self._prefill_form(batch, n_kv, n_q // n_kv), st), "attn_prefill_fp8")
             N.count(2)
             return out
         splits = self.attn_splits
@@ -500,6 +517,13 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
             int(cfg.attn_gated), st), "attn_paged_fp8")
         N.count(2 + (1 if splits > 1 else 0))
         return out
+
+    def _prefill_form(self, batch, n_kv: int, g: int) -> int:
+        if g > 4 or not batch.host_q_len:
+            return -1
+        if n_kv not in batch.prefill_forms:
+            batch.prefill_forms[n_kv] = prefill_form(batch.host_q_len, batch.host_kv_len, n_kv, g, self.sms)
+        return batch.prefill_forms[n_kv]
 
     def _pick_splits(self, batch, t: int, n_kv: int, keys: int = 32) -> int:
         """Enough CTAs to fill the GPU when few tokens attend to long contexts; a split covers at
