@@ -820,8 +820,8 @@ TRL_API int trl_gemv_bf16(const void* x, int ldx, const void* w, const void* nor
   if (trl_gemv_bf16_one_pass(M, K) && (epi == EPI_STORE || epi == EPI_STORE_F32 || epi == EPI_RESIDUAL)) {
     // up to 16 rows: one pass over the weights on the tensor cores
     const int nt = M <= 8 ? 1 : 2;
-    // Warps that share K.  A barrier a group costs about as much as five steps of a warp, so K up to 5120 is shared by fewer
-    // than 16 (10 steps a warp at most) as long as there are two rounds of blocks; the
+    // Warps that share K.  A barrier a group costs about as much as five steps of a warp, so K up to 2560 is shared by 8 and up
+    // to 1280 by 4 (10 steps a warp at most) as long as there are two rounds of blocks; the
     // activation rows are then kept once for each group of rows, which fits at these K.  The set of loads is 4 or 5 steps,
     // whichever leaves less of the last one unused (128 256 x 4096, 16 rows: 192 us with 4, 235 with 5).
     int kw = BR_WARPS;

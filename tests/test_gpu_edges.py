@@ -22,9 +22,11 @@ def _rel(a, b):
 @pytest.mark.parametrize("m,n,k,shift", [
     (1, 1, 32, 0), (2, 17, 96, 0), (8, 15, 544, 0), (9, 33, 512, 0), (16, 40, 1056, 0), (1, 16 * 149, 5120, 0), (3, 4100, 5120, 8),
     (5, 2500, 2592, 1), (8, 700, 13824, 0), (16, 900, 6240, 0), (16, 900, 6656, 0), (7, 64, 13856, 0), (16, 64, 6688, 0),
-    (1, 19000, 1024, 0), (13, 19001, 1280, 0), (4, 10100, 2560, 0), (16, 9999, 2048, 4)])
+    (1, 19000, 1024, 0), (13, 19001, 1280, 0), (4, 10100, 2560, 0), (16, 9999, 2048, 4),
+    (4, 32761, 1024, 0), (8, 19001, 1280, 0), (5, 9999, 2048, 0), (12, 32761, 1024, 0), (16, 9999, 2560, 0)])
 def test_bf16_rows_for_every_split_of_k(ops, m, n, k, shift):
-    """K shorter than the 16 warps that share it (4 or 8 with many rows), shared unevenly, and up to what shared memory holds with two, one and no
+    """K shared by 4, 8 and 16 warps in sets of 4 and 5 loads, with one and two tiles of activation rows; K shorter than the 16
+    warps, shared unevenly, and up to what shared memory holds with two, one and no
     reduction buffers; rows that are no multiple of a tile; activations that start off a 16-byte boundary.  Products of bf16
     values are exact in fp32, so sums differ from 64 bits by fp32 rounding alone: below k * 2^-24 of the summed magnitudes,
     and their square root's share of it on average."""
