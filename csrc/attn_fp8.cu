@@ -249,8 +249,8 @@ attn_split_fp8_kernel(const bf16* q, const bf16* gate_src, int gate_ld,
 // a chain is two products long and what it gives is added in fp32.
 // Query rows are scaled by a power of two into f16's range: exact for elements above 2^-27 of the row's largest, within
 // 2^-35 of the largest for those below.  12 sequences of 3 000 to 6 000 keys, 4 kv heads x 6:
-// 620 us a layer with the one-key-a-warp kernel (products on the FMA pipe, a shuffle reduction for each score), 59 here with the
-// merge of the splits (the bytes: 17).
+// 620 us a layer with the one-key-a-warp kernel (products on the FMA pipe, a shuffle reduction for each score), 56 here with the
+// merge of the splits, 51 without (the bytes: 17).
 constexpr int F8_WARPS = 4, F8_D = 256;
 
 __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {

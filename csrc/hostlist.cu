@@ -1,8 +1,8 @@
 // Host-side steps of a tick that the interpreter is slow at (no device code): Python lists into int32 staging memory.
 //
-// A decode tick hands over its sequences as dicts with lists of block ids, some thousands of ids in all; numpy converts ten to
-// twenty a microsecond, which for one 2 000-block list or 32 short ones is as long as three projections of the tick.  Reading
-// the objects directly takes 8 ns each and one call a tick: 1 x 2 047 blocks 44 us before, 8 here; 8 x 260 blocks 41 us,
+// A decode tick hands over its sequences as dicts with lists of block ids, some thousands of ids in all; numpy converts forty to
+// fifty a microsecond, which for one 2 000-block list or 32 short ones is as long as three projections of the tick.  Reading
+// the objects directly takes 4 to 5 ns each and one call a tick: 1 x 2 047 blocks 44 us before, 8 here; 8 x 260 blocks 41 us,
 // 8; 32 x 76 blocks 59 us, 12.  It needs the interpreter (loaded with ctypes.PyDLL); without Python's headers at build time the
 // entry points are left out and the callers keep to numpy.  No counterpart in the reference, whose tick fills its inputs in
 // Python (src/tilerl/decode_graph.py:112).
