@@ -822,7 +822,7 @@ gdn_scan_wy_kernel(const float* qn, const float* kn,
 // state scan, chunk output), here one kernel.
 constexpr int GC_C = 16, GC_D = 128, GC_ROW = GC_D * 2;     // chunk, head dim, bytes of a bf16 row over dk
 constexpr int GC_NS = 2, GC_DV = GC_D / GC_NS, GC_VROW = GC_DV * 2;   // value columns per CTA, bytes of such a row
-constexpr int GC_SLOTS = 4, GC_GROUP = 256, GC_THREADS = 3 * GC_GROUP;
+constexpr int GC_GROUP = 256, GC_SERIAL_CTAS = 3;      // threads of a group; blocks an SM of the form without preparing groups
 struct GcPre {                                   // working memory of one group of preparing warps
   float sq[GC_C][GC_D], sk[GC_C][GC_D];          // fp32 q, k of its chunk
   float sv[GC_C][GC_DV];                         // fp32 v, this CTA's columns
@@ -839,12 +839,14 @@ struct GcSlot {                                  // what a chunk hands to the wa
   __align__(16) float4 u[GC_GROUP];                                      // U in accumulator fragments
   float g_last;
 };
+template <bool PIPE>
 struct GcSmem {
-  GcPre pre[2];
-  GcSlot slot[GC_SLOTS];
+  static constexpr int PRE = PIPE ? 2 : 1, SLOTS = PIPE ? 4 : 1, THREADS = PIPE ? 3 * GC_GROUP : GC_GROUP;
+  GcPre pre[PRE];
+  GcSlot slot[SLOTS];
   __align__(128) unsigned char vn[GC_C * GC_VROW];                       // bf16 [16][64 dv]
   __align__(128) unsigned char sbf[GC_D * GC_VROW];                      // bf16 copy of the state [dk][64 dv], swizzled
-  unsigned long long full[GC_SLOTS], empty[GC_SLOTS];
+  unsigned long long full[SLOTS], empty[SLOTS];
   int abort;
 };
 __device__ __forceinline__ void gc_cp4(void* smem_dst, const void* gsrc) {
@@ -874,20 +876,23 @@ __device__ __forceinline__ void gc_mma(float (&c)[4], const uint32_t (&a)[4], ui
 // from v) does not wait for the state: two groups of eight warps prepare the chunks, one the even, one the odd ones, up to four
 // chunks ahead, and eight warps that hold the state take them over with two block-wide meetings a chunk.  In one sequence of
 // phases, as before, a chunk took 2.9 us (a 2000-token layer 360 us); here 2.0 us (251 us).  The chain of the chunks bounds it: products of
-// 16 rows, no unit is busy.  Raw outputs go to o_scratch (fp32); the gated RMSNorm, which needs whole rows, is the small
+// 16 rows, no unit is busy.  Without PIPE eight warps do all of it, one thing after the other, with 72 KB instead of 157: three blocks an SM,
+// for many short sequences.  Raw outputs go to o_scratch (fp32); the gated RMSNorm, which needs whole rows, is the small
 // kernel below.
-__global__ void __launch_bounds__(GC_THREADS, 1)
+template <bool PIPE>
+__global__ void __launch_bounds__(GcSmem<PIPE>::THREADS, PIPE ? 1 : GC_SERIAL_CTAS)
 gdn_chunk_mma_kernel(const float* qn, const float* kn, const float* vc, const float* gin, const float* bin,
                      float* states, int* cur, bf16* ring, const bf16* inp, int ld, const int* q_start,
                      const int* q_len, const int* positions, const int* state_slots, long state_slot_stride,
                      long plane_stride, long ring_slot_stride, float* o_scratch, int nk, int nv) {
-  constexpr int D = GC_D, C = GC_C, DV = GC_DV;
+  using Smem = GcSmem<PIPE>;
+  constexpr int D = GC_D, C = GC_C, DV = GC_DV, SLOTS = Smem::SLOTS;
   extern __shared__ __align__(128) unsigned char gc_raw[];
-  GcSmem& sm = *reinterpret_cast<GcSmem*>(gc_raw);
+  Smem& sm = *reinterpret_cast<Smem*>(gc_raw);
   pdl_launch_dependents(2);
   pdl_wait();
   const int h = blockIdx.x / GC_NS, c0 = (blockIdx.x % GC_NS) * DV, seq = blockIdx.y;
-  const int group = threadIdx.x / GC_GROUP, tid = threadIdx.x % GC_GROUP, warp = tid >> 5, lane = tid & 31;
+  const int group = PIPE ? threadIdx.x / GC_GROUP : 0, tid = threadIdx.x % GC_GROUP, warp = tid >> 5, lane = tid & 31;
   const int T = q_len[seq], t0 = q_start[seq];
   if (T == 0) return;
   const int chunks = (T + C - 1) / C;
@@ -898,7 +903,7 @@ gdn_chunk_mma_kernel(const float* qn, const float* kn, const float* vc, const fl
   auto u32 = [](const void* p) { return (uint32_t)__cvta_generic_to_shared(p); };
   volatile int* abort_flag = &sm.abort;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < GC_SLOTS; ++i) mbar_init(u32(&sm.full[i]), GC_GROUP), mbar_init(u32(&sm.empty[i]), GC_GROUP);
+    for (int i = 0; i < SLOTS; ++i) mbar_init(u32(&sm.full[i]), GC_GROUP), mbar_init(u32(&sm.empty[i]), GC_GROUP);
     sm.abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -915,195 +920,203 @@ gdn_chunk_mma_kernel(const float* qn, const float* kn, const float* vc, const fl
     return r != 0;
   };
 
-  if (group > 0) {
-    // ---------------- preparing groups ----------------
-    const int first = group - 1;
-    GcPre& w = sm.pre[first];
-    const uint32_t a_qraw = u32(w.qraw), a_kraw = u32(w.kraw), a_kb = u32(w.kb), a_vb = u32(w.vb), a_thi = u32(w.t_hi), a_tlo = u32(w.t_lo);
-    auto stage = [&](int i0, int b) {      // fp32 q, k, v rows and the gates of chunk i0 .. i0 + 15 (rows past T: zeros)
-      for (int x = tid; x < C * (D / 4); x += GC_GROUP) {
-        const int tt = x / (D / 4), e = (x % (D / 4)) * 4;
-        if (i0 + tt < T) {
-          const size_t src = ((size_t)(t0 + i0 + tt) * nk + kh) * D + e;
-          cp_async16(&w.sq[tt][e], qn + src);
-          cp_async16(&w.sk[tt][e], kn + src);
-        } else {
-          *reinterpret_cast<float4*>(&w.sq[tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
-          *reinterpret_cast<float4*>(&w.sk[tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+  // ---------------- what a chunk needs before the state is known ----------------
+  const int first = group > 0 ? group - 1 : 0;
+  GcPre& w = sm.pre[first];
+  auto stage = [&](int i0, int b) {      // fp32 q, k, v rows and the gates of chunk i0 .. i0 + 15 (rows past T: zeros)
+    for (int x = tid; x < C * (D / 4); x += GC_GROUP) {
+      const int tt = x / (D / 4), e = (x % (D / 4)) * 4;
+      if (i0 + tt < T) {
+        const size_t src = ((size_t)(t0 + i0 + tt) * nk + kh) * D + e;
+        cp_async16(&w.sq[tt][e], qn + src);
+        cp_async16(&w.sk[tt][e], kn + src);
+      } else {
+        *reinterpret_cast<float4*>(&w.sq[tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(&w.sk[tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      {
-        const int tt = tid >> 4, e = (tid & 15) * 4;
-        if (i0 + tt < T) cp_async16(&w.sv[tt][e], vc + ((size_t)(t0 + i0 + tt) * nv + h) * D + c0 + e);
-        else *reinterpret_cast<float4*>(&w.sv[tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      if (tid < C) {                       // gates: asynchronous too, nothing of the next chunk is waited for here
-        if (i0 + tid < T) {
-          gc_cp4(&w.sg[b][tid], gin + (size_t)(t0 + i0 + tid) * nv + h);
-          gc_cp4(&w.sb[b][tid], bin + (size_t)(t0 + i0 + tid) * nv + h);
-        } else {
-          w.sg[b][tid] = 0.f, w.sb[b][tid] = 0.f;                           // padding rows: no decay, no update
-        }
-      }
-      cp_async_commit();
-    };
-    if (first < chunks) stage(first * C, 0);
-    int b = 0;
-    for (int c = first; c < chunks; c += 2, b ^= 1) {
-      GcSlot& o = sm.slot[c % GC_SLOTS];
-      const bool ok = c < GC_SLOTS || mbar_wait(u32(&sm.empty[c % GC_SLOTS]), (uint32_t)(c / GC_SLOTS - 1) & 1u, abort_flag);
-      cp_async_wait<0>();
-      if (!meet(ok)) break;                // the chunk landed; this group's tiles and the slot are free
-      // running sums of the log-decays, recomputed where they are needed (16 broadcast reads)
-      float g_last = 0.f;
-#pragma unroll
-      for (int j = 0; j < C; ++j) g_last += w.sg[b][j];
-      if (tid == 0) o.g_last = g_last;
-      // ---- operand tiles (bf16) from the staged fp32 rows: thread = (token, 8 columns)
-      {
-        const int tt = tid >> 4, ch = tid & 15, e = ch * 8;
-        float gi = 0.f;
-        for (int j = 0; j <= tt; ++j) gi += w.sg[b][j];
-        const float eg = __expf(gi), beta = w.sb[b][tt], kbs = beta * eg;
-        const float4 q0 = *reinterpret_cast<const float4*>(&w.sq[tt][e]), q1 = *reinterpret_cast<const float4*>(&w.sq[tt][e + 4]);
-        const float4 k0 = *reinterpret_cast<const float4*>(&w.sk[tt][e]), k1 = *reinterpret_cast<const float4*>(&w.sk[tt][e + 4]);
-        const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        const float kv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
-        uint32_t oq[4], ok_[4], oqe[4], okb[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          oq[j] = f2_to_bf162_bits(qv[2 * j], qv[2 * j + 1]);
-          ok_[j] = f2_to_bf162_bits(kv[2 * j], kv[2 * j + 1]);
-          oqe[j] = f2_to_bf162_bits(qv[2 * j] * eg, qv[2 * j + 1] * eg);
-          okb[j] = f2_to_bf162_bits(kv[2 * j] * kbs, kv[2 * j + 1] * kbs);
-        }
-        const uint32_t off = gc_off(tt, ch);
-        *reinterpret_cast<uint4*>(w.qraw + off) = make_uint4(oq[0], oq[1], oq[2], oq[3]);
-        *reinterpret_cast<uint4*>(w.kraw + off) = make_uint4(ok_[0], ok_[1], ok_[2], ok_[3]);
-        *reinterpret_cast<uint4*>(o.qe + off) = make_uint4(oqe[0], oqe[1], oqe[2], oqe[3]);
-        *reinterpret_cast<uint4*>(w.kb + off) = make_uint4(okb[0], okb[1], okb[2], okb[3]);
-        if (ch < DV / 8) {
-          const float4 v0 = *reinterpret_cast<const float4*>(&w.sv[tt][e]), v1 = *reinterpret_cast<const float4*>(&w.sv[tt][e + 4]);
-          *reinterpret_cast<uint4*>(w.vb + gc_offv(tt, ch)) =
-              make_uint4(f2_to_bf162_bits(v0.x * beta, v0.y * beta), f2_to_bf162_bits(v0.z * beta, v0.w * beta),
-                         f2_to_bf162_bits(v1.x * beta, v1.y * beta), f2_to_bf162_bits(v1.z * beta, v1.w * beta));
-        }
-      }
-      {
-        // transposed decayed keys [dk][token]: thread = (dk row, 8 tokens), one 16-byte store
-        const int r = tid & 127, half = tid >> 7;
-        float gi = 0.f;
-        for (int j = 0; j < half * 8; ++j) gi += w.sg[b][j];
-        uint32_t ov[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          gi += w.sg[b][half * 8 + 2 * j];
-          const float x0 = w.sk[half * 8 + 2 * j][r] * __expf(g_last - gi);
-          gi += w.sg[b][half * 8 + 2 * j + 1];
-          const float x1 = w.sk[half * 8 + 2 * j + 1][r] * __expf(g_last - gi);
-          ov[j] = f2_to_bf162_bits(x0, x1);
-        }
-        *reinterpret_cast<uint4*>(o.kdt + (size_t)r * 32 + half * 16) = make_uint4(ov[0], ov[1], ov[2], ov[3]);
-      }
-      meet(true);
-      if (c + 2 < chunks) stage((c + 2) * C, b ^ 1);       // the fp32 rows have been read
-      // ---- warp 0: KK -> A -> T = (I + A)^-1;  warp 1: QK'
-      if (warp < 2) {
-        float gc[C];                         // inclusive running sums
-        {
-          float acc = 0.f;
-#pragma unroll
-          for (int j = 0; j < C; ++j) acc += w.sg[b][j], gc[j] = acc;
-        }
-        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        const uint32_t a_base = warp == 0 ? a_kraw : a_qraw;
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          uint32_t af[4], bfr[4];
-          gc_ldsm(af, a_base + gc_off(lrow, kk * 2 + (lane >> 4)));
-          gc_ldsm(bfr, a_kraw + gc_off((lane & 7) + (lane >> 4) * 8, kk * 2 + ((lane >> 3) & 1)));
-          gc_mma(acc[0], af, bfr[0], bfr[1]);
-          gc_mma(acc[1], af, bfr[2], bfr[3]);
-        }
-#pragma unroll
-        for (int n8 = 0; n8 < 2; ++n8)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = g8 + (e >> 1) * 8, j = n8 * 8 + t4 * 2 + (e & 1);
-            float gi_ = 0.f, gj_ = 0.f;
-#pragma unroll
-            for (int q = 0; q < C; ++q) gi_ = q == i ? gc[q] : gi_, gj_ = q == j ? gc[q] : gj_;
-            const float dec = j <= i ? __expf(gi_ - gj_) : 0.f;
-            if (warp == 0) w.a[i][j] = j < i ? w.sb[b][i] * acc[n8][e] * dec : 0.f;
-            else *reinterpret_cast<bf16*>(o.qkm + i * 32 + j * 2) = __float2bfloat16(acc[n8][e] * dec);
-          }
-        if (warp == 0) {
-          __syncwarp();
-          if (lane < C) {                    // lane j solves column j of T by forward substitution
-            float tcol[C];
-#pragma unroll
-            for (int i = 0; i < C; ++i) {
-              float v = i == lane ? 1.f : 0.f;
-#pragma unroll
-              for (int m = 0; m < i; ++m) v -= w.a[i][m] * tcol[m];
-              tcol[i] = i < lane ? 0.f : v;
-            }
-#pragma unroll
-            for (int i = 0; i < C; ++i) {
-              const bf16 hi = __float2bfloat16(tcol[i]);
-              *reinterpret_cast<bf16*>(w.t_hi + i * 32 + lane * 2) = hi;
-              *reinterpret_cast<bf16*>(w.t_lo + i * 32 + lane * 2) = __float2bfloat16(tcol[i] - __bfloat162float(hi));
-            }
-          }
-        }
-      }
-      meet(true);
-      // ---- W = T (K beta e^G) over all of dk (16 columns per warp); U = T (V beta), this warp's 8 value columns
-      {
-        float U[4] = {0.f, 0.f, 0.f, 0.f};
-        float Wf[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        uint32_t thi[4], tlo[4], bk[4], bv[2];
-        const uint32_t trow = (uint32_t)(lrow * 32 + (lane >> 4) * 16);
-        gc_ldsm(thi, a_thi + trow);
-        gc_ldsm(tlo, a_tlo + trow);
-        gc_ldsm_t(bk, a_kb + gc_off(lrow, 2 * warp + (lane >> 4)));
-        gc_ldsm2_t(bv, a_vb + gc_offv(lrow, warp));
-        gc_mma(Wf[0], thi, bk[0], bk[1]), gc_mma(Wf[1], thi, bk[2], bk[3]);
-        gc_mma(Wf[0], tlo, bk[0], bk[1]), gc_mma(Wf[1], tlo, bk[2], bk[3]);
-        gc_mma(U, thi, bv[0], bv[1]);
-        gc_mma(U, tlo, bv[0], bv[1]);
-#pragma unroll
-        for (int n8 = 0; n8 < 2; ++n8) {
-          *reinterpret_cast<uint32_t*>(o.ws + gc_off(g8, 2 * warp + n8) + t4 * 4) = f2_to_bf162_bits(Wf[n8][0], Wf[n8][1]);
-          *reinterpret_cast<uint32_t*>(o.ws + gc_off(g8 + 8, 2 * warp + n8) + t4 * 4) = f2_to_bf162_bits(Wf[n8][2], Wf[n8][3]);
-        }
-        o.u[tid] = make_float4(U[0], U[1], U[2], U[3]);
-      }
-      mbar_arrive(u32(&sm.full[c % GC_SLOTS]));
     }
-    // ---- conv ring refresh for the last tokens (as the token-serial scan does)
-    if (group == 2 && c0 == 0) {
-      const int cw = 2 * nk * D + nv * D;
-      bf16* rg = ring + (size_t)slot * ring_slot_stride;
-      const int rep = nv / nk;
-      for (int i = max(0, T - RING); i < T; ++i) {
-        const int t = t0 + i;
-        const bf16* src = inp + (size_t)t * ld;
-        bf16* dst = rg + (size_t)(positions[t] % RING) * cw;
-        if (h % rep == 0) {
-          for (int c = tid; c < 2 * D; c += GC_GROUP) {
-            const int cc = (c < D) ? kh * D + c : nk * D + kh * D + (c - D);
-            dst[cc] = src[cc];
+    {
+      const int tt = tid >> 4, e = (tid & 15) * 4;
+      if (i0 + tt < T) cp_async16(&w.sv[tt][e], vc + ((size_t)(t0 + i0 + tt) * nv + h) * D + c0 + e);
+      else *reinterpret_cast<float4*>(&w.sv[tt][e]) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (tid < C) {                       // gates: asynchronous too, nothing of the next chunk is waited for here
+      if (i0 + tid < T) {
+        gc_cp4(&w.sg[b][tid], gin + (size_t)(t0 + i0 + tid) * nv + h);
+        gc_cp4(&w.sb[b][tid], bin + (size_t)(t0 + i0 + tid) * nv + h);
+      } else {
+        w.sg[b][tid] = 0.f, w.sb[b][tid] = 0.f;                           // padding rows: no decay, no update
+      }
+    }
+    cp_async_commit();
+  };
+  // chunk c, staged in buffer b, into slot o; starts the loads of this group's next chunk
+  auto prepare = [&](int c, int b, GcSlot& o) {
+    const uint32_t a_qraw = u32(w.qraw), a_kraw = u32(w.kraw), a_kb = u32(w.kb), a_vb = u32(w.vb), a_thi = u32(w.t_hi), a_tlo = u32(w.t_lo);
+    // running sums of the log-decays, recomputed where they are needed (16 broadcast reads)
+    float g_last = 0.f;
+#pragma unroll
+    for (int j = 0; j < C; ++j) g_last += w.sg[b][j];
+    if (tid == 0) o.g_last = g_last;
+    // ---- operand tiles (bf16) from the staged fp32 rows: thread = (token, 8 columns)
+    {
+      const int tt = tid >> 4, ch = tid & 15, e = ch * 8;
+      float gi = 0.f;
+      for (int j = 0; j <= tt; ++j) gi += w.sg[b][j];
+      const float eg = __expf(gi), beta = w.sb[b][tt], kbs = beta * eg;
+      const float4 q0 = *reinterpret_cast<const float4*>(&w.sq[tt][e]), q1 = *reinterpret_cast<const float4*>(&w.sq[tt][e + 4]);
+      const float4 k0 = *reinterpret_cast<const float4*>(&w.sk[tt][e]), k1 = *reinterpret_cast<const float4*>(&w.sk[tt][e + 4]);
+      const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+      const float kv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+      uint32_t oq[4], ok_[4], oqe[4], okb[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        oq[j] = f2_to_bf162_bits(qv[2 * j], qv[2 * j + 1]);
+        ok_[j] = f2_to_bf162_bits(kv[2 * j], kv[2 * j + 1]);
+        oqe[j] = f2_to_bf162_bits(qv[2 * j] * eg, qv[2 * j + 1] * eg);
+        okb[j] = f2_to_bf162_bits(kv[2 * j] * kbs, kv[2 * j + 1] * kbs);
+      }
+      const uint32_t off = gc_off(tt, ch);
+      *reinterpret_cast<uint4*>(w.qraw + off) = make_uint4(oq[0], oq[1], oq[2], oq[3]);
+      *reinterpret_cast<uint4*>(w.kraw + off) = make_uint4(ok_[0], ok_[1], ok_[2], ok_[3]);
+      *reinterpret_cast<uint4*>(o.qe + off) = make_uint4(oqe[0], oqe[1], oqe[2], oqe[3]);
+      *reinterpret_cast<uint4*>(w.kb + off) = make_uint4(okb[0], okb[1], okb[2], okb[3]);
+      if (ch < DV / 8) {
+        const float4 v0 = *reinterpret_cast<const float4*>(&w.sv[tt][e]), v1 = *reinterpret_cast<const float4*>(&w.sv[tt][e + 4]);
+        *reinterpret_cast<uint4*>(w.vb + gc_offv(tt, ch)) =
+            make_uint4(f2_to_bf162_bits(v0.x * beta, v0.y * beta), f2_to_bf162_bits(v0.z * beta, v0.w * beta),
+                       f2_to_bf162_bits(v1.x * beta, v1.y * beta), f2_to_bf162_bits(v1.z * beta, v1.w * beta));
+      }
+    }
+    {
+      // transposed decayed keys [dk][token]: thread = (dk row, 8 tokens), one 16-byte store
+      const int r = tid & 127, half = tid >> 7;
+      float gi = 0.f;
+      for (int j = 0; j < half * 8; ++j) gi += w.sg[b][j];
+      uint32_t ov[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        gi += w.sg[b][half * 8 + 2 * j];
+        const float x0 = w.sk[half * 8 + 2 * j][r] * __expf(g_last - gi);
+        gi += w.sg[b][half * 8 + 2 * j + 1];
+        const float x1 = w.sk[half * 8 + 2 * j + 1][r] * __expf(g_last - gi);
+        ov[j] = f2_to_bf162_bits(x0, x1);
+      }
+      *reinterpret_cast<uint4*>(o.kdt + (size_t)r * 32 + half * 16) = make_uint4(ov[0], ov[1], ov[2], ov[3]);
+    }
+    meet(true);
+    if (c + Smem::PRE < chunks) stage((c + Smem::PRE) * C, b ^ 1);       // the fp32 rows have been read
+    // ---- warp 0: KK -> A -> T = (I + A)^-1;  warp 1: QK'
+    if (warp < 2) {
+      float gc[C];                         // inclusive running sums
+      {
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < C; ++j) acc += w.sg[b][j], gc[j] = acc;
+      }
+      float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      const uint32_t a_base = warp == 0 ? a_kraw : a_qraw;
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) {
+        uint32_t af[4], bfr[4];
+        gc_ldsm(af, a_base + gc_off(lrow, kk * 2 + (lane >> 4)));
+        gc_ldsm(bfr, a_kraw + gc_off((lane & 7) + (lane >> 4) * 8, kk * 2 + ((lane >> 3) & 1)));
+        gc_mma(acc[0], af, bfr[0], bfr[1]);
+        gc_mma(acc[1], af, bfr[2], bfr[3]);
+      }
+#pragma unroll
+      for (int n8 = 0; n8 < 2; ++n8)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = g8 + (e >> 1) * 8, j = n8 * 8 + t4 * 2 + (e & 1);
+          float gi_ = 0.f, gj_ = 0.f;
+#pragma unroll
+          for (int q = 0; q < C; ++q) gi_ = q == i ? gc[q] : gi_, gj_ = q == j ? gc[q] : gj_;
+          const float dec = j <= i ? __expf(gi_ - gj_) : 0.f;
+          if (warp == 0) w.a[i][j] = j < i ? w.sb[b][i] * acc[n8][e] * dec : 0.f;
+          else *reinterpret_cast<bf16*>(o.qkm + i * 32 + j * 2) = __float2bfloat16(acc[n8][e] * dec);
+        }
+      if (warp == 0) {
+        __syncwarp();
+        if (lane < C) {                    // lane j solves column j of T by forward substitution
+          float tcol[C];
+#pragma unroll
+          for (int i = 0; i < C; ++i) {
+            float v = i == lane ? 1.f : 0.f;
+#pragma unroll
+            for (int m = 0; m < i; ++m) v -= w.a[i][m] * tcol[m];
+            tcol[i] = i < lane ? 0.f : v;
+          }
+#pragma unroll
+          for (int i = 0; i < C; ++i) {
+            const bf16 hi = __float2bfloat16(tcol[i]);
+            *reinterpret_cast<bf16*>(w.t_hi + i * 32 + lane * 2) = hi;
+            *reinterpret_cast<bf16*>(w.t_lo + i * 32 + lane * 2) = __float2bfloat16(tcol[i] - __bfloat162float(hi));
           }
         }
-        for (int c = tid; c < D; c += GC_GROUP) {
-          const int cc = 2 * nk * D + h * D + c;
+      }
+    }
+    meet(true);
+    // ---- W = T (K beta e^G) over all of dk (16 columns per warp); U = T (V beta), this warp's 8 value columns
+    {
+      float U[4] = {0.f, 0.f, 0.f, 0.f};
+      float Wf[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      uint32_t thi[4], tlo[4], bk[4], bv[2];
+      const uint32_t trow = (uint32_t)(lrow * 32 + (lane >> 4) * 16);
+      gc_ldsm(thi, a_thi + trow);
+      gc_ldsm(tlo, a_tlo + trow);
+      gc_ldsm_t(bk, a_kb + gc_off(lrow, 2 * warp + (lane >> 4)));
+      gc_ldsm2_t(bv, a_vb + gc_offv(lrow, warp));
+      gc_mma(Wf[0], thi, bk[0], bk[1]), gc_mma(Wf[1], thi, bk[2], bk[3]);
+      gc_mma(Wf[0], tlo, bk[0], bk[1]), gc_mma(Wf[1], tlo, bk[2], bk[3]);
+      gc_mma(U, thi, bv[0], bv[1]);
+      gc_mma(U, tlo, bv[0], bv[1]);
+#pragma unroll
+      for (int n8 = 0; n8 < 2; ++n8) {
+        *reinterpret_cast<uint32_t*>(o.ws + gc_off(g8, 2 * warp + n8) + t4 * 4) = f2_to_bf162_bits(Wf[n8][0], Wf[n8][1]);
+        *reinterpret_cast<uint32_t*>(o.ws + gc_off(g8 + 8, 2 * warp + n8) + t4 * 4) = f2_to_bf162_bits(Wf[n8][2], Wf[n8][3]);
+      }
+      o.u[tid] = make_float4(U[0], U[1], U[2], U[3]);
+    }
+  };
+  // conv ring refresh for the last tokens (as the token-serial scan does)
+  auto refresh = [&]() {
+    if (c0 != 0) return;
+    const int cw = 2 * nk * D + nv * D;
+    bf16* rg = ring + (size_t)slot * ring_slot_stride;
+    const int rep = nv / nk;
+    for (int i = max(0, T - RING); i < T; ++i) {
+      const int t = t0 + i;
+      const bf16* src = inp + (size_t)t * ld;
+      bf16* dst = rg + (size_t)(positions[t] % RING) * cw;
+      if (h % rep == 0) {
+        for (int c = tid; c < 2 * D; c += GC_GROUP) {
+          const int cc = (c < D) ? kh * D + c : nk * D + kh * D + (c - D);
           dst[cc] = src[cc];
         }
       }
+      for (int c = tid; c < D; c += GC_GROUP) {
+        const int cc = 2 * nk * D + h * D + c;
+        dst[cc] = src[cc];
+      }
     }
+  };
+  bool good = true;
+  if (group > 0) {
+    // ---------------- preparing groups ----------------
+    if (first < chunks) stage(first * C, 0);
+    int b = 0;
+    for (int c = first; c < chunks; c += 2, b ^= 1) {
+      const bool ok = c < SLOTS || mbar_wait(u32(&sm.empty[c % SLOTS]), (uint32_t)(c / SLOTS - 1) & 1u, abort_flag);
+      cp_async_wait<0>();
+      if (!meet(ok)) break;                // the chunk landed; this group's tiles and the slot are free
+      prepare(c, b, sm.slot[c % SLOTS]);
+      mbar_arrive(u32(&sm.full[c % SLOTS]));
+    }
+    if (group == 2) refresh();
   } else {
     // ---------------- the state: rows 16 warp .. 16 warp + 15, this CTA's 64 columns, as accumulator fragments ----------------
+    if (!PIPE) stage(0, 0);
     float* sp = states + (size_t)slot * state_slot_stride + (size_t)h * D * D + (size_t)cur[slot] * plane_stride + c0;
     const uint32_t a_vn = u32(sm.vn), a_sbf = u32(sm.sbf);
     float S[DV / 8][4];
@@ -1121,12 +1134,9 @@ gdn_chunk_mma_kernel(const float* qn, const float* kn, const float* vc, const fl
       }
     };
     store_sbf();
-    bool good = true;
-    for (int c = 0; c < chunks; ++c) {
-      const GcSlot& o = sm.slot[c % GC_SLOTS];
+    auto advance = [&](int c) {
+      const GcSlot& o = sm.slot[c % SLOTS];
       const uint32_t a_qe = u32(o.qe), a_ws = u32(o.ws), a_kdt = u32(o.kdt), a_qkm = u32(o.qkm);
-      good = meet(mbar_wait(u32(&sm.full[c % GC_SLOTS]), (uint32_t)(c / GC_SLOTS) & 1u, abort_flag));   // and: the state's copy is whole
-      if (!good) break;
       // ---- O = (Q e^G) S and V' = U - W S, this warp's 8 value columns of both
       float O[4] = {0.f, 0.f, 0.f, 0.f}, acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -1161,12 +1171,24 @@ gdn_chunk_mma_kernel(const float* qn, const float* kn, const float* vc, const fl
         }
         store_sbf();
         gc_mma(O, aq, bvn[0], bvn[1]);
-        mbar_arrive(u32(&sm.empty[c % GC_SLOTS]));
+        if (PIPE) mbar_arrive(u32(&sm.empty[c % SLOTS]));
         const int i0 = c * C;
         float* orow = o_scratch + ((size_t)(t0 + i0) * nv + h) * D + c0 + 8 * warp + t4 * 2;
         if (i0 + g8 < T) *reinterpret_cast<float2*>(orow + (size_t)g8 * nv * D) = make_float2(O[0], O[1]);
         if (i0 + g8 + 8 < T) *reinterpret_cast<float2*>(orow + (size_t)(g8 + 8) * nv * D) = make_float2(O[2], O[3]);
       }
+    };
+    for (int c = 0; c < chunks; ++c) {
+      if (PIPE) {
+        good = meet(mbar_wait(u32(&sm.full[c % SLOTS]), (uint32_t)(c / SLOTS) & 1u, abort_flag));   // and: the state's copy is whole
+        if (!good) break;
+      } else {
+        cp_async_wait<0>();
+        meet(true);                          // the chunk landed; the last chunk's tiles have been read
+        prepare(c, c & 1, sm.slot[0]);
+        meet(true);                          // the slot and the state's copy are whole
+      }
+      advance(c);
     }
     // ---- state back to its plane
     if (good) {
@@ -1176,6 +1198,7 @@ gdn_chunk_mma_kernel(const float* qn, const float* kn, const float* vc, const fl
         *reinterpret_cast<float2*>(sp + (size_t)(16 * warp + g8 + 8) * D + nt * 8 + t4 * 2) = make_float2(S[nt][2], S[nt][3]);
       }
     }
+    if (!PIPE) refresh();
   }
   trl_trace_end();
 }
@@ -1563,14 +1586,25 @@ TRL_API void trl_gdn_set_wy(int on) { g_gdn_wy = on ? 1 : 0; }
 // Prefill scan on the tensor cores (gdn_chunk_mma_kernel): 1 on, 0 off (token-serial scan), -1 = the environment's choice.
 TRL_API void trl_gdn_set_mma(int on) { g_gdn_mma = on; }
 
+// Whether the chunk kernel does without preparing groups: with that many blocks that three an SM are worth more than chunks
+// prepared ahead, and the longest sequence no longer than it takes the others to go through the SMs.  us a layer with its
+// preparation, with groups and without (48 heads): 3 x 24 tokens 35.3 and 34.2, 4 x 24 45.7 and 38.0, 16 x 24 149 and 122, 9 x 64
+// 128 and 110, 31 of one token and one of 100 159 and 149, 3 and one of 100 47.8 and 63.0, 6 and 3 x 330 182 and 205.  What lies
+// between one and two blocks an SM is slower than two blocks of 256 threads an SM were (3 x 37 tokens 39 us, 37 then).
+static bool gc_serial(int B, int nv, int longest, int sms) {
+  const long ctas = (long)nv * GC_NS * B;
+  return longest > 0 && 4 * ctas > 9L * sms && (long)(longest + GC_C - 1) / GC_C * sms <= ctas;
+}
+
 // Scratch (fp32): qn, kn [T*nk*D]; vc, o_scratch [T*nv*D]; g, beta [T*nv].
-TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_bias, const void* a_log,
-                    const void* norm_w, void* states, void* cur, void* ring, const void* positions,
-                    const void* seq_ids, const void* q_start, const void* q_len,
-                    const void* state_slots, const void* keep_flags, long state_slot_stride,
-                    long plane_stride, long ring_slot_stride, void* qn, void* kn, void* vc, void* g,
-                    void* beta, void* o_scratch, void* out, int T, int B, int nk, int nv, int D, int KW,
-                    int planes, float eps, void* stream) {
+// longest: tokens of the longest sequence (0: not known); form of the chunk kernel: 0 with preparing groups, 1 without, -1 by rule.
+TRL_API int trl_gdn_form(const void* inp, int ld, const void* conv_w, const void* dt_bias, const void* a_log,
+                         const void* norm_w, void* states, void* cur, void* ring, const void* positions,
+                         const void* seq_ids, const void* q_start, const void* q_len,
+                         const void* state_slots, const void* keep_flags, long state_slot_stride,
+                         long plane_stride, long ring_slot_stride, void* qn, void* kn, void* vc, void* g,
+                         void* beta, void* o_scratch, void* out, int T, int B, int nk, int nv, int D, int KW,
+                         int planes, float eps, int longest, int form, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   if (KW > 4) return (int)cudaErrorInvalidValue;
   if ((D != 64 && D != 128) || (ld % 2) != 0) return (int)cudaErrorInvalidValue;
@@ -1618,16 +1652,22 @@ TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_
   // tensor-core chunk kernel; TRL_GDN_MMA=0 (or trl_gdn_set_mma(0)) falls back to the token-serial scan
   if (g_gdn_mma < 0) g_gdn_mma = (getenv("TRL_GDN_MMA") && atoi(getenv("TRL_GDN_MMA")) == 0) ? 0 : 1;
   if (g_gdn_mma != 0 && D == 128 && T > B && keep_flags == nullptr) {
-    static bool configured = false;
-    if (!configured) {
-      if (cudaFuncSetAttribute(gdn_chunk_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GcSmem)) != cudaSuccess)
-        return 3;
-      configured = true;
-    }
-    e = trl_launch(gdn_chunk_mma_kernel, dim3(nv * GC_NS, B), dim3(GC_THREADS), sizeof(GcSmem), st, (const float*)qn,
-                   (const float*)kn, (const float*)vc, (const float*)g, (const float*)beta, (float*)states, (int*)cur,
-                   (bf16*)ring, (const bf16*)inp, ld, (const int*)q_start, (const int*)q_len, (const int*)positions,
-                   (const int*)state_slots, state_slot_stride, plane_stride, ring_slot_stride, (float*)o_scratch, nk, nv);
+    const bool serial = form >= 0 ? form == 1 : gc_serial(B, nv, longest, num_sms());
+#define CHUNK(PIPE)                                                                                                              \
+  {                                                                                                                              \
+    auto kern = gdn_chunk_mma_kernel<PIPE>;                                                                                      \
+    static bool configured = false;                                                                                              \
+    if (!configured) {                                                                                                           \
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GcSmem<PIPE>)) != cudaSuccess) return 3; \
+      configured = true;                                                                                                         \
+    }                                                                                                                            \
+    e = trl_launch(kern, dim3(nv * GC_NS, B), dim3(GcSmem<PIPE>::THREADS), sizeof(GcSmem<PIPE>), st, (const float*)qn,           \
+                   (const float*)kn, (const float*)vc, (const float*)g, (const float*)beta, (float*)states, (int*)cur,           \
+                   (bf16*)ring, (const bf16*)inp, ld, (const int*)q_start, (const int*)q_len, (const int*)positions,             \
+                   (const int*)state_slots, state_slot_stride, plane_stride, ring_slot_stride, (float*)o_scratch, nk, nv);       \
+  }
+    if (serial) CHUNK(false) else CHUNK(true)
+#undef CHUNK
     if (e != cudaSuccess) return (int)e;
     return (int)trl_launch(gdn_gated_norm_kernel, dim3((T * nv + 7) / 8), dim3(256), 0, st, (const float*)o_scratch,
                            (const bf16*)inp, ld, (const float*)norm_w, eps, (bf16*)out, T * nv, nk, nv);
@@ -1655,6 +1695,17 @@ TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_
 #undef SCAN
 #undef SCANWY
   return (int)e;
+}
+
+TRL_API int trl_gdn(const void* inp, int ld, const void* conv_w, const void* dt_bias, const void* a_log,
+                    const void* norm_w, void* states, void* cur, void* ring, const void* positions,
+                    const void* seq_ids, const void* q_start, const void* q_len,
+                    const void* state_slots, const void* keep_flags, long state_slot_stride,
+                    long plane_stride, long ring_slot_stride, void* qn, void* kn, void* vc, void* g,
+                    void* beta, void* o_scratch, void* out, int T, int B, int nk, int nv, int D, int KW,
+                    int planes, float eps, void* stream) {
+  return trl_gdn_form(inp, ld, conv_w, dt_bias, a_log, norm_w, states, cur, ring, positions, seq_ids, q_start, q_len, state_slots, keep_flags, state_slot_stride, plane_stride, ring_slot_stride,
+                      qn, kn, vc, g, beta, o_scratch, out, T, B, nk, nv, D, KW, planes, eps, 0, -1, stream);
 }
 
 // Decode tick of a Gated-DeltaNet layer in ONE launch: every sequence carries exactly one token

@@ -662,3 +662,38 @@ def test_prefill_attention_forms(ops, g_heads, fp8, form):
         want = (want * torch.sigmoid(gate[rows].double().view(n, n_q, 2, d)[:, :, 1])).reshape(n, -1)
         assert _rel(out[rows], want) < 2 ** -7, (n, h, _rel(out[rows], want))
     assert N.read_error()[0] == 0
+
+
+@pytest.mark.parametrize("lens", [[2], [16, 1], [17, 1, 15], [33, 2, 1, 48, 31, 100], [1] * 40 + [2]])
+@pytest.mark.parametrize("nk,nv", [(2, 2), (1, 3)])
+def test_delta_rule_chunk_kernel_with_and_without_preparing_groups(ops, lens, nk, nv):
+    """The two forms of the chunk kernel take the same steps in the same order: the same bits in outputs, states and ring,
+    over one chunk, a slot's reuse, rows that fill no chunk and sequences of one token."""
+    from tilerl_b200.batch import Batch
+    from tilerl_b200.config import GDN, ModelConfig
+    from tilerl_b200.kv import GdnStatePool
+    from tilerl_b200.ops import native as N
+    d = 128
+    cfg = ModelConfig("t", hidden=64, ffn=64, vocab=64, layer_types=(GDN,), n_q_heads=2, n_kv_heads=1, head_dim=64, rotary_dim=64,
+                      rope_theta=1e6, gdn_k_heads=nk, gdn_v_heads=nv, gdn_head_dim=d)
+    g = torch.Generator().manual_seed(sum(lens) + nv)
+    lp = dict(conv=(torch.randn(cfg.gdn_conv_dim, 4, generator=g) * 0.3).to(DEV), dt_bias=torch.rand(nv, generator=g).to(DEV),
+              a_log=torch.log(1 + 3 * torch.rand(nv, generator=g)).to(DEV), gdn_norm=(1 + 0.1 * torch.randn(d, generator=g)).to(DEV))
+    batch = Batch.build([dict(tokens=[0] * n, start=7, blocks=list(range(1 + 8 * i, 9 + 8 * i)), slot=i + 1) for i, n in enumerate(lens)], DEV)
+    inp = torch.randn(batch.n_tokens, cfg.gdn_in_rows, generator=g).to(DEV, torch.bfloat16)
+    got = []
+    try:
+        for form in (0, 1, -1):
+            pool = GdnStatePool(cfg, len(lens) + 1, DEV, planes=1, ring_dtype=torch.bfloat16)
+            for i, x in enumerate((pool.states, pool.ring)):
+                x.copy_(torch.randn(x.shape, generator=torch.Generator().manual_seed(i)))
+            before = pool.states.clone()
+            ops.gdn_form = form
+            out = ops.gdn(inp, lp, batch, pool, 0, cfg, nk, nv).clone()
+            got.append((out, pool.states.clone(), pool.ring.clone()))
+    finally:
+        ops.gdn_form = -1
+    assert not torch.equal(got[0][1], before) and N.read_error()[0] == 0
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert torch.equal(a, b)

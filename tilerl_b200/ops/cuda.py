@@ -117,6 +117,7 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
         # register-streamed kernels on the checkpoint layout)
         self.gemv_stream = os.environ.get("TRL_GEMV_STREAM", "1") != "0"
         self.prefill_attn = os.environ.get("TRL_PREFILL_ATTN", "1") != "0"   # tiled kernel for q_len >= 16
+        self.gdn_form = -1            # chunk kernel of prompt ticks: -1 by rule, 0 with preparing groups of warps, 1 without
         self.gdn_fused_decode = os.environ.get("TRL_GDN_FUSED", "1") != "0"    # decode ticks: prep inside the scan kernel
         from .. import tape as _tape
         _tape.set_dequant(self.dequantize_nvfp4)   # frozen-base linears of the training forward
@@ -583,7 +584,7 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
                 cfg.gdn_conv, cfg.rms_eps, N.stream()), "gdn_decode")
             N.count()
             return out
-        N.check(self.lib.trl_gdn(
+        N.check(self.lib.trl_gdn_form(
             inp.data_ptr(), inp.stride(0), self._f32(lp["conv"]).data_ptr(),
             self._f32(lp["dt_bias"]).data_ptr(), self._f32(lp["a_log"]).data_ptr(),
             self._f32(lp["gdn_norm"]).data_ptr(), s_l.data_ptr(), spool.cur.data_ptr(), r_l.data_ptr(),
@@ -592,7 +593,7 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
             states.stride(0), states.stride(2), ring.stride(0),
             qn.data_ptr(), kn.data_ptr(), vc.data_ptr(), g.data_ptr(), beta.data_ptr(), osc.data_ptr(),
             out.data_ptr(), t, batch.n_seqs, nk, nv, d, cfg.gdn_conv, spool.planes, cfg.rms_eps,
-            N.stream()), "gdn")
+            batch.max_q_len, self.gdn_form, N.stream()), "gdn")
         N.count(2)
         return out
 
