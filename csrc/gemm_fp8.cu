@@ -86,7 +86,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   const int n_work = p.n_tiles * p.t_tiles;
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int st = 0;
       uint32_t ph = 0;
       long issued = 0;
@@ -114,7 +114,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     pdl_wait();
-    if (lane == 0) {
+    if (elect_one()) {
       // dense f8f6f4: fp32 accumulator, e4m3 x e4m3, both K-major, N = F8_BN, M = 128
       constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(F8_BN >> 3) << 17) | ((uint32_t)(F8_TILE >> 4) << 24);
       const uint64_t d0 = desc_sw128(smem_u32(smem));

@@ -463,7 +463,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const int n_units = (int)(u1 - u0);
       const uint32_t smem_a0 = smem_u32(smem), smem_b0 = smem_u32(smem_b);
       // two cursors over the same unit sequence: weights run up to SA units ahead of the MMA,
@@ -557,7 +557,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     pdl_wait();
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TILE_N >> 4) << 24);
       long long u = u0;
       int it = 0, seg = 0, sa_i = 0, sb_i = 0;

@@ -77,7 +77,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int st = 0;
       uint32_t ph = 0;
       long issued = 0;
@@ -98,7 +98,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t d0 = desc_sw128(smem_u32(smem));
       const uint32_t lo0 = (uint32_t)d0, hi = (uint32_t)(d0 >> 32);
       int st = 0, count = 0;

@@ -12,6 +12,17 @@ constexpr int TC_SF_ATOM = 512;                     // bytes: 128 rows x 4 scale
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// True in one lane of a converged warp, always the same one.  tcgen05, TMA and bulk-copy instructions take their operands from
+// uniform registers.  Behind `lane == 0` the compiler does not know that one lane is left and spends 45 clocks an instruction
+// on moving them there; behind elect.sync a scale copy issues in 8 and an NVFP4 MMA of 16 columns in 39.  A k-tile of 12 scale
+// copies and four MMAs of 256 columns takes 873 clocks the one way and 512, the MMAs alone, the other; 8 copies and four MMAs
+// of 32 columns 589 and 224 (a loop of nothing else, one CTA an SM).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
