@@ -1,0 +1,24 @@
+// The NVFP4 GEMM's form for many activation columns (gemm_pair.cu), as gemm_tc.cu calls it.
+#pragma once
+#include <stdint.h>
+#include <cuda_runtime.h>
+
+struct GemmPairArgs {
+  const void* wq;        // weights, [N, K/2] or tile-contiguous (w_tiled)
+  const void* sfw;       // weight scales, tiled
+  const float* tscale;
+  const void* xq;        // [tokens * 2, K/2]
+  const void* sfx;       // activation scales, tiled
+  const float* rs;       // [tokens * 2]
+  const void* residual;  // bf16 [tokens, ldr]
+  void* out;
+  int ldr, ldo, tokens, J, N, K, epi, w_tiled;
+  int pairs;             // pairs of SMs there are
+  int parts;             // pairs that share a tile, each a part of K
+};
+
+// Launches it with `bn` (128 or 192) columns a tile.
+int gemm_pair_launch(const GemmPairArgs& a, int bn, cudaStream_t stream);
+
+// Clusters of `parts` pairs that fit the GPU at a time.
+int gemm_pair_clusters(int parts);

@@ -33,6 +33,9 @@
 //   byte offset = ((row/128) * KT4 + k64) * 512 + (row%32)*16 + ((row%128)/32)*4 + (k16%4)
 // so that one k-tile of a 128-row atom is 2 KB contiguous.
 //
+// Most products go to the form on pairs of SMs (gemm_pair.cu), which this file's launcher picks: the kernel here serves tiles
+// split over CTAs as asked for, more than four terms, and outputs that 16-byte stores do not fit.
+//
 // No counterpart exists in the reference: its Blackwell kernel cell is empty
 // (packages/tilerl-kernels/src/tilerl_kernels/registry.py:188-189); functionally this
 // replaces linear_fp4_fp8 / linear_fp4_gemv / linear_fp4_mma8 (kernels_linear.py:924-1687).
@@ -41,6 +44,7 @@
 
 #include "common.cuh"
 #include "tcgen05.cuh"
+#include "gemm_pair.cuh"
 
 namespace {
 
@@ -99,22 +103,6 @@ __device__ __forceinline__ void epi_store(const GemmParams& p, int tok, int n, i
   }
 }
 
-// The finished values of one row and up to 128 tokens, out.
-template <int V, int EPI>
-__device__ __forceinline__ void store_values(const GemmParams& p, const float (&v)[V], int tok, int n, int lane) {
-  constexpr int GRP = V < 16 ? V : 16;
-#pragma unroll
-  for (int c = 0; c < V; c += GRP) {
-    float res[GRP];
-#pragma unroll
-    for (int t = 0; t < GRP; ++t)                // issued before any store of these tokens
-      res[t] = (EPI == EPI_RESIDUAL && tok + c + t < p.tokens && n < p.N)
-                   ? __bfloat162float(p.residual[(size_t)(tok + c + t) * p.ldr + n]) : 0.f;
-#pragma unroll
-    for (int t = 0; t < GRP; ++t) epi_store<EPI>(p, tok + c + t, n, lane, v[c + t], res[t]);
-  }
-}
-
 // Epilogue of one accumulator tile: TMEM -> registers in chunks of CH columns, J columns summed per token with their activation
 // scales, then either the final store (WHOLE) or this CTA's split-K slot.  tok_first = first token of the tile; slot_row =
 // slot + row.
@@ -149,103 +137,9 @@ __device__ __forceinline__ void epilogue_chunks(const GemmParams& p, uint32_t ta
   }
 }
 
-// The same for a whole tile that this CTA's next one follows: up to 128 tokens a thread into registers, the accumulator given
-// back, and only then the stores, which the next tile's MMAs run beside.  With the stores between the TMEM reads the tensor
-// cores stood still for 5 (plain), 8 (SwiGLU) and 20 us (residual) a tile of 256 columns, against 14 for its 20 k-tiles.
-// 2000 tokens, 34 816 x 5120 SwiGLU 677 -> 542 us; 5120 x 6144 residual 189 -> 126.
 template <int BN, int J>
-__device__ __forceinline__ void epilogue_ahead(const GemmParams& p, uint32_t taddr0, const float* rs_s, float ts,
-                                               int tok_first, int n, int lane, uint32_t accum_empty) {
-  constexpr int CH = BN >= 32 ? 32 : 16, TPC = CH / J, V = BN / J < 128 ? BN / J : 128;
-#pragma unroll 1
-  for (int t0 = 0; t0 < BN / J; t0 += V) {
-    float v[V];
-#pragma unroll
-    for (int c = 0; c < V / TPC; ++c) {
-      uint32_t r[32];
-      const int col = t0 * J + c * CH;
-      if (CH == 32) tc_ld32(taddr0 + (uint32_t)col, r); else tc_ld16(taddr0 + (uint32_t)col, r);
-      tc_wait_ld();
-#pragma unroll
-      for (int t = 0; t < TPC; ++t) {
-        float a = 0.f;
-#pragma unroll
-        for (int j = 0; j < J; ++j) a = fmaf(__uint_as_float(r[t * J + j]), rs_s[col + t * J + j], a);
-        v[c * TPC + t] = a * ts;
-      }
-    }
-    if (t0 + V >= BN / J) {
-      tc_fence_before();
-      mbar_arrive(accum_empty);
-    }
-    if (p.epi == EPI_SWIGLU) {
-      store_values<V, EPI_SWIGLU>(p, v, tok_first + t0, n, lane);
-    } else if (p.epi == EPI_RESIDUAL) {
-      store_values<V, EPI_RESIDUAL>(p, v, tok_first + t0, n, lane);
-    } else {
-      store_values<V, EPI_STORE_F32>(p, v, tok_first + t0, n, lane);
-    }
-  }
-}
-
-// Plain bf16 results wait in registers as pairs: half as many.  2000 tokens, 20 000 x 2048: 171 us as fp32, 143 here.
-template <int BN, int J>
-__device__ __forceinline__ void epilogue_ahead_bf16(const GemmParams& p, uint32_t taddr0, const float* rs_s, float ts,
-                                                    int tok_first, int n, uint32_t accum_empty) {
-  constexpr int CH = BN >= 32 ? 32 : 16, TPC = CH / J, V = BN / J < 128 ? BN / J : 128;
-#pragma unroll 1
-  for (int t0 = 0; t0 < BN / J; t0 += V) {
-    uint32_t pk[V / 2];
-#pragma unroll
-    for (int c = 0; c < V / TPC; ++c) {
-      uint32_t r[32];
-      const int col = t0 * J + c * CH;
-      if (CH == 32) tc_ld32(taddr0 + (uint32_t)col, r); else tc_ld16(taddr0 + (uint32_t)col, r);
-      tc_wait_ld();
-#pragma unroll
-      for (int t = 0; t < TPC; t += 2) {
-        float a = 0.f, b = 0.f;
-#pragma unroll
-        for (int j = 0; j < J; ++j) {
-          a = fmaf(__uint_as_float(r[t * J + j]), rs_s[col + t * J + j], a);
-          b = fmaf(__uint_as_float(r[(t + 1) * J + j]), rs_s[col + (t + 1) * J + j], b);
-        }
-        pk[(c * TPC + t) / 2] = f2_to_bf162_bits(a * ts + 0.f, b * ts + 0.f);      // (+ 0: no negative zero, as epi_store)
-      }
-    }
-    if (t0 + V >= BN / J) {
-      tc_fence_before();
-      mbar_arrive(accum_empty);
-    }
-    uint16_t* out = reinterpret_cast<uint16_t*>(p.out) + n;
-#pragma unroll
-    for (int t = 0; t < V; ++t) {
-      const int tok = tok_first + t0 + t;
-      if (tok < p.tokens && n < p.N) out[(size_t)tok * p.ldo] = (uint16_t)(t & 1 ? pk[t / 2] >> 16 : pk[t / 2]);
-    }
-  }
-}
-
-// How a kernel stores its tiles (the forms are kept apart: together they spill registers in one another's loops).  CHUNKS: a
-// CTA has a tile or parts of some.  AHEAD, AHEAD_BF16 (plain bf16 results): CTAs that go through whole tiles one after the
-// other.  `follows`: this CTA has another one.  The last tile's stores run beside nothing and go out chunk by chunk, but for
-// residuals, whose loads wait for one another there.
-enum { STORES_CHUNKS = 0, STORES_AHEAD = 1, STORES_AHEAD_BF16 = 2 };
-template <int BN, int J, int STORES>
-__device__ __forceinline__ void epilogue_tile(const GemmParams& p, bool whole, bool follows, uint32_t taddr0, const float* rs_s,
-                                              float ts, int tok_first, int n, int lane, float* slot_row, uint32_t accum_empty) {
-  if constexpr (STORES == STORES_AHEAD_BF16) {
-    if (whole && follows) {
-      epilogue_ahead_bf16<BN, J>(p, taddr0, rs_s, ts, tok_first, n, accum_empty);
-      return;
-    }
-  }
-  if constexpr (STORES == STORES_AHEAD) {
-    if (whole && (follows || p.epi == EPI_RESIDUAL)) {
-      epilogue_ahead<BN, J>(p, taddr0, rs_s, ts, tok_first, n, lane, accum_empty);
-      return;
-    }
-  }
+__device__ __forceinline__ void epilogue_tile(const GemmParams& p, bool whole, uint32_t taddr0, const float* rs_s, float ts,
+                                              int tok_first, int n, int lane, float* slot_row, uint32_t accum_empty) {
   if (!whole) epilogue_chunks<BN, J, EPI_STORE, false>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
   else if (p.epi == EPI_SWIGLU) epilogue_chunks<BN, J, EPI_SWIGLU, true>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
   else if (p.epi == EPI_RESIDUAL) epilogue_chunks<BN, J, EPI_RESIDUAL, true>(p, taddr0, rs_s, ts, tok_first, n, lane, slot_row);
@@ -404,7 +298,7 @@ __device__ __forceinline__ void finish_split_tile(const GemmParams& p, const flo
   }
 }
 
-template <int BN, int STORES>
+template <int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                   const GemmParams p) {
@@ -654,10 +548,9 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       if (seg == 0 && threadIdx.x == 64) trace_stamp(5);
       {
         const uint32_t taddr0 = tmem_base + ((uint32_t)(quad * 32) << 16);
-        const bool follows = u + len < u1;
-        if (J == 4) epilogue_tile<BN, 4, STORES>(p, whole, follows, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
-        else if (J == 2) epilogue_tile<BN, 2, STORES>(p, whole, follows, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
-        else epilogue_tile<BN, 1, STORES>(p, whole, follows, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
+        if (J == 4) epilogue_tile<BN, 4>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
+        else if (J == 2) epilogue_tile<BN, 2>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
+        else epilogue_tile<BN, 1>(p, whole, taddr0, rs_s, ts, tok0, n, lane, slot + row, accum_empty);
       }
       if (threadIdx.x == 64) trace_stamp(6);
       if (!whole) {
@@ -997,10 +890,10 @@ int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t row_bytes
   return r == CUDA_SUCCESS ? 0 : 2;
 }
 
-template <int BN, int STORES>
+template <int BN>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, GemmParams p, int grid, cudaStream_t st) {
   using C = Cfg<BN>;
-  auto kern = gemm_nvfp4_kernel<BN, STORES>;
+  auto kern = gemm_nvfp4_kernel<BN>;
   // default: equal rings (one barrier pair per stage); unequal rings are an experiment knob --
   // measured on the 27B shapes they did not pay for their second wait / commit per unit
   int sa = C::RING_BYTES / (C::A_STAGE + C::B_STAGE);
@@ -1051,9 +944,6 @@ TRL_API int trl_quant_act_nvfp4(const void* x, int ldx, const void* norm_w, floa
                          swiglu_in, (int)staged);
 }
 
-// k-tiles from which the stores of a tile run beside the next one's MMAs: with fewer, the stores bound either way.
-constexpr int AHEAD_NK = 8;
-
 // How a product is laid out: columns a tile, CTAs, whole tiles or split ones.
 struct GemmPlan {
   int BN, n_tiles, c_tiles, nk, grid, split, max_seg;
@@ -1080,12 +970,43 @@ TRL_API int trl_gemm_trace_read(void* out, int n_ctas) {
   return (int)cudaMemcpyFromSymbol(out, g_gemm_trace, (size_t)n_ctas * TRACE_SLOTS * sizeof(unsigned long long));
 }
 
-// split: 1 / 0 as the caller wants it, -1 by the rule below.  Tiles are split along K when there are fewer than SMs, or when the
-// last round of whole tiles would leave more of the GPU idle than adding up the partial tiles costs.  In units of one k-tile of
-// one tile (0.55 us with up to 128 columns, 0.7 us with 256) the addition costs about ten and 16: measured at 8, 32 and 37 rows
-// 5.4 us, at 512 rows 11 us.  512 rows x 5120 x 17 408: 136 against 73.5 + 16, 141 us against 96.  The 5 %: not for every last
-// round its scratch memory.  Nearly as many tiles as SMs (8 rows x 16 480: 129) are faster whole when alone, 23.6 us against 27.6,
-// but not in a tick (8 sequences 590 us whole, 593 split; verify 2 x 8 rows 662 and 656): split, as fewer tiles are.
+// Columns a tile, pairs that share a tile along K (1, 2 or 3: a cluster of up to six CTAs), and pairs there are; bn 0: not for
+// the pair form (more than four terms, tiles split over CTAs as asked for, less than a pair of SMs).  Costs in units of a k-tile
+// of 128 columns, 0.2 us: one of 192 takes 1.25 (256 columns of 34 816 x 5120: 31.5 us in tiles of 128, 33.3 of 192; 512
+// columns, 8 rounds against 6: 51.1 and 46.0), one of 64 or 32, where the weights bound, a little less; parts cost the exchange
+// of their sums, more of them more.  5120 x 17 408 with its quantiser, one, two, three parts: 8 rows 22.6, 17.2, 16.3 us;
+// 32 rows 20.9, 16.3, 16.2; 64 rows 23.2, 17.5, 18.4; 96 rows 25.1, 22.0, 21.6 (24.0 in tiles of 128 columns, one part).
+// 5120 x 6144, 8 rows 10.7, 9.8, 9.0; 64 rows 11.4, 11.1, 11.5.
+struct PairPlan {
+  int bn, parts, pairs;
+};
+static PairPlan plan_pair(int tokens, int J, int N, int K, int max_ctas, int split) {
+  PairPlan best{0, 1, 0};
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int pairs = (max_ctas > 0 ? min(sms, max_ctas) : sms) / 2;
+  if (split == 1 || (J != 1 && J != 2 && J != 4) || pairs < 1) return best;
+  static const struct { int bn; double unit, exchange; } forms[] = {{32, 0.85, 1}, {64, 0.9, 2}, {128, 1, 9}, {192, 1.25, 12}};
+  const int cols = tokens * J, nk = (K + KT_ELEMS - 1) / KT_ELEMS, r_tiles = (N + 2 * TILE_N - 1) / (2 * TILE_N);
+  double least = 0;
+  for (const auto& f : forms) {
+    if (cols > f.bn && f.bn < 128) continue;              // (up to 64 columns in one tile)
+    const long long T = (long long)r_tiles * ((cols + f.bn - 1) / f.bn);
+    for (int S = 1; S <= 3; ++S) {
+      if (S > 1 && (split == 0 || nk < 8 * S || T * S > pairs || T > gemm_pair_clusters(S))) break;
+      const double cost = (double)((T * S + pairs - 1) / pairs) * nk / S * f.unit + f.exchange * S * (S - 1) / 2;
+      if (!best.bn || cost < least) best = PairPlan{f.bn, S, pairs}, least = cost;
+    }
+    if (cols <= f.bn) break;
+  }
+  return best;
+}
+
+// For what the pair form does not take.  split: 1 / 0 as the caller wants it, -1 by the rule below.  Tiles are split along K when
+// there are fewer than SMs, or when the last round of whole tiles would leave more of the GPU idle than adding up the partial tiles
+// costs: in units of one k-tile of one tile, about ten, and 16 with 256 columns.  The 5 %: not for every last round its scratch
+// memory.
 static GemmPlan plan_gemm(int tokens, int J, int N, int K, int max_ctas, int split) {
   GemmPlan g;
   const int cols = tokens * J;
@@ -1104,6 +1025,7 @@ static GemmPlan plan_gemm(int tokens, int J, int N, int K, int max_ctas, int spl
 }
 
 TRL_API long trl_gemm_nvfp4_scratch_bytes(int tokens, int J, int N, int K, int max_ctas, int split) {
+  if (plan_pair(tokens, J, N, K, max_ctas, split).bn) return 0;
   const GemmPlan g = plan_gemm(tokens, J, N, K, max_ctas, split);
   return g.split ? (long)g.n_tiles * g.c_tiles * g.max_seg * (g.BN / J) * TILE_N * (long)sizeof(float) : 0;
 }
@@ -1117,6 +1039,18 @@ TRL_API int trl_gemm_nvfp4(const void* wq, const void* sfw, const void* tscale, 
                            int split, int w_tiled, void* stream) {
   if (K % 32 != 0 || J < 1 || (32 % J) != 0 || J > 16) return (int)cudaErrorInvalidValue;
   const int cols = tokens * J;
+  const PairPlan pp = plan_pair(tokens, J, N, K, max_ctas, split);
+  if (pp.bn) {
+    // its stores are 8 rows of a token at a time (4 results of SwiGLU)
+    const int wide = epi == EPI_STORE_F32 || epi == EPI_SWIGLU ? 4 : 8, bytes = epi == EPI_SWIGLU ? 8 : 16;
+    if (N % 8 == 0 && ldo % wide == 0 && reinterpret_cast<uintptr_t>(out) % bytes == 0 &&
+        (epi != EPI_RESIDUAL || (ldr % 8 == 0 && reinterpret_cast<uintptr_t>(residual) % 16 == 0))) {
+      const GemmPairArgs a{wq, sfw, (const float*)tscale, xq, sfx, (const float*)rs, residual, out, ldr, ldo, tokens, J, N, K, epi,
+                           w_tiled, pp.pairs, pp.parts};
+      return gemm_pair_launch(a, pp.bn, (cudaStream_t)stream);
+    }
+    split = 0;                                            // no scratch was asked for
+  }
   const GemmPlan g = plan_gemm(tokens, J, N, K, max_ctas, split);
   CUtensorMap mw, mx;
   {
@@ -1136,16 +1070,7 @@ TRL_API int trl_gemm_nvfp4(const void* wq, const void* sfw, const void* tscale, 
     return (int)cudaErrorMemoryAllocation;
   cudaStream_t st = (cudaStream_t)stream;
   const int grid = g.grid;
-  const long long tiles = (long long)g.n_tiles * g.c_tiles;
-  // (SwiGLU of little more than a wide tile a CTA: 128 rows x 34 816, 272 tiles, 50.3 us ahead, 48.9 in chunks; residuals
-  // already with four k-tiles: 4096 rows x 1024 x 1024 30.7 us in chunks, 28.5 ahead)
-  const bool ahead = tiles > grid && g.nk >= (epi == EPI_RESIDUAL ? AHEAD_NK / 2 : AHEAD_NK) &&
-                     (epi != EPI_SWIGLU || g.BN < 256 || tiles >= 2 * grid);
-  const int stores = !ahead ? STORES_CHUNKS : epi == EPI_STORE ? STORES_AHEAD_BF16 : STORES_AHEAD;
-#define GEMM_CASE(B)                                                                     \
-  return stores == STORES_CHUNKS  ? launch<B, STORES_CHUNKS>(mw, mx, p, grid, st)        \
-         : stores == STORES_AHEAD ? launch<B, STORES_AHEAD>(mw, mx, p, grid, st)         \
-                                  : launch<B, STORES_AHEAD_BF16>(mw, mx, p, grid, st)
+#define GEMM_CASE(B) return launch<B>(mw, mx, p, grid, st)
   switch (g.BN) {
     case 16: GEMM_CASE(16);
     case 32: GEMM_CASE(32);

@@ -511,6 +511,35 @@ def test_gemm_stores_beside_the_next_tile(ops, tokens, n, k):
     assert native.read_error()[0] == 0
 
 
+@pytest.mark.parametrize("tokens,terms", [(1, 4), (8, 4), (9, 4), (16, 2), (17, 2), (32, 2), (33, 2), (64, 2), (65, 2), (96, 2), (97, 2), (31, 1), (193, 1), (500, 2)])
+@pytest.mark.parametrize("n,k", [(264, 544), (1288, 4128), (5120, 6144), (19072, 288)])
+def test_gemm_on_pairs_of_sms(ops, tokens, terms, n, k):
+    """Every width of a tile with columns that fill it, one more and one less, rows that leave the second SM of a pair half or
+    nothing, tiles that one pair and two or three go through, every epilogue, against one CTA alone (the one-SM kernel).  The
+    same products in fp32, summed in another order."""
+    from tilerl_b200 import formats as F
+    from tilerl_b200.ops import native
+    from tilerl_b200.ops.gemm_tc import gemm_nvfp4
+    g = torch.Generator().manual_seed(tokens + n)
+    w = F.quantize_nvfp4(torch.randn(n, k, generator=g) * 0.02).to(DEV)
+    x = torch.randn(tokens, k, generator=g).to(DEV, torch.bfloat16)
+    got, want = (torch.full((tokens, n), float("nan"), device=DEV) for _ in range(2))
+    gemm_nvfp4(ops, x, w, want, terms=terms, epi=3, max_ctas=1, split=False)
+    for _ in range(2):
+        gemm_nvfp4(ops, x, w, got, terms=terms, epi=3)
+        assert _rel(got, want) < 1e-6
+    a, r = torch.full((tokens, n), float("nan"), dtype=torch.bfloat16, device=DEV), torch.randn(tokens, n, generator=g).to(DEV, torch.bfloat16)
+    gemm_nvfp4(ops, x, w, a, terms=terms)
+    assert _rel(a, want) < 2 ** -8
+    acc = r.clone()
+    gemm_nvfp4(ops, x, w, acc, terms=terms, epi=1, residual=acc)
+    assert _rel(acc, want.double() + r.double()) < 2 ** -8
+    h = torch.full((tokens, n // 2), float("nan"), dtype=torch.bfloat16, device=DEV)
+    gemm_nvfp4(ops, x, w, h, terms=terms, epi=2)
+    assert _rel(h, torch.nn.functional.silu(want[:, 0::2].double()) * want[:, 1::2].double()) < 2 ** -8
+    assert native.read_error()[0] == 0
+
+
 @pytest.mark.parametrize("k", [1040, 18464, 24576, 28672])
 @pytest.mark.parametrize("terms,swiglu", [(1, False), (2, False), (2, True), (4, False)])
 def test_activation_quantiser_with_the_row_staged(ops, k, terms, swiglu):
