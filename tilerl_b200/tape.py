@@ -409,10 +409,19 @@ def gdn_block_torch(inp, conv_w, dt_bias, a_log, norm_w, *, nk, nv, dk, dv, eps,
 def gdn_block(tape: Tape, inp: torch.Tensor, conv_w, dt_bias, a_log, norm_w, **kw) -> torch.Tensor:
     """GDN block as one tape op.  Forward runs without a graph; backward recomputes
     the block (activation checkpointing at block granularity) and differentiates
-    the chunked form locally."""
+    the chunked form locally; on CUDA both are kernels (``csrc/gdn_train.cu``) for the shapes
+    they take."""
+    params = (conv_w, dt_bias, a_log, norm_w)
+    if inp.is_cuda:
+        from .ops import gdn_train
+        if gdn_train.takes(inp, *params, **kw):
+            with torch.no_grad():
+                out = gdn_train.forward(inp, *params, **kw)
+            tape.record("gdn", (inp,) + params, (out,),
+                        lambda g: gdn_train.backward(inp, *params, g, need=[id(p) in tape.leaves for p in params], **kw))
+            return out
     with torch.no_grad():
         out = gdn_block_torch(inp, conv_w, dt_bias, a_log, norm_w, **kw)
-    params = (conv_w, dt_bias, a_log, norm_w)
 
     def bwd(g):
         with torch.enable_grad():
