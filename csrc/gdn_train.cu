@@ -23,6 +23,8 @@
 // kept, then norm, scan backwards, everything of a chunk that needs both states (a block a chunk and head), and prep's gradient
 // in two steps.  All fp32 on the CUDA cores, as the torch ops were; products go through shared memory in tiles of 4 x 4 or
 // 2 x 4 a thread, rows padded by four floats.  Sums over heads and tokens are in a fixed order.
+//
+// In the place of the reference's tape handlers of the block (src/tilerl/autograd.py:113-301).
 #include "common.cuh"
 
 namespace {

@@ -22,6 +22,8 @@
 // half of the columns.  A warp turns 32 rows x 16 tokens round through its own piece of shared memory, so that results leave
 // as 16-byte stores along a token's row (2 bytes a lane along the rows were 3.7 us a tile in the open).  Weights' and
 // activations' scales come by tiled copies too, since only these may count on the other SM's barrier; none is multicast.
+//
+// In the reference's place: linear_fp4_fp8 / linear_fp4_mma8 (packages/tilerl-kernels/src/tilerl_kernels/kernels_linear.py:924-1687).
 #include <cuda.h>
 #include "common.cuh"
 #include "tcgen05.cuh"
