@@ -60,51 +60,89 @@ __device__ __forceinline__ void fma4(float4& d, float a, float4 b) {
 }
 __device__ __forceinline__ float4 mul4(float4 a, float b) { return make_float4(a.x * b, a.y * b, a.z * b, a.w * b); }
 
-// The convolution's four channels c .. c + 3 at token t of a sequence (zeros before its beginning).
-__device__ __forceinline__ float4 conv4(const GdnTrain& a, const float* seq, int ld, int t, int c) {
-  float4 y = f4(0.f);
-  for (int j = 0; j < a.kw; ++j) {
-    const int s = t - (a.kw - 1) + j;
-    if (s < 0) continue;
-    const float4 x = ld4(seq + (size_t)s * ld + c);
-    y.x = fmaf(x.x, a.conv[(c + 0) * a.kw + j], y.x), y.y = fmaf(x.y, a.conv[(c + 1) * a.kw + j], y.y);
-    y.z = fmaf(x.z, a.conv[(c + 2) * a.kw + j], y.z), y.w = fmaf(x.w, a.conv[(c + 3) * a.kw + j], y.w);
+// A run of RUN tokens, a warp a head of 128 channels: taps and the window of rows stay in registers (a token alone read four taps of
+// four channels again for each row: 74 us at 4 x 512 tokens of 16 heads).  Convolutions of up to four taps; longer ones reread.
+constexpr int RUN = 8, TAPS = 4;
+struct Conv {
+  float4 tap[TAPS];                                 // of four channels: tap[j].x is channel c's
+  __device__ __forceinline__ void load(const GdnTrain& a, int c) {
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) {
+      const int at = j - (TAPS - a.kw);             // shorter ones: zeros in front
+      tap[j] = at >= 0 && a.kw <= TAPS ? make_float4(a.conv[c * a.kw + at], a.conv[(c + 1) * a.kw + at], a.conv[(c + 2) * a.kw + at], a.conv[(c + 3) * a.kw + at])
+                                       : f4(0.f);
+    }
   }
-  return y;
+};
+__device__ __forceinline__ void fma44(float4& d, float4 a, float4 b) {
+  d.x = fmaf(a.x, b.x, d.x), d.y = fmaf(a.y, b.y, d.y), d.z = fmaf(a.z, b.z, d.z), d.w = fmaf(a.w, b.w, d.w);
+}
+// Its four channels at tokens t0 .. t0 + RUN - 1 of a sequence (zeros before its beginning and from its end on).
+__device__ __forceinline__ void conv_run(const GdnTrain& a, const float* seq, int ld, int t0, int c, float4 (&y)[RUN]) {
+  Conv cv;
+  cv.load(a, c);
+  if (a.kw <= TAPS) {
+    float4 x[RUN + TAPS - 1];
+#pragma unroll
+    for (int i = 0; i < RUN + TAPS - 1; ++i) {
+      const int t = t0 + i - (TAPS - 1);
+      x[i] = t >= 0 && t < a.T ? ld4(seq + (size_t)t * ld + c) : f4(0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) {
+      y[i] = f4(0.f);
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) fma44(y[i], x[i + j], cv.tap[j]);
+    }
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < RUN; ++i) {
+    y[i] = f4(0.f);
+    for (int j = 0; j < a.kw; ++j) {
+      const int t = t0 + i - (a.kw - 1) + j;
+      if (t < 0 || t0 + i >= a.T) continue;
+      fma44(y[i], ld4(seq + (size_t)t * ld + c), make_float4(a.conv[c * a.kw + j], a.conv[(c + 1) * a.kw + j], a.conv[(c + 2) * a.kw + j], a.conv[(c + 3) * a.kw + j]));
+    }
+  }
 }
 
-// ---- prep: a block a token (of the padded sequence), a warp a head -----------------------------------------------
+// ---- prep: a block a run of tokens (of the padded sequence) and eight heads ---------------------------------------------
 __global__ void __launch_bounds__(256) gt_prep_kernel(const GdnTrain a) {
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int tp = a.n * C, b = blockIdx.x / tp, t = blockIdx.x % tp, ck = t / C, i = t % C;
+  const int lane = threadIdx.x & 31;
+  const int runs = a.n * C / RUN, b = blockIdx.x / runs, t0 = blockIdx.x % runs * RUN, ck = t0 / C, i0 = t0 % C;
   const int ch = (2 * a.nk + a.nv) * D, ld = ch + a.nv * D + 2 * a.nv;
   const float* seq = a.inp + (size_t)b * a.T * ld;
-  for (int h = threadIdx.x >> 5; h < 2 * a.nk + a.nv; h += nw) {
-    float4 x = f4(0.f);
-    if (t < a.T) {
-      x = conv4(a, seq, ld, t, h * D + lane * 4);
-      x = make_float4(silu(x.x), silu(x.y), silu(x.z), silu(x.w));
-      if (h < 2 * a.nk) {
-        const float inv = 1.f / sqrtf(warp_sum(dot4(x, x)) + 1e-12f);
-        x = mul4(x, h < a.nk ? inv * rsqrtf((float)D) : inv);
-      }
-    }
+  const int h = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (h < 2 * a.nk + a.nv) {
+    float4 x[RUN];
+    conv_run(a, seq, ld, t0, h * D + lane * 4, x);
     float* dst = h < a.nk ? a.q + ((size_t)(b * a.nk + h) * a.n + ck) * C * D
                  : h < 2 * a.nk ? a.k + ((size_t)(b * a.nk + h - a.nk) * a.n + ck) * C * D
                                 : a.v + ((size_t)(b * a.nv + h - 2 * a.nk) * a.n + ck) * C * D;
-    st4(dst + i * D + lane * 4, x);
-  }
-  for (int h = threadIdx.x; h < a.nv; h += blockDim.x) {
-    float g = 0.f, be = 0.f;
-    if (t < a.T) {
-      const float* row = seq + (size_t)t * ld + ch + a.nv * D;
-      const float x = row[h] + a.dt_bias[h];
-      g = -expf(a.a_log[h]) * (x > 20.f ? x : log1pf(expf(x)));
-      be = 1.f / (1.f + expf(-row[a.nv + h]));
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) {
+      x[i] = t0 + i < a.T ? make_float4(silu(x[i].x), silu(x[i].y), silu(x[i].z), silu(x[i].w)) : f4(0.f);
+      if (h < 2 * a.nk) {
+        const float inv = 1.f / sqrtf(warp_sum(dot4(x[i], x[i])) + 1e-12f);
+        x[i] = mul4(x[i], h < a.nk ? inv * rsqrtf((float)D) : inv);
+      }
+      st4(dst + (i0 + i) * D + lane * 4, x[i]);
     }
-    const size_t at = ((size_t)(b * a.nv + h) * a.n + ck) * C + i;
-    a.g[at] = g, a.beta[at] = be;                  // (the chunk kernel makes sums of the decays)
   }
+  if (blockIdx.y == 0)
+    for (int e = threadIdx.x; e < a.nv * RUN; e += blockDim.x) {
+      const int hv = e / RUN, i = e % RUN, t = t0 + i;
+      float g = 0.f, be = 0.f;
+      if (t < a.T) {
+        const float* row = seq + (size_t)t * ld + ch + a.nv * D;
+        const float x = row[hv] + a.dt_bias[hv];
+        g = -expf(a.a_log[hv]) * (x > 20.f ? x : log1pf(expf(x)));
+        be = 1.f / (1.f + expf(-row[a.nv + hv]));
+      }
+      const size_t at = ((size_t)(b * a.nv + hv) * a.n + ck) * C + i0 + i;
+      a.g[at] = g, a.beta[at] = be;                // (the chunk kernel makes sums of the decays)
+    }
 }
 
 // Rows 4 rg .. 4 rg + 3 against row `lane` of two padded [32, 128] tiles: acc[r] += x_r . y_lane
@@ -498,56 +536,81 @@ __global__ void __launch_bounds__(GC_T) gt_chunk_grad_kernel(const GdnTrain a, c
   }
 }
 
-// Gradients of norms, SiLU and gates: a block a token, a warp a head.
+// Gradients of norms, SiLU and gates: a block a run of tokens and eight heads.
 __global__ void __launch_bounds__(256) gt_prep_grad_kernel(const GdnTrain a, const GdnTrainGrad d) {
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int b = blockIdx.x / a.T, t = blockIdx.x % a.T, ck = t / C, i = t % C, rep = a.nv / a.nk;
+  const int lane = threadIdx.x & 31, rep = a.nv / a.nk;
+  const int runs = a.n * C / RUN, b = blockIdx.x / runs, t0 = blockIdx.x % runs * RUN, ck = t0 / C, i0 = t0 % C;
+  if (t0 >= a.T) return;
   const int ch = (2 * a.nk + a.nv) * D, ld = ch + a.nv * D + 2 * a.nv;
   const float* seq = a.inp + (size_t)b * a.T * ld;
-  for (int h = threadIdx.x >> 5; h < 2 * a.nk + a.nv; h += nw) {
-    const float4 y = conv4(a, seq, ld, t, h * D + lane * 4);
-    float4 e = f4(0.f);
-    if (h < 2 * a.nk) {
-      const bool is_q = h < a.nk;
-      const int hk = is_q ? h : h - a.nk;
-      const float* src = is_q ? d.dq : d.dk;
-      for (int r = 0; r < rep; ++r) {
-        const float4 x = ld4(src + (((size_t)(b * a.nv + hk * rep + r) * a.n + ck) * C + i) * D + lane * 4);
+  const int h = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (h < 2 * a.nk + a.nv) {
+    float4 y[RUN];
+    conv_run(a, seq, ld, t0, h * D + lane * 4, y);
+    const bool is_v = h >= 2 * a.nk, is_q = h < a.nk;
+    const int first = is_v ? h - 2 * a.nk : (is_q ? h : h - a.nk) * rep, heads = is_v ? 1 : rep;
+    const float* src = (is_v ? d.dv : is_q ? d.dq : d.dk) + (((size_t)(b * a.nv + first) * a.n + ck) * C + i0) * D + lane * 4;
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) {
+      if (t0 + i >= a.T) break;
+      float4 e = f4(0.f);
+      for (int r = 0; r < heads; ++r) {
+        const float4 x = ld4(src + ((size_t)r * a.n * C + i) * D);
         e.x += x.x, e.y += x.y, e.z += x.z, e.w += x.w;
       }
-      const float4 c = make_float4(silu(y.x), silu(y.y), silu(y.z), silu(y.w));
-      const float inv = 1.f / sqrtf(warp_sum(dot4(c, c)) + 1e-12f), sc = is_q ? inv * rsqrtf((float)D) : inv;
-      const float m = warp_sum(dot4(c, e)) * inv * inv;
-      e = make_float4(sc * (e.x - c.x * m), sc * (e.y - c.y * m), sc * (e.z - c.z * m), sc * (e.w - c.w * m));
-    } else {
-      e = ld4(d.dv + (((size_t)(b * a.nv + h - 2 * a.nk) * a.n + ck) * C + i) * D + lane * 4);
+      if (!is_v) {
+        const float4 c = make_float4(silu(y[i].x), silu(y[i].y), silu(y[i].z), silu(y[i].w));
+        const float inv = 1.f / sqrtf(warp_sum(dot4(c, c)) + 1e-12f), sc = is_q ? inv * rsqrtf((float)D) : inv;
+        const float m = warp_sum(dot4(c, e)) * inv * inv;
+        e = make_float4(sc * (e.x - c.x * m), sc * (e.y - c.y * m), sc * (e.z - c.z * m), sc * (e.w - c.w * m));
+      }
+      st4(d.dy + ((size_t)b * a.T + t0 + i) * ch + h * D + lane * 4,
+          make_float4(e.x * silu_grad(y[i].x), e.y * silu_grad(y[i].y), e.z * silu_grad(y[i].z), e.w * silu_grad(y[i].w)));
     }
-    st4(d.dy + ((size_t)b * a.T + t) * ch + h * D + lane * 4,
-        make_float4(e.x * silu_grad(y.x), e.y * silu_grad(y.y), e.z * silu_grad(y.z), e.w * silu_grad(y.w)));
   }
-  for (int h = threadIdx.x; h < a.nv; h += blockDim.x) {
-    const size_t at = ((size_t)(b * a.nv + h) * a.n + ck) * C + i, row = ((size_t)b * a.T + t) * ld + ch + a.nv * D;
-    const float x = a.inp[row + h] + a.dt_bias[h], be = a.beta[at];
-    d.dinp[row + h] = -d.dg[at] * expf(a.a_log[h]) / (1.f + expf(-x));
-    d.dinp[row + a.nv + h] = d.dbeta[at] * be * (1.f - be);
-  }
+  if (blockIdx.y == 0)
+    for (int e = threadIdx.x; e < a.nv * RUN; e += blockDim.x) {
+      const int hv = e / RUN, i = e % RUN, t = t0 + i;
+      if (t >= a.T) continue;
+      const size_t at = ((size_t)(b * a.nv + hv) * a.n + ck) * C + i0 + i, row = ((size_t)b * a.T + t) * ld + ch + a.nv * D;
+      const float x = a.inp[row + hv] + a.dt_bias[hv], be = a.beta[at];
+      d.dinp[row + hv] = -d.dg[at] * expf(a.a_log[hv]) / (1.f + expf(-x));
+      d.dinp[row + a.nv + hv] = d.dbeta[at] * be * (1.f - be);
+    }
 }
 
-// The convolution backwards: four channels of a token a thread.
+// The convolution backwards: a run of tokens and eight heads' channels a block.
 __global__ void __launch_bounds__(256) gt_conv_grad_kernel(const GdnTrain a, const GdnTrainGrad d) {
   const int ch = (2 * a.nk + a.nv) * D, ld = ch + a.nv * D + 2 * a.nv;
-  const long long x = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (x >= (long long)a.B * a.T * (ch / 4)) return;
-  const int c = (int)(x % (ch / 4)) * 4, t = (int)(x / (ch / 4) % a.T), b = (int)(x / (ch / 4) / a.T);
-  float4 e = f4(0.f);
-  for (int j = 0; j < a.kw; ++j) {
-    const int s = t + a.kw - 1 - j;
-    if (s >= a.T) continue;
-    const float4 y = ld4(d.dy + ((size_t)b * a.T + s) * ch + c);
-    e.x = fmaf(y.x, a.conv[(c + 0) * a.kw + j], e.x), e.y = fmaf(y.y, a.conv[(c + 1) * a.kw + j], e.y);
-    e.z = fmaf(y.z, a.conv[(c + 2) * a.kw + j], e.z), e.w = fmaf(y.w, a.conv[(c + 3) * a.kw + j], e.w);
+  const int runs = (a.T + RUN - 1) / RUN, b = blockIdx.x / runs, t0 = blockIdx.x % runs * RUN, c = (blockIdx.y * 256 + threadIdx.x) * 4;
+  if (c >= ch) return;
+  const float* dy = d.dy + (size_t)b * a.T * ch + c;
+  float* dst = d.dinp + ((size_t)b * a.T + t0) * ld + c;
+  Conv cv;
+  cv.load(a, c);
+  if (a.kw <= TAPS) {
+    float4 y[RUN + TAPS - 1];
+#pragma unroll
+    for (int i = 0; i < RUN + TAPS - 1; ++i) y[i] = t0 + i < a.T ? ld4(dy + (size_t)(t0 + i) * ch) : f4(0.f);
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) {
+      if (t0 + i >= a.T) break;
+      float4 e = f4(0.f);
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) fma44(e, y[i + TAPS - 1 - j], cv.tap[j]);
+      st4(dst + (size_t)i * ld, e);
+    }
+    return;
   }
-  st4(d.dinp + ((size_t)b * a.T + t) * ld + c, e);
+  for (int i = 0; i < RUN && t0 + i < a.T; ++i) {
+    float4 e = f4(0.f);
+    for (int j = 0; j < a.kw; ++j) {
+      const int t = t0 + i + a.kw - 1 - j;
+      if (t >= a.T) continue;
+      fma44(e, ld4(dy + (size_t)t * ch), make_float4(a.conv[c * a.kw + j], a.conv[(c + 1) * a.kw + j], a.conv[(c + 2) * a.kw + j], a.conv[(c + 3) * a.kw + j]));
+    }
+    st4(dst + (size_t)i * ld, e);
+  }
 }
 
 // Pieces of the workspace, in order; `grad`: those of a gradient too.  Returns the floats used.
@@ -587,7 +650,7 @@ bool fits(int B, int T, int nk, int nv, int kw) {
 }
 
 int run_forward(const GdnTrain& a, int keep, cudaStream_t st) {
-  gt_prep_kernel<<<a.B * a.n * C, 256, 0, st>>>(a);
+  gt_prep_kernel<<<dim3(a.B * a.n * (C / RUN), (2 * a.nk + a.nv + 7) / 8), 256, 0, st>>>(a);
   gt_chunk_kernel<<<a.B * a.nv * a.n, 256, CHUNK_SMEM, st>>>(a);
   gt_scan_kernel<<<dim3(a.B * a.nv, D / SLICE), 256, SCAN_SMEM, st>>>(a, keep);
   return (int)cudaGetLastError();
@@ -632,8 +695,8 @@ TRL_API int trl_gdn_train_backward(const void* inp, const void* conv, const void
   gt_norm_grad_kernel<<<(B * a.n * C * nv + 7) / 8, 256, 0, st>>>(a, d);
   gt_scan_grad_kernel<<<dim3(B * nv, D / SLICE), 256, SCAN_SMEM, st>>>(a, d);
   gt_chunk_grad_kernel<<<B * nv * a.n, GC_T, sizeof(ChunkGradSmem), st>>>(a, d);
-  gt_prep_grad_kernel<<<B * T, 256, 0, st>>>(a, d);
-  gt_conv_grad_kernel<<<(int)(((long long)B * T * ((2 * nk + nv) * D / 4) + 255) / 256), 256, 0, st>>>(a, d);
+  gt_prep_grad_kernel<<<dim3(B * a.n * (C / RUN), (2 * nk + nv + 7) / 8), 256, 0, st>>>(a, d);
+  gt_conv_grad_kernel<<<dim3(B * ((T + RUN - 1) / RUN), ((2 * nk + nv) * D / 4 + 255) / 256), 256, 0, st>>>(a, d);
   where[0] = a.o - (float*)ws, where[1] = d.dg - (float*)ws, where[2] = d.dy - (float*)ws;
   return (int)cudaGetLastError();
 }

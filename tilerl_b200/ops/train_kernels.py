@@ -1,0 +1,225 @@
+"""The training tape's elementwise and low-rank ops on the kernels of ``csrc/train.cu``.  Each function says what it takes with a
+``*_takes`` of its own or returns ``None``; the tape runs its torch form where it does not."""
+from __future__ import annotations
+
+import ctypes
+from typing import Dict, List, Optional, Sequence
+
+import torch
+
+from . import native as N
+
+N.register("trl_train_rmsnorm", [N.P] * 3 + [N.I] * 2 + [N.F, N.P])
+N.register("trl_train_rmsnorm_grad", [N.P] * 4 + [N.I] * 2 + [N.F, N.P])
+N.register("trl_train_swiglu", [N.P] * 3 + [N.L, N.P])
+N.register("trl_train_lowrank", [N.P] * 3 + [N.I] * 4 + [N.F, N.P])
+N.register("trl_train_expand", [N.P] * 4 + [N.I] * 4 + [N.F, N.P])
+N.register("trl_train_outer_parts", [N.I] * 2)
+N.register("trl_train_outer", [N.P] * 4 + [N.I] * 4 + [N.F, N.P])
+N.register("trl_train_attn_prep", [N.P] * 8 + [N.I] * 8 + [N.F, N.P])
+N.register("trl_train_attn_prep_grad", [N.P] * 11 + [N.I] * 8 + [N.F, N.P])
+N.register("trl_train_attn_gate", [N.P] * 3 + [N.I] * 7 + [N.P])
+N.register("trl_train_softmax", [N.P] * 2 + [N.I] * 4 + [N.F, N.P])
+N.register("trl_train_softmax_grad", [N.P] * 2 + [N.L, N.I, N.F, N.P])
+N.register("trl_train_lse", [N.P] * 2 + [N.L] * 2 + [N.P])
+N.register("trl_train_ce_grad", [N.P] * 6 + [N.L] * 2 + [N.P])
+N.register("trl_train_adamw", [N.P] * 8 + [N.I] + [N.F] * 6 + [N.P])
+N.register("trl_train_squares", [N.P, N.P, N.I, N.P, N.P])
+N.register("trl_train_scale", [N.P, N.P, N.I, N.F, N.P])
+
+MAX_TENSORS = 32          # a launch of the many-tensor kernels
+
+
+def plain(*tensors) -> bool:
+    """fp32, contiguous, not empty and on 16-byte boundaries, all on the current CUDA device."""
+    return all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() and t.data_ptr() % 16 == 0
+               and t.device.index == torch.cuda.current_device() for t in tensors)
+
+
+def _grad(g: torch.Tensor) -> torch.Tensor:
+    g = g.float().contiguous()
+    return g if g.data_ptr() % 16 == 0 else g.clone()
+
+
+# ---- RMSNorm ---------------------------------------------------------------------------------------------
+def rmsnorm_takes(x, w) -> bool:
+    h = x.shape[-1]
+    return h % 4 == 0 and h <= 8192 and w.dim() == 1 and w.numel() == h and plain(x, w) and x.numel() // h < 1 << 31
+
+
+def rmsnorm(x, w, eps):
+    out = torch.empty_like(x)
+    h = x.shape[-1]
+    N.check(N.lib().trl_train_rmsnorm(x.data_ptr(), w.data_ptr(), out.data_ptr(), x.numel() // h, h, eps, N.stream()), "train_rmsnorm")
+    N.count()
+    return out
+
+
+def rmsnorm_grad(x, w, g, eps):
+    g, dx, h = _grad(g), torch.empty_like(x), x.shape[-1]
+    N.check(N.lib().trl_train_rmsnorm_grad(x.data_ptr(), w.data_ptr(), g.data_ptr(), dx.data_ptr(), x.numel() // h, h, eps, N.stream()), "train_rmsnorm_grad")
+    N.count()
+    return dx
+
+
+# ---- SwiGLU ------------------------------------------------------------------------------------------------
+def swiglu_takes(gu) -> bool:
+    return gu.shape[-1] % 2 == 0 and gu.numel() % 8 == 0 and gu.numel() < 1 << 40 and plain(gu)
+
+
+def swiglu(gu):
+    out = torch.empty(*gu.shape[:-1], gu.shape[-1] // 2, dtype=torch.float32, device=gu.device)
+    N.check(N.lib().trl_train_swiglu(gu.data_ptr(), None, out.data_ptr(), out.numel(), N.stream()), "train_swiglu")
+    N.count()
+    return out
+
+
+def swiglu_grad(gu, g):
+    g, d = _grad(g), torch.empty_like(gu)
+    N.check(N.lib().trl_train_swiglu(gu.data_ptr(), g.data_ptr(), d.data_ptr(), g.numel(), N.stream()), "train_swiglu_grad")
+    N.count()
+    return d
+
+
+# ---- adapters: y + s (x A^T) B^T -----------------------------------------------------------------------------
+def lora_takes(y, x, a, b) -> bool:
+    r, k = a.shape
+    return (r in (4, 8, 16, 32) and k % 4 == 0 and b.shape[0] % 4 == 0 and b.shape[1] == r and x.shape[-1] == k and y.shape[-1] == b.shape[0]
+            and x.shape[:-1] == y.shape[:-1] and plain(y, x, a, b) and x.numel() // k <= 16 * 65535)
+
+
+def lora(y, x, a, b, s):
+    """The result, and ``x A^T`` for the gradient."""
+    (r, k), n, m = a.shape, b.shape[0], x.numel() // x.shape[-1]
+    xa, out = torch.empty(m, r, dtype=torch.float32, device=x.device), torch.empty_like(y)
+    N.check(N.lib().trl_train_lowrank(x.data_ptr(), a.data_ptr(), xa.data_ptr(), m, k, r, 0, 1.0, N.stream()), "train_lowrank")
+    N.check(N.lib().trl_train_expand(y.data_ptr(), xa.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, r, 0, s, N.stream()), "train_expand")
+    N.count(2)
+    return out, xa
+
+
+def lora_grad(x, xa, a, b, s, g):
+    """Gradients of (x, a, b) for that of the result."""
+    (r, k), n, m = a.shape, b.shape[0], x.numel() // x.shape[-1]
+    lib, st = N.lib(), N.stream()
+    dxa, dx, da, db = torch.empty_like(xa), torch.empty_like(x), torch.empty_like(a), torch.empty_like(b)
+    part = torch.empty(r * max(lib.trl_train_outer_parts(m, n) * n, lib.trl_train_outer_parts(m, k) * k), dtype=torch.float32, device=x.device)
+    N.check(lib.trl_train_lowrank(g.data_ptr(), b.data_ptr(), dxa.data_ptr(), m, n, r, 1, s, st), "train_lowrank")
+    N.check(lib.trl_train_outer(g.data_ptr(), xa.data_ptr(), part.data_ptr(), db.data_ptr(), m, n, r, 0, s, st), "train_outer")
+    N.check(lib.trl_train_outer(x.data_ptr(), dxa.data_ptr(), part.data_ptr(), da.data_ptr(), m, k, r, 1, 1.0, st), "train_outer")
+    N.check(lib.trl_train_expand(None, dxa.data_ptr(), a.data_ptr(), dx.data_ptr(), m, k, r, 1, 1.0, st), "train_expand")
+    N.count(6)
+    return dx, da, db
+
+
+# ---- attention block --------------------------------------------------------------------------------------------
+def attention_takes(qkv, q_norm_w, k_norm_w, positions, *, n_q, n_kv, head_dim, rotary_dim, gated) -> bool:
+    if qkv.dim() != 3 or n_q % n_kv or head_dim % 4 or head_dim > 512 or rotary_dim % 2 or rotary_dim > head_dim or rotary_dim < 2:
+        return False
+    b, t, rows = qkv.shape
+    return (rows == n_q * head_dim * (2 if gated else 1) + 2 * n_kv * head_dim and t <= 4096 and b * n_q * t < 1 << 31
+            and tuple(positions.shape) in ((t,), (b, t), (1, t)) and q_norm_w.numel() == head_dim and k_norm_w.numel() == head_dim
+            and positions.device == qkv.device and plain(qkv, q_norm_w, k_norm_w))
+
+
+def attention(qkv, q_norm_w, k_norm_w, positions, *, n_q, n_kv, head_dim, rotary_dim, theta, eps, gated):
+    """Output ``[B, T, n_q * head_dim]`` and the function of its gradient that gives qkv's."""
+    (b, t, rows), d, half, lib = qkv.shape, head_dim, rotary_dim // 2, N.lib()
+    inv = theta ** (-torch.arange(half, dtype=torch.float64, device=qkv.device) * 2.0 / rotary_dim)
+    pos = positions.reshape(-1, t).to(torch.int64).contiguous()
+    ang = pos.to(torch.float64)[..., None] * inv
+    cs, sn, pr = ang.cos().float(), ang.sin().float(), pos.shape[0]
+    dims = (b, t, n_q, n_kv, d, half, int(gated), pr, eps)
+    new = lambda *shape: torch.empty(*shape, dtype=torch.float32, device=qkv.device)
+    head = (qkv.data_ptr(), q_norm_w.data_ptr(), k_norm_w.data_ptr(), cs.data_ptr(), sn.data_ptr())
+    q, k, v = new(b * n_kv, n_q // n_kv * t, d), new(b * n_kv, t, d), new(b * n_kv, t, d)
+    N.check(lib.trl_train_attn_prep(*head, q.data_ptr(), k.data_ptr(), v.data_ptr(), *dims, N.stream()), "train_attn_prep")
+    sc = 1.0 / d ** 0.5
+    p = torch.bmm(q, k.transpose(1, 2))
+    N.check(lib.trl_train_softmax(p.data_ptr(), pos.data_ptr(), pr, b, n_q, t, sc, N.stream()), "train_softmax")
+    o = torch.bmm(p, v)
+    out = new(b, t, n_q * d)
+    N.check(lib.trl_train_attn_gate(o.data_ptr(), qkv.data_ptr(), out.data_ptr(), b, t, n_q, d, rows, int(gated), 0, N.stream()), "train_attn_gate")
+    N.count(3)
+
+    def backward(gout):
+        up, go, dqkv = _grad(gout), torch.empty_like(o), torch.empty_like(qkv)
+        N.check(lib.trl_train_attn_gate(up.data_ptr(), qkv.data_ptr(), go.data_ptr(), b, t, n_q, d, rows, int(gated), 1, N.stream()), "train_attn_gate")
+        dv = torch.bmm(p.transpose(1, 2), go)
+        ds = torch.bmm(go, v.transpose(1, 2))
+        N.check(lib.trl_train_softmax_grad(p.data_ptr(), ds.data_ptr(), b * n_q * t, t, sc, N.stream()), "train_softmax_grad")
+        dq, dk = torch.bmm(ds, k), torch.bmm(ds.transpose(1, 2), q)
+        N.check(lib.trl_train_attn_prep_grad(qkv.data_ptr(), q_norm_w.data_ptr(), k_norm_w.data_ptr(), cs.data_ptr(), sn.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+                                             dv.data_ptr(), o.data_ptr(), up.data_ptr(), dqkv.data_ptr(), *dims, N.stream()), "train_attn_prep_grad")
+        N.count(3)
+        return dqkv
+
+    return out, backward
+
+
+# ---- cross-entropy ------------------------------------------------------------------------------------------------
+def cross_entropy_takes(logits, targets, weights) -> bool:
+    return logits.shape[-1] % 4 == 0 and plain(logits) and targets.device == logits.device and weights.device == logits.device \
+        and targets.numel() == weights.numel() == logits.numel() // logits.shape[-1] < 1 << 31
+
+
+def lse(lg):
+    """``[3, rows]``: largest value, sum of exponentials below it, log-sum-exp."""
+    out = torch.empty(3, lg.shape[0], dtype=torch.float32, device=lg.device)
+    N.check(N.lib().trl_train_lse(lg.data_ptr(), out.data_ptr(), lg.shape[0], lg.shape[1], N.stream()), "train_lse")
+    N.count()
+    return out
+
+
+def cross_entropy_grad(lg, stats, targets, weights, up):
+    g, up = torch.empty_like(lg), up.reshape(1).float()
+    N.check(N.lib().trl_train_ce_grad(lg.data_ptr(), stats.data_ptr(), targets.data_ptr(), weights.data_ptr(), up.data_ptr(), g.data_ptr(),
+                                      lg.shape[0], lg.shape[1], N.stream()), "train_ce_grad")
+    N.count()
+    return g
+
+
+# ---- many tensors at a time -------------------------------------------------------------------------------------------
+def _pointers(tensors: Sequence[torch.Tensor]):
+    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+
+
+def _lengths(tensors: Sequence[torch.Tensor]):
+    return (ctypes.c_long * len(tensors))(*[t.numel() for t in tensors])
+
+
+def _floats(v: Sequence[float]):
+    return (ctypes.c_float * len(v))(*v)
+
+
+def adamw(items: List[tuple], lr: float, betas, eps: float) -> None:
+    """``items``: (parameter, m, v, gradient, decay factor, 1 - b1^t, 1 - b2^t), tensors plain."""
+    for i in range(0, len(items), MAX_TENSORS):
+        p, m, v, g, decay, c1, c2 = zip(*items[i:i + MAX_TENSORS])
+        N.check(N.lib().trl_train_adamw(_pointers(p), _pointers(m), _pointers(v), _pointers(g), _lengths(p), _floats(decay), _floats(c1), _floats(c2),
+                                        len(p), lr, betas[0], 1 - betas[0], betas[1], 1 - betas[1], eps, N.stream()), "train_adamw")
+        torch.autograd.graph.increment_version(p + m + v)         # written in place, as ``copy_`` says it
+        N.count()
+
+
+def squares(grads: Dict[str, torch.Tensor]) -> Optional[torch.Tensor]:
+    """Sum of squares of every gradient in fp64, in the order of the dict; ``None`` where the kernel does not take them all."""
+    gs = list(grads.values())
+    if not gs or not plain(*gs):
+        return None
+    part = torch.empty(len(gs), 16, dtype=torch.float64, device=gs[0].device)
+    for i in range(0, len(gs), MAX_TENSORS):
+        some = gs[i:i + MAX_TENSORS]
+        N.check(N.lib().trl_train_squares(_pointers(some), _lengths(some), len(some), part[i:].data_ptr(), N.stream()), "train_squares")
+        N.count()
+    return part.sum(1)
+
+
+def scale(tensors: Sequence[torch.Tensor], c: float) -> None:
+    """All of them times ``c``, in place (plain ones)."""
+    tensors = list(tensors)
+    for i in range(0, len(tensors), MAX_TENSORS):
+        some = tensors[i:i + MAX_TENSORS]
+        N.check(N.lib().trl_train_scale(_pointers(some), _lengths(some), len(some), c, N.stream()), "train_scale")
+        torch.autograd.graph.increment_version(some)
+        N.count()

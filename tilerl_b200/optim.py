@@ -33,10 +33,17 @@ def clip_grad_norm(grads: Dict[str, torch.Tensor], max_norm: float, *, sharded: 
     summed across ranks while replicated tensors are counted once: one all-reduce
     of two numbers in fp64."""
     dev = next(iter(grads.values())).device if grads else torch.device("cpu")
+    many = None
+    if dev.type == "cuda":
+        from .ops import train_kernels as many
+        parts = many.squares(grads)
+        many = many if parts is not None else None
     sh = torch.zeros((), dtype=torch.float64, device=dev)
     rep = torch.zeros((), dtype=torch.float64, device=dev)
-    for k, g in grads.items():
-        s = g.double().pow(2).sum()
+    if many and sharded is None:
+        rep += parts.sum()
+    for i, (k, g) in enumerate(grads.items() if not many or sharded is not None else ()):
+        s = parts[i] if many else g.double().pow(2).sum()
         if sharded is not None and sharded(k):
             sh += s
         else:
@@ -54,8 +61,11 @@ def clip_grad_norm(grads: Dict[str, torch.Tensor], max_norm: float, *, sharded: 
     norm = math.sqrt(total)
     if max_norm > 0 and norm > max_norm:
         c = max_norm / (norm + 1e-6)
-        for g in grads.values():
-            g.mul_(c)
+        if many:
+            many.scale(grads.values(), c)
+        else:
+            for g in grads.values():
+                g.mul_(c)
     return norm
 
 
@@ -90,8 +100,23 @@ class AdamW:
         p.copy_(w.to(p.dtype))
 
     def step(self, grads: Dict[str, torch.Tensor], lr: Optional[float] = None) -> None:
+        items, rate, (b1, b2) = [], self.lr if lr is None else lr, self.betas
         for k, g in grads.items():
-            self.step_param(k, g, lr)
+            p = self.params[k]
+            if not (p.is_cuda and p.dtype == torch.float32):
+                self.step_param(k, g, lr)
+                continue
+            from .ops import train_kernels
+            if k not in self.m:
+                self.m[k], self.v[k], self.t[k] = torch.zeros_like(p), torch.zeros_like(p), 0
+            if not train_kernels.plain(p, g, self.m[k], self.v[k]) or g.shape != p.shape:
+                self.step_param(k, g, lr)
+                continue
+            self.t[k] += 1
+            t = self.t[k]
+            items.append((p, self.m[k], self.v[k], g, 1 - rate * self.wd if self.wd and p.dim() >= 2 else 1.0, 1 - b1 ** t, 1 - b2 ** t))
+        if items:
+            train_kernels.adamw(items, rate, self.betas, self.eps)
 
     def state_dict(self) -> Dict[str, object]:
         return dict(m=self.m, v=self.v, t=self.t, lr=self.lr)

@@ -123,6 +123,14 @@ def _nograd(fn):
     return wrapped
 
 
+def _kernels(x: torch.Tensor):
+    """The CUDA kernels of the ops below for a tensor on the GPU; each says which shapes it takes, the torch forms serve the rest."""
+    if not x.is_cuda:
+        return None
+    from .ops import train_kernels
+    return train_kernels
+
+
 @_nograd
 def embedding(tape: Tape, table: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
     out = table[ids.long()].float()
@@ -139,6 +147,18 @@ def embedding(tape: Tape, table: torch.Tensor, ids: torch.Tensor) -> torch.Tenso
 
 @_nograd
 def rmsnorm(tape: Tape, x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
+    K = _kernels(x)
+    if K is not None and K.rmsnorm_takes(x, w):
+        out = K.rmsnorm(x, w, eps)
+
+        def bwd_kernel(g):
+            gw = None
+            if id(w) in tape.leaves:
+                gw = (g.float() * x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps)).reshape(-1, x.shape[-1]).sum(0)
+            return K.rmsnorm_grad(x, w, g, eps), gw
+
+        tape.record("rmsnorm", (x, w), (out,), bwd_kernel)
+        return out
     xf = x.float()
     rstd = torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)
     xn = xf * rstd
@@ -223,6 +243,11 @@ def scale(tape: Tape, a: torch.Tensor, s: float) -> torch.Tensor:
 
 @_nograd
 def swiglu(tape: Tape, gu: torch.Tensor) -> torch.Tensor:
+    K = _kernels(gu)
+    if K is not None and K.swiglu_takes(gu):
+        out = K.swiglu(gu)
+        tape.record("swiglu", (gu,), (out,), lambda g: (K.swiglu_grad(gu, g),))
+        return out
     g_, u_ = gu[..., 0::2].float(), gu[..., 1::2].float()
     sig = torch.sigmoid(g_)
     out = g_ * sig * u_
@@ -245,6 +270,13 @@ def attention_block(tape: Tape, qkv: torch.Tensor, q_norm_w: torch.Tensor, k_nor
     hand (softmax Jacobian, RoPE transpose rotation, RMSNorm).  With a context-parallel
     ``cp`` the rotated K, V and their absolute positions are all-gathered over the ranks
     (the mask compares absolute positions) and dK / dV are reduce-scattered in backward."""
+    K = _kernels(qkv)
+    if K is not None and cp is None and id(q_norm_w) not in tape.leaves and id(k_norm_w) not in tape.leaves and K.attention_takes(
+            qkv, q_norm_w, k_norm_w, positions, n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim, gated=gated):
+        out, grad = K.attention(qkv, q_norm_w, k_norm_w, positions, n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim,
+                                theta=theta, eps=eps, gated=gated)
+        tape.record("attention", (qkv, q_norm_w, k_norm_w), (out,), lambda g: (grad(g), None, None))
+        return out
     b, t, _ = qkv.shape
     d, g = head_dim, n_q // n_kv
     x = qkv.float()
@@ -440,6 +472,13 @@ def cross_entropy(tape: Tape, logits: torch.Tensor, targets: torch.Tensor,
     """``sum_i w_i * nll_i`` over flattened rows; the gradient is produced together
     with the loss (the form used by SFT and by the policy-gradient step)."""
     lg = logits.reshape(-1, logits.shape[-1])
+    K = _kernels(logits)
+    if K is not None and K.cross_entropy_takes(logits, targets, weights):
+        # the gradient is written once, in the backward pass, from each row's largest value and sum
+        tg, w, stats = targets.reshape(-1).long().contiguous(), weights.reshape(-1).float().contiguous(), K.lse(lg)
+        loss = (w * (stats[2] - lg.gather(-1, tg[:, None]).squeeze(-1))).sum()
+        tape.record("cross_entropy", (logits,), (loss,), lambda g: (K.cross_entropy_grad(lg, stats, tg, w, g).view_as(logits),))
+        return loss
     loss, grad = ref.cross_entropy_grad(lg, targets.reshape(-1), weights.reshape(-1).float())
     grad = grad.view_as(logits)
     tape.record("cross_entropy", (logits,), (loss,), lambda g: (grad * g,))
@@ -556,6 +595,16 @@ def all_reduce(tape: Tape, x: torch.Tensor) -> torch.Tensor:
 def lora(tape: Tape, y: torch.Tensor, x: torch.Tensor, a: torch.Tensor, b: torch.Tensor,
          s: float) -> torch.Tensor:
     """``y + s * (x A^T) B^T`` with gradients for x, A and B."""
+    K = _kernels(y)
+    if K is not None and K.lora_takes(y, x, a, b):
+        out, xa = K.lora(y, x, a, b, s)
+
+        def bwd_kernel(g):
+            g = K._grad(g)
+            return (g,) + K.lora_grad(x, xa, a, b, s, g)
+
+        tape.record("lora", (y, x, a, b), (out,), bwd_kernel)
+        return out
     xa = x.float() @ a.float().t()
     out = y + (xa @ b.float().t()) * s
 
