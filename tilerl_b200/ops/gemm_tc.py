@@ -20,7 +20,7 @@ from . import native as N
 N.register("trl_quant_act_nvfp4", [N.P, N.I, N.P, N.F, N.P, N.P, N.P, N.I, N.I, N.I, N.I, N.P])
 N.register("trl_gemm_nvfp4", [N.P, N.P, N.P, N.P, N.P, N.P, N.P, N.I, N.P, N.I, N.P, N.P, N.L,
                               N.I, N.I, N.I, N.I, N.I, N.I, N.I, N.I, N.P])
-N.register("trl_gemm_nvfp4_scratch_bytes", [N.I, N.I, N.I, N.I, N.I, N.I])
+N.register("trl_gemm_nvfp4_scratch_bytes", [N.I, N.I, N.I, N.I, N.I, N.I], N.L)
 N.register("trl_gemv_stream_bytes", [N.I, N.I])
 N.register("trl_gemv_stream_pack", [N.P, N.P, N.P, N.I, N.I, N.P])
 N.register("trl_gemv2_nvfp4", [N.P, N.I, N.P, N.P, N.P, N.F, N.P, N.I, N.P, N.I, N.I, N.I, N.I, N.I, N.P])
@@ -171,7 +171,6 @@ def gemm_nvfp4(ops, x: torch.Tensor, w: NVFP4Tensor, y: torch.Tensor, *, terms: 
         bn *= 2
     c_tiles = (cols + bn - 1) // bn
     n_tiles = (n + 127) // 128
-    ops.lib.trl_gemm_nvfp4_scratch_bytes.restype = __import__("ctypes").c_long
     split = _want_split() if split is None else int(split)
     nbytes = ops.lib.trl_gemm_nvfp4_scratch_bytes(t, terms, n, k, max_ctas, split)
     partial, counters = _scratch(ops, nbytes, n_tiles * c_tiles)

@@ -200,13 +200,15 @@ def _pylib():
     return _PYLIB
 
 
-def register(name: str, sig) -> None:
+def register(name: str, sig, restype=c_int) -> None:
     """Declare the signature of an entry point defined by another source file."""
     _SIGS[name] = sig
+    if restype is not c_int:
+        _RESTYPE[name] = restype
     if _LIB is not None and hasattr(_LIB, name):
         fn = getattr(_LIB, name)
         fn.argtypes = sig
-        fn.restype = c_int
+        fn.restype = restype
 
 
 class KernelError(RuntimeError):
@@ -223,7 +225,13 @@ def ptr(t) -> Optional[int]:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device, as ``torch.cuda.current_stream().cuda_stream`` (which builds an object a
+    call, 6 us; an eager tick of the 27B model asks 40 times for every four layers)."""
+    return _raw_stream(_device()) if torch.cuda.is_initialized() else torch.cuda.current_stream().cuda_stream
+
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", lambda d: torch.cuda.current_stream(d).cuda_stream)
+_device = getattr(torch._C, "_cuda_getDevice", lambda: torch.cuda.current_device())
 
 
 def read_error(clear: bool = True):
