@@ -104,17 +104,17 @@ __device__ __forceinline__ void gp_mma(uint32_t d_tmem, uint32_t alo, uint32_t b
       ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory");
 }
 
-// Eight finished values of a row block and token, out.
-__device__ __forceinline__ void gp_store8(const PairParams& p, int tok, int row, float4 lo, float4 hi, uint4 res) {
+// Eight values of a row block and token, times s, out.
+__device__ __forceinline__ void gp_store8(const PairParams& p, int tok, int row, float4 lo, float4 hi, float s, uint4 res) {
   if (p.epi == GP_SWIGLU) {                          // rows in (gate, up) pairs
-    auto act = [](float g, float u) { return __fdividef(g, 1.f + __expf(-g)) * u; };
+    auto act = [s](float g, float u) { return __fdividef(g * s, 1.f + __expf(-(g * s))) * (u * s); };
     *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(p.out) + (size_t)tok * p.ldo + (row >> 1)) =
         make_uint2(f2_to_bf162_bits(act(lo.x, lo.y), act(lo.z, lo.w)), f2_to_bf162_bits(act(hi.x, hi.y), act(hi.z, hi.w)));
     return;
   }
   const float2 a = bf162_bits_to_f2(res.x), b = bf162_bits_to_f2(res.y), c = bf162_bits_to_f2(res.z), d = bf162_bits_to_f2(res.w);
-  lo = make_float4(lo.x + a.x, lo.y + a.y, lo.z + b.x, lo.w + b.y);          // (no residual: zeros)
-  hi = make_float4(hi.x + c.x, hi.y + c.y, hi.z + d.x, hi.w + d.y);
+  lo = make_float4(fmaf(lo.x, s, a.x), fmaf(lo.y, s, a.y), fmaf(lo.z, s, b.x), fmaf(lo.w, s, b.y));      // (no residual: zeros)
+  hi = make_float4(fmaf(hi.x, s, c.x), fmaf(hi.y, s, c.y), fmaf(hi.z, s, d.x), fmaf(hi.w, s, d.y));
   if (p.epi == GP_STORE_F32) {
     float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (size_t)tok * p.ldo + row);
     o[0] = lo, o[1] = hi;
@@ -299,10 +299,14 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         }
 #pragma unroll
         for (int t = 0; t < TPC; ++t) {
-          float a = 0.f;                             // a token's terms, the smallest first
+          // a token's terms: two in their order, as the one-SM kernel adds them (whole tiles: the same bits), four the smallest first
+          float a = 0.f;
 #pragma unroll
-          for (int j = J - 1; j >= 0; --j) a = fmaf(__uint_as_float(r[t * J + j]), rs_s[t * J + j], a);
-          a *= ts;
+          for (int i = 0; i < J; ++i) {
+            const int j = J == 4 ? J - 1 - i : i;
+            a = fmaf(__uint_as_float(r[t * J + j]), rs_s[t * J + j], a);
+          }
+          if (SPLIT || J == 4) a *= ts;
           if (SPLIT) sum[(size_t)(half * (C::COLS_WARP / J) + c * TPC + t) * GP_ROWS + quad * 32 + lane] = a;
           else tr[t * GP_TR_STRIDE + lane] = a;
         }
@@ -312,7 +316,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
           for (int i = 0; i < VECS; ++i) {
             const int t = (i * 32 + lane) >> 2, tok = tok0 + c * TPC + t, row = n0 + (lane & 3) * 8;
             const float4* v = reinterpret_cast<const float4*>(tr + t * GP_TR_STRIDE + (lane & 3) * 8);
-            if (tok < p.tokens && row < p.N) gp_store8(p, tok, row, v[0], v[1], res[c][i]);
+            if (tok < p.tokens && row < p.N) gp_store8(p, tok, row, v[0], v[1], J == 4 ? 1.f : ts, res[c][i]);
           }
           __syncwarp();
         }
@@ -336,7 +340,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         lo.x += a.x, lo.y += a.y, lo.z += a.z, lo.w += a.w;
         hi.x += b.x, hi.y += b.y, hi.z += b.z, hi.w += b.w;
       }
-      gp_store8(p, tok, row, lo, hi, res);
+      gp_store8(p, tok, row, lo, hi, 1.f, res);
     }
   }
 
