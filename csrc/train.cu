@@ -80,15 +80,16 @@ __global__ void __launch_bounds__(256) tr_swiglu_grad_kernel(const float* gu, co
 }
 
 // ---- adapters of rank up to 32 ---------------------------------------------------------------------------------------
-// out [M, R] = scale * x [M, K] . A, A(k, r) = a[r][k] or (by_k) a[k][r].  Four warps a block, four rows a warp, the lanes share K; 16
-// ranks a block's y, their factors staged 128 k at a time, rows and factors of the next 128 on their way meanwhile (in the open,
-// 2048 x 6144 took 100 us).
-constexpr int LR = 16, LR_T = 128;
-__global__ void __launch_bounds__(128) tr_lowrank_kernel(const float* x, const float* a, float* out, int M, int K, int R, int by_k, float scale) {
-  __shared__ __align__(16) float s[2][LR][LR_T + 4];
-  const int lane = threadIdx.x & 31, row0 = blockIdx.x * 16 + (threadIdx.x >> 5) * 4, r0 = blockIdx.y * LR;
+// out [M, R] = scale * x [M, K] . A, A(k, r) = a[r][k] or (by_k) a[k][r].  Sixteen rows a block: four rows a warp, two groups of four
+// warps that take every other 128 k and are added up at the end, the lanes share K; 16 ranks a block's y, their factors staged,
+// rows and factors of a group's next 128 on their way meanwhile.  2048 x 6144: 100 us with the loads in the open, 45 with one
+// group, and what the rows take to read is 8.
+constexpr int LR = 16, LR_T = 128, LR_S = LR_T + 4;
+__global__ void __launch_bounds__(256) tr_lowrank_kernel(const float* x, const float* a, float* out, int M, int K, int R, int by_k, float scale) {
+  __shared__ __align__(16) float s[2][2][LR][LR_S];
+  const int group = threadIdx.x >> 7, tid = threadIdx.x & 127, lane = tid & 31, row0 = blockIdx.x * 16 + (tid >> 5) * 4, r0 = blockIdx.y * LR;
   // the factors this thread stages: by_k, 4 ranks of four k (R % 4 == 0), else 4 k of four ranks
-  const int fr = by_k ? (threadIdx.x & 3) * 4 : threadIdx.x >> 5, fk = by_k ? threadIdx.x >> 2 : lane * 4;
+  const int fr = by_k ? (tid & 3) * 4 : tid >> 5, fk = by_k ? tid >> 2 : lane * 4;
   float4 v[4], f[4];
   float acc[4][LR] = {};
   auto fetch = [&](int k0) {
@@ -99,68 +100,95 @@ __global__ void __launch_bounds__(128) tr_lowrank_kernel(const float* x, const f
       f[m] = q < R && k < K ? ld4(a + (by_k ? (size_t)k * R + q : (size_t)q * K + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   };
-  fetch(0);
-  for (int k0 = 0, b = 0; k0 < K; k0 += LR_T, b ^= 1) {
+  if (group * LR_T < K) fetch(group * LR_T);
+  for (int k0 = group * LR_T, b = 0; k0 < K; k0 += 2 * LR_T, b ^= 1) {
     float4 now[4];
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
       now[m] = v[m];
       if (by_k) {
-        float* d = &s[b][fr][fk + 32 * m];
-        d[0] = f[m].x, d[LR_T + 4] = f[m].y, d[2 * (LR_T + 4)] = f[m].z, d[3 * (LR_T + 4)] = f[m].w;
+        float* d = &s[group][b][fr][fk + 32 * m];
+        d[0] = f[m].x, d[LR_S] = f[m].y, d[2 * LR_S] = f[m].z, d[3 * LR_S] = f[m].w;
       } else {
-        st4(&s[b][fr + 4 * m][fk], f[m]);
+        st4(&s[group][b][fr + 4 * m][fk], f[m]);
       }
     }
-    __syncthreads();                                // (the other half was read before the barrier of the tile before)
-    if (k0 + LR_T < K) fetch(k0 + LR_T);
+    asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory");     // (the other half was read before the barrier of the tile before)
+    if (k0 + 2 * LR_T < K) fetch(k0 + 2 * LR_T);
 #pragma unroll
     for (int r = 0; r < LR; ++r) {
-      const float4 w = ld4(&s[b][r][lane * 4]);
+      const float4 w = ld4(&s[group][b][r][lane * 4]);
 #pragma unroll
       for (int m = 0; m < 4; ++m) acc[m][r] += dot4(now[m], w);
     }
   }
+  __syncthreads();
+  float* other = &s[0][0][0][0];                    // the second group's sums: [16 rows][16 ranks]
 #pragma unroll
   for (int m = 0; m < 4; ++m)
 #pragma unroll
     for (int r = 0; r < LR; ++r) {
-      const float t = warp_sum(acc[m][r]);
-      if (lane == r && row0 + m < M && r0 + r < R) out[(size_t)(row0 + m) * R + r0 + r] = t * scale;
+      acc[m][r] = warp_sum(acc[m][r]);
+      if (group == 1 && lane == r) other[((tid >> 5) * 4 + m) * LR + r] = acc[m][r];
     }
+  __syncthreads();
+  if (group == 1) return;
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+#pragma unroll
+    for (int r = 0; r < LR; ++r)
+      if (lane == r && row0 + m < M && r0 + r < R) out[(size_t)(row0 + m) * R + r0 + r] = (acc[m][r] + other[((tid >> 5) * 4 + m) * LR + r]) * scale;
 }
 
-// out [M, N] = base + scale * z [M, R] . b, b(r, n) = b[n][r] or (by_r) b[r][n]; base may be null.  A thread four columns (two from
-// rank 32 on), their factors in registers, 16 rows a block.
+// out [M, N] = base + scale * z [M, R] . b, b(r, n) = b[n][r] or (by_r) b[r][n]; base may be null, or bf16 (a dense product's result).
+// A thread four columns (two from rank 32 on), their factors in registers, 16 rows a block, four of them on their way.  Measured
+// against it and slower: eight rows on their way and 32 a block (29.6 us a call of a training step, 23.5 here), factors in shared memory.
+constexpr int EX_ROWS = 16;
 template <int R>
-__global__ void __launch_bounds__(128) tr_expand_kernel(const float* base, const float* z, const float* b, float* out, int M, int N, int by_r, float scale) {
-  constexpr int W = R > 16 ? 2 : 4, ROWS = 16;
-  __shared__ __align__(16) float s[ROWS][R];
-  const int n = (blockIdx.x * 128 + threadIdx.x) * W, m0 = blockIdx.y * ROWS, rows = min(ROWS, M - m0);
+__global__ void __launch_bounds__(128) tr_expand_kernel(const float* base, const bf16* base16, const float* z, const float* b, float* out, int M, int N,
+                                                        int by_r, float scale) {
+  constexpr int W = R > 16 ? 2 : 4;
+  __shared__ __align__(16) float s[EX_ROWS][R];
+  const int n = (blockIdx.x * 128 + threadIdx.x) * W, m0 = blockIdx.y * EX_ROWS, rows = min(EX_ROWS, M - m0);
   for (int i = threadIdx.x; i < rows * R; i += 128) s[i / R][i % R] = z[(size_t)m0 * R + i];
   float f[W][R];
+  if (!by_r) {
 #pragma unroll
-  for (int w = 0; w < W; ++w)
+    for (int w = 0; w < W; ++w)
 #pragma unroll
-    for (int r = 0; r < R; r += 4)
-      if (!by_r) {
+      for (int r = 0; r < R; r += 4) {
         const float4 v = n < N ? ld4(b + (size_t)(n + w) * R + r) : make_float4(0.f, 0.f, 0.f, 0.f);
         f[w][r] = v.x, f[w][r + 1] = v.y, f[w][r + 2] = v.z, f[w][r + 3] = v.w;
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) f[w][r + q] = n < N ? b[(size_t)(r + q) * N + n + w] : 0.f;
       }
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (n < N && W == 4) v = ld4(b + (size_t)r * N + n);
+      else if (n < N) v.x = b[(size_t)r * N + n], v.y = b[(size_t)r * N + n + 1];
+      f[0][r] = v.x, f[1][r] = v.y;
+      if (W == 4) f[2 % W][r] = v.z, f[3 % W][r] = v.w;
+    }
+  }
   __syncthreads();
   if (n >= N) return;
   for (int m = 0; m < rows; m += 4) {
     float y[4][W];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int w = 0; w < W; w += 2) {
-        const float2 v = base && m + q < rows ? *reinterpret_cast<const float2*>(base + (size_t)(m0 + m + q) * N + n + w) : make_float2(0.f, 0.f);
-        y[q][w] = v.x, y[q][w + 1] = v.y;
+    for (int q = 0; q < 4; ++q) {
+      const size_t at = (size_t)(m0 + m + q) * N + n;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (m + q < rows && base) {
+        if (W == 4) v = ld4(base + at);
+        else v.x = base[at], v.y = base[at + 1];
+      } else if (m + q < rows && base16) {
+        const uint2 u = W == 4 ? *reinterpret_cast<const uint2*>(base16 + at) : make_uint2(*reinterpret_cast<const uint32_t*>(base16 + at), 0u);
+        const float2 lo = bf162_bits_to_f2(u.x), hi = bf162_bits_to_f2(u.y);
+        v = make_float4(lo.x, lo.y, hi.x, hi.y);
       }
+      y[q][0] = v.x, y[q][1] = v.y;
+      if (W == 4) y[q][2 % W] = v.z, y[q][3 % W] = v.w;
+    }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (m + q >= rows) break;
@@ -173,8 +201,10 @@ __global__ void __launch_bounds__(128) tr_expand_kernel(const float* base, const
           t[w] = fmaf(v.x, f[w][r], t[w]), t[w] = fmaf(v.y, f[w][r + 1], t[w]), t[w] = fmaf(v.z, f[w][r + 2], t[w]), t[w] = fmaf(v.w, f[w][r + 3], t[w]);
       }
 #pragma unroll
-      for (int w = 0; w < W; w += 2)
-        *reinterpret_cast<float2*>(out + (size_t)(m0 + m + q) * N + n + w) = make_float2(fmaf(t[w], scale, y[q][w]), fmaf(t[w + 1], scale, y[q][w + 1]));
+      for (int w = 0; w < W; ++w) t[w] = fmaf(t[w], scale, y[q][w]);
+      float* o = out + (size_t)(m0 + m + q) * N + n;
+      if (W == 4) st4(o, make_float4(t[0], t[1], t[2 % W], t[3 % W]));
+      else *reinterpret_cast<float2*>(o) = make_float2(t[0], t[1]);
     }
   }
 }
@@ -191,7 +221,7 @@ __global__ void __launch_bounds__(128) tr_outer_kernel(const float* v, const flo
     for (int i = threadIdx.x; i < cnt * R; i += 128) s[i / R][i % R] = z[(size_t)m0 * R + i];
     __syncthreads();
     if (n < N)
-#pragma unroll 8
+#pragma unroll 16
       for (int m = 0; m < cnt; ++m) {
         const float x = v[(size_t)(m0 + m) * N + n];
 #pragma unroll
@@ -480,12 +510,12 @@ TRL_API int trl_train_swiglu(const void* gu, const void* up, void* out, long n, 
   }
 TRL_API int trl_train_lowrank(const void* x, const void* a, void* out, int M, int K, int R, int by_k, float scale, void* stream) {
   if (M < 1 || K < 4 || K % 4 || R < 4 || R % 4) return (int)cudaErrorInvalidValue;
-  tr_lowrank_kernel<<<dim3((M + 15) / 16, (R + LR - 1) / LR), 128, 0, (cudaStream_t)stream>>>((const float*)x, (const float*)a, (float*)out, M, K, R, by_k, scale);
+  tr_lowrank_kernel<<<dim3((M + 15) / 16, (R + LR - 1) / LR), 256, 0, (cudaStream_t)stream>>>((const float*)x, (const float*)a, (float*)out, M, K, R, by_k, scale);
   return (int)cudaGetLastError();
 }
-TRL_API int trl_train_expand(const void* base, const void* z, const void* b, void* out, int M, int N, int R, int by_r, float scale, void* stream) {
-  if (M < 1 || N < 4 || N % 4 || (M + 15) / 16 > 65535) return (int)cudaErrorInvalidValue;
-  BY_RANK((tr_expand_kernel<RR><<<dim3((N / (RR > 16 ? 2 : 4) + 127) / 128, (M + 15) / 16), 128, 0, (cudaStream_t)stream>>>((const float*)base, (const float*)z, (const float*)b,
+TRL_API int trl_train_expand(const void* base, int bf16_base, const void* z, const void* b, void* out, int M, int N, int R, int by_r, float scale, void* stream) {
+  if (M < 1 || N < 4 || N % 4 || (M + EX_ROWS - 1) / EX_ROWS > 65535) return (int)cudaErrorInvalidValue;
+  BY_RANK((tr_expand_kernel<RR><<<dim3((N / (RR > 16 ? 2 : 4) + 127) / 128, (M + EX_ROWS - 1) / EX_ROWS), 128, 0, (cudaStream_t)stream>>>(bf16_base ? nullptr : (const float*)base, bf16_base ? (const bf16*)base : nullptr, (const float*)z, (const float*)b,
                                                                                                         (float*)out, M, N, by_r, scale)))
   return (int)cudaGetLastError();
 }

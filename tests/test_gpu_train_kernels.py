@@ -93,6 +93,31 @@ def test_adapters(m, k, n, r):
     _both(lambda t, y, x, a, b: T.lora(t, y, x, a, b, 0.7), (*m, n), (*m, k), (r, k), (n, r), seed=n)
 
 
+@pytest.mark.parametrize("m,k,n,r", [((3, 11), 64, 132, 16), ((700,), 1024, 516, 8)])
+@pytest.mark.parametrize("quantised", [True, False])
+def test_frozen_linear_with_adapter(m, k, n, r, quantised):
+    """One op against the two it stands for, on the same device: the dense products are the same calls, sums around them in another
+    order."""
+    from tilerl_b200 import formats as F
+    from tilerl_b200 import tape as T
+    from tilerl_b200.ops.cuda import CudaOps
+    CudaOps(DEV)                                      # installs the weights' decoder
+    g = torch.Generator().manual_seed(n)
+    w = torch.randn(n, k, generator=g) * 0.05
+    w = F.quantize_nvfp4(w).to(DEV) if quantised else w.to(DEV)
+    x, a, b, up = (torch.randn(*s, generator=g).to(DEV) for s in ((*m, k), (r, k), (n, r), (*m, n)))
+    res = []
+    for one in (True, False):
+        tape = T.Tape()
+        tape.watch(x, a, b)
+        y = T.linear_lora(tape, x, w, True, a, b, 0.5) if one else T.lora(tape, T.linear(tape, x, w, frozen=True), x, a, b, 0.5)
+        assert len(tape.nodes) == (1 if one else 2)
+        gs = tape.backward(y, up)
+        res.append([y] + [gs[id(t)] for t in (x, a, b)])
+    for got, want in zip(*res):
+        assert _rel(got, want) < 1e-6
+
+
 @pytest.mark.parametrize("b,t,n_q,n_kv,d,rot,gated", [(1, 1, 1, 1, 4, 2, True), (2, 33, 4, 2, 64, 32, True), (1, 300, 6, 1, 256, 64, True), (2, 40, 2, 2, 512, 512, False)])
 def test_attention_block(b, t, n_q, n_kv, d, rot, gated):
     """Positions as they come, shared and one row a sequence out of order; heads narrower than a warp and the widest."""

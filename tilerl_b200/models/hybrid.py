@@ -287,11 +287,10 @@ class HybridModel:
     def _tlinear(self, tape, x, name: str):
         from .. import tape as T
         w, frozen = self._w(name)
-        y = T.linear(tape, x, w, frozen=frozen)
         lo = self.lora.get(name)
         if lo is not None:
-            y = T.lora(tape, y, x, lo[0], lo[1], lo[2])
-        return y
+            return T.linear_lora(tape, x, w, frozen, lo[0], lo[1], lo[2])
+        return T.linear(tape, x, w, frozen=frozen)
 
     def forward_dense(self, tape, ids: torch.Tensor, *, checkpoint_layers: bool = False,
                       positions: Optional[torch.Tensor] = None, hook=None, cp=None,

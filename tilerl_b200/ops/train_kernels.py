@@ -13,7 +13,7 @@ N.register("trl_train_rmsnorm", [N.P] * 3 + [N.I] * 2 + [N.F, N.P])
 N.register("trl_train_rmsnorm_grad", [N.P] * 4 + [N.I] * 2 + [N.F, N.P])
 N.register("trl_train_swiglu", [N.P] * 3 + [N.L, N.P])
 N.register("trl_train_lowrank", [N.P] * 3 + [N.I] * 4 + [N.F, N.P])
-N.register("trl_train_expand", [N.P] * 4 + [N.I] * 4 + [N.F, N.P])
+N.register("trl_train_expand", [N.P, N.I] + [N.P] * 3 + [N.I] * 4 + [N.F, N.P])
 N.register("trl_train_outer_parts", [N.I] * 2)
 N.register("trl_train_outer", [N.P] * 4 + [N.I] * 4 + [N.F, N.P])
 N.register("trl_train_attn_prep", [N.P] * 8 + [N.I] * 8 + [N.F, N.P])
@@ -83,23 +83,24 @@ def swiglu_grad(gu, g):
 
 # ---- adapters: y + s (x A^T) B^T -----------------------------------------------------------------------------
 def lora_takes(y, x, a, b) -> bool:
+    """``y`` may be ``None`` (a dense product's bf16 result to come)."""
     r, k = a.shape
-    return (r in (4, 8, 16, 32) and k % 4 == 0 and b.shape[0] % 4 == 0 and b.shape[1] == r and x.shape[-1] == k and y.shape[-1] == b.shape[0]
-            and x.shape[:-1] == y.shape[:-1] and plain(y, x, a, b) and x.numel() // k <= 16 * 65535)
+    return (r in (4, 8, 16, 32) and k % 4 == 0 and b.shape[0] % 4 == 0 and b.shape[1] == r and x.shape[-1] == k and plain(x, a, b)
+            and x.numel() // k <= 16 * 65535 and (y is None or (y.shape[-1] == b.shape[0] and x.shape[:-1] == y.shape[:-1] and plain(y))))
 
 
 def lora(y, x, a, b, s):
-    """The result, and ``x A^T`` for the gradient."""
+    """The result, and ``x A^T`` for the gradient.  ``y``: fp32, or bf16 as a dense product leaves it."""
     (r, k), n, m = a.shape, b.shape[0], x.numel() // x.shape[-1]
-    xa, out = torch.empty(m, r, dtype=torch.float32, device=x.device), torch.empty_like(y)
+    xa, out = torch.empty(m, r, dtype=torch.float32, device=x.device), torch.empty(y.shape, dtype=torch.float32, device=y.device)
     N.check(N.lib().trl_train_lowrank(x.data_ptr(), a.data_ptr(), xa.data_ptr(), m, k, r, 0, 1.0, N.stream()), "train_lowrank")
-    N.check(N.lib().trl_train_expand(y.data_ptr(), xa.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, r, 0, s, N.stream()), "train_expand")
+    N.check(N.lib().trl_train_expand(y.data_ptr(), int(y.dtype == torch.bfloat16), xa.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, r, 0, s, N.stream()), "train_expand")
     N.count(2)
     return out, xa
 
 
-def lora_grad(x, xa, a, b, s, g):
-    """Gradients of (x, a, b) for that of the result."""
+def lora_grad(x, xa, a, b, s, g, dx16=None):
+    """Gradients of (x, a, b) for that of the result; ``dx16``: what is to be added to x's (bf16)."""
     (r, k), n, m = a.shape, b.shape[0], x.numel() // x.shape[-1]
     lib, st = N.lib(), N.stream()
     dxa, dx, da, db = torch.empty_like(xa), torch.empty_like(x), torch.empty_like(a), torch.empty_like(b)
@@ -107,7 +108,7 @@ def lora_grad(x, xa, a, b, s, g):
     N.check(lib.trl_train_lowrank(g.data_ptr(), b.data_ptr(), dxa.data_ptr(), m, n, r, 1, s, st), "train_lowrank")
     N.check(lib.trl_train_outer(g.data_ptr(), xa.data_ptr(), part.data_ptr(), db.data_ptr(), m, n, r, 0, s, st), "train_outer")
     N.check(lib.trl_train_outer(x.data_ptr(), dxa.data_ptr(), part.data_ptr(), da.data_ptr(), m, k, r, 1, 1.0, st), "train_outer")
-    N.check(lib.trl_train_expand(None, dxa.data_ptr(), a.data_ptr(), dx.data_ptr(), m, k, r, 1, 1.0, st), "train_expand")
+    N.check(lib.trl_train_expand(N.ptr(dx16), int(dx16 is not None), dxa.data_ptr(), a.data_ptr(), dx.data_ptr(), m, k, r, 1, 1.0, st), "train_expand")
     N.count(6)
     return dx, da, db
 

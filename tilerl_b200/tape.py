@@ -228,6 +228,25 @@ def linear(tape: Tape, x: torch.Tensor, w, frozen: bool = False) -> torch.Tensor
 
 
 @_nograd
+def linear_lora(tape: Tape, x: torch.Tensor, w, frozen: bool, a: torch.Tensor, b: torch.Tensor, s: float) -> torch.Tensor:
+    """``linear`` and ``lora`` on its result.  On CUDA, over a frozen weight, as one op: the dense products' bf16 results go into
+    the adapters' kernels as they are, without fp32 copies between, and x's gradient is summed there."""
+    K = _kernels(x)
+    if K is None or (isinstance(w, torch.Tensor) and not frozen) or DEQUANT_BF16 is None or not (hasattr(w, "wq") or isinstance(w, torch.Tensor)) \
+            or not K.lora_takes(None, x, a, b) or b.shape[0] != w.shape[0]:
+        return lora(tape, linear(tape, x, w, frozen=frozen), x, a, b, s)
+    wf = DEQUANT_BF16(w) if hasattr(w, "wq") else w.to(torch.bfloat16)
+    out, xa = K.lora(x.to(torch.bfloat16) @ wf.t(), x, a, b, s)
+
+    def bwd(g):
+        g = K._grad(g)
+        return K.lora_grad(x, xa, a, b, s, g, g.to(torch.bfloat16) @ wf)
+
+    tape.record("linear_lora", (x, a, b), (out,), bwd)
+    return out
+
+
+@_nograd
 def add(tape: Tape, a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     out = a + b
     tape.record("add", (a, b), (out,), lambda g: (g, g))
