@@ -32,16 +32,6 @@ struct TcArgs {
   int N, nkb, ldo, act, per_item;
 };
 
-__device__ __forceinline__ void tc_mma_bf16_lh(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{ .reg .pred p; .reg .b64 da, db;\n"
-      "  mov.b64 da, {%1, %3}; mov.b64 db, {%2, %3};\n"
-      "  setp.ne.b32 p, %5, 0;\n"
-      "  tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p; }\n"
-      ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 template <int KIND>
 __global__ void __launch_bounds__(MT_THREADS, 1)
 moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const TcArgs p) {

@@ -159,5 +159,15 @@ __device__ __forceinline__ void tc_mma_f8_lh(uint32_t d_tmem, uint32_t alo, uint
       ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Dense bf16 MMA, fp32 accumulate.
+__device__ __forceinline__ void tc_mma_bf16_lh(uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{ .reg .pred p; .reg .b64 da, db;\n"
+      "  mov.b64 da, {%1, %3}; mov.b64 db, {%2, %3};\n"
+      "  setp.ne.b32 p, %5, 0;\n"
+      "  tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p; }\n"
+      ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 
 }  // namespace

@@ -726,3 +726,22 @@ def test_delta_rule_chunk_kernel_with_and_without_preparing_groups(ops, lens, nk
     for other in got[1:]:
         for a, b in zip(got[0], other):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("m", [9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("n,k", [(130, 72), (999, 1032), (15520, 5120), (40003, 640)])
+def test_logits_of_many_rows(ops, m, n, k):
+    """Every width of a tile, vocabularies that fill none of 128, K that fills no stage and one of many accumulators, more tiles than
+    CTAs, against fp64 from the same normed rows: fp32 sums over K."""
+    from tilerl_b200.ops import native
+    g = torch.Generator().manual_seed(m + n)
+    w, nw = (torch.randn(n, k, generator=g) * 0.02).to(DEV, torch.bfloat16), (1 + 0.1 * torch.randn(k, generator=g)).to(DEV)
+    x = torch.randn(m, k, generator=g).to(DEV, torch.bfloat16)
+    before = native.launch_count
+    got = ops.lm_head(x, nw, w, 1e-6).clone()
+    assert native.launch_count - before == 2 and got.dtype == torch.float32
+    want = ops._rmsnorm(x, nw, 1e-6).double() @ w.double().t()
+    assert _rel(got, want) < 2e-6
+    # few rows and many: within the few roundings of the normed rows' bf16
+    assert _rel(ops.lm_head(x[:4].contiguous(), nw, w, 1e-6), want[:4]) < 2 ** -8
+    assert native.read_error()[0] == 0

@@ -43,6 +43,9 @@ class ChainOp(ctypes.Structure):
                 ("ldx", ctypes.c_int), ("ldr", ctypes.c_int), ("ldy", ctypes.c_int), ("N", ctypes.c_int),
                 ("K", ctypes.c_int), ("epi", ctypes.c_int), ("coop", ctypes.c_int), ("eps", ctypes.c_float)]
 GEMV_MAX_M = 8
+# Rows of bf16 logits that go to the tcgen05 kernel (csrc/head_tc.cu), the lower ones to the kernel for rows: as fast up to 8 rows in a
+# tick of the 27B model (8 sequences 432 us either way), faster there with the small model's short rows (151 us against 160).
+HEAD_MIN_M, HEAD_MAX_M = 9, 64
 MMA_MAX_M = 16     # rows served by the mma.sync NVFP4 kernel (csrc/gemv_mma.cu)
 
 
@@ -611,6 +614,12 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
         m = x.shape[0]
         n = w.shape[0]
         logits = self.ws.get("logits", (m, n), torch.float32)
+        if HEAD_MIN_M <= m <= HEAD_MAX_M and isinstance(w, torch.Tensor) and w.dtype == torch.bfloat16 and w.is_contiguous() \
+                and w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0 and x.dtype == torch.bfloat16:
+            h = self._rmsnorm(x.contiguous(), self._f32(norm_w), eps, name="h_head")
+            N.check(self.lib.trl_head_bf16(h.data_ptr(), w.data_ptr(), logits.data_ptr(), n, m, n, w.shape[1], N.stream()), "head_bf16")
+            N.count()
+            return logits
         if m <= GEMV_MAX_M or (m <= 16 and isinstance(w, torch.Tensor) and w.dtype == torch.bfloat16):
             # bf16 head: up to 16 rows share one pass over the vocabulary matrix (tensor-core GEMV)
             self._gemv(x.contiguous(), w, logits, norm_w=self._f32(norm_w), eps=eps, epi=EPI_STORE_F32)

@@ -28,6 +28,7 @@ _SIGS = {
     "trl_gemv_nvfp4": [P, I, P, P, P, P, F, P, I, P, I, I, I, I, I, P],
     "trl_gemv_bf16_one_pass": [I, I],
     "trl_gemv_bf16": [P, I, P, P, F, P, I, P, I, I, I, I, I, P],
+    "trl_head_bf16": [P, P, P, L, I, I, I, P],
     "trl_set_pdl": [I],
     "trl_trace_read": [P, I, I],
     "trl_error_read": [P, I],
