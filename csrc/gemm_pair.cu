@@ -75,8 +75,12 @@ __device__ __forceinline__ float4 gp_ld_cluster(uint32_t addr) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
+// Not the .aligned forms: the warps come here from loops and branches that their lanes left at different times, and a warp
+// that is not converged would count more than once.
 __device__ __forceinline__ void gp_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+  __syncwarp();
 }
 __device__ __forceinline__ void gp_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
@@ -156,13 +160,16 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // TMEM of a pair is taken by both SMs together: only once both CTAs are known to run (and the other SM's barriers are there).
+  // An allocation that waits for its other half has no limit on its wait, as the mbarriers have.
+  gp_cluster_sync();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(C::TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
-  gp_cluster_sync();                                // the other SM's barriers are there
+  gp_cluster_sync();                                // both halves are allocated
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();
@@ -203,6 +210,11 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         load_x(x_ct, x_kt, st);
         if (++x_kt == k1) { x_kt = k0; if (++x_ct == p.c_tiles) x_ct = 0; }
         if (++st == STAGES) st = 0, ph ^= 1u;
+      }
+      // the last arrivals of the even SM's MMAs on this CTA's barriers, before its memory goes away
+      for (int s = 0; s < pre; ++s) {
+        const int u = units - pre + s;              // the last unit of its stage
+        if (!mbar_wait(empty(u % STAGES), (uint32_t)(u / STAGES) & 1u, abort_flag)) break;
       }
     }
     __syncwarp();
@@ -357,6 +369,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   tc_fence_after();
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::TMEM_COLS) : "memory");
+  gp_cluster_sync();                                // no CTA leaves while the other's half is being given back
 }
 
 typedef CUresult (*EncodeTiledFnP)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
