@@ -11,11 +11,12 @@
 // cluster share a tile along K and add their parts through each other's shared memory, no scratch, no counters, in a fixed
 // order (rules at gemm_tc.cu::plan_pair).  With the quantiser, one-SM form (behind elect.sync too) and here, us:
 //     rows                 8          32          128          512         2000
-//     34 816 x 5120   25.3 21.4   26.2 21.4   42.6  30.4   125  89.7   402  282   (2.5 PFLOP/s counted once a row)
-//     5120 x 17 408   23.7 16.9   22.6 16.8   37.1  24.8   84.7 53.8   230  183
-//     16 480 x 5120   20.1 13.1   20.2 13.4   30.6  18.1   52.3 45.8   169  142
-//     5120 x 6144     14.8  8.7   15.5  9.5   28.3  12.2   45.1 23.1   117   60
-//     1024 x 3072      8.4  7.4    8.5  6.9   23.3   7.8   29.6  9.8    29   19   (3, 16, 128, 512, 2000 rows)
+//     34 816 x 5120   25.3 21.4   26.2 21.5   42.6  30.8   125  90.4   402  283   (2.5 PFLOP/s counted once a row)
+//     5120 x 17 408   23.7 17.0   22.6 16.6   37.1  24.5   84.7 53.5   230  186
+//     16 480 x 5120   20.1 13.4   20.2 13.7   30.6  18.3   52.3 46.6   169  142
+//     5120 x 6144     14.8  9.7   15.5  9.8   28.3  12.1   45.1 23.6   117   60
+//     1024 x 3072      8.4  7.4    8.5  6.9   23.3   7.8   29.6  9.8    29   19   (3, 16, 128, 512, 2000 rows; without
+//                              the barriers round the TMEM allocation, which the rest has: 0.3 to 1 us a product)
 //
 // Roles (10 warps): warp 0 = TMA producer of its SM's operands (a stage = 256 k; both SMs' copies count on the even one's
 // barrier), warp 1 = TMEM owner and, in the even SM, MMA issuer for both, warps 2-9 = epilogue: two groups of four, each

@@ -976,7 +976,8 @@ TRL_API int trl_gemm_trace_read(void* out, int n_ctas) {
 // columns, 8 rounds against 6: 51.1 and 46.0), one of 64 or 32, where the weights bound, a little less; parts cost the exchange
 // of their sums, more of them more.  5120 x 17 408 with its quantiser, one, two, three parts: 8 rows 22.6, 17.2, 16.3 us;
 // 32 rows 20.9, 16.3, 16.2; 64 rows 23.2, 17.5, 18.4; 96 rows 25.1, 22.0, 21.6 (24.0 in tiles of 128 columns, one part).
-// 5120 x 6144, 8 rows 10.7, 9.8, 9.0; 64 rows 11.4, 11.1, 11.5.
+// 5120 x 6144, 8 rows 10.7, 9.8, 9.0; 64 rows 11.4, 11.1, 11.5.  (All before the barriers round the TMEM allocation, which add
+// 0.3 to 1 us to each; three parts of 5120 x 6144, 8 rows: 9.7.)
 struct PairPlan {
   int bn, parts, pairs;
 };

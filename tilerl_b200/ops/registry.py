@@ -102,7 +102,8 @@ register("nvfp4", "sm100", {
     "linear_nvfp4_rows16": Kernel("gemv_nvfp4_mma_kernel", "csrc/gemv_mma.cu", "trl_gemv_nvfp4_mma",
                                   note="3..16 rows: weights as the mma.sync A operand, f16 activations, every epilogue"),
     "linear_nvfp4_gemm": Kernel("gemm_nvfp4_kernel", "csrc/gemm_tc.cu", "trl_gemm_nvfp4", "tilerl_b200.ops.gemm_tc",
-                                note="tcgen05.mma kind::mxf4nvf4.block_scale, TMA, TMEM accumulator, stream-K"),
+                                note="tcgen05.mma kind::mxf4nvf4.block_scale; on pairs of SMs (gemm_nvfp4_pair_kernel, csrc/gemm_pair.cu) but for forced stream-K, "
+                                     "more than four terms and outputs off 16 bytes"),
     "quant_act_nvfp4": Kernel("quant_act_rows_kernel / quant_act_kernel", "csrc/gemm_tc.cu", "trl_quant_act_nvfp4", "tilerl_b200.ops.gemm_tc",
                               note="RMSNorm / SwiGLU + J NVFP4 residual terms per token"),
     "quantize_nvfp4": Kernel("quant_nvfp4_kernel", "csrc/misc.cu", "trl_quant_nvfp4", note="weights, in place (resync)"),
@@ -112,6 +113,7 @@ register("bf16", "sm100", {
     "linear_bf16_gemv": Kernel("gemv_bf16_kernel", "csrc/gemv.cu", "trl_gemv_bf16"),
     "linear_bf16_gemv_rows16": Kernel("gemv_bf16_rows_kernel", "csrc/gemv.cu", "trl_gemv_bf16",
                                       note="1..16 rows (lm_head): one mma.sync pass over the weights, K shared by a block's warps"),
+    "logits_rows64": Kernel("head_bf16_kernel", "csrc/head_tc.cu", "trl_head_bf16", note="lm_head of 9..64 rows: tcgen05 kind::f16, fp32 results"),
     "linear_stream_rows": Kernel("linear_rows_kernel", "csrc/linear_rows.cu", "trl_linear_rows",
                                  note="few rows out of / into an fp32 stream: norm prologue, cp.async weight ring, mma.sync"),
     "linear_bf16_gemm": Kernel("torch.matmul (cuBLAS)", "tilerl_b200/ops/gemm.py", note="plain library GEMM"),
@@ -159,6 +161,15 @@ register("any", "sm100", {
                           note="greedy accept length + GDN state-plane selection of a verify tick, inside its graph"),
     "lora": Kernel("lora_a_kernel + lora_b_kernel", "csrc/misc.cu", "trl_lora_add"),
     "adamw": Kernel("adamw_kernel", "csrc/misc.cu", "trl_adamw"),
+    "train_adamw": Kernel("tr_adamw_kernel", "csrc/train.cu", "trl_train_adamw", "tilerl_b200.ops.train_kernels", note="up to 32 tensors a launch; squares and scaling of gradients beside it"),
+    "train_rmsnorm": Kernel("tr_rmsnorm_kernel + tr_rmsnorm_grad_kernel", "csrc/train.cu", "trl_train_rmsnorm", "tilerl_b200.ops.train_kernels"),
+    "train_swiglu": Kernel("tr_swiglu_kernel + tr_swiglu_grad_kernel", "csrc/train.cu", "trl_train_swiglu", "tilerl_b200.ops.train_kernels"),
+    "train_lora": Kernel("tr_lowrank_kernel + tr_expand_kernel + tr_outer_kernel", "csrc/train.cu", "trl_train_lowrank", "tilerl_b200.ops.train_kernels", note="ranks 4, 8, 16, 32"),
+    "train_attention": Kernel("tr_attn_prep_kernel + tr_softmax_kernel + tr_attn_gate_kernel", "csrc/train.cu", "trl_train_attn_prep", "tilerl_b200.ops.train_kernels",
+                              note="norms, rotation, masked softmax, gate and their gradients; the products are library GEMMs"),
+    "train_cross_entropy": Kernel("tr_lse_kernel + tr_ce_grad_kernel", "csrc/train.cu", "trl_train_lse", "tilerl_b200.ops.train_kernels"),
+    "train_gdn": Kernel("gt_prep_kernel + gt_chunk_kernel + gt_scan_kernel + gt_norm_kernel", "csrc/gdn_train.cu", "trl_gdn_train_forward", "tilerl_b200.ops.gdn_train",
+                        note="forward and gradient of the block, fp32, chunks of 32, heads of 128"),
     "decode_advance": Kernel("decode_advance_kernel", "csrc/misc.cu", "trl_decode_advance"),
     "zero_all_gather": Kernel("zero_allgather_kernel", "csrc/zero.cu", "trl_zero_allgather", "tilerl_b200.parallel.zero3"),
     "zero_reduce_scatter": Kernel("zero_reduce_scatter_kernel", "csrc/zero.cu", "trl_zero_reduce_scatter",

@@ -79,7 +79,7 @@ def main():
     ap.add_argument("--reps", type=int, default=20)
     ap.add_argument("--shapes", default="")
     ap.add_argument("--max-ctas", type=int, default=0)
-    ap.add_argument("--split", type=int, default=1)
+    ap.add_argument("--split", type=int, default=-1, help="GEMM: 1 stream-K on the one-SM kernel, 0 whole tiles, -1 by the launcher's rule (--trace: 1)")
     ap.add_argument("--tiled", type=int, default=1)
     ap.add_argument("--trace", action="store_true", help="gemm: per-phase timestamps of one launch (median, max over CTAs)")
     ap.add_argument("--ctx", type=int, default=32768, help="attn: context length")
@@ -139,21 +139,22 @@ def main():
             res["gemv_simt_us"] = round(us, 2)
             res["gemv_simt_TBs"] = round(wbytes / us / 1e6, 3)
         if args.only in ("", "gemm"):
-            us = timeit(lambda w: gemm_nvfp4(ops, x, w, y, terms=args.terms, max_ctas=args.max_ctas, split=bool(args.split)))
+            split = 1 if args.trace and args.split < 0 else args.split      # (phase stamps: the one-SM kernel has them)
+            us = timeit(lambda w: gemm_nvfp4(ops, x, w, y, terms=args.terms, max_ctas=args.max_ctas, split=None if split < 0 else bool(split)))
             res["quant+gemm_tc_us"] = round(us, 2)
             res["quant+gemm_tc_TBs"] = round(wbytes / us / 1e6, 3)
             xq, sfx, rs = quant_act(ops, x, k, args.terms)
             from tilerl_b200.ops.gemm_tc import _scratch
             import ctypes
             ops.lib.trl_gemm_nvfp4_scratch_bytes.restype = ctypes.c_long
-            nb = ops.lib.trl_gemm_nvfp4_scratch_bytes(args.m, args.terms, n, k, args.max_ctas, int(args.split))
+            nb = ops.lib.trl_gemm_nvfp4_scratch_bytes(args.m, args.terms, n, k, args.max_ctas, split)
             partial, counters = _scratch(ops, nb, 8192)
 
             def gemm_only(w):
                 native.check(ops.lib.trl_gemm_nvfp4(
                     (w.wq_tiled if args.tiled else w.wq).data_ptr(), w.sf_tiled.data_ptr(), w.tscale.data_ptr(), xq.data_ptr(), sfx.data_ptr(),
                     rs.data_ptr(), None, 0, y.data_ptr(), y.stride(0), partial.data_ptr(), counters.data_ptr(),
-                    partial.numel() * 4, args.m, args.terms, n, k, 0, args.max_ctas, args.split, args.tiled, native.stream()))
+                    partial.numel() * 4, args.m, args.terms, n, k, 0, args.max_ctas, split, args.tiled, native.stream()))
             us = timeit(gemm_only)
             res["gemm_tc_us"] = round(us, 2)
             res["gemm_tc_TBs"] = round(wbytes / us / 1e6, 3)
