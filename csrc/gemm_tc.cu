@@ -974,10 +974,10 @@ TRL_API int trl_gemm_trace_read(void* out, int n_ctas) {
 // the pair form (more than four terms, tiles split over CTAs as asked for, less than a pair of SMs).  Costs in units of a k-tile
 // of 128 columns, 0.2 us: one of 192 takes 1.25 (256 columns of 34 816 x 5120: 31.5 us in tiles of 128, 33.3 of 192; 512
 // columns, 8 rounds against 6: 51.1 and 46.0), one of 64 or 32, where the weights bound, a little less; parts cost the exchange
-// of their sums, more of them more.  5120 x 17 408 with its quantiser, one, two, three parts: 8 rows 22.6, 17.2, 16.3 us;
-// 32 rows 20.9, 16.3, 16.2; 64 rows 23.2, 17.5, 18.4; 96 rows 25.1, 22.0, 21.6 (24.0 in tiles of 128 columns, one part).
-// 5120 x 6144, 8 rows 10.7, 9.8, 9.0; 64 rows 11.4, 11.1, 11.5.  (All before the barriers round the TMEM allocation, which add
-// 0.3 to 1 us to each; three parts of 5120 x 6144, 8 rows: 9.7.)
+// of their sums, more of them more.  With the quantiser, one, two, three parts: 5120 x 17 408, 8 rows 22.7, 18.0, 16.9 us, 32
+// rows 21.1, 16.8, 16.6; 5120 x 6144, 8 rows 10.9, 10.6, 9.8, 32 rows 10.8, 9.8, 9.9; and without the barriers round the TMEM
+// allocation 5120 x 17 408, 64 rows 23.2, 17.5, 18.4, 96 rows 25.1, 22.0, 21.6 (24.0 in tiles of 128 columns, one part);
+// 5120 x 6144, 64 rows 11.4, 11.1, 11.5.
 struct PairPlan {
   int bn, parts, pairs;
 };
