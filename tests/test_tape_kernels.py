@@ -1,0 +1,134 @@
+"""What the tape hands to the training kernels, on the CPU: stand-ins that read as many values as the kernels do take their place."""
+import types
+
+import pytest
+import torch
+
+from tilerl_b200 import tape as T
+from tilerl_b200.ops import gdn_train, ref, train_kernels
+
+
+def _grad_of(fn, g, *xs):
+    with torch.enable_grad():
+        leaves = [x.clone().requires_grad_(True) for x in xs]
+        y = fn(*leaves)
+        return torch.autograd.grad(y, leaves, g)
+
+
+@pytest.fixture
+def kernels(monkeypatch):
+    """A namespace in the place of ``ops.train_kernels``: its checks, and its functions in torch on flat memory of the sizes that the
+    kernels go through.  ``calls`` counts what went to them."""
+    calls = []
+
+    def flat(t, n):
+        calls.append(n)
+        assert t.numel() >= n, "read past the end"
+        return t.reshape(-1)[:n]
+
+    def rmsnorm(x, w, eps):
+        return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * w
+
+    def swiglu(gu):
+        return torch.nn.functional.silu(gu[..., 0::2]) * gu[..., 1::2]
+
+    def lora(y, x, a, b, s):
+        xa = x.reshape(-1, x.shape[-1]) @ a.t()
+        return y.float() + (xa @ b.t()).view(y.shape) * s, xa
+
+    def lora_grad(x, xa, a, b, s, g, dx16=None):
+        m, n = xa.shape[0], b.shape[0]
+        g2 = flat(g, m * n).view(m, n)
+        dxa = g2 @ b * s
+        dx = (dxa @ a).view(x.shape)
+        return dx if dx16 is None else dx + dx16.float(), dxa.t() @ x.reshape(m, -1), g2.t() @ xa * s
+
+    def attention(qkv, qw, kw, pos, **k):
+        out, bwd = T._attention_torch(qkv, qw, kw, pos.to(torch.int64), **k)
+        return out, lambda g: bwd(flat(g, out.numel()).view(out.shape))[0]
+
+    def cross_entropy_grad(lg, stats, tg, w, up):
+        return ref.cross_entropy_grad(lg, tg, w)[1] * flat(up, 1)
+
+    K = types.SimpleNamespace(
+        calls=calls, grad_takes=train_kernels.grad_takes, _grad=train_kernels._grad,
+        rmsnorm_takes=lambda x, w: True, rmsnorm=rmsnorm,
+        rmsnorm_grad=lambda x, w, g, eps: _grad_of(lambda x_: rmsnorm(x_, w, eps), flat(g, x.numel()).view(x.shape), x)[0],
+        swiglu_takes=lambda gu: True, swiglu=swiglu,
+        swiglu_grad=lambda gu, g: _grad_of(swiglu, flat(g, gu.numel() // 2).view(*gu.shape[:-1], -1), gu)[0],
+        lora_takes=lambda y, x, a, b: True, lora=lora, lora_grad=lora_grad,
+        attention_takes=lambda *a, **k: True, attention=attention,
+        cross_entropy_takes=lambda lg, tg, w: True, lse=lambda lg: torch.stack([lg.amax(-1), torch.exp(lg - lg.amax(-1, keepdim=True)).sum(-1), torch.logsumexp(lg, -1)]),
+        cross_entropy_grad=cross_entropy_grad)
+    monkeypatch.setattr(T, "_kernels", lambda x: K)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: None)        # (a CPU tensor's device has no index)
+    return K
+
+
+def _ops():
+    g = torch.Generator().manual_seed(0)
+    r = lambda *s: torch.randn(*s, generator=g)
+    pos = torch.arange(5)
+    return {
+        "rmsnorm": (lambda t, x, w: T.rmsnorm(t, x, w, 1e-6), [r(3, 8), r(8)]),
+        "swiglu": (lambda t, x: T.swiglu(t, x), [r(3, 8)]),
+        "lora": (lambda t, y, x, a, b: T.lora(t, y, x, a, b, 0.5), [r(3, 6), r(3, 8), r(4, 8), r(6, 4)]),
+        "attention": (lambda t, x: T.attention_block(t, x, torch.ones(4), torch.ones(4), pos, n_q=2, n_kv=1, head_dim=4, rotary_dim=4, theta=1e4, eps=1e-6), [r(1, 5, 24)]),
+    }
+
+
+@pytest.mark.parametrize("op", ["rmsnorm", "swiglu", "lora"])
+def test_gradient_that_broadcasts_is_not_read_past_its_end(op, kernels):
+    """A root gradient of one row: no kernel gets it, and what comes back is what the torch form gives (the adapters' refuses it)."""
+    fn, xs = _ops()[op]
+    with torch.no_grad():
+        tape = T.Tape()
+        tape.watch(*xs)
+        y = fn(tape, *xs)
+        one = torch.randn(1, y.shape[-1], generator=torch.Generator().manual_seed(1))
+        if op == "lora":
+            with pytest.raises(RuntimeError):
+                tape.backward(y, one)
+            assert not kernels.calls
+            return
+        got = tape.backward(y, one)
+        assert not kernels.calls
+        whole = T.Tape()
+        whole.watch(*xs)
+        want = whole.backward(fn(whole, *xs), one.expand(y.shape).contiguous())
+        assert kernels.calls
+    for x in xs:
+        assert got[id(x)].shape in (x.shape, one.shape)
+        if got[id(x)].shape == x.shape:
+            assert torch.allclose(got[id(x)], want[id(x)], rtol=1e-5, atol=1e-6)
+
+
+def test_gradient_seen_in_another_shape(kernels):
+    """The attention block's torch form takes a gradient of as many values in another shape."""
+    fn, (x,) = _ops()["attention"]
+    tape = T.Tape()
+    tape.watch(x)
+    y = fn(tape, x)
+    up = torch.randn(y.shape, generator=torch.Generator().manual_seed(1))
+    got = tape.backward(y, up.view(5, 8))[id(x)]
+    assert not kernels.calls
+    tape.watch(x)
+    assert torch.allclose(got, tape.backward(fn(tape, x), up)[id(x)], rtol=1e-5, atol=1e-6)
+
+
+def test_loss_gradient_of_another_shape(kernels):
+    x, tg, w = torch.randn(4, 8, generator=torch.Generator().manual_seed(2)), torch.tensor([1, 7, 0, 3]), torch.rand(4)
+    tape = T.Tape()
+    tape.watch(x)
+    rows = torch.tensor([[1.0], [2.0], [0.0], [4.0]])                    # one number a row: broadcasts over the gradient
+    got = tape.backward(T.cross_entropy(tape, x, tg, w), rows)[id(x)]
+    assert not kernels.calls and torch.allclose(got, ref.cross_entropy_grad(x, tg, w)[1] * rows)
+
+
+def test_gradients_that_the_kernels_read():
+    """Of the output's shape and device only; a number on the CPU for a loss elsewhere is not one."""
+    out = torch.empty(2, 3, device="meta")
+    for takes in (train_kernels.grad_takes, gdn_train.grad_takes):
+        assert not takes(torch.empty(1, 3, device="meta"), out) and not takes(torch.empty(2, 3), out)
+        assert not takes(torch.ones(()), torch.empty((), device="meta"))
+    assert gdn_train.grad_takes(torch.empty(2, 3, device="meta"), out)

@@ -22,6 +22,11 @@ def takes(inp, conv_w, dt_bias, a_log, norm_w, *, nk, nv, dk, dv, eps, chunk=64,
             and all(p.device == inp.device for p in (conv_w, dt_bias, a_log, norm_w)))
 
 
+def grad_takes(g, out) -> bool:
+    """A gradient of ``out``'s shape, on its device: what broadcasts to it (which autograd refuses) has fewer values than the kernels read."""
+    return g.shape == out.shape and g.device == out.device
+
+
 def _ready(*tensors):
     """fp32, contiguous and on a 16-byte boundary, as the kernels read them."""
     out = []

@@ -36,6 +36,12 @@ def plain(*tensors) -> bool:
                and t.device.index == torch.cuda.current_device() for t in tensors)
 
 
+def grad_takes(g: torch.Tensor, out: torch.Tensor) -> bool:
+    """A gradient that the kernels can read as that of ``out``: the same shape (torch ops also take one that broadcasts, or a number
+    on the CPU; a kernel would read past its end), on the same device, which still is the current one."""
+    return g.shape == out.shape and g.device == out.device and g.device.index == torch.cuda.current_device()
+
+
 def _grad(g: torch.Tensor) -> torch.Tensor:
     g = g.float().contiguous()
     return g if g.data_ptr() % 16 == 0 else g.clone()

@@ -145,24 +145,10 @@ def embedding(tape: Tape, table: torch.Tensor, ids: torch.Tensor) -> torch.Tenso
     return out
 
 
-@_nograd
-def rmsnorm(tape: Tape, x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
-    K = _kernels(x)
-    if K is not None and K.rmsnorm_takes(x, w):
-        out = K.rmsnorm(x, w, eps)
-
-        def bwd_kernel(g):
-            gw = None
-            if id(w) in tape.leaves:
-                gw = (g.float() * x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps)).reshape(-1, x.shape[-1]).sum(0)
-            return K.rmsnorm_grad(x, w, g, eps), gw
-
-        tape.record("rmsnorm", (x, w), (out,), bwd_kernel)
-        return out
+def _rmsnorm_torch(x: torch.Tensor, w: torch.Tensor, eps: float):
     xf = x.float()
     rstd = torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)
     xn = xf * rstd
-    out = xn * w.float()
 
     def bwd(g):
         g = g.float()
@@ -171,6 +157,26 @@ def rmsnorm(tape: Tape, x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.T
         dx = rstd * (gx - xn * (gx * xn).mean(-1, keepdim=True))
         return dx, gw
 
+    return xn * w.float(), bwd
+
+
+@_nograd
+def rmsnorm(tape: Tape, x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
+    K = _kernels(x)
+    if K is not None and K.rmsnorm_takes(x, w):
+        out = K.rmsnorm(x, w, eps)
+
+        def bwd_kernel(g):
+            if not K.grad_takes(g, x):
+                return _rmsnorm_torch(x, w, eps)[1](g)
+            gw = None
+            if id(w) in tape.leaves:
+                gw = (g.float() * x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps)).reshape(-1, x.shape[-1]).sum(0)
+            return K.rmsnorm_grad(x, w, g, eps), gw
+
+        tape.record("rmsnorm", (x, w), (out,), bwd_kernel)
+        return out
+    out, bwd = _rmsnorm_torch(x, w, eps)
     tape.record("rmsnorm", (x, w), (out,), bwd)
     return out
 
@@ -239,6 +245,9 @@ def linear_lora(tape: Tape, x: torch.Tensor, w, frozen: bool, a: torch.Tensor, b
     out, xa = K.lora(x.to(torch.bfloat16) @ wf.t(), x, a, b, s)
 
     def bwd(g):
+        if not K.grad_takes(g, out):
+            _, dx, da, db = _lora_torch(out, x, a, b, s)[1](g)
+            return dx + (g.to(torch.bfloat16) @ wf).float(), da, db
         g = K._grad(g)
         return K.lora_grad(x, xa, a, b, s, g, g.to(torch.bfloat16) @ wf)
 
@@ -260,22 +269,26 @@ def scale(tape: Tape, a: torch.Tensor, s: float) -> torch.Tensor:
     return out
 
 
-@_nograd
-def swiglu(tape: Tape, gu: torch.Tensor) -> torch.Tensor:
-    K = _kernels(gu)
-    if K is not None and K.swiglu_takes(gu):
-        out = K.swiglu(gu)
-        tape.record("swiglu", (gu,), (out,), lambda g: (K.swiglu_grad(gu, g),))
-        return out
+def _swiglu_torch(gu: torch.Tensor):
     g_, u_ = gu[..., 0::2].float(), gu[..., 1::2].float()
     sig = torch.sigmoid(g_)
-    out = g_ * sig * u_
 
     def bwd(g):
         dg = g * u_ * sig * (1 + g_ * (1 - sig))
         du = g * g_ * sig
         return (torch.stack([dg, du], -1).flatten(-2),)
 
+    return g_ * sig * u_, bwd
+
+
+@_nograd
+def swiglu(tape: Tape, gu: torch.Tensor) -> torch.Tensor:
+    K = _kernels(gu)
+    if K is not None and K.swiglu_takes(gu):
+        out = K.swiglu(gu)
+        tape.record("swiglu", (gu,), (out,), lambda g: (K.swiglu_grad(gu, g),) if K.grad_takes(g, out) else _swiglu_torch(gu)[1](g))
+        return out
+    out, bwd = _swiglu_torch(gu)
     tape.record("swiglu", (gu,), (out,), bwd)
     return out
 
@@ -292,10 +305,18 @@ def attention_block(tape: Tape, qkv: torch.Tensor, q_norm_w: torch.Tensor, k_nor
     K = _kernels(qkv)
     if K is not None and cp is None and id(q_norm_w) not in tape.leaves and id(k_norm_w) not in tape.leaves and K.attention_takes(
             qkv, q_norm_w, k_norm_w, positions, n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim, gated=gated):
-        out, grad = K.attention(qkv, q_norm_w, k_norm_w, positions, n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim,
-                                theta=theta, eps=eps, gated=gated)
-        tape.record("attention", (qkv, q_norm_w, k_norm_w), (out,), lambda g: (grad(g), None, None))
+        dims = dict(n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim, theta=theta, eps=eps, gated=gated)
+        out, grad = K.attention(qkv, q_norm_w, k_norm_w, positions, **dims)
+        tape.record("attention", (qkv, q_norm_w, k_norm_w), (out,), lambda g: (grad(g), None, None) if K.grad_takes(g, out)
+                    else _attention_torch(qkv, q_norm_w, k_norm_w, positions, **dims)[1](g))
         return out
+    out, bwd = _attention_torch(qkv, q_norm_w, k_norm_w, positions, n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim,
+                                theta=theta, eps=eps, gated=gated, cp=cp)
+    tape.record("attention", (qkv, q_norm_w, k_norm_w), (out,), bwd)
+    return out
+
+
+def _attention_torch(qkv, q_norm_w, k_norm_w, positions, *, n_q, n_kv, head_dim, rotary_dim, theta, eps, gated, cp=None):
     b, t, _ = qkv.shape
     d, g = head_dim, n_q // n_kv
     x = qkv.float()
@@ -383,8 +404,7 @@ def attention_block(tape: Tape, qkv: torch.Tensor, q_norm_w: torch.Tensor, k_nor
         parts += [dk_raw.reshape(b, t, -1), dv.reshape(b, t, -1)]
         return torch.cat(parts, -1), gqw, gkw
 
-    tape.record("attention", (qkv, q_norm_w, k_norm_w), (out,), bwd)
-    return out
+    return out, bwd
 
 
 def _gdn_block_cp(inp, conv_w, dt_bias, a_log, norm_w, *, nk, nv, dk, dv, eps, chunk, cp):
@@ -463,16 +483,6 @@ def gdn_block(tape: Tape, inp: torch.Tensor, conv_w, dt_bias, a_log, norm_w, **k
     the chunked form locally; on CUDA both are kernels (``csrc/gdn_train.cu``) for the shapes
     they take."""
     params = (conv_w, dt_bias, a_log, norm_w)
-    if inp.is_cuda:
-        from .ops import gdn_train
-        if gdn_train.takes(inp, *params, **kw):
-            with torch.no_grad():
-                out = gdn_train.forward(inp, *params, **kw)
-            tape.record("gdn", (inp,) + params, (out,),
-                        lambda g: gdn_train.backward(inp, *params, g, need=[id(p) in tape.leaves for p in params], **kw))
-            return out
-    with torch.no_grad():
-        out = gdn_block_torch(inp, conv_w, dt_bias, a_log, norm_w, **kw)
 
     def bwd(g):
         with torch.enable_grad():
@@ -481,6 +491,21 @@ def gdn_block(tape: Tape, inp: torch.Tensor, conv_w, dt_bias, a_log, norm_w, **k
             gs = torch.autograd.grad(y, leaves, g.float(), allow_unused=True)
         return tuple(gs)
 
+    if inp.is_cuda:
+        from .ops import gdn_train
+        if gdn_train.takes(inp, *params, **kw):
+            with torch.no_grad():
+                out = gdn_train.forward(inp, *params, **kw)
+
+            def bwd_kernel(g):
+                if not gdn_train.grad_takes(g, out):
+                    return bwd(g)
+                return gdn_train.backward(inp, *params, g, need=[id(p) in tape.leaves for p in params], **kw)
+
+            tape.record("gdn", (inp,) + params, (out,), bwd_kernel)
+            return out
+    with torch.no_grad():
+        out = gdn_block_torch(inp, conv_w, dt_bias, a_log, norm_w, **kw)
     tape.record("gdn", (inp,) + params, (out,), bwd)
     return out
 
@@ -496,7 +521,13 @@ def cross_entropy(tape: Tape, logits: torch.Tensor, targets: torch.Tensor,
         # the gradient is written once, in the backward pass, from each row's largest value and sum
         tg, w, stats = targets.reshape(-1).long().contiguous(), weights.reshape(-1).float().contiguous(), K.lse(lg)
         loss = (w * (stats[2] - lg.gather(-1, tg[:, None]).squeeze(-1))).sum()
-        tape.record("cross_entropy", (logits,), (loss,), lambda g: (K.cross_entropy_grad(lg, stats, tg, w, g).view_as(logits),))
+
+        def bwd_kernel(g):
+            if not K.grad_takes(g, loss):
+                return (ref.cross_entropy_grad(lg, tg, w)[1].view_as(logits) * g,)
+            return (K.cross_entropy_grad(lg, stats, tg, w, g).view_as(logits),)
+
+        tape.record("cross_entropy", (logits,), (loss,), bwd_kernel)
         return loss
     loss, grad = ref.cross_entropy_grad(lg, targets.reshape(-1), weights.reshape(-1).float())
     grad = grad.view_as(logits)
@@ -610,22 +641,8 @@ def all_reduce(tape: Tape, x: torch.Tensor) -> torch.Tensor:
     return out
 
 
-@_nograd
-def lora(tape: Tape, y: torch.Tensor, x: torch.Tensor, a: torch.Tensor, b: torch.Tensor,
-         s: float) -> torch.Tensor:
-    """``y + s * (x A^T) B^T`` with gradients for x, A and B."""
-    K = _kernels(y)
-    if K is not None and K.lora_takes(y, x, a, b):
-        out, xa = K.lora(y, x, a, b, s)
-
-        def bwd_kernel(g):
-            g = K._grad(g)
-            return (g,) + K.lora_grad(x, xa, a, b, s, g)
-
-        tape.record("lora", (y, x, a, b), (out,), bwd_kernel)
-        return out
+def _lora_torch(y, x, a, b, s):
     xa = x.float() @ a.float().t()
-    out = y + (xa @ b.float().t()) * s
 
     def bwd(g):
         g = g.float()
@@ -635,5 +652,25 @@ def lora(tape: Tape, y: torch.Tensor, x: torch.Tensor, a: torch.Tensor, b: torch
         da = dxa.reshape(-1, dxa.shape[-1]).t() @ x.float().reshape(-1, x.shape[-1])
         return g, dxa @ a.float(), da, db
 
+    return y + (xa @ b.float().t()) * s, bwd
+
+
+@_nograd
+def lora(tape: Tape, y: torch.Tensor, x: torch.Tensor, a: torch.Tensor, b: torch.Tensor,
+         s: float) -> torch.Tensor:
+    """``y + s * (x A^T) B^T`` with gradients for x, A and B."""
+    K = _kernels(y)
+    if K is not None and K.lora_takes(y, x, a, b):
+        out, xa = K.lora(y, x, a, b, s)
+
+        def bwd_kernel(g):
+            if not K.grad_takes(g, out):
+                return _lora_torch(y, x, a, b, s)[1](g)
+            g = K._grad(g)
+            return (g,) + K.lora_grad(x, xa, a, b, s, g)
+
+        tape.record("lora", (y, x, a, b), (out,), bwd_kernel)
+        return out
+    out, bwd = _lora_torch(y, x, a, b, s)
     tape.record("lora", (y, x, a, b), (out,), bwd)
     return out
