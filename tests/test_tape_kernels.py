@@ -132,3 +132,20 @@ def test_gradients_that_the_kernels_read():
         assert not takes(torch.empty(1, 3, device="meta"), out) and not takes(torch.empty(2, 3), out)
         assert not takes(torch.ones(()), torch.empty((), device="meta"))
     assert gdn_train.grad_takes(torch.empty(2, 3, device="meta"), out)
+
+
+def test_positions_and_vectors_that_the_kernels_take(monkeypatch):
+    """Fractional positions are rotated by their fraction (a cast to whole ones would drop it); vectors and taps of another rank
+    mean something else to the torch form, or are refused there."""
+    monkeypatch.setattr(train_kernels, "plain", lambda *t: True)
+    qkv, w = torch.randn(1, 3, 24), torch.ones(4)
+    dims = dict(n_q=2, n_kv=1, head_dim=4, rotary_dim=4, gated=True)
+    pos = torch.arange(3)
+    assert train_kernels.attention_takes(qkv, w, w, pos, **dims) and train_kernels.attention_takes(qkv, w, w, pos.int()[None], **dims)
+    assert not train_kernels.attention_takes(qkv, w, w, pos * 0.5, **dims)
+    nk, nv = 1, 2
+    inp, conv, v, nw = torch.zeros(1, 3, (2 * nk + 2 * nv) * 128 + 2 * nv), torch.zeros((2 * nk + nv) * 128, 4), torch.zeros(nv), torch.ones(128)
+    kw = dict(nk=nk, nv=nv, dk=128, dv=128, eps=1e-6)
+    assert gdn_train.takes(inp, conv, v, v, nw, **kw)
+    assert not gdn_train.takes(inp, conv[:, None], v, v, nw, **kw) and not gdn_train.takes(inp, conv, v[:, None], v, nw, **kw)
+    assert not gdn_train.takes(inp, conv, v, v[None], nw, **kw) and not gdn_train.takes(inp, conv, v, v, nw[None], **kw)

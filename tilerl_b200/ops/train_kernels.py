@@ -27,6 +27,7 @@ N.register("trl_train_adamw", [N.P] * 8 + [N.I] + [N.F] * 6 + [N.P])
 N.register("trl_train_squares", [N.P, N.P, N.I, N.P, N.P])
 N.register("trl_train_scale", [N.P, N.P, N.I, N.F, N.P])
 
+INTEGERS = (torch.int64, torch.int32, torch.int16, torch.int8, torch.uint8)       # (positions between two tokens: the torch form)
 MAX_TENSORS = 32          # a launch of the many-tensor kernels
 
 
@@ -126,7 +127,7 @@ def attention_takes(qkv, q_norm_w, k_norm_w, positions, *, n_q, n_kv, head_dim, 
     b, t, rows = qkv.shape
     return (rows == n_q * head_dim * (2 if gated else 1) + 2 * n_kv * head_dim and t <= 4096 and b * n_q * t < 1 << 31
             and tuple(positions.shape) in ((t,), (b, t), (1, t)) and q_norm_w.numel() == head_dim and k_norm_w.numel() == head_dim
-            and positions.device == qkv.device and plain(qkv, q_norm_w, k_norm_w))
+            and positions.device == qkv.device and positions.dtype in INTEGERS and plain(qkv, q_norm_w, k_norm_w))
 
 
 def attention(qkv, q_norm_w, k_norm_w, positions, *, n_q, n_kv, head_dim, rotary_dim, theta, eps, gated):
