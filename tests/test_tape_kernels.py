@@ -149,3 +149,39 @@ def test_positions_and_vectors_that_the_kernels_take(monkeypatch):
     assert gdn_train.takes(inp, conv, v, v, nw, **kw)
     assert not gdn_train.takes(inp, conv[:, None], v, v, nw, **kw) and not gdn_train.takes(inp, conv, v[:, None], v, nw, **kw)
     assert not gdn_train.takes(inp, conv, v, v[None], nw, **kw) and not gdn_train.takes(inp, conv, v, v, nw[None], **kw)
+
+
+@pytest.mark.parametrize("late", [False, True])
+def test_weights_that_an_op_made_or_that_are_watched_later_get_their_gradient(late, kernels):
+    """A norm's weight that comes out of another op on the tape passes its gradient on; a tensor may be watched after the ops that read it."""
+    g = torch.Generator().manual_seed(3)
+    x, qkv, base = torch.randn(3, 4, generator=g), torch.randn(1, 5, 24, generator=g), 1 + 0.1 * torch.randn(4, generator=g)
+    dims = dict(n_q=2, n_kv=1, head_dim=4, rotary_dim=4, theta=1e4, eps=1e-6)
+    for fn in (lambda t, w: T.rmsnorm(t, x, w, 1e-6), lambda t, w: T.attention_block(t, qkv, w, w, torch.arange(5), **dims)):
+        res = []
+        for K in (kernels, None):
+            T._kernels = lambda x: K               # (the fixture puts the module's own back)
+            tape = T.Tape()
+            if not late:
+                tape.watch(base)
+            y = fn(tape, base if late else T.scale(tape, base, 2.0))
+            tape.watch(base)
+            res.append(tape.backward(y, torch.ones_like(y))[id(base)])
+        assert torch.allclose(*res, rtol=1e-4, atol=1e-5)
+
+
+@pytest.mark.parametrize("late", [False, True])
+def test_delta_rule_parameters_that_an_op_made_get_their_gradient(late, monkeypatch):
+    asked = []
+    monkeypatch.setattr(gdn_train, "takes", lambda *a, **k: True)
+    monkeypatch.setattr(gdn_train, "forward", lambda inp, *a, **k: inp * 1.0)
+    monkeypatch.setattr(gdn_train, "backward", lambda inp, *p, need, **k: asked.append(need) or (inp,) + tuple(q if n else None for q, n in zip(p, need)))
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True, raising=False)
+    params = [torch.ones(2) for _ in range(4)]
+    tape = T.Tape()
+    if not late:
+        tape.watch(params[0])
+    used = params if late else [T.scale(tape, params[0], 2.0)] + params[1:]
+    y = T.gdn_block(tape, torch.ones(2), *used, nk=1, nv=2, dk=128, dv=128, eps=1e-6)
+    tape.watch(params[0])
+    assert id(params[0]) in tape.backward(y, torch.ones_like(y)) and asked == [[True, False, False, False]]

@@ -39,6 +39,7 @@ class Tape:
     def __init__(self, tp_group=None, tp_world: int = 1):
         self.nodes: List[_Node] = []
         self.leaves: Dict[int, torch.Tensor] = {}
+        self.made: set = set()            # ids of the recorded ops' outputs
         self.tp_group, self.tp_world = tp_group, tp_world
         self.enabled = True
 
@@ -51,6 +52,11 @@ class Tape:
                bwd: Callable) -> None:
         if self.enabled:
             self.nodes.append(_Node(name, tuple(inputs), tuple(outputs), bwd))
+            self.made.update(map(id, outputs))
+
+    def wants(self, t: torch.Tensor) -> bool:
+        """Whether a gradient of ``t`` goes anywhere: it is watched, or an op on this tape made it."""
+        return id(t) in self.leaves or id(t) in self.made
 
     # ---- backward ----------------------------------------------------------------
     def backward(self, root: torch.Tensor, grad: Optional[torch.Tensor] = None,
@@ -82,6 +88,7 @@ class Tape:
                     if first_use.get(k) == idx and k in grads:
                         on_grad(t, grads.pop(k))
         self.nodes.clear()
+        self.made.clear()
         return {k: g for k, g in grads.items() if k in self.leaves}
 
     def grad_of(self, grads: Dict[int, torch.Tensor], t: torch.Tensor) -> Optional[torch.Tensor]:
@@ -170,7 +177,7 @@ def rmsnorm(tape: Tape, x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.T
             if not K.grad_takes(g, x):
                 return _rmsnorm_torch(x, w, eps)[1](g)
             gw = None
-            if id(w) in tape.leaves:
+            if tape.wants(w):
                 gw = (g.float() * x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps)).reshape(-1, x.shape[-1]).sum(0)
             return K.rmsnorm_grad(x, w, g, eps), gw
 
@@ -303,12 +310,17 @@ def attention_block(tape: Tape, qkv: torch.Tensor, q_norm_w: torch.Tensor, k_nor
     ``cp`` the rotated K, V and their absolute positions are all-gathered over the ranks
     (the mask compares absolute positions) and dK / dV are reduce-scattered in backward."""
     K = _kernels(qkv)
-    if K is not None and cp is None and id(q_norm_w) not in tape.leaves and id(k_norm_w) not in tape.leaves and K.attention_takes(
+    if K is not None and cp is None and not tape.wants(q_norm_w) and not tape.wants(k_norm_w) and K.attention_takes(
             qkv, q_norm_w, k_norm_w, positions, n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim, gated=gated):
         dims = dict(n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim, theta=theta, eps=eps, gated=gated)
         out, grad = K.attention(qkv, q_norm_w, k_norm_w, positions, **dims)
-        tape.record("attention", (qkv, q_norm_w, k_norm_w), (out,), lambda g: (grad(g), None, None) if K.grad_takes(g, out)
-                    else _attention_torch(qkv, q_norm_w, k_norm_w, positions, **dims)[1](g))
+
+        def bwd_kernel(g):
+            if not K.grad_takes(g, out) or tape.wants(q_norm_w) or tape.wants(k_norm_w):       # (watched since)
+                return _attention_torch(qkv, q_norm_w, k_norm_w, positions, **dims)[1](g)
+            return grad(g), None, None
+
+        tape.record("attention", (qkv, q_norm_w, k_norm_w), (out,), bwd_kernel)
         return out
     out, bwd = _attention_torch(qkv, q_norm_w, k_norm_w, positions, n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim,
                                 theta=theta, eps=eps, gated=gated, cp=cp)
@@ -500,7 +512,7 @@ def gdn_block(tape: Tape, inp: torch.Tensor, conv_w, dt_bias, a_log, norm_w, **k
             def bwd_kernel(g):
                 if not gdn_train.grad_takes(g, out):
                     return bwd(g)
-                return gdn_train.backward(inp, *params, g, need=[id(p) in tape.leaves for p in params], **kw)
+                return gdn_train.backward(inp, *params, g, need=[tape.wants(p) for p in params], **kw)
 
             tape.record("gdn", (inp,) + params, (out,), bwd_kernel)
             return out
