@@ -185,3 +185,26 @@ def test_delta_rule_parameters_that_an_op_made_get_their_gradient(late, monkeypa
     y = T.gdn_block(tape, torch.ones(2), *used, nk=1, nv=2, dk=128, dv=128, eps=1e-6)
     tape.watch(params[0])
     assert id(params[0]) in tape.backward(y, torch.ones_like(y)) and asked == [[True, False, False, False]]
+
+
+def test_tensors_changed_between_the_passes(kernels):
+    """Targets and weights may be written into after the forward pass; logits, a norm's rows and an attention block's may not: the
+    gradient of other values would come back."""
+    g = torch.Generator().manual_seed(4)
+    x, tg, w = torch.randn(4, 8, generator=g), torch.tensor([1, 7, 0, 3]), torch.rand(4, generator=g)
+    want = ref.cross_entropy_grad(x, tg, w)[1]
+    tape = T.Tape()
+    tape.watch(x)
+    loss = T.cross_entropy(tape, x, tg, w)
+    tg.zero_(), w.zero_()
+    assert torch.allclose(tape.backward(loss)[id(x)], want)
+    for fn, t in ((lambda tape, t: T.cross_entropy(tape, t, tg, w), x), (lambda tape, t: T.rmsnorm(tape, t, torch.ones(8), 1e-6), x),
+                  (_ops()["attention"][0], torch.randn(1, 5, 24, generator=g))):
+        tape = T.Tape()
+        tape.watch(t)
+        y = fn(tape, t)
+        t.mul_(2.0)
+        with pytest.raises(RuntimeError, match="in place"):
+            tape.backward(y)
+        with torch.inference_mode():                 # (no count to look at)
+            fn(T.Tape(), t * 1.0)

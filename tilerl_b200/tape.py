@@ -138,6 +138,17 @@ def _kernels(x: torch.Tensor):
     return train_kernels
 
 
+def _unchanged(*kept: torch.Tensor) -> Callable[[], None]:
+    """For tensors that a backward kernel reads again: the check that nothing was written into them since (their torch forms keep
+    what they need, and would give the gradient of the old values; inference tensors keep no count)."""
+    kept = [(t, t._version) for t in kept if not t.is_inference()]
+
+    def check():
+        if any(t._version != v for t, v in kept):
+            raise RuntimeError("a tensor that the backward pass needs was changed in place after the forward pass")
+    return check
+
+
 @_nograd
 def embedding(tape: Tape, table: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
     out = table[ids.long()].float()
@@ -171,9 +182,10 @@ def _rmsnorm_torch(x: torch.Tensor, w: torch.Tensor, eps: float):
 def rmsnorm(tape: Tape, x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
     K = _kernels(x)
     if K is not None and K.rmsnorm_takes(x, w):
-        out = K.rmsnorm(x, w, eps)
+        out, unchanged = K.rmsnorm(x, w, eps), _unchanged(x)
 
         def bwd_kernel(g):
+            unchanged()
             if not K.grad_takes(g, x):
                 return _rmsnorm_torch(x, w, eps)[1](g)
             gw = None
@@ -314,8 +326,10 @@ def attention_block(tape: Tape, qkv: torch.Tensor, q_norm_w: torch.Tensor, k_nor
             qkv, q_norm_w, k_norm_w, positions, n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim, gated=gated):
         dims = dict(n_q=n_q, n_kv=n_kv, head_dim=head_dim, rotary_dim=rotary_dim, theta=theta, eps=eps, gated=gated)
         out, grad = K.attention(qkv, q_norm_w, k_norm_w, positions, **dims)
+        unchanged = _unchanged(qkv)
 
         def bwd_kernel(g):
+            unchanged()
             if not K.grad_takes(g, out) or tape.wants(q_norm_w) or tape.wants(k_norm_w):       # (watched since)
                 return _attention_torch(qkv, q_norm_w, k_norm_w, positions, **dims)[1](g)
             return grad(g), None, None
@@ -531,10 +545,11 @@ def cross_entropy(tape: Tape, logits: torch.Tensor, targets: torch.Tensor,
     K = _kernels(logits)
     if K is not None and K.cross_entropy_takes(logits, targets, weights):
         # the gradient is written once, in the backward pass, from each row's largest value and sum
-        tg, w, stats = targets.reshape(-1).long().contiguous(), weights.reshape(-1).float().contiguous(), K.lse(lg)
-        loss = (w * (stats[2] - lg.gather(-1, tg[:, None]).squeeze(-1))).sum()
+        tg, w, stats = targets.reshape(-1).to(torch.int64, copy=True), weights.reshape(-1).to(torch.float32, copy=True), K.lse(lg)
+        loss, unchanged = (w * (stats[2] - lg.gather(-1, tg[:, None]).squeeze(-1))).sum(), _unchanged(lg)
 
         def bwd_kernel(g):
+            unchanged()
             if not K.grad_takes(g, loss):
                 return (ref.cross_entropy_grad(lg, tg, w)[1].view_as(logits) * g,)
             return (K.cross_entropy_grad(lg, stats, tg, w, g).view_as(logits),)
