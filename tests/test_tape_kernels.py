@@ -208,3 +208,35 @@ def test_tensors_changed_between_the_passes(kernels):
             tape.backward(y)
         with torch.inference_mode():                 # (no count to look at)
             fn(T.Tape(), t * 1.0)
+
+
+def test_training_without_the_kernels(monkeypatch, tmp_path):
+    """A library without these entry points (one that serves a single architecture), or none at all: the ops, clipping and the
+    optimizer run in torch."""
+    from tilerl_b200.ops import native
+    from tilerl_b200.optim import AdamW, clip_grad_norm
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True, raising=False)
+
+    class Device(str):                                # a "cuda" whose tensors live on the CPU
+        type = "cuda"
+    g = torch.Generator().manual_seed(5)
+    x, w = torch.randn(3, 8, generator=g), torch.ones(8)
+    params = [torch.zeros(4 * 128, 2), torch.zeros(2), torch.zeros(2), torch.ones(128)]
+    inp = torch.randn(1, 3, 6 * 128 + 4, generator=g)
+    for lib, path in ((object(), __file__), (None, str(tmp_path / "none.so"))):
+        monkeypatch.setattr(native, "_LIB", lib), monkeypatch.setattr(native, "_PATH", path)
+        assert not native.has("trl_train_adamw")
+        tape = T.Tape()
+        tape.watch(x)
+        assert tape.backward(T.rmsnorm(tape, x, w, 1e-6), torch.ones(3, 8))[id(x)].shape == (3, 8)
+        assert not gdn_train.takes(inp, *params, nk=1, nv=2, dk=128, dv=128, eps=1e-6)
+        p, grads = {"w": torch.ones(4)}, {"w": torch.ones(4)}
+        opt = AdamW(p, lr=0.1)
+        opt.step(grads)
+        assert float(p["w"][0]) < 1 and opt.t == {"w": 1}
+        monkeypatch.setattr(torch.Tensor, "device", Device("cpu"), raising=False)
+        assert abs(clip_grad_norm(grads, 10.0) - 2.0) < 1e-6
+        monkeypatch.undo()
+        monkeypatch.setattr(torch.Tensor, "is_cuda", True, raising=False)
+    monkeypatch.setattr(native, "_LIB", type("L", (), {"trl_x": 1})())
+    assert native.has("trl_x") and not native.has("trl_y")

@@ -16,6 +16,8 @@ N.register("trl_gdn_train_backward", [N.P] * 9 + [N.I] * 5 + [N.F, N.P])
 def takes(inp, conv_w, dt_bias, a_log, norm_w, *, nk, nv, dk, dv, eps, chunk=64, state=None, cp=None) -> bool:
     if cp is not None or state is not None or dk != 128 or dv != 128 or nv % nk or nv % 2 or inp.dim() != 3 or inp.numel() == 0:
         return False
+    if not N.has("trl_gdn_train_forward"):           # (a library of one architecture)
+        return False
     rows = 2 * nk * dk + 2 * nv * dv + 2 * nv
     return (inp.shape[2] == rows and inp.numel() < 1 << 29 and conv_w.dim() == 2 and conv_w.shape[0] == (2 * nk + nv) * dk
             and dt_bias.shape == a_log.shape == (nv,) and norm_w.shape == (dv,)

@@ -171,6 +171,11 @@ def lib() -> ctypes.CDLL:
     return _LIB
 
 
+def has(name: str) -> bool:
+    """The library is there and has this entry point (one that serves a single architecture has some only)."""
+    return (_LIB is not None or os.path.exists(_PATH)) and hasattr(lib(), name)
+
+
 _PYLIB = None        # the same library called with the interpreter locked: False when it has no such entry point
 
 

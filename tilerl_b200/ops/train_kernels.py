@@ -31,6 +31,11 @@ INTEGERS = (torch.int64, torch.int32, torch.int16, torch.int8, torch.uint8)     
 MAX_TENSORS = 32          # a launch of the many-tensor kernels
 
 
+def there() -> bool:
+    """The library has these kernels: one of a single architecture does not, and training runs in torch as it does without one."""
+    return N.has("trl_train_adamw")
+
+
 def plain(*tensors) -> bool:
     """fp32, contiguous, not empty and on 16-byte boundaries, all on the current CUDA device."""
     return all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() and t.data_ptr() % 16 == 0

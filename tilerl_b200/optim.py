@@ -36,7 +36,7 @@ def clip_grad_norm(grads: Dict[str, torch.Tensor], max_norm: float, *, sharded: 
     many = None
     if dev.type == "cuda":
         from .ops import train_kernels as many
-        parts = many.squares(grads)
+        parts = many.squares(grads) if many.there() else None
         many = many if parts is not None else None
     sh = torch.zeros((), dtype=torch.float64, device=dev)
     rep = torch.zeros((), dtype=torch.float64, device=dev)
@@ -107,6 +107,9 @@ class AdamW:
                 self.step_param(k, g, lr)
                 continue
             from .ops import train_kernels
+            if not train_kernels.there():
+                self.step_param(k, g, lr)
+                continue
             if k not in self.m:
                 self.m[k], self.v[k], self.t[k] = torch.zeros_like(p), torch.zeros_like(p), 0
             if not train_kernels.plain(p, g, self.m[k], self.v[k]) or g.shape != p.shape:

@@ -135,7 +135,7 @@ def _kernels(x: torch.Tensor):
     if not x.is_cuda:
         return None
     from .ops import train_kernels
-    return train_kernels
+    return train_kernels if train_kernels.there() else None
 
 
 def _unchanged(*kept: torch.Tensor) -> Callable[[], None]:
