@@ -240,3 +240,35 @@ def test_training_without_the_kernels(monkeypatch, tmp_path):
         monkeypatch.setattr(torch.Tensor, "is_cuda", True, raising=False)
     monkeypatch.setattr(native, "_LIB", type("L", (), {"trl_x": 1})())
     assert native.has("trl_x") and not native.has("trl_y")
+
+
+def test_tensors_that_share_memory_are_not_in_one_launch(monkeypatch):
+    """A weight under two names is updated by one after the other, as the loop over the names does; a gradient given twice is scaled
+    by one after the other.  Gradients that only are read may be shared."""
+    launches = []
+
+    class Lib:
+        def trl_train_adamw(self, p, m, v, g, n, decay, c1, c2, count, *rest):
+            launches.append([int(p[i]) for i in range(count)])
+            return 0
+
+        def trl_train_scale(self, p, n, count, c, stream):
+            launches.append([int(p[i]) for i in range(count)])
+            return 0
+    monkeypatch.setattr(train_kernels.N, "lib", lambda: Lib())
+    monkeypatch.setattr(train_kernels.N, "stream", lambda: 0)
+    t = [torch.ones(8) for _ in range(12)]
+    item = lambda p, m, v, g: (p, m, v, g, 1.0, 0.1, 0.1)
+    run = lambda *items: (launches.clear(), train_kernels.adamw(list(items), 0.1, (0.9, 0.99), 1e-8), [list(x) for x in launches])[2]
+    at = lambda x: x.data_ptr()
+    assert run(item(*t[:4]), item(*t[4:8])) == [[at(t[0]), at(t[4])]]
+    assert run(item(*t[:4]), item(t[4], t[5], t[6], t[3])) == [[at(t[0]), at(t[4])]]
+    assert run(item(*t[:4]), item(t[0], t[5], t[6], t[7])) == [[at(t[0])], [at(t[0])]]
+    assert run(item(*t[:4]), item(t[4], t[5], t[6], t[0])) == [[at(t[0])], [at(t[4])]]
+    whole = torch.ones(16)
+    assert run(item(whole[:8], *t[1:4]), item(whole[8:], *t[5:8])) == [[at(whole), at(whole[8:])]]
+    assert len(run(item(whole[:8], *t[1:4]), item(whole[4:12], *t[5:8]))) == 2
+    for tensors, want in (([t[0], t[1]], [[at(t[0]), at(t[1])]]), ([t[0], t[1], t[0]], [[at(t[0])], [at(t[1])], [at(t[0])]])):
+        launches.clear()
+        train_kernels.scale(tensors, 0.5)
+        assert launches == want

@@ -205,10 +205,23 @@ def _floats(v: Sequence[float]):
     return (ctypes.c_float * len(v))(*v)
 
 
+def apart(written: Sequence[torch.Tensor], read: Sequence[torch.Tensor] = ()) -> bool:
+    """No tensor that is written shares memory with another one (a weight under two names, a gradient given twice): the tensors of a
+    launch are worked on at the same time."""
+    any_end = written_end = 0
+    for start, end, w in sorted([(t.data_ptr(), t.data_ptr() + t.nbytes, True) for t in written] + [(t.data_ptr(), t.data_ptr() + t.nbytes, False) for t in read]):
+        if start < (any_end if w else written_end):
+            return False
+        any_end = max(any_end, end)
+        written_end = max(written_end, end) if w else written_end
+    return True
+
+
 def adamw(items: List[tuple], lr: float, betas, eps: float) -> None:
-    """``items``: (parameter, m, v, gradient, decay factor, 1 - b1^t, 1 - b2^t), tensors plain."""
-    for i in range(0, len(items), MAX_TENSORS):
-        p, m, v, g, decay, c1, c2 = zip(*items[i:i + MAX_TENSORS])
+    """``items``: (parameter, m, v, gradient, decay factor, 1 - b1^t, 1 - b2^t), tensors plain.  One after the other where some share memory."""
+    most = MAX_TENSORS if apart([t for it in items for t in it[:3]], [it[3] for it in items]) else 1
+    for i in range(0, len(items), most):
+        p, m, v, g, decay, c1, c2 = zip(*items[i:i + most])
         N.check(N.lib().trl_train_adamw(_pointers(p), _pointers(m), _pointers(v), _pointers(g), _lengths(p), _floats(decay), _floats(c1), _floats(c2),
                                         len(p), lr, betas[0], 1 - betas[0], betas[1], 1 - betas[1], eps, N.stream()), "train_adamw")
         torch.autograd.graph.increment_version(p + m + v)         # written in place, as ``copy_`` says it
@@ -229,10 +242,11 @@ def squares(grads: Dict[str, torch.Tensor]) -> Optional[torch.Tensor]:
 
 
 def scale(tensors: Sequence[torch.Tensor], c: float) -> None:
-    """All of them times ``c``, in place (plain ones)."""
+    """All of them times ``c``, in place (plain ones), one after the other where some share memory."""
     tensors = list(tensors)
-    for i in range(0, len(tensors), MAX_TENSORS):
-        some = tensors[i:i + MAX_TENSORS]
+    most = MAX_TENSORS if apart(tensors) else 1
+    for i in range(0, len(tensors), most):
+        some = tensors[i:i + most]
         N.check(N.lib().trl_train_scale(_pointers(some), _lengths(some), len(some), c, N.stream()), "train_scale")
         torch.autograd.graph.increment_version(some)
         N.count()
