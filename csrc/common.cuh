@@ -254,6 +254,21 @@ __device__ __forceinline__ uint32_t f2_to_bf162_bits(float a, float b) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// ---- once a device (host) ----------------------------------------------------------------------
+// What is set or asked once for each GPU that the process uses, zero at first: a kernel's shared-memory limit belongs to the device
+// that was current when it was raised.  (Threads that meet here write the same.)
+template <typename T>
+struct TrlPerDevice {
+  static constexpr int MOST = 64;
+  T v[MOST] = {};
+  T last{};                                          // of a device past the table: set again on every call
+  T& here() {
+    int d = 0;
+    if (cudaGetDevice(&d) == cudaSuccess && d >= 0 && d < MOST) return v[d];
+    return last = T{};
+  }
+};
+
 // ---- launch helper (host) ---------------------------------------------------------------------
 // Launch with the programmatic-stream-serialization attribute so consecutive
 // kernels of a tick overlap their tails/prologues (also inside CUDA graphs).

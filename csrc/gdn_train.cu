@@ -638,10 +638,13 @@ constexpr int CHUNK_SMEM = (3 * C * LD + 2 * C * LC + 2 * C) * 4;
 constexpr int SCAN_SMEM = (int)(2 * sizeof(ScanStage)) + (D * LS + C * LS) * 4;
 
 int shared_memory() {
-  static const bool ok = cudaFuncSetAttribute(gt_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM) == cudaSuccess &&
-                         cudaFuncSetAttribute(gt_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM) == cudaSuccess &&
-                         cudaFuncSetAttribute(gt_scan_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM) == cudaSuccess &&
-                         cudaFuncSetAttribute(gt_chunk_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChunkGradSmem)) == cudaSuccess;
+  static TrlPerDevice<bool> set;
+  bool& ok = set.here();
+  if (!ok)
+    ok = cudaFuncSetAttribute(gt_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM) == cudaSuccess &&
+         cudaFuncSetAttribute(gt_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM) == cudaSuccess &&
+         cudaFuncSetAttribute(gt_scan_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM) == cudaSuccess &&
+         cudaFuncSetAttribute(gt_chunk_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChunkGradSmem)) == cudaSuccess;
   return ok ? 0 : 3;
 }
 

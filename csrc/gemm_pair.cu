@@ -394,7 +394,8 @@ bool gp_tensor(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dim
 template <int BN, int J, bool SPLIT>
 int launch_pair(const CUtensorMap (&m)[4], const PairParams& p, int pairs, cudaStream_t stream) {
   auto kern = gemm_nvfp4_pair_kernel<BN, J, SPLIT>;
-  static bool configured = false;
+  static TrlPerDevice<bool> set;
+  bool& configured = set.here();
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<BN, J>::SMEM) != cudaSuccess) return 3;
     configured = true;
@@ -428,9 +429,10 @@ int launch_pair(const CUtensorMap (&m)[4], const PairParams& p, int bn, int pair
 }  // namespace
 
 int gemm_pair_clusters(int parts) {
-  static int known[4] = {};                          // (threads that meet here write the same)
+  static TrlPerDevice<int> counts[4];
   if (parts < 1 || parts > 3) return 0;
-  if (known[parts] == 0) {
+  int& known = counts[parts].here();
+  if (known == 0) {
     auto kern = gemm_nvfp4_pair_kernel<64, 2, true>;
     constexpr int smem = PairCfg<64, 2>::SMEM;
     cudaLaunchConfig_t cfg = {};
@@ -445,9 +447,9 @@ int gemm_pair_clusters(int parts) {
       cudaGetLastError();
       n = 0;
     }
-    known[parts] = n > 0 ? n : -1;
+    known = n > 0 ? n : -1;
   }
-  return known[parts];
+  return known;
 }
 
 int gemm_pair_launch(const GemmPairArgs& a, int bn, cudaStream_t stream) {

@@ -191,7 +191,8 @@ bool head_map(CUtensorMap* m, const void* base, long rows, long K, int box) {
 template <int BN>
 int launch_head(const CUtensorMap& mw, const CUtensorMap& mx, float* out, long ldo, int M, int N, int nk, int grid, cudaStream_t st) {
   auto kern = head_bf16_kernel<BN>;
-  static bool configured = false;
+  static TrlPerDevice<bool> set;
+  bool& configured = set.here();
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, HeadCfg<BN>::SMEM) != cudaSuccess) return 3;
     configured = true;

@@ -179,3 +179,20 @@ def test_adamw_and_clipping_of_many_tensors():
         for a, b in ((g0[k], g1[k]), (o0.m[k], o1.m[k]), (o0.v[k], o1.v[k])):
             assert torch.allclose(a.float(), b.float().cpu(), rtol=2e-6, atol=1e-9), k
         assert torch.allclose(p0[k].float(), p1[k].float().cpu(), rtol=2 ** -8 if k == "half" else 2e-6, atol=1e-7), k
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs in one process")
+def test_delta_rule_block_on_a_second_gpu_of_the_process():
+    """Its kernels' shared-memory limits are raised on the device that they run on, not once for the process."""
+    from tilerl_b200 import tape as T
+    g = torch.Generator().manual_seed(1)
+    args = [torch.randn(1, 40, 768 + 4, generator=g), torch.randn(512, 4, generator=g) * 0.4, torch.randn(2, generator=g), torch.randn(2, generator=g), torch.ones(128)]
+    outs = []
+    for dev in ("cuda:0", "cuda:1"):
+        here = [a.to(dev) for a in args]
+        tape = T.Tape()
+        tape.watch(*here)
+        y = T.gdn_block(tape, *here, nk=1, nv=2, dk=128, dv=128, eps=1e-6)
+        outs.append([y.cpu()] + [tape.backward(y, torch.ones_like(y))[id(a)].cpu() for a in here[:1]])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
