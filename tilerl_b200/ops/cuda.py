@@ -615,7 +615,7 @@ class CudaOps(StreamOps, MixerOps, BlockOps, GatedOps):
         n = w.shape[0]
         logits = self.ws.get("logits", (m, n), torch.float32)
         if HEAD_MIN_M <= m <= HEAD_MAX_M and isinstance(w, torch.Tensor) and w.dtype == torch.bfloat16 and w.is_contiguous() \
-                and w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0 and x.dtype == torch.bfloat16:
+                and w.shape[1] % 8 == 0 and w.shape[1] == x.shape[1] and w.data_ptr() % 16 == 0 and x.dtype == torch.bfloat16:
             h = self._rmsnorm(x.contiguous(), self._f32(norm_w), eps, name="h_head")
             N.check(self.lib.trl_head_bf16(h.data_ptr(), w.data_ptr(), logits.data_ptr(), n, m, n, w.shape[1], N.stream()), "head_bf16")
             N.count()
