@@ -28,3 +28,12 @@ def test_head_of_another_width_is_not_read_past_its_rows(monkeypatch):
     with pytest.raises(RuntimeError):
         _head(x(32, 48), w)
     assert _head(x(12, 48), w) == ["rows"]
+
+
+def test_workspace_takes_shapes_of_every_form():
+    """Lists as well as tuples; a buffer that was replaced gives no old view."""
+    ws = cuda.Workspace("cpu")
+    a = ws.get("a", [2, 3], torch.float32)
+    assert a.shape == (2, 3) and ws.get("a", (2, 3), torch.float32) is a and ws.get("a", torch.Size([2, 3]), torch.float32) is a
+    b = ws.get("a", (4, 3), torch.float32)
+    assert ws.get("a", (2, 3), torch.float32).data_ptr() == b.data_ptr() != a.data_ptr() and ws.retired[0].data_ptr() == a.data_ptr()

@@ -61,7 +61,7 @@ class Workspace:
         self.views: Dict[tuple, tuple] = {}       # (name, shape, dtype) -> (buffer, view of it): two tensor ops a call, 4 us
 
     def get(self, name: str, shape, dtype) -> torch.Tensor:
-        key = (name, shape, dtype)
+        key = (name, tuple(shape), dtype)
         hit = self.views.get(key)
         if hit is not None and hit[0] is self.bufs.get(name):
             return hit[1]
