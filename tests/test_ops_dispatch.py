@@ -30,8 +30,9 @@ def test_head_of_another_width_is_not_read_past_its_rows(monkeypatch):
     assert _head(x(12, 48), w) == ["rows"]
 
 
-def test_workspace_takes_shapes_of_every_form():
+def test_workspace_takes_shapes_of_every_form(monkeypatch):
     """Lists as well as tuples; a buffer that was replaced gives no old view."""
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     ws = cuda.Workspace("cpu")
     a = ws.get("a", [2, 3], torch.float32)
     assert a.shape == (2, 3) and ws.get("a", (2, 3), torch.float32) is a and ws.get("a", torch.Size([2, 3]), torch.float32) is a
