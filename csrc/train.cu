@@ -17,8 +17,9 @@ __device__ __forceinline__ float dot4(float4 a, float4 b) { return a.x * b.x + a
 __device__ __forceinline__ float sigm(float x) { return 1.f / (1.f + expf(-x)); }
 
 // ---- RMSNorm: a block a row, up to 8192 values ---------------------------------------------------------------------
+// kept (or null): a copy of the rows for the gradient, since the caller may write into x between the passes.
 template <int RN_V>                                 // vectors a thread keeps
-__global__ void __launch_bounds__(256) tr_rmsnorm_kernel(const float* x, const float* w, float* out, int h, float eps) {
+__global__ void __launch_bounds__(256) tr_rmsnorm_kernel(const float* x, const float* w, float* out, float* kept, int h, float eps) {
   __shared__ float red[32];
   const float* row = x + (size_t)blockIdx.x * h;
   float4 v[RN_V];
@@ -33,6 +34,7 @@ __global__ void __launch_bounds__(256) tr_rmsnorm_kernel(const float* x, const f
   for (int i = 0; i < RN_V; ++i) {
     const int c = (threadIdx.x + i * 256) * 4;
     if (c >= h) continue;
+    if (kept) st4(kept + (size_t)blockIdx.x * h + c, v[i]);
     const float4 g = ld4(w + c);
     st4(out + (size_t)blockIdx.x * h + c, make_float4(v[i].x * r * g.x, v[i].y * r * g.y, v[i].z * r * g.z, v[i].w * r * g.w));
   }
@@ -392,8 +394,8 @@ __global__ void __launch_bounds__(256) tr_softmax_grad_kernel(const float* p, fl
 
 // ---- cross-entropy -------------------------------------------------------------------------------------------------------
 // A row's largest value, sum of exponentials below it and log-sum-exp, [3, rows]; read once.  As torch for rows with infinities
-// and NaN.
-__global__ void __launch_bounds__(512) tr_lse_kernel(const float* lg, float* out, long V) {
+// and NaN.  kept (or null): a copy of the rows for the gradient, as the norm's.
+__global__ void __launch_bounds__(512) tr_lse_kernel(const float* lg, float* out, float* kept, long V) {
   __shared__ float red[32];
   const float* x = lg + (size_t)blockIdx.x * V;
   float m = -INFINITY, s = 0.f;
@@ -401,6 +403,7 @@ __global__ void __launch_bounds__(512) tr_lse_kernel(const float* lg, float* out
 #pragma unroll 4
   for (long c = threadIdx.x * 4; c < V; c += 2048) {
     const float4 v = ld4(x + c);
+    if (kept) st4(kept + (size_t)blockIdx.x * V + c, v);
     const float n = fmaxf(fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)), m);
     nan |= v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
     if (n > m) s *= expf(m - n), m = n;
@@ -481,9 +484,9 @@ AttnRows rows_of(const void* qkv, const void* qw, const void* kw, const void* cs
 }  // namespace
 
 // Rows of h values (h % 4 == 0, up to 8192), 16-byte aligned; so are all buffers below.
-TRL_API int trl_train_rmsnorm(const void* x, const void* w, void* out, int rows, int h, float eps, void* stream) {
+TRL_API int trl_train_rmsnorm(const void* x, const void* w, void* out, void* kept, int rows, int h, float eps, void* stream) {
   if (h % 4 || h > 8192 || rows < 1) return (int)cudaErrorInvalidValue;
-  (h <= 1024 ? tr_rmsnorm_kernel<1> : h <= 2048 ? tr_rmsnorm_kernel<2> : tr_rmsnorm_kernel<8>)<<<rows, 256, 0, (cudaStream_t)stream>>>((const float*)x, (const float*)w, (float*)out, h, eps);
+  (h <= 1024 ? tr_rmsnorm_kernel<1> : h <= 2048 ? tr_rmsnorm_kernel<2> : tr_rmsnorm_kernel<8>)<<<rows, 256, 0, (cudaStream_t)stream>>>((const float*)x, (const float*)w, (float*)out, (float*)kept, h, eps);
   return (int)cudaGetLastError();
 }
 TRL_API int trl_train_rmsnorm_grad(const void* x, const void* w, const void* up, void* dx, int rows, int h, float eps, void* stream) {
@@ -569,9 +572,9 @@ TRL_API int trl_train_softmax_grad(const void* p, void* dp, long rows, int T, fl
   return (int)cudaGetLastError();
 }
 
-TRL_API int trl_train_lse(const void* lg, void* stats, long rows, long V, void* stream) {
+TRL_API int trl_train_lse(const void* lg, void* stats, void* kept, long rows, long V, void* stream) {
   if (rows < 1 || rows >= 1l << 31 || V < 4 || V % 4) return (int)cudaErrorInvalidValue;
-  tr_lse_kernel<<<(int)rows, 512, 0, (cudaStream_t)stream>>>((const float*)lg, (float*)stats, V);
+  tr_lse_kernel<<<(int)rows, 512, 0, (cudaStream_t)stream>>>((const float*)lg, (float*)stats, (float*)kept, V);
   return (int)cudaGetLastError();
 }
 TRL_API int trl_train_ce_grad(const void* lg, const void* stats, const void* target, const void* weight, const void* up, void* grad, long rows, long V,

@@ -26,7 +26,9 @@ def kernels(monkeypatch):
         assert t.numel() >= n, "read past the end"
         return t.reshape(-1)[:n]
 
-    def rmsnorm(x, w, eps):
+    def rmsnorm(x, w, eps, kept=None):
+        if kept is not None:
+            kept.copy_(x)
         return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * w
 
     def swiglu(gu):
@@ -47,18 +49,23 @@ def kernels(monkeypatch):
         out, bwd = T._attention_torch(qkv, qw, kw, pos.to(torch.int64), **k)
         return out, lambda g: bwd(flat(g, out.numel()).view(out.shape))[0]
 
+    def lse(lg, kept=None):
+        if kept is not None:
+            kept.copy_(lg)
+        return torch.stack([lg.amax(-1), torch.exp(lg - lg.amax(-1, keepdim=True)).sum(-1), torch.logsumexp(lg, -1)])
+
     def cross_entropy_grad(lg, stats, tg, w, up):
         return ref.cross_entropy_grad(lg, tg, w)[1] * flat(up, 1)
 
     K = types.SimpleNamespace(
         calls=calls, grad_takes=train_kernels.grad_takes, _grad=train_kernels._grad,
         rmsnorm_takes=lambda x, w: True, rmsnorm=rmsnorm,
-        rmsnorm_grad=lambda x, w, g, eps: _grad_of(lambda x_: rmsnorm(x_, w, eps), flat(g, x.numel()).view(x.shape), x)[0],
+        rmsnorm_grad=lambda x, w, g, eps: T._rmsnorm_torch(x, w, eps)[1](flat(g, x.numel()).view(x.shape))[0],
         swiglu_takes=lambda gu: True, swiglu=swiglu,
         swiglu_grad=lambda gu, g: _grad_of(swiglu, flat(g, gu.numel() // 2).view(*gu.shape[:-1], -1), gu)[0],
         lora_takes=lambda y, x, a, b: True, lora=lora, lora_grad=lora_grad,
         attention_takes=lambda *a, **k: True, attention=attention,
-        cross_entropy_takes=lambda lg, tg, w: True, lse=lambda lg: torch.stack([lg.amax(-1), torch.exp(lg - lg.amax(-1, keepdim=True)).sum(-1), torch.logsumexp(lg, -1)]),
+        cross_entropy_takes=lambda lg, tg, w: True, lse=lse,
         cross_entropy_grad=cross_entropy_grad)
     monkeypatch.setattr(T, "_kernels", lambda x: K)
     monkeypatch.setattr(torch.cuda, "current_device", lambda: None)        # (a CPU tensor's device has no index)
@@ -188,26 +195,32 @@ def test_delta_rule_parameters_that_an_op_made_get_their_gradient(late, monkeypa
 
 
 def test_tensors_changed_between_the_passes(kernels):
-    """Targets and weights may be written into after the forward pass; logits, a norm's rows and an attention block's may not: the
-    gradient of other values would come back."""
+    """Logits, targets, weights and a norm's rows may be written into after the forward pass: the gradient is that of the values
+    that it saw.  An attention block's rows may not: both forms read some of them again."""
     g = torch.Generator().manual_seed(4)
     x, tg, w = torch.randn(4, 8, generator=g), torch.tensor([1, 7, 0, 3]), torch.rand(4, generator=g)
     want = ref.cross_entropy_grad(x, tg, w)[1]
-    tape = T.Tape()
-    tape.watch(x)
-    loss = T.cross_entropy(tape, x, tg, w)
-    tg.zero_(), w.zero_()
-    assert torch.allclose(tape.backward(loss)[id(x)], want)
-    for fn, t in ((lambda tape, t: T.cross_entropy(tape, t, tg, w), x), (lambda tape, t: T.rmsnorm(tape, t, torch.ones(8), 1e-6), x),
-                  (_ops()["attention"][0], torch.randn(1, 5, 24, generator=g))):
-        tape = T.Tape()
-        tape.watch(t)
-        y = fn(tape, t)
-        t.mul_(2.0)
-        with pytest.raises(RuntimeError, match="in place"):
-            tape.backward(y)
-        with torch.inference_mode():                 # (no count to look at)
-            fn(T.Tape(), t * 1.0)
+    up = torch.randn(4, 8, generator=g)
+    want_norm = T._rmsnorm_torch(x, torch.ones(8), 1e-6)[1](up)[0]
+    for inference in (False, True):                  # (whose tensors keep no count of the writes)
+        with torch.inference_mode(inference):
+            lg, t, v = x * 1.0, tg * 1, w * 1.0
+            tape = T.Tape()
+            tape.watch(lg)
+            loss = T.cross_entropy(tape, lg, t, v)
+            lg.zero_(), t.zero_(), v.zero_()
+            assert torch.allclose(tape.backward(loss)[id(lg)], want)
+            rows = x * 1.0
+            tape.watch(rows)
+            y = T.rmsnorm(tape, rows, torch.ones(8), 1e-6)
+            rows.zero_()
+            assert torch.allclose(tape.backward(y, up * 1.0)[id(rows)], want_norm, rtol=1e-5, atol=1e-6)
+    tape, qkv = T.Tape(), torch.randn(1, 5, 24, generator=g)
+    tape.watch(qkv)
+    y = _ops()["attention"][0](tape, qkv)
+    qkv.mul_(2.0)
+    with pytest.raises(RuntimeError, match="in place"):
+        tape.backward(y)
 
 
 def test_training_without_the_kernels(monkeypatch, tmp_path):

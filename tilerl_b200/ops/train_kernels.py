@@ -9,7 +9,7 @@ import torch
 
 from . import native as N
 
-N.register("trl_train_rmsnorm", [N.P] * 3 + [N.I] * 2 + [N.F, N.P])
+N.register("trl_train_rmsnorm", [N.P] * 4 + [N.I] * 2 + [N.F, N.P])
 N.register("trl_train_rmsnorm_grad", [N.P] * 4 + [N.I] * 2 + [N.F, N.P])
 N.register("trl_train_swiglu", [N.P] * 3 + [N.L, N.P])
 N.register("trl_train_lowrank", [N.P] * 3 + [N.I] * 4 + [N.F, N.P])
@@ -21,7 +21,7 @@ N.register("trl_train_attn_prep_grad", [N.P] * 11 + [N.I] * 8 + [N.F, N.P])
 N.register("trl_train_attn_gate", [N.P] * 3 + [N.I] * 7 + [N.P])
 N.register("trl_train_softmax", [N.P] * 2 + [N.I] * 4 + [N.F, N.P])
 N.register("trl_train_softmax_grad", [N.P] * 2 + [N.L, N.I, N.F, N.P])
-N.register("trl_train_lse", [N.P] * 2 + [N.L] * 2 + [N.P])
+N.register("trl_train_lse", [N.P] * 3 + [N.L] * 2 + [N.P])
 N.register("trl_train_ce_grad", [N.P] * 6 + [N.L] * 2 + [N.P])
 N.register("trl_train_adamw", [N.P] * 8 + [N.I] + [N.F] * 6 + [N.P])
 N.register("trl_train_squares", [N.P, N.P, N.I, N.P, N.P])
@@ -59,10 +59,11 @@ def rmsnorm_takes(x, w) -> bool:
     return h % 4 == 0 and h <= 8192 and w.dim() == 1 and w.numel() == h and plain(x, w) and x.numel() // h < 1 << 31
 
 
-def rmsnorm(x, w, eps):
+def rmsnorm(x, w, eps, kept=None):
+    """``kept``: gets a copy of ``x`` for the gradient, since the caller may write into ``x`` between the passes."""
     out = torch.empty_like(x)
     h = x.shape[-1]
-    N.check(N.lib().trl_train_rmsnorm(x.data_ptr(), w.data_ptr(), out.data_ptr(), x.numel() // h, h, eps, N.stream()), "train_rmsnorm")
+    N.check(N.lib().trl_train_rmsnorm(x.data_ptr(), w.data_ptr(), out.data_ptr(), N.ptr(kept), x.numel() // h, h, eps, N.stream()), "train_rmsnorm")
     N.count()
     return out
 
@@ -176,10 +177,10 @@ def cross_entropy_takes(logits, targets, weights) -> bool:
         and targets.numel() == weights.numel() == logits.numel() // logits.shape[-1] < 1 << 31
 
 
-def lse(lg):
-    """``[3, rows]``: largest value, sum of exponentials below it, log-sum-exp."""
+def lse(lg, kept=None):
+    """``[3, rows]``: largest value, sum of exponentials below it, log-sum-exp.  ``kept`` gets a copy of the rows, as :func:`rmsnorm`'s."""
     out = torch.empty(3, lg.shape[0], dtype=torch.float32, device=lg.device)
-    N.check(N.lib().trl_train_lse(lg.data_ptr(), out.data_ptr(), lg.shape[0], lg.shape[1], N.stream()), "train_lse")
+    N.check(N.lib().trl_train_lse(lg.data_ptr(), out.data_ptr(), N.ptr(kept), lg.shape[0], lg.shape[1], N.stream()), "train_lse")
     N.count()
     return out
 

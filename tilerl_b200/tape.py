@@ -139,8 +139,8 @@ def _kernels(x: torch.Tensor):
 
 
 def _unchanged(*kept: torch.Tensor) -> Callable[[], None]:
-    """For tensors that a backward kernel reads again: the check that nothing was written into them since (their torch forms keep
-    what they need, and would give the gradient of the old values; inference tensors keep no count)."""
+    """For tensors that a backward kernel reads again, as the torch form does: the check that nothing was written into them since
+    (inference tensors keep no count)."""
     kept = [(t, t._version) for t in kept if not t.is_inference()]
 
     def check():
@@ -182,16 +182,16 @@ def _rmsnorm_torch(x: torch.Tensor, w: torch.Tensor, eps: float):
 def rmsnorm(tape: Tape, x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
     K = _kernels(x)
     if K is not None and K.rmsnorm_takes(x, w):
-        out, unchanged = K.rmsnorm(x, w, eps), _unchanged(x)
+        kept = torch.empty_like(x) if tape.enabled else None
+        out = K.rmsnorm(x, w, eps, kept)
 
         def bwd_kernel(g):
-            unchanged()
-            if not K.grad_takes(g, x):
-                return _rmsnorm_torch(x, w, eps)[1](g)
+            if not K.grad_takes(g, kept):
+                return _rmsnorm_torch(kept, w, eps)[1](g)
             gw = None
             if tape.wants(w):
-                gw = (g.float() * x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps)).reshape(-1, x.shape[-1]).sum(0)
-            return K.rmsnorm_grad(x, w, g, eps), gw
+                gw = (g.float() * kept * torch.rsqrt(kept.pow(2).mean(-1, keepdim=True) + eps)).reshape(-1, kept.shape[-1]).sum(0)
+            return K.rmsnorm_grad(kept, w, g, eps), gw
 
         tape.record("rmsnorm", (x, w), (out,), bwd_kernel)
         return out
@@ -545,14 +545,15 @@ def cross_entropy(tape: Tape, logits: torch.Tensor, targets: torch.Tensor,
     K = _kernels(logits)
     if K is not None and K.cross_entropy_takes(logits, targets, weights):
         # the gradient is written once, in the backward pass, from each row's largest value and sum
-        tg, w, stats = targets.reshape(-1).to(torch.int64, copy=True), weights.reshape(-1).to(torch.float32, copy=True), K.lse(lg)
-        loss, unchanged = (w * (stats[2] - lg.gather(-1, tg[:, None]).squeeze(-1))).sum(), _unchanged(lg)
+        tg, w = targets.reshape(-1).to(torch.int64, copy=True), weights.reshape(-1).to(torch.float32, copy=True)
+        kept = torch.empty_like(lg) if tape.enabled else None
+        stats = K.lse(lg, kept)
+        loss = (w * (stats[2] - lg.gather(-1, tg[:, None]).squeeze(-1))).sum()
 
         def bwd_kernel(g):
-            unchanged()
             if not K.grad_takes(g, loss):
-                return (ref.cross_entropy_grad(lg, tg, w)[1].view_as(logits) * g,)
-            return (K.cross_entropy_grad(lg, stats, tg, w, g).view_as(logits),)
+                return (ref.cross_entropy_grad(kept, tg, w)[1].view_as(logits) * g,)
+            return (K.cross_entropy_grad(kept, stats, tg, w, g).view_as(logits),)
 
         tape.record("cross_entropy", (logits,), (loss,), bwd_kernel)
         return loss
