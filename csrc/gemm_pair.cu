@@ -21,7 +21,13 @@
 // Roles (10 warps): warp 0 = TMA producer of its SM's operands (a stage = 256 k; both SMs' copies count on the even one's
 // barrier), warp 1 = TMEM owner and, in the even SM, MMA issuer for both, warps 2-9 = epilogue: two groups of four, each
 // half of the columns.  A warp turns 32 rows x 16 tokens round through its own piece of shared memory, so that results leave
-// as 16-byte stores along a token's row (2 bytes a lane along the rows were 3.7 us a tile in the open).  Weights' and
+// as 16-byte stores along a token's row (2 bytes a lane along the rows were 3.7 us a tile in the open), or as 8-byte ones or one by
+// one where rows, strides or bases are no multiple (a rank's 2060 rows).  Before, those went to the one-SM kernel in whole tiles; that, here
+// as 8-byte stores, and a multiple of eight beside it, us with the quantiser, plain and with a residual:
+//     rows                    128                             512                             2000
+//     2060 x 5120      16.3 10.7 10.6, 23.9 11.4 10.7   18.9 14.2 13.9, 27.1 14.2 14.2   39.6 33.2 32.5, 56.2 34.4 33.5
+//     16 484 x 5120    20.7 18.3 18.1, 29.3 18.5 18.3   59.5 47.5 46.4, 104  49.6 51.4   209  151  142,  369  184  169
+// (one by one 11.7, 22.5; 16.9, 20.3; 44.2, 57.9 and 23.0, 29.0; 64.2, 96.4; 204, 318, residuals not yet requested ahead).  Weights' and
 // activations' scales come by tiled copies too, since only these may count on the other SM's barrier; none is multicast.
 //
 // In the reference's place: linear_fp4_fp8 / linear_fp4_mma8 (packages/tilerl-kernels/src/tilerl_kernels/kernels_linear.py:924-1687).
@@ -63,6 +69,7 @@ struct PairParams {
   const bf16* residual;
   void* out;
   int N, tokens, cols, ldr, ldo, r_tiles, c_tiles, nk, w_tiled, epi;
+  int vec;               // rows of a token that leave as one vector: 8, 4 or 1
   int parts;             // pairs that share a tile (a cluster), each a part of K; 1: a pair goes through whole tiles
 };
 
@@ -109,12 +116,36 @@ __device__ __forceinline__ void gp_mma(uint32_t d_tmem, uint32_t alo, uint32_t b
       ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory");
 }
 
+__device__ __forceinline__ float gp_swiglu(float g, float u, float s) { return __fdividef(g * s, 1.f + __expf(-(g * s))) * (u * s); }
+
+// A value of a row and token, times s, out; SwiGLU (rows in (gate, up) pairs): the pair of an even row.
+__device__ __forceinline__ void gp_store1(const PairParams& p, int tok, int row, float v, float up, float s, float res) {
+  const size_t at = (size_t)tok * p.ldo;
+  if (p.epi == GP_SWIGLU) {
+    if (!(row & 1) && row + 1 < p.N) reinterpret_cast<bf16*>(p.out)[at + (row >> 1)] = __float2bfloat16(gp_swiglu(v, up, s));
+  } else if (p.epi == GP_STORE_F32) {
+    reinterpret_cast<float*>(p.out)[at + row] = fmaf(v, s, res);
+  } else {
+    reinterpret_cast<bf16*>(p.out)[at + row] = __float2bfloat16(fmaf(v, s, res));
+  }
+}
+// Four of them.
+__device__ __forceinline__ void gp_store4(const PairParams& p, int tok, int row, float4 v, float s, uint2 res) {
+  const size_t at = (size_t)tok * p.ldo;
+  if (p.epi == GP_SWIGLU) {
+    *reinterpret_cast<uint32_t*>(reinterpret_cast<bf16*>(p.out) + at + (row >> 1)) = f2_to_bf162_bits(gp_swiglu(v.x, v.y, s), gp_swiglu(v.z, v.w, s));
+    return;
+  }
+  const float2 a = bf162_bits_to_f2(res.x), b = bf162_bits_to_f2(res.y);
+  v = make_float4(fmaf(v.x, s, a.x), fmaf(v.y, s, a.y), fmaf(v.z, s, b.x), fmaf(v.w, s, b.y));
+  if (p.epi == GP_STORE_F32) *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at + row) = v;
+  else *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(p.out) + at + row) = make_uint2(f2_to_bf162_bits(v.x, v.y), f2_to_bf162_bits(v.z, v.w));
+}
 // Eight values of a row block and token, times s, out.
 __device__ __forceinline__ void gp_store8(const PairParams& p, int tok, int row, float4 lo, float4 hi, float s, uint4 res) {
   if (p.epi == GP_SWIGLU) {                          // rows in (gate, up) pairs
-    auto act = [s](float g, float u) { return __fdividef(g * s, 1.f + __expf(-(g * s))) * (u * s); };
     *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(p.out) + (size_t)tok * p.ldo + (row >> 1)) =
-        make_uint2(f2_to_bf162_bits(act(lo.x, lo.y), act(lo.z, lo.w)), f2_to_bf162_bits(act(hi.x, hi.y), act(hi.z, hi.w)));
+        make_uint2(f2_to_bf162_bits(gp_swiglu(lo.x, lo.y, s), gp_swiglu(lo.z, lo.w, s)), f2_to_bf162_bits(gp_swiglu(hi.x, hi.y, s), gp_swiglu(hi.z, hi.w, s)));
     return;
   }
   const float2 a = bf162_bits_to_f2(res.x), b = bf162_bits_to_f2(res.y), c = bf162_bits_to_f2(res.z), d = bf162_bits_to_f2(res.w);
@@ -128,9 +159,50 @@ __device__ __forceinline__ void gp_store8(const PairParams& p, int tok, int row,
         make_uint4(f2_to_bf162_bits(lo.x, lo.y), f2_to_bf162_bits(lo.z, lo.w), f2_to_bf162_bits(hi.x, hi.y), f2_to_bf162_bits(hi.z, hi.w));
   }
 }
+// Residuals of V rows from `row` on, one vector (V = 1: in the low half).
+template <int V>
 __device__ __forceinline__ uint4 gp_residual(const PairParams& p, int tok, int row) {
-  return p.epi == GP_RESIDUAL && tok < p.tokens && row < p.N
-             ? __ldcg(reinterpret_cast<const uint4*>(p.residual + (size_t)tok * p.ldr + row)) : make_uint4(0u, 0u, 0u, 0u);
+  uint4 r = make_uint4(0u, 0u, 0u, 0u);
+  if (p.epi != GP_RESIDUAL || tok >= p.tokens || row >= p.N) return r;
+  const bf16* src = p.residual + (size_t)tok * p.ldr + row;
+  if constexpr (V == 8) {
+    r = __ldcg(reinterpret_cast<const uint4*>(src));
+  } else if constexpr (V == 4) {
+    const uint2 v = __ldcg(reinterpret_cast<const uint2*>(src));
+    r.x = v.x, r.y = v.y;
+  } else {
+    r.x = __ldcg(reinterpret_cast<const unsigned short*>(src));
+  }
+  return r;
+}
+
+// A warp's piece of 32 rows x T tokens, V rows a lane and vector: V tokens at a time, 64 bytes of each.  `res`: the residuals in the
+// order in which the values leave.
+template <int V, int T>
+__device__ __forceinline__ void gp_piece_residual(const PairParams& p, int tok0, int n0, int lane, uint32_t (&res)[T / 2]) {
+#pragma unroll
+  for (int i = 0; i < T / V; ++i) {
+    const uint4 r = gp_residual<V>(p, tok0 + i * V + lane / (32 / V), n0 + lane % (32 / V) * V);
+    if constexpr (V == 8) res[i * 4] = r.x, res[i * 4 + 1] = r.y, res[i * 4 + 2] = r.z, res[i * 4 + 3] = r.w;
+    else if constexpr (V == 4) res[i * 2] = r.x, res[i * 2 + 1] = r.y;
+    else res[i / 2] = i % 2 ? res[i / 2] | r.x << 16 : r.x;
+  }
+}
+template <int V, int T>
+__device__ __forceinline__ void gp_piece_store(const PairParams& p, int tok0, int n0, int lane, const float* tr, float s, const uint32_t (&res)[T / 2]) {
+#pragma unroll
+  for (int i = 0; i < T / V; ++i) {
+    const int t = i * V + lane / (32 / V), tok = tok0 + t, col = lane % (32 / V) * V, row = n0 + col;
+    const float* v = tr + t * GP_TR_STRIDE + col;
+    if (tok >= p.tokens || row >= p.N) continue;
+    if constexpr (V == 8) {
+      gp_store8(p, tok, row, reinterpret_cast<const float4*>(v)[0], reinterpret_cast<const float4*>(v)[1], s, make_uint4(res[i * 4], res[i * 4 + 1], res[i * 4 + 2], res[i * 4 + 3]));
+    } else if constexpr (V == 4) {
+      gp_store4(p, tok, row, *reinterpret_cast<const float4*>(v), s, make_uint2(res[i * 2], res[i * 2 + 1]));
+    } else {
+      gp_store1(p, tok, row, v[0], v[lane < 31], s, __uint_as_float(i % 2 ? res[i / 2] & 0xffff0000u : res[i / 2] << 16));
+    }
+  }
 }
 
 template <int BN, int J, bool SPLIT>
@@ -269,7 +341,6 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     pdl_wait();
     const int quad = warp & 3, half = (warp - 2) >> 2;
     constexpr int CHUNKS = C::COLS_WARP / C::CH, TPC = C::CH / J;    // a chunk's tokens: 8 or 16
-    constexpr int VECS = TPC / 8;                   // vectors of 8 rows a lane and chunk
     float* tr = reinterpret_cast<float*>(turn + (warp - 2) * GP_TR_BYTES);
     float* rs_s = tr + 16 * GP_TR_STRIDE;
     float* sum = reinterpret_cast<float*>(smem);    // parts: [token][128 rows] of this CTA's, in the ring, which is through by then
@@ -283,15 +354,16 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
       // what the values need besides the accumulator, requested before it is waited for: column scales (a lane a column), and
       // the residuals as they will leave (vectors of 8 rows)
       float rs[CHUNKS];
-      uint4 res[CHUNKS][VECS];
+      uint32_t res[CHUNKS][TPC / 2];
 #pragma unroll
       for (int c = 0; c < CHUNKS; ++c) {
         const int col = col0 + c * C::CH + lane;
         rs[c] = lane < C::CH && col < p.cols ? __ldcg(p.rs + col) : 0.f;
-#pragma unroll
-        for (int i = 0; i < VECS; ++i)
-          res[c][i] = SPLIT ? make_uint4(0u, 0u, 0u, 0u)
-                                  : gp_residual(p, tok0 + c * TPC + ((i * 32 + lane) >> 2), n0 + (lane & 3) * 8);
+        if (!SPLIT) {
+          if (p.vec == 8) gp_piece_residual<8, TPC>(p, tok0 + c * TPC, n0, lane, res[c]);
+          else if (p.vec == 4) gp_piece_residual<4, TPC>(p, tok0 + c * TPC, n0, lane, res[c]);
+          else gp_piece_residual<1, TPC>(p, tok0 + c * TPC, n0, lane, res[c]);
+        }
       }
       // (the warps of a group do not meet: each has its own barrier phase and its own piece of shared memory)
       if (!__all_sync(0xffffffffu, mbar_wait(acc_full(buf), (uint32_t)(n >> 1) & 1u, abort_flag))) break;
@@ -325,12 +397,10 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         }
         __syncwarp();
         if (!SPLIT) {
-#pragma unroll
-          for (int i = 0; i < VECS; ++i) {
-            const int t = (i * 32 + lane) >> 2, tok = tok0 + c * TPC + t, row = n0 + (lane & 3) * 8;
-            const float4* v = reinterpret_cast<const float4*>(tr + t * GP_TR_STRIDE + (lane & 3) * 8);
-            if (tok < p.tokens && row < p.N) gp_store8(p, tok, row, v[0], v[1], J == 4 ? 1.f : ts, res[c][i]);
-          }
+          const float s = J == 4 ? 1.f : ts;
+          if (p.vec == 8) gp_piece_store<8, TPC>(p, tok0 + c * TPC, n0, lane, tr, s, res[c]);
+          else if (p.vec == 4) gp_piece_store<4, TPC>(p, tok0 + c * TPC, n0, lane, tr, s, res[c]);
+          else gp_piece_store<1, TPC>(p, tok0 + c * TPC, n0, lane, tr, s, res[c]);
           __syncwarp();
         }
       }
@@ -345,7 +415,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     for (int i = t0 * 16 + (int)threadIdx.x; i < t1 * 16; i += GP_THREADS) {
       const int t = i >> 4, r = (i & 15) * 8, tok = ct * TOKENS + t, row = (rt * 2 + rank) * GP_ROWS + r;
       if (tok >= p.tokens || row >= p.N) continue;
-      const uint4 res = gp_residual(p, tok, row);
+      const uint4 res = p.vec == 8 ? gp_residual<8>(p, tok, row) : make_uint4(0u, 0u, 0u, 0u);
       float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
       for (int q = 0; q < p.parts; ++q) {
         const uint32_t src = gp_map(smem_u32(smem) + (uint32_t)(t * GP_ROWS + r) * 4u, 2 * q + rank);
@@ -353,7 +423,18 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         lo.x += a.x, lo.y += a.y, lo.z += a.z, lo.w += a.w;
         hi.x += b.x, hi.y += b.y, hi.z += b.z, hi.w += b.w;
       }
-      gp_store8(p, tok, row, lo, hi, 1.f, res);
+      if (p.vec == 8) {
+        gp_store8(p, tok, row, lo, hi, 1.f, res);
+      } else if (p.vec == 4) {
+        const uint4 a = gp_residual<4>(p, tok, row), b = gp_residual<4>(p, tok, row + 4);
+        gp_store4(p, tok, row, lo, 1.f, make_uint2(a.x, a.y));
+        if (row + 4 < p.N) gp_store4(p, tok, row + 4, hi, 1.f, make_uint2(b.x, b.y));
+      } else {
+        const float v[9] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w, 0.f};
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (row + e < p.N) gp_store1(p, tok, row + e, v[e], v[e + 1], 1.f, __uint_as_float(gp_residual<1>(p, tok, row + e).x << 16));
+      }
     }
   }
 
@@ -479,7 +560,7 @@ int gemm_pair_launch(const GemmPairArgs& a, int bn, cudaStream_t stream) {
   PairParams p;
   p.tscale = a.tscale, p.rs = a.rs, p.residual = (const bf16*)a.residual, p.out = a.out;
   p.N = a.N, p.tokens = a.tokens, p.cols = cols, p.ldr = a.ldr, p.ldo = a.ldo;
-  p.r_tiles = (n_tiles + 1) / 2, p.c_tiles = (cols + bn - 1) / bn, p.nk = nk, p.w_tiled = a.w_tiled, p.epi = a.epi, p.parts = a.parts;
+  p.r_tiles = (n_tiles + 1) / 2, p.c_tiles = (cols + bn - 1) / bn, p.nk = nk, p.w_tiled = a.w_tiled, p.epi = a.epi, p.parts = a.parts, p.vec = a.vec;
   const long long tiles = (long long)p.r_tiles * p.c_tiles;
   const int pairs = a.parts > 1 ? (int)tiles * a.parts : (int)(tiles < a.pairs ? tiles : a.pairs);
   if (bn == 32 && p.c_tiles > 1) return (int)cudaErrorInvalidValue;      // (its scales would start on an odd column of TMEM)

@@ -15,6 +15,7 @@ struct GemmPairArgs {
   int ldr, ldo, tokens, J, N, K, epi, w_tiled;
   int pairs;             // pairs of SMs there are
   int parts;             // pairs that share a tile, each a part of K
+  int vec;               // rows of a token that are one aligned vector in the output (of SwiGLU half as many results) and the residual: 8, 4 or 1
 };
 
 // Launches it with `bn` (128 or 192) columns a tile.

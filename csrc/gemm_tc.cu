@@ -34,7 +34,7 @@
 // so that one k-tile of a 128-row atom is 2 KB contiguous.
 //
 // Most products go to the form on pairs of SMs (gemm_pair.cu), which this file's launcher picks: the kernel here serves tiles
-// split over CTAs as asked for, more than four terms, and outputs that 16-byte stores do not fit.
+// split over CTAs as asked for and more than four terms.
 //
 // No counterpart exists in the reference: its Blackwell kernel cell is empty
 // (packages/tilerl-kernels/src/tilerl_kernels/registry.py:188-189); functionally this
@@ -1042,15 +1042,15 @@ TRL_API int trl_gemm_nvfp4(const void* wq, const void* sfw, const void* tscale, 
   const int cols = tokens * J;
   const PairPlan pp = plan_pair(tokens, J, N, K, max_ctas, split);
   if (pp.bn) {
-    // its stores are 8 rows of a token at a time (4 results of SwiGLU)
-    const int wide = epi == EPI_STORE_F32 || epi == EPI_SWIGLU ? 4 : 8, bytes = epi == EPI_SWIGLU ? 8 : 16;
-    if (N % 8 == 0 && ldo % wide == 0 && reinterpret_cast<uintptr_t>(out) % bytes == 0 &&
-        (epi != EPI_RESIDUAL || (ldr % 8 == 0 && reinterpret_cast<uintptr_t>(residual) % 16 == 0))) {
-      const GemmPairArgs a{wq, sfw, (const float*)tscale, xq, sfx, (const float*)rs, residual, out, ldr, ldo, tokens, J, N, K, epi,
-                           w_tiled, pp.pairs, pp.parts};
-      return gemm_pair_launch(a, pp.bn, (cudaStream_t)stream);
-    }
-    split = 0;                                            // no scratch was asked for
+    // rows of a token that leave at a time: 8 (16 bytes; SwiGLU: 4 results) where the output and the residual allow it, 4 or one
+    auto fits = [&](int v) {
+      const int results = epi == EPI_SWIGLU ? v / 2 : v, bytes = epi == EPI_STORE_F32 ? 16 : 2 * results;
+      return N % v == 0 && ldo % (epi == EPI_STORE_F32 ? 4 : results) == 0 && reinterpret_cast<uintptr_t>(out) % bytes == 0 &&
+             (epi != EPI_RESIDUAL || (ldr % v == 0 && reinterpret_cast<uintptr_t>(residual) % (2 * v) == 0));
+    };
+    const GemmPairArgs a{wq, sfw, (const float*)tscale, xq, sfx, (const float*)rs, residual, out, ldr, ldo, tokens, J, N, K, epi,
+                         w_tiled, pp.pairs, pp.parts, fits(8) ? 8 : fits(4) ? 4 : 1};
+    return gemm_pair_launch(a, pp.bn, (cudaStream_t)stream);
   }
   const GemmPlan g = plan_gemm(tokens, J, N, K, max_ctas, split);
   CUtensorMap mw, mx;

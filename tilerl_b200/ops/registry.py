@@ -102,8 +102,8 @@ register("nvfp4", "sm100", {
     "linear_nvfp4_rows16": Kernel("gemv_nvfp4_mma_kernel", "csrc/gemv_mma.cu", "trl_gemv_nvfp4_mma",
                                   note="3..16 rows: weights as the mma.sync A operand, f16 activations, every epilogue"),
     "linear_nvfp4_gemm": Kernel("gemm_nvfp4_kernel", "csrc/gemm_tc.cu", "trl_gemm_nvfp4", "tilerl_b200.ops.gemm_tc",
-                                note="tcgen05.mma kind::mxf4nvf4.block_scale; on pairs of SMs (gemm_nvfp4_pair_kernel, csrc/gemm_pair.cu) but for forced stream-K, "
-                                     "more than four terms and outputs off 16 bytes"),
+                                note="tcgen05.mma kind::mxf4nvf4.block_scale; on pairs of SMs (gemm_nvfp4_pair_kernel, csrc/gemm_pair.cu) but for forced stream-K "
+                                     "and more than four terms"),
     "quant_act_nvfp4": Kernel("quant_act_rows_kernel / quant_act_kernel", "csrc/gemm_tc.cu", "trl_quant_act_nvfp4", "tilerl_b200.ops.gemm_tc",
                               note="RMSNorm / SwiGLU + J NVFP4 residual terms per token"),
     "quantize_nvfp4": Kernel("quant_nvfp4_kernel", "csrc/misc.cu", "trl_quant_nvfp4", note="weights, in place (resync)"),
