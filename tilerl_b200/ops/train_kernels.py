@@ -24,7 +24,8 @@ N.register("trl_train_softmax_grad", [N.P] * 2 + [N.L, N.I, N.F, N.P])
 N.register("trl_train_lse", [N.P] * 3 + [N.L] * 2 + [N.P])
 N.register("trl_train_ce_grad", [N.P] * 6 + [N.L] * 2 + [N.P])
 N.register("trl_train_adamw", [N.P] * 8 + [N.I] + [N.F] * 6 + [N.P])
-N.register("trl_train_squares", [N.P, N.P, N.I, N.P, N.P])
+N.register("trl_train_squares_blocks", [N.L])
+N.register("trl_train_squares", [N.P, N.P, N.I, N.I, N.P, N.P])
 N.register("trl_train_scale", [N.P, N.P, N.I, N.F, N.P])
 
 INTEGERS = (torch.int64, torch.int32, torch.int16, torch.int8, torch.uint8)       # (positions between two tokens: the torch form)
@@ -230,16 +231,18 @@ def adamw(items: List[tuple], lr: float, betas, eps: float) -> None:
 
 
 def squares(grads: Dict[str, torch.Tensor]) -> Optional[torch.Tensor]:
-    """Sum of squares of every gradient in fp64, in the order of the dict; ``None`` where the kernel does not take them all."""
+    """Parts of the sum of squares of every gradient in fp64, a row each, in the order of the dict; ``None`` where the kernel does not
+    take them all."""
     gs = list(grads.values())
     if not gs or not plain(*gs):
         return None
-    part = torch.empty(len(gs), 16, dtype=torch.float64, device=gs[0].device)
+    blocks = N.lib().trl_train_squares_blocks(max(g.numel() for g in gs))
+    part = torch.empty(len(gs), blocks, dtype=torch.float64, device=gs[0].device)
     for i in range(0, len(gs), MAX_TENSORS):
         some = gs[i:i + MAX_TENSORS]
-        N.check(N.lib().trl_train_squares(_pointers(some), _lengths(some), len(some), part[i:].data_ptr(), N.stream()), "train_squares")
+        N.check(N.lib().trl_train_squares(_pointers(some), _lengths(some), len(some), blocks, part[i:].data_ptr(), N.stream()), "train_squares")
         N.count()
-    return part.sum(1)
+    return part
 
 
 def scale(tensors: Sequence[torch.Tensor], c: float) -> None:

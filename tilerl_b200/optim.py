@@ -38,12 +38,13 @@ def clip_grad_norm(grads: Dict[str, torch.Tensor], max_norm: float, *, sharded: 
         from .ops import train_kernels as many
         parts = many.squares(grads) if many.there() else None
         many = many if parts is not None else None
+    if many and sharded is None and tp_world <= 1:
+        return _scaled(grads, math.sqrt(float(parts.sum())), max_norm, many)
     sh = torch.zeros((), dtype=torch.float64, device=dev)
     rep = torch.zeros((), dtype=torch.float64, device=dev)
-    if many and sharded is None:
-        rep += parts.sum()
-    for i, (k, g) in enumerate(grads.items() if not many or sharded is not None else ()):
-        s = parts[i] if many else g.double().pow(2).sum()
+    sums = parts.sum(1) if many else None
+    for i, (k, g) in enumerate(grads.items()):
+        s = sums[i] if many else g.double().pow(2).sum()
         if sharded is not None and sharded(k):
             sh += s
         else:
@@ -58,7 +59,10 @@ def clip_grad_norm(grads: Dict[str, torch.Tensor], max_norm: float, *, sharded: 
         total = float(buf[0] + buf[1] / tp_world)
     else:
         total = float(sh + rep)
-    norm = math.sqrt(total)
+    return _scaled(grads, math.sqrt(total), max_norm, many)
+
+
+def _scaled(grads, norm: float, max_norm: float, many) -> float:
     if max_norm > 0 and norm > max_norm:
         c = max_norm / (norm + 1e-6)
         if many:
