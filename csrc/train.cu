@@ -394,8 +394,8 @@ __global__ void __launch_bounds__(256) tr_softmax_grad_kernel(const float* p, fl
 
 // ---- cross-entropy -------------------------------------------------------------------------------------------------------
 // A row's largest value, sum of exponentials below it and log-sum-exp, [3, rows]; read once.  As torch for rows with infinities
-// and NaN.  kept (or null): a copy of the rows for the gradient, as the norm's.
-__global__ void __launch_bounds__(512) tr_lse_kernel(const float* lg, float* out, float* kept, long V) {
+// and NaN.
+__global__ void __launch_bounds__(512) tr_lse_kernel(const float* lg, float* out, long V) {
   __shared__ float red[32];
   const float* x = lg + (size_t)blockIdx.x * V;
   float m = -INFINITY, s = 0.f;
@@ -403,7 +403,6 @@ __global__ void __launch_bounds__(512) tr_lse_kernel(const float* lg, float* out
 #pragma unroll 4
   for (long c = threadIdx.x * 4; c < V; c += 2048) {
     const float4 v = ld4(x + c);
-    if (kept) st4(kept + (size_t)blockIdx.x * V + c, v);
     const float n = fmaxf(fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)), m);
     nan |= v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
     if (n > m) s *= expf(m - n), m = n;
@@ -418,12 +417,12 @@ __global__ void __launch_bounds__(512) tr_lse_kernel(const float* lg, float* out
     out[2 * gridDim.x + blockIdx.x] = nan ? NAN : fabsf(all) < INFINITY ? all + logf(s) : all;
   }
 }
-// grad = (exp(lg - max) / sum - [c == target]) * weight * up.  (Not exp(lg - lse): an lse of 20 is rounded to 1e-6, and so would
+// grad = (exp(lg - max) / sum - [c == target]) * weight, in the forward pass: the caller may write into the logits before the other.  (Not exp(lg - lse): an lse of 20 is rounded to 1e-6, and so would
 // every probability be.)
-__global__ void __launch_bounds__(256) tr_ce_grad_kernel(const float* lg, const float* stats, const long long* target, const float* weight, const float* up,
+__global__ void __launch_bounds__(256) tr_ce_grad_kernel(const float* lg, const float* stats, const long long* target, const float* weight,
                                                          float* grad, long V) {
   const size_t at = (size_t)blockIdx.x * V;
-  const float m = stats[blockIdx.x], inv = 1.f / stats[gridDim.x + blockIdx.x], w = weight[blockIdx.x] * *up;
+  const float m = stats[blockIdx.x], inv = 1.f / stats[gridDim.x + blockIdx.x], w = weight[blockIdx.x];
   const long long t = target[blockIdx.x];
 #pragma unroll 4
   for (long c = threadIdx.x * 4; c < V; c += 1024) {
@@ -431,6 +430,16 @@ __global__ void __launch_bounds__(256) tr_ce_grad_kernel(const float* lg, const 
     float e[4] = {expf(v.x - m) * inv, expf(v.y - m) * inv, expf(v.z - m) * inv, expf(v.w - m) * inv};
     if (t >= c && t < c + 4) e[t - c] -= 1.f;
     st4(grad + at + c, make_float4(e[0] * w, e[1] * w, e[2] * w, e[3] * w));
+  }
+}
+
+// x times *up; no pass over the values where that is 1, as it is for a loss that is differentiated itself.
+__global__ void __launch_bounds__(256) tr_scale_by_kernel(float* x, const float* up, long n4) {
+  const float u = *up;
+  if (u == 1.f) return;
+  for (long i = (long)blockIdx.x * 256 + threadIdx.x; i < n4; i += (long)gridDim.x * 256) {
+    const float4 v = ld4(x + i * 4);
+    st4(x + i * 4, make_float4(v.x * u, v.y * u, v.z * u, v.w * u));
   }
 }
 
@@ -614,16 +623,21 @@ TRL_API int trl_train_softmax_grad(const void* p, void* dp, long rows, int T, fl
   return (int)cudaGetLastError();
 }
 
-TRL_API int trl_train_lse(const void* lg, void* stats, void* kept, long rows, long V, void* stream) {
+TRL_API int trl_train_lse(const void* lg, void* stats, long rows, long V, void* stream) {
   if (rows < 1 || rows >= 1l << 31 || V < 4 || V % 4) return (int)cudaErrorInvalidValue;
-  tr_lse_kernel<<<(int)rows, 512, 0, (cudaStream_t)stream>>>((const float*)lg, (float*)stats, (float*)kept, V);
+  tr_lse_kernel<<<(int)rows, 512, 0, (cudaStream_t)stream>>>((const float*)lg, (float*)stats, V);
   return (int)cudaGetLastError();
 }
-TRL_API int trl_train_ce_grad(const void* lg, const void* stats, const void* target, const void* weight, const void* up, void* grad, long rows, long V,
-                              void* stream) {
+TRL_API int trl_train_ce_grad(const void* lg, const void* stats, const void* target, const void* weight, void* grad, long rows, long V, void* stream) {
   if (rows < 1 || rows >= 1l << 31 || V < 4 || V % 4) return (int)cudaErrorInvalidValue;
   tr_ce_grad_kernel<<<(int)rows, 256, 0, (cudaStream_t)stream>>>((const float*)lg, (const float*)stats, (const long long*)target, (const float*)weight,
-                                                                (const float*)up, (float*)grad, V);
+                                                                (float*)grad, V);
+  return (int)cudaGetLastError();
+}
+TRL_API int trl_train_scale_by(void* x, const void* up, long n, void* stream) {
+  if (n < 4 || n % 4) return (int)cudaErrorInvalidValue;
+  const long blocks = (n / 4 + 1023) / 1024;
+  tr_scale_by_kernel<<<(int)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, (cudaStream_t)stream>>>((float*)x, (const float*)up, n / 4);
   return (int)cudaGetLastError();
 }
 

@@ -49,13 +49,11 @@ def kernels(monkeypatch):
         out, bwd = T._attention_torch(qkv, qw, kw, pos.to(torch.int64), **k)
         return out, lambda g: bwd(flat(g, out.numel()).view(out.shape))[0]
 
-    def lse(lg, kept=None):
-        if kept is not None:
-            kept.copy_(lg)
+    def lse(lg):
         return torch.stack([lg.amax(-1), torch.exp(lg - lg.amax(-1, keepdim=True)).sum(-1), torch.logsumexp(lg, -1)])
 
-    def cross_entropy_grad(lg, stats, tg, w, up):
-        return ref.cross_entropy_grad(lg, tg, w)[1] * flat(up, 1)
+    def cross_entropy_grad(lg, stats, tg, w):
+        return ref.cross_entropy_grad(lg, tg, w)[1]
 
     K = types.SimpleNamespace(
         calls=calls, grad_takes=train_kernels.grad_takes, _grad=train_kernels._grad,
@@ -66,7 +64,7 @@ def kernels(monkeypatch):
         lora_takes=lambda y, x, a, b: True, lora=lora, lora_grad=lora_grad,
         attention_takes=lambda *a, **k: True, attention=attention,
         cross_entropy_takes=lambda lg, tg, w: True, lse=lse,
-        cross_entropy_grad=cross_entropy_grad)
+        cross_entropy_grad=cross_entropy_grad, scale_by=lambda t, up: t.mul_(flat(up, 1)))
     monkeypatch.setattr(T, "_kernels", lambda x: K)
     monkeypatch.setattr(torch.cuda, "current_device", lambda: None)        # (a CPU tensor's device has no index)
     return K

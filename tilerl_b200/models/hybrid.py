@@ -317,7 +317,7 @@ class HybridModel:
             p = f"L{i}."
             if hook is not None:
                 hook.pre_layer(i)
-            h = T.rmsnorm(tape, x, P[p + "norm1"], eps)
+            h = T.rmsnorm(tape, x, P[p + "norm1"], eps, own=True)
             if tp:
                 h = T.tp_fork(tape, h)
             if cfg.layer_types[i] == ATTN:
@@ -336,7 +336,7 @@ class HybridModel:
             if tp:
                 y = T.all_reduce(tape, y)
             x = T.add(tape, x, y)
-            h = T.rmsnorm(tape, x, P[p + "norm2"], eps)
+            h = T.rmsnorm(tape, x, P[p + "norm2"], eps, own=True)
             if tp:
                 h = T.tp_fork(tape, h)
             act = T.swiglu(tape, self._tlinear(tape, h, p + "gate_up"))
@@ -355,7 +355,7 @@ class HybridModel:
                 x = layer(tape, x, i)
             if hook is not None and checkpoint_layers:
                 hook.post_layer(i)
-        h = T.rmsnorm(tape, x, P["final_norm"], eps)
+        h = T.rmsnorm(tape, x, P["final_norm"], eps, own=True)
         if tp:
             h = T.tp_fork(tape, h)
         head = "embed" if cfg.tie_embeddings else "lm_head"

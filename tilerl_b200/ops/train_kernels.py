@@ -21,8 +21,9 @@ N.register("trl_train_attn_prep_grad", [N.P] * 11 + [N.I] * 8 + [N.F, N.P])
 N.register("trl_train_attn_gate", [N.P] * 3 + [N.I] * 7 + [N.P])
 N.register("trl_train_softmax", [N.P] * 2 + [N.I] * 4 + [N.F, N.P])
 N.register("trl_train_softmax_grad", [N.P] * 2 + [N.L, N.I, N.F, N.P])
-N.register("trl_train_lse", [N.P] * 3 + [N.L] * 2 + [N.P])
-N.register("trl_train_ce_grad", [N.P] * 6 + [N.L] * 2 + [N.P])
+N.register("trl_train_lse", [N.P] * 2 + [N.L] * 2 + [N.P])
+N.register("trl_train_ce_grad", [N.P] * 5 + [N.L] * 2 + [N.P])
+N.register("trl_train_scale_by", [N.P] * 2 + [N.L, N.P])
 N.register("trl_train_adamw", [N.P] * 8 + [N.I] + [N.F] * 6 + [N.P])
 N.register("trl_train_squares_blocks", [N.L])
 N.register("trl_train_squares", [N.P, N.P, N.I, N.I, N.P, N.P])
@@ -178,20 +179,29 @@ def cross_entropy_takes(logits, targets, weights) -> bool:
         and targets.numel() == weights.numel() == logits.numel() // logits.shape[-1] < 1 << 31
 
 
-def lse(lg, kept=None):
-    """``[3, rows]``: largest value, sum of exponentials below it, log-sum-exp.  ``kept`` gets a copy of the rows, as :func:`rmsnorm`'s."""
+def lse(lg):
+    """``[3, rows]``: largest value, sum of exponentials below it, log-sum-exp."""
     out = torch.empty(3, lg.shape[0], dtype=torch.float32, device=lg.device)
-    N.check(N.lib().trl_train_lse(lg.data_ptr(), out.data_ptr(), N.ptr(kept), lg.shape[0], lg.shape[1], N.stream()), "train_lse")
+    N.check(N.lib().trl_train_lse(lg.data_ptr(), out.data_ptr(), lg.shape[0], lg.shape[1], N.stream()), "train_lse")
     N.count()
     return out
 
 
-def cross_entropy_grad(lg, stats, targets, weights, up):
-    g, up = torch.empty_like(lg), up.reshape(1).float()
-    N.check(N.lib().trl_train_ce_grad(lg.data_ptr(), stats.data_ptr(), targets.data_ptr(), weights.data_ptr(), up.data_ptr(), g.data_ptr(),
+def cross_entropy_grad(lg, stats, targets, weights):
+    g = torch.empty_like(lg)
+    N.check(N.lib().trl_train_ce_grad(lg.data_ptr(), stats.data_ptr(), targets.data_ptr(), weights.data_ptr(), g.data_ptr(),
                                       lg.shape[0], lg.shape[1], N.stream()), "train_ce_grad")
     N.count()
     return g
+
+
+def scale_by(t, up):
+    """``t`` times a number on the device, in place (nothing is touched where it is 1)."""
+    up = up.reshape(1).float()
+    N.check(N.lib().trl_train_scale_by(t.data_ptr(), up.data_ptr(), t.numel(), N.stream()), "train_scale_by")
+    torch.autograd.graph.increment_version(t)
+    N.count()
+    return t
 
 
 # ---- many tensors at a time -------------------------------------------------------------------------------------------

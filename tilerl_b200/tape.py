@@ -179,13 +179,18 @@ def _rmsnorm_torch(x: torch.Tensor, w: torch.Tensor, eps: float):
 
 
 @_nograd
-def rmsnorm(tape: Tape, x: torch.Tensor, w: torch.Tensor, eps: float) -> torch.Tensor:
+def rmsnorm(tape: Tape, x: torch.Tensor, w: torch.Tensor, eps: float, own: bool = False) -> torch.Tensor:
+    """``own``: nobody writes into ``x`` before the backward pass, which then reads it again (checked) instead of a copy."""
     K = _kernels(x)
     if K is not None and K.rmsnorm_takes(x, w):
-        kept = torch.empty_like(x) if tape.enabled else None
+        kept = torch.empty_like(x) if tape.enabled and not own else None
         out = K.rmsnorm(x, w, eps, kept)
+        if kept is None:
+            kept = x
+        unchanged = _unchanged(kept)
 
         def bwd_kernel(g):
+            unchanged()
             if not K.grad_takes(g, kept):
                 return _rmsnorm_torch(kept, w, eps)[1](g)
             gw = None
@@ -544,16 +549,14 @@ def cross_entropy(tape: Tape, logits: torch.Tensor, targets: torch.Tensor,
     lg = logits.reshape(-1, logits.shape[-1])
     K = _kernels(logits)
     if K is not None and K.cross_entropy_takes(logits, targets, weights):
-        # the gradient is written once, in the backward pass, from each row's largest value and sum
-        tg, w = targets.reshape(-1).to(torch.int64, copy=True), weights.reshape(-1).to(torch.float32, copy=True)
-        kept = torch.empty_like(lg) if tape.enabled else None
-        stats = K.lse(lg, kept)
+        tg, w, stats = targets.reshape(-1).long().contiguous(), weights.reshape(-1).float().contiguous(), K.lse(lg)
         loss = (w * (stats[2] - lg.gather(-1, tg[:, None]).squeeze(-1))).sum()
+        grad = K.cross_entropy_grad(lg, stats, tg, w) if tape.enabled else None
 
         def bwd_kernel(g):
             if not K.grad_takes(g, loss):
-                return (ref.cross_entropy_grad(kept, tg, w)[1].view_as(logits) * g,)
-            return (K.cross_entropy_grad(kept, stats, tg, w, g).view_as(logits),)
+                return (grad.view_as(logits) * g,)
+            return (K.scale_by(grad, g).view_as(logits),)
 
         tape.record("cross_entropy", (logits,), (loss,), bwd_kernel)
         return loss
