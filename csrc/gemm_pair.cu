@@ -205,7 +205,8 @@ __device__ __forceinline__ void gp_piece_store(const PairParams& p, int tok0, in
   }
 }
 
-template <int BN, int J, bool SPLIT>
+// V: p.vec where it is 8; else 0 (the branches on it cost a tick of 32 sequences 0.5 %, as one kernel for all).
+template <int BN, int J, bool SPLIT, int V>
 __global__ void __launch_bounds__(GP_THREADS, 1)
 gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_sfw,
                        const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_sfx, const PairParams p) {
@@ -360,7 +361,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         const int col = col0 + c * C::CH + lane;
         rs[c] = lane < C::CH && col < p.cols ? __ldcg(p.rs + col) : 0.f;
         if (!SPLIT) {
-          if (p.vec == 8) gp_piece_residual<8, TPC>(p, tok0 + c * TPC, n0, lane, res[c]);
+          if (V == 8) gp_piece_residual<8, TPC>(p, tok0 + c * TPC, n0, lane, res[c]);
           else if (p.vec == 4) gp_piece_residual<4, TPC>(p, tok0 + c * TPC, n0, lane, res[c]);
           else gp_piece_residual<1, TPC>(p, tok0 + c * TPC, n0, lane, res[c]);
         }
@@ -398,7 +399,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         __syncwarp();
         if (!SPLIT) {
           const float s = J == 4 ? 1.f : ts;
-          if (p.vec == 8) gp_piece_store<8, TPC>(p, tok0 + c * TPC, n0, lane, tr, s, res[c]);
+          if (V == 8) gp_piece_store<8, TPC>(p, tok0 + c * TPC, n0, lane, tr, s, res[c]);
           else if (p.vec == 4) gp_piece_store<4, TPC>(p, tok0 + c * TPC, n0, lane, tr, s, res[c]);
           else gp_piece_store<1, TPC>(p, tok0 + c * TPC, n0, lane, tr, s, res[c]);
           __syncwarp();
@@ -415,7 +416,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     for (int i = t0 * 16 + (int)threadIdx.x; i < t1 * 16; i += GP_THREADS) {
       const int t = i >> 4, r = (i & 15) * 8, tok = ct * TOKENS + t, row = (rt * 2 + rank) * GP_ROWS + r;
       if (tok >= p.tokens || row >= p.N) continue;
-      const uint4 res = p.vec == 8 ? gp_residual<8>(p, tok, row) : make_uint4(0u, 0u, 0u, 0u);
+      const uint4 res = V == 8 ? gp_residual<8>(p, tok, row) : make_uint4(0u, 0u, 0u, 0u);
       float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
       for (int q = 0; q < p.parts; ++q) {
         const uint32_t src = gp_map(smem_u32(smem) + (uint32_t)(t * GP_ROWS + r) * 4u, 2 * q + rank);
@@ -423,7 +424,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         lo.x += a.x, lo.y += a.y, lo.z += a.z, lo.w += a.w;
         hi.x += b.x, hi.y += b.y, hi.z += b.z, hi.w += b.w;
       }
-      if (p.vec == 8) {
+      if (V == 8) {
         gp_store8(p, tok, row, lo, hi, 1.f, res);
       } else if (p.vec == 4) {
         const uint4 a = gp_residual<4>(p, tok, row), b = gp_residual<4>(p, tok, row + 4);
@@ -472,9 +473,9 @@ bool gp_tensor(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dim
                 swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, int J, bool SPLIT>
+template <int BN, int J, bool SPLIT, int V>
 int launch_pair(const CUtensorMap (&m)[4], const PairParams& p, int pairs, cudaStream_t stream) {
-  auto kern = gemm_nvfp4_pair_kernel<BN, J, SPLIT>;
+  auto kern = gemm_nvfp4_pair_kernel<BN, J, SPLIT, V>;
   static TrlPerDevice<bool> set;
   bool& configured = set.here();
   if (!configured) {
@@ -494,7 +495,8 @@ int launch_pair(const CUtensorMap (&m)[4], const PairParams& p, int pairs, cudaS
 
 template <int BN, int J>
 int launch_pair(const CUtensorMap (&m)[4], const PairParams& p, int pairs, cudaStream_t stream) {
-  return p.parts > 1 ? launch_pair<BN, J, true>(m, p, pairs, stream) : launch_pair<BN, J, false>(m, p, pairs, stream);
+  if (p.vec == 8) return p.parts > 1 ? launch_pair<BN, J, true, 8>(m, p, pairs, stream) : launch_pair<BN, J, false, 8>(m, p, pairs, stream);
+  return p.parts > 1 ? launch_pair<BN, J, true, 0>(m, p, pairs, stream) : launch_pair<BN, J, false, 0>(m, p, pairs, stream);
 }
 
 template <int J>
@@ -514,7 +516,7 @@ int gemm_pair_clusters(int parts) {
   if (parts < 1 || parts > 3) return 0;
   int& known = counts[parts].here();
   if (known == 0) {
-    auto kern = gemm_nvfp4_pair_kernel<64, 2, true>;
+    auto kern = gemm_nvfp4_pair_kernel<64, 2, true, 8>;
     constexpr int smem = PairCfg<64, 2>::SMEM;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * parts), cfg.blockDim = dim3(GP_THREADS), cfg.dynamicSmemBytes = smem;
