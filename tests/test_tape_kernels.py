@@ -283,3 +283,16 @@ def test_tensors_that_share_memory_are_not_in_one_launch(monkeypatch):
         launches.clear()
         train_kernels.scale(tensors, 0.5)
         assert launches == want
+
+
+def test_adapters_go_to_the_kernels_where_they_are_faster(monkeypatch):
+    """Few wide rows, and rank 32 over many, stay with the library's products."""
+    monkeypatch.setattr(train_kernels, "plain", lambda *t: True)
+    e = lambda *s: torch.empty(*s, device="meta")
+    takes = lambda m, k, n, r: train_kernels.lora_takes(None, e(m, k), e(r, k), e(n, r))
+    for m, k, n, r, want in ((1, 1024, 3072, 16, True), (1, 6144, 5120, 32, True), (31, 5120, 34816, 8, False), (32, 5120, 34816, 8, True), (16, 17408, 5120, 16, False),
+                             (2048, 1024, 6144, 32, True), (4096, 1024, 3072, 32, True), (8192, 1024, 3072, 32, False), (1024, 17408, 5120, 32, True),
+                             (2048, 17408, 5120, 32, False), (256, 5120, 34816, 32, False), (16384, 17408, 5120, 16, True), (64, 1024, 3072, 12, False)):
+        assert takes(m, k, n, r) == want, (m, k, n, r)
+        y = e(m, n)
+        assert train_kernels.lora_takes(y, e(m, k), e(r, k), e(n, r)) == want

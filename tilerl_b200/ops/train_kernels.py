@@ -99,9 +99,20 @@ def swiglu_grad(gu, g):
 # ---- adapters: y + s (x A^T) B^T -----------------------------------------------------------------------------
 def lora_takes(y, x, a, b) -> bool:
     """``y`` may be ``None`` (a dense product's bf16 result to come)."""
-    r, k = a.shape
-    return (r in (4, 8, 16, 32) and k % 4 == 0 and b.shape[0] % 4 == 0 and b.shape[1] == r and x.shape[-1] == k and plain(x, a, b)
-            and x.numel() // k <= 16 * 65535 and (y is None or (y.shape[-1] == b.shape[0] and x.shape[:-1] == y.shape[:-1] and plain(y))))
+    (r, k), n = a.shape, b.shape[0]
+    return (r in (4, 8, 16, 32) and k % 4 == 0 and n % 4 == 0 and b.shape[1] == r and x.shape[-1] == k and _lora_pays(x.numel() // k, k, n, r) and plain(x, a, b)
+            and x.numel() // k <= 16 * 65535 and (y is None or (y.shape[-1] == n and x.shape[:-1] == y.shape[:-1] and plain(y))))
+
+
+def _lora_pays(m: int, k: int, n: int, r: int) -> bool:
+    """Sizes where the kernels beat the torch ops (whose products are the library's).  Forward and gradient over a frozen weight, torch and
+    here, us.  Few wide rows leave most of the GPU idle, a block going through all of them: 5120 -> 34 816, 16 rows of rank 16 271, 381, 32 rows 375,
+    377; 16 480 16 rows 213, 231, 32 rows 273, 234; 6144 -> 5120 from one row on 194, 133.  Rank 32 passes over the rows twice, and a good GEMM does
+    not: 1024 -> 3072, 4096 rows 407, 388, 8192 rows 658, 725; 6144 -> 5120 2048 rows 660, 610, 8192 1958, 2158; 17 408 -> 5120 1024 rows 706, 652,
+    2048 rows 1226, 1223, 8192 4246, 4582; 34 816 at no length."""
+    if m < 32 and max(k, n) > 8192:
+        return False
+    return r < 32 or (m <= 4096 and k + n <= 32768 and m * (k + n) <= 2048 * 16384)
 
 
 def lora(y, x, a, b, s):
