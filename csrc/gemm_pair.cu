@@ -61,6 +61,7 @@ struct PairCfg {
   // TMEM: accumulators at 0 and BN, two buffers of 64 columns of scale factors behind them
   static constexpr int TMEM_COLS = BN <= 64 ? 256 : 512, SF_COL0 = TMEM_COLS - 128;
   static_assert(OFF_SFB + SFB_BYTES == STAGE && STAGE % 1024 == 0 && SMEM <= 227 * 1024 && 2 * BN <= SF_COL0, "layout");
+  static_assert(SMEM >= 208 * 1024, "no other kernel with TMEM fits beside it on an SM");
 };
 
 struct PairParams {
@@ -83,6 +84,13 @@ __device__ __forceinline__ float4 gp_ld_cluster(uint32_t addr) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
+// What a CTA waits for without a limit, and why it ends.  A cluster barrier takes the place of __syncthreads for two to six CTAs
+// that the hardware starts together; shared memory of another CTA may only be touched once one has been passed, and no CTA may
+// leave before the last access to its own, so an mbarrier with a limit can stand in for neither the first nor the last.  Every thread
+// comes to each of them: no path returns early, and all waits in between (the ring, the accumulators, the producers' tail) have
+// a limit, after which they leave their loop.  The allocation of TMEM waits for the other CTA's, right behind the first barrier, and
+// for columns to be free: a CTA leaves too little shared memory on its SM for any other kernel that holds some (the smallest takes
+// more, and gives its columns back on every path).  The release waits for the other CTA's, behind a barrier too.
 // Not the .aligned forms: the warps come here from loops and branches that their lanes left at different times, and a warp
 // that is not converged would count more than once.
 __device__ __forceinline__ void gp_cluster_sync() {

@@ -971,7 +971,7 @@ TRL_API int trl_gemm_trace_read(void* out, int n_ctas) {
 }
 
 // Columns a tile, pairs that share a tile along K (1, 2 or 3: a cluster of up to six CTAs), and pairs there are; bn 0: not for
-// the pair form (more than four terms, tiles split over CTAs as asked for, less than a pair of SMs).  Costs in units of a k-tile
+// the pair form (more than four terms, tiles split over CTAs as asked for, the one-SM form as asked for, less than a pair of SMs).  Costs in units of a k-tile
 // of 128 columns, 0.2 us: one of 192 takes 1.25 (256 columns of 34 816 x 5120: 31.5 us in tiles of 128, 33.3 of 192; 512
 // columns, 8 rounds against 6: 51.1 and 46.0), one of 64 or 32, where the weights bound, a little less; parts cost the exchange
 // of their sums, more of them more.  With the quantiser, one, two, three parts: 5120 x 17 408, 8 rows 22.7, 18.0, 16.9 us, 32
@@ -981,13 +981,14 @@ TRL_API int trl_gemm_trace_read(void* out, int n_ctas) {
 struct PairPlan {
   int bn, parts, pairs;
 };
+enum { SPLIT_ONE_SM = -2, SPLIT_ONE_SM_WHOLE = 2 };      // of `split`: as -1 and 0, on one SM
 static PairPlan plan_pair(int tokens, int J, int N, int K, int max_ctas, int split) {
   PairPlan best{0, 1, 0};
   int sms = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int pairs = (max_ctas > 0 ? min(sms, max_ctas) : sms) / 2;
-  if (split == 1 || (J != 1 && J != 2 && J != 4) || pairs < 1) return best;
+  if (split == 1 || split == SPLIT_ONE_SM || split == SPLIT_ONE_SM_WHOLE || (J != 1 && J != 2 && J != 4) || pairs < 1) return best;
   static const struct { int bn; double unit, exchange; } forms[] = {{32, 0.85, 1}, {64, 0.9, 2}, {128, 1, 9}, {192, 1.25, 12}};
   const int cols = tokens * J, nk = (K + KT_ELEMS - 1) / KT_ELEMS, r_tiles = (N + 2 * TILE_N - 1) / (2 * TILE_N);
   double least = 0;
@@ -1019,7 +1020,7 @@ static GemmPlan plan_gemm(int tokens, int J, int N, int K, int max_ctas, int spl
   if (max_ctas > 0) sms = min(sms, max_ctas);
   const long long T = (long long)g.n_tiles * g.c_tiles, U = T * g.nk;
   const double whole = (double)((T + sms - 1) / sms) * g.nk, even = (double)U / sms + (g.BN == 256 ? 16 : 10);
-  g.split = split >= 0 ? split : (T < sms || whole > 1.05 * even);
+  g.split = split == SPLIT_ONE_SM_WHOLE ? 0 : split >= 0 ? split : (T < sms || whole > 1.05 * even);
   g.grid = (int)min((long long)sms, g.split ? U : T);
   g.max_seg = g.split ? max_segments(U, g.grid, g.nk) : 1;
   return g;

@@ -82,3 +82,21 @@ def test_rows_that_are_no_multiple_of_eight_cost_little_more(ops, tokens):
     torch.cuda.synchronize()
     us = {n: statistics.median(a.elapsed_time(b) for a, b in t) for n, t in times.items()}
     assert us[2060] < 1.45 * us[2064], us
+
+
+def test_one_sm_as_asked_for(ops, monkeypatch):
+    """``TRL_GEMM_PAIR=0``: by its own rules the one-SM kernel gives what it gives when asked for by the number of CTAs, and needs scratch
+    where it splits tiles, which the form on pairs never does."""
+    lib = ops.lib
+    assert lib.trl_gemm_nvfp4_scratch_bytes(8, 4, 5120, 17408, 0, -1) == 0 < lib.trl_gemm_nvfp4_scratch_bytes(8, 4, 5120, 17408, 0, -2)
+    assert lib.trl_gemm_nvfp4_scratch_bytes(8, 4, 5120, 17408, 0, 2) == 0
+    g = torch.Generator().manual_seed(0)
+    w = F.quantize_nvfp4(torch.randn(1288, 4128, generator=g) * 0.02).to(DEV)
+    x = torch.randn(100, 4128, generator=g).to(DEV, torch.bfloat16)
+    want, got = torch.empty(100, 1288, device=DEV), torch.empty(100, 1288, device=DEV)
+    gemm_nvfp4(ops, x, w, want, terms=2, epi=3, max_ctas=1, split=False)
+    monkeypatch.setenv("TRL_GEMM_PAIR", "0")
+    gemm_nvfp4(ops, x, w, got, terms=2, epi=3, split=False)
+    assert torch.equal(got, want)
+    gemm_nvfp4(ops, x, w, got, terms=2, epi=3)
+    assert _rel(got, want) < 1e-6

@@ -38,3 +38,16 @@ def test_workspace_takes_shapes_of_every_form(monkeypatch):
     assert a.shape == (2, 3) and ws.get("a", (2, 3), torch.float32) is a and ws.get("a", torch.Size([2, 3]), torch.float32) is a
     b = ws.get("a", (4, 3), torch.float32)
     assert ws.get("a", (2, 3), torch.float32).data_ptr() == b.data_ptr() != a.data_ptr() and ws.retired[0].data_ptr() == a.data_ptr()
+
+
+def test_gemm_on_one_sm_as_asked_for(monkeypatch):
+    """``TRL_GEMM_PAIR=0`` keeps every layout off the kernel on pairs; without it nothing changes."""
+    from tilerl_b200.ops.gemm_tc import _want_split
+    for pair, forms in (("1", {None: -1, False: 0, True: 1}), ("0", {None: -2, False: 2, True: 1})):
+        monkeypatch.setenv("TRL_GEMM_PAIR", pair)
+        for split, want in forms.items():
+            assert _want_split(split) == want
+    monkeypatch.setenv("TRL_SPLITK", "0")
+    assert _want_split() == 2 and _want_split(True) == 1
+    monkeypatch.delenv("TRL_GEMM_PAIR")
+    assert _want_split() == 0

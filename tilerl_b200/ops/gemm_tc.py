@@ -10,6 +10,7 @@
 """
 from __future__ import annotations
 
+import os
 from typing import Optional
 
 import torch
@@ -152,11 +153,12 @@ def _scratch(ops, nbytes: int, tiles: int):
     return buf, ops.ws.bufs["tc_counters"]
 
 
-def _want_split() -> int:
-    """Split tiles along K: 1 / 0 forced by ``TRL_SPLITK``, -1: by the launcher's rule (``csrc/gemm_tc.cu::plan_gemm``)."""
-    import os
+def _want_split(split: Optional[bool] = None) -> int:
+    """How tiles are laid out: 1 split along K on the kernel of one SM, 0 whole, -1 by the launcher's rules (``csrc/gemm_tc.cu::plan_pair``,
+    ``plan_gemm``); ``TRL_SPLITK`` forces 1 or 0 where the caller leaves it open.  ``TRL_GEMM_PAIR=0``: 0 and -1 on the kernel of one SM too (2, -2)."""
     mode = os.environ.get("TRL_SPLITK", "auto")
-    return int(mode) if mode in ("0", "1") else -1
+    want = int(split) if split is not None else int(mode) if mode in ("0", "1") else -1
+    return want if os.environ.get("TRL_GEMM_PAIR", "1") != "0" else {0: 2, -1: -2}.get(want, want)
 
 
 def gemm_nvfp4(ops, x: torch.Tensor, w: NVFP4Tensor, y: torch.Tensor, *, terms: int = 1, norm_w=None,
@@ -171,7 +173,7 @@ def gemm_nvfp4(ops, x: torch.Tensor, w: NVFP4Tensor, y: torch.Tensor, *, terms: 
         bn *= 2
     c_tiles = (cols + bn - 1) // bn
     n_tiles = (n + 127) // 128
-    split = _want_split() if split is None else int(split)
+    split = _want_split(split)
     nbytes = ops.lib.trl_gemm_nvfp4_scratch_bytes(t, terms, n, k, max_ctas, split)
     partial, counters = _scratch(ops, nbytes, n_tiles * c_tiles)
     tiled = getattr(ops, "tile_weights", True)
