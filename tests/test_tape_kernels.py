@@ -296,3 +296,17 @@ def test_adapters_go_to_the_kernels_where_they_are_faster(monkeypatch):
         assert takes(m, k, n, r) == want, (m, k, n, r)
         y = e(m, n)
         assert train_kernels.lora_takes(y, e(m, k), e(r, k), e(n, r)) == want
+
+
+def test_narrow_rows_and_short_sequences_in_numbers_stay_with_torch(monkeypatch):
+    monkeypatch.setattr(train_kernels, "plain", lambda *t: True), monkeypatch.setattr(gdn_train.N, "has", lambda name: True)
+    e = lambda *s: torch.empty(*s, device="meta")
+    for rows, h, want in ((65536, 64, True), (65537, 64, False), (262144, 252, False), (262144, 256, True), (512, 64, True)):
+        assert train_kernels.rmsnorm_takes(e(rows, h), e(h)) == want
+    for rows, v, want in ((8192, 128, True), (262144, 128, False), (65536, 512, True)):
+        assert train_kernels.cross_entropy_takes(e(rows, v), e(rows), e(rows)) == want
+    for m, k, want in ((16384, 64, True), (262144, 64, False), (65536, 512, True), (65537, 512, False), (131072, 1024, True), (65536, 256, False)):
+        assert train_kernels.lora_takes(None, e(m, k), e(16, k), e(k, 16)) == want
+    for b, t, nv, want in ((512, 1, 8, False), (512, 8, 8, True), (1, 1, 2, True), (256, 1, 8, True)):
+        ch = (2 + nv) * 128
+        assert gdn_train.takes(e(b, t, ch + nv * 130), e(ch, 4), e(nv), e(nv), e(128), nk=1, nv=nv, dk=128, dv=128, eps=1e-6) == want

@@ -16,6 +16,10 @@ N.register("trl_gdn_train_backward", [N.P] * 9 + [N.I] * 5 + [N.F, N.P])
 def takes(inp, conv_w, dt_bias, a_log, norm_w, *, nk, nv, dk, dv, eps, chunk=64, state=None, cp=None) -> bool:
     if cp is not None or state is not None or dk != 128 or dv != 128 or nv % nk or nv % 2 or inp.dim() != 3 or inp.numel() == 0:
         return False
+    # a sequence is a whole chunk of 32 tokens at least: 512 of one token with eight heads 4522 us with the gradient, 3634 as torch ops; of eight
+    # tokens 4609 and 5520
+    if inp.shape[1] < 8 and inp.shape[0] * nv > 2048:
+        return False
     if not N.has("trl_gdn_train_forward"):           # (a library of one architecture)
         return False
     rows = 2 * nk * dk + 2 * nv * dv + 2 * nv

@@ -57,7 +57,10 @@ def _grad(g: torch.Tensor) -> torch.Tensor:
 
 # ---- RMSNorm ---------------------------------------------------------------------------------------------
 def rmsnorm_takes(x, w) -> bool:
+    """Not many narrow rows, of which a block each is mostly idle: 262 144 x 64 722 us with its gradient, 570 as torch ops; 65 536 x 256 218 and 501."""
     h = x.shape[-1]
+    if h < 256 and x.numel() > 65536 * h:
+        return False
     return h % 4 == 0 and h <= 8192 and w.dim() == 1 and w.numel() == h and plain(x, w) and x.numel() // h < 1 << 31
 
 
@@ -109,7 +112,9 @@ def _lora_pays(m: int, k: int, n: int, r: int) -> bool:
     here, us.  Few wide rows leave most of the GPU idle, a block going through all of them: 5120 -> 34 816, 16 rows of rank 16 271, 381, 32 rows 375,
     377; 16 480 16 rows 213, 231, 32 rows 273, 234; 6144 -> 5120 from one row on 194, 133.  Rank 32 passes over the rows twice, and a good GEMM does
     not: 1024 -> 3072, 4096 rows 407, 388, 8192 rows 658, 725; 6144 -> 5120 2048 rows 660, 610, 8192 1958, 2158; 17 408 -> 5120 1024 rows 706, 652,
-    2048 rows 1226, 1223, 8192 4246, 4582; 34 816 at no length."""
+    2048 rows 1226, 1223, 8192 4246, 4582; 34 816 at no length.  Many narrow rows: 262 144 x 256 rank 16 1273, 2216, 65 536 x 512 827, 782, 131 072 x 1024 rank 8 2004, 1748."""
+    if m > (65536 if min(k, n) >= 512 else 16384) and min(k, n) < 1024:
+        return False
     if m < 32 and max(k, n) > 8192:
         return False
     return r < 32 or (m <= 4096 and k + n <= 32768 and m * (k + n) <= 2048 * 16384)
@@ -186,6 +191,9 @@ def attention(qkv, q_norm_w, k_norm_w, positions, *, n_q, n_kv, head_dim, rotary
 
 # ---- cross-entropy ------------------------------------------------------------------------------------------------
 def cross_entropy_takes(logits, targets, weights) -> bool:
+    """Not many rows of few classes: 262 144 x 128 1714 us with its gradient, 830 as torch ops; 65 536 x 1000 601 and 986."""
+    if logits.shape[-1] < 512 and logits.numel() > 8192 * logits.shape[-1]:
+        return False
     return logits.shape[-1] % 4 == 0 and plain(logits) and targets.device == logits.device and weights.device == logits.device \
         and targets.numel() == weights.numel() == logits.numel() // logits.shape[-1] < 1 << 31
 
