@@ -1,7 +1,7 @@
 // Gated delta rule over whole sequences for training: forward, and its gradient, in fp32.
 //
 // The tape's op used to run the chunked form as torch ops and differentiate it with autograd: over a thousand launches of a few
-// microseconds a layer and step, bound by the host.  Here a forward is four launches and a gradient nine.  Chunks of 32 tokens: the
+// microseconds a layer and step, bound by the host.  Here a forward is four launches and a gradient eight.  Chunks of 32 tokens: the
 // products within a chunk grow with its length, what goes from chunk to chunk is a [128, 128] state, and a warp has a lane a
 // token for everything that is one number a token.  Per chunk, head, with S the state before it, G the running sum of the log
 // decays, D_ij = exp(G_i - G_j):

@@ -89,8 +89,8 @@ __device__ __forceinline__ float4 gp_ld_cluster(uint32_t addr) {
 // leave before the last access to its own, so an mbarrier with a limit can stand in for neither the first nor the last.  Every thread
 // comes to each of them: no path returns early, and all waits in between (the ring, the accumulators, the producers' tail) have
 // a limit, after which they leave their loop.  The allocation of TMEM waits for the other CTA's, right behind the first barrier, and
-// for columns to be free: a CTA leaves too little shared memory on its SM for any other kernel that holds some (the smallest takes
-// more, and gives its columns back on every path).  The release waits for the other CTA's, behind a barrier too.
+// for columns to be free: a CTA leaves too little shared memory on its SM for any other kernel that holds some (each takes
+// 190 KB or more, and gives its columns back on every path).  The release waits for the other CTA's, behind a barrier too.
 // Not the .aligned forms: the warps come here from loops and branches that their lanes left at different times, and a warp
 // that is not converged would count more than once.
 __device__ __forceinline__ void gp_cluster_sync() {

@@ -6,10 +6,12 @@
 // rounded the logits to bf16.  Here copies go to shared memory, 160 KB an SM on their way, the first of them before the rows are
 // known, and rows up to 64 are one operand: a tile is 128 vocabulary rows (the MMA's A: TMEM lanes) by 16, 32 or 64 activation rows
 // (its B: TMEM columns), K in stages of 128 values.  The tensor cores' fp32 sums lose 6e-6 of the logits over 5120 terms in a row; so
-// accumulators of 256 values of K each (512 above 16 rows) share it, as the warps of the kernel for rows do, and are added up at the
+// accumulators of 256 values of K each (of 5120 values with 17 to 32 rows 512, above that 640) share it, as the warps of the kernel for rows do, and are added up at the
 // end: 2.5e-7 off 64 bits with 16 rows (3.0e-7 there), 6e-7 with 64 (1.7e-3 with results in bf16).  15 520 x 5120 with its norm, one after the other, us before and
 // here (24 to read): 8 rows 31.6, 35.3; 12 and 16 rows 45.5, 35.6; 32 rows 40.6, 36.7; 64 rows 42.5, 39.5.  In a tick, where the kernel
-// for rows waits: 8 sequences 432 both, 12 sequences 500 and 485, 2 x 8 rows 505 and 492.
+// for rows waits: 8 sequences 432 both, 12 sequences 500 and 485, 2 x 8 rows 505 and 492.  The whole vocabulary, 248 320 x 5120 (394 to read), where a CTA goes
+// through 13 tiles and there is no second accumulator: 8 rows 385, 386; 9 rows 541, 382; 16 rows 532, 387; 17 rows 410, 386; 32 rows 429, 395;
+// 64 rows 505, 437; and 62 080 x 5120 8 rows 110, 117; 16 rows 147, 113; 64 rows 139, 126.
 //
 // Warp roles (192 threads): warp 0 = TMA producer, warp 1 = TMEM owner and MMA issuer, warps 2..5 = epilogue.  Every mbarrier wait is
 // bounded (error word, abort flag, TMEM freed).

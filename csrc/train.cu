@@ -2,7 +2,8 @@
 // softmax and gate, cross-entropy, AdamW over many tensors, each with its gradient.
 //
 // As torch ops each of these was four to forty launches that pass over the rows once apiece, and a step waited for the host.  All
-// are bound by memory: a kernel reads its rows once, keeps them in registers between the passes, and moves 16 bytes a lane.
+// are bound by memory: a kernel reads its rows once and keeps them in registers between the passes; norms, SwiGLU, gate, loss and AdamW
+// move 16 bytes a lane, softmax, the attention's preparation and the outer products 4.  The adapters are bound by what their products read from shared memory.
 // (The dense products beside them stay library GEMMs.)  Sums are in a fixed order; nothing is added with atomics.
 //
 // In the place of the reference's tape handlers and optimizer (src/tilerl/autograd.py:113-301, :466, :661) and its loss
@@ -84,8 +85,8 @@ __global__ void __launch_bounds__(256) tr_swiglu_grad_kernel(const float* gu, co
 // ---- adapters of rank up to 32 ---------------------------------------------------------------------------------------
 // out [M, R] = scale * x [M, K] . A, A(k, r) = a[r][k] or (by_k) a[k][r].  Sixteen rows a block: four rows a warp, two groups of four
 // warps that take every other 128 k and are added up at the end, the lanes share K; 16 ranks a block's y, their factors staged,
-// rows and factors of a group's next 128 on their way meanwhile.  2048 x 6144: 100 us with the loads in the open, 45 with one
-// group, and what the rows take to read is 8.
+// rows and factors of a group's next 128 on their way meanwhile.  2048 x 6144 with 16 ranks: 100 us with the loads in the open, 45 with
+// one group, 31 so; the rows take 8 to read, the products 5.4 at the rate of fp32 FMAs, their factors twice that from shared memory; 32 ranks 56.
 constexpr int LR = 16, LR_T = 128, LR_S = LR_T + 4;
 __global__ void __launch_bounds__(256) tr_lowrank_kernel(const float* x, const float* a, float* out, int M, int K, int R, int by_k, float scale) {
   __shared__ __align__(16) float s[2][2][LR][LR_S];

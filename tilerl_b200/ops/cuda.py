@@ -44,7 +44,8 @@ class ChainOp(ctypes.Structure):
                 ("K", ctypes.c_int), ("epi", ctypes.c_int), ("coop", ctypes.c_int), ("eps", ctypes.c_float)]
 GEMV_MAX_M = 8
 # Rows of bf16 logits that go to the tcgen05 kernel (csrc/head_tc.cu), the lower ones to the kernel for rows: as fast up to 8 rows in a
-# tick of the 27B model (8 sequences 432 us either way), faster there with the small model's short rows (151 us against 160).
+# tick of the 27B model (8 sequences 432 us either way) and alone over its whole vocabulary (385 and 386), faster there with the small
+# model's short rows (151 us against 160).  Nine rows of the whole vocabulary: 541 us there, 382 here.
 HEAD_MIN_M, HEAD_MAX_M = 9, 64
 MMA_MAX_M = 16     # rows served by the mma.sync NVFP4 kernel (csrc/gemv_mma.cu)
 

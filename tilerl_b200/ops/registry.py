@@ -112,7 +112,7 @@ register("nvfp4", "sm100", {
 register("bf16", "sm100", {
     "linear_bf16_gemv": Kernel("gemv_bf16_kernel", "csrc/gemv.cu", "trl_gemv_bf16"),
     "linear_bf16_gemv_rows16": Kernel("gemv_bf16_rows_kernel", "csrc/gemv.cu", "trl_gemv_bf16",
-                                      note="1..16 rows (lm_head): one mma.sync pass over the weights, K shared by a block's warps"),
+                                      note="1..16 rows (lm_head: up to 8): one mma.sync pass over the weights, K shared by a block's warps"),
     "logits_rows64": Kernel("head_bf16_kernel", "csrc/head_tc.cu", "trl_head_bf16", note="lm_head of 9..64 rows: tcgen05 kind::f16, fp32 results"),
     "linear_stream_rows": Kernel("linear_rows_kernel", "csrc/linear_rows.cu", "trl_linear_rows",
                                  note="few rows out of / into an fp32 stream: norm prologue, cp.async weight ring, mma.sync"),
