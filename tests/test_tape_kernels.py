@@ -310,3 +310,23 @@ def test_narrow_rows_and_short_sequences_in_numbers_stay_with_torch(monkeypatch)
     for b, t, nv, want in ((512, 1, 8, False), (512, 8, 8, True), (1, 1, 2, True), (256, 1, 8, True)):
         ch = (2 + nv) * 128
         assert gdn_train.takes(e(b, t, ch + nv * 130), e(ch, 4), e(nv), e(nv), e(128), nk=1, nv=nv, dk=128, dv=128, eps=1e-6) == want
+
+
+def test_tensors_that_autograd_or_inference_mode_keeps_are_refused_as_before(monkeypatch):
+    """A followed leaf, and an inference tensor outside that mode, are not written into by a kernel: torch refuses them."""
+    from tilerl_b200 import optim
+    monkeypatch.setattr(train_kernels, "there", lambda: True), monkeypatch.setattr(train_kernels, "plain", lambda *t: True)
+    monkeypatch.setattr(train_kernels, "adamw", lambda items, *a: [it[0].data.zero_() for it in items])
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True, raising=False)
+    with torch.inference_mode():
+        kept = torch.ones(4)
+    for p in (torch.ones(4, requires_grad=True), kept):
+        with pytest.raises(RuntimeError):
+            optim.AdamW({"w": p}).step({"w": torch.ones(4)})
+    p = torch.ones(4, requires_grad=True)
+    with torch.no_grad():
+        optim.AdamW({"w": p}).step({"w": torch.ones(4)})
+    assert float(p.detach().sum()) == 0.0
+    assert not train_kernels.writable(kept) and train_kernels.writable(torch.ones(4))
+    with torch.inference_mode():
+        assert train_kernels.writable(kept)

@@ -44,6 +44,12 @@ def plain(*tensors) -> bool:
                and t.device.index == torch.cuda.current_device() for t in tensors)
 
 
+def writable(*tensors) -> bool:
+    """Tensors that torch would write into without a word: autograd refuses leaves that it follows (and records the others), inference
+    mode its tensors outside it.  Kernels ask neither."""
+    return not any(t.requires_grad and torch.is_grad_enabled() or t.is_inference() and not torch.is_inference_mode_enabled() for t in tensors)
+
+
 def grad_takes(g: torch.Tensor, out: torch.Tensor) -> bool:
     """A gradient that the kernels can read as that of ``out``: the same shape (torch ops also take one that broadcasts, or a number
     on the CPU; a kernel would read past its end), on the same device, which still is the current one."""

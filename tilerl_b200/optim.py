@@ -36,7 +36,7 @@ def clip_grad_norm(grads: Dict[str, torch.Tensor], max_norm: float, *, sharded: 
     many = None
     if dev.type == "cuda":
         from .ops import train_kernels as many
-        parts = many.squares(grads) if many.there() else None
+        parts = many.squares(grads) if many.there() and many.writable(*grads.values()) else None
         many = many if parts is not None else None
     if many and sharded is None and tp_world <= 1:
         return _scaled(grads, math.sqrt(float(parts.sum())), max_norm, many)
@@ -116,7 +116,7 @@ class AdamW:
                 continue
             if k not in self.m:
                 self.m[k], self.v[k], self.t[k] = torch.zeros_like(p), torch.zeros_like(p), 0
-            if not train_kernels.plain(p, g, self.m[k], self.v[k]) or g.shape != p.shape:
+            if not train_kernels.plain(p, g, self.m[k], self.v[k]) or not train_kernels.writable(p, g, self.m[k], self.v[k]) or g.shape != p.shape:
                 self.step_param(k, g, lr)
                 continue
             self.t[k] += 1
