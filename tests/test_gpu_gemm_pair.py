@@ -95,7 +95,7 @@ def test_one_sm_as_asked_for(ops, monkeypatch):
     x = torch.randn(100, 4128, generator=g).to(DEV, torch.bfloat16)
     want, got = torch.empty(100, 1288, device=DEV), torch.empty(100, 1288, device=DEV)
     gemm_nvfp4(ops, x, w, want, terms=2, epi=3, max_ctas=1, split=False)
-    monkeypatch.setenv("TRL_GEMM_PAIR", "0")
+    monkeypatch.setattr("tilerl_b200.ops.gemm_tc._PAIR", False)
     gemm_nvfp4(ops, x, w, got, terms=2, epi=3, split=False)
     assert torch.equal(got, want)
     gemm_nvfp4(ops, x, w, got, terms=2, epi=3)

@@ -42,12 +42,13 @@ def test_workspace_takes_shapes_of_every_form(monkeypatch):
 
 def test_gemm_on_one_sm_as_asked_for(monkeypatch):
     """``TRL_GEMM_PAIR=0`` keeps every layout off the kernel on pairs; without it nothing changes."""
+    from tilerl_b200.ops import gemm_tc
     from tilerl_b200.ops.gemm_tc import _want_split
-    for pair, forms in (("1", {None: -1, False: 0, True: 1}), ("0", {None: -2, False: 2, True: 1})):
-        monkeypatch.setenv("TRL_GEMM_PAIR", pair)
+    for pair, forms in ((True, {None: -1, False: 0, True: 1}), (False, {None: -2, False: 2, True: 1})):
+        monkeypatch.setattr(gemm_tc, "_PAIR", pair)
         for split, want in forms.items():
             assert _want_split(split) == want
     monkeypatch.setenv("TRL_SPLITK", "0")
     assert _want_split() == 2 and _want_split(True) == 1
-    monkeypatch.delenv("TRL_GEMM_PAIR")
+    monkeypatch.setattr(gemm_tc, "_PAIR", True)
     assert _want_split() == 0

@@ -153,12 +153,15 @@ def _scratch(ops, nbytes: int, tiles: int):
     return buf, ops.ws.bufs["tc_counters"]
 
 
+_PAIR = os.environ.get("TRL_GEMM_PAIR", "1") != "0"       # (asked once: a look at the environment is 0.8 us a product)
+
+
 def _want_split(split: Optional[bool] = None) -> int:
     """How tiles are laid out: 1 split along K on the kernel of one SM, 0 whole, -1 by the launcher's rules (``csrc/gemm_tc.cu::plan_pair``,
     ``plan_gemm``); ``TRL_SPLITK`` forces 1 or 0 where the caller leaves it open.  ``TRL_GEMM_PAIR=0``: 0 and -1 on the kernel of one SM too (2, -2)."""
     mode = os.environ.get("TRL_SPLITK", "auto")
     want = int(split) if split is not None else int(mode) if mode in ("0", "1") else -1
-    return want if os.environ.get("TRL_GEMM_PAIR", "1") != "0" else {0: 2, -1: -2}.get(want, want)
+    return want if _PAIR else {0: 2, -1: -2}.get(want, want)
 
 
 def gemm_nvfp4(ops, x: torch.Tensor, w: NVFP4Tensor, y: torch.Tensor, *, terms: int = 1, norm_w=None,

@@ -40,14 +40,16 @@ def there() -> bool:
 
 def plain(*tensors) -> bool:
     """fp32, contiguous, not empty and on 16-byte boundaries, all on the current CUDA device."""
+    here = torch.cuda.current_device() if tensors and tensors[0].is_cuda else None
     return all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.numel() and t.data_ptr() % 16 == 0
-               and t.device.index == torch.cuda.current_device() for t in tensors)
+               and t.device.index == here for t in tensors)
 
 
 def writable(*tensors) -> bool:
     """Tensors that torch would write into without a word: autograd refuses leaves that it follows (and records the others), inference
     mode its tensors outside it.  Kernels ask neither."""
-    return not any(t.requires_grad and torch.is_grad_enabled() or t.is_inference() and not torch.is_inference_mode_enabled() for t in tensors)
+    followed, outside = torch.is_grad_enabled(), not torch.is_inference_mode_enabled()
+    return not any(followed and t.requires_grad or outside and t.is_inference() for t in tensors)
 
 
 def grad_takes(g: torch.Tensor, out: torch.Tensor) -> bool:
@@ -230,23 +232,30 @@ def scale_by(t, up):
 
 
 # ---- many tensors at a time -------------------------------------------------------------------------------------------
-def _pointers(tensors: Sequence[torch.Tensor]):
-    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+def _addresses(tensors: Sequence[torch.Tensor]) -> List[int]:
+    return [t.data_ptr() for t in tensors]
 
 
-def _lengths(tensors: Sequence[torch.Tensor]):
-    return (ctypes.c_long * len(tensors))(*[t.numel() for t in tensors])
+def _pointers(addresses: Sequence[int]):
+    return (ctypes.c_void_p * len(addresses))(*addresses)
+
+
+def _lengths(lengths: Sequence[int]):
+    return (ctypes.c_long * len(lengths))(*lengths)
 
 
 def _floats(v: Sequence[float]):
     return (ctypes.c_float * len(v))(*v)
 
 
-def apart(written: Sequence[torch.Tensor], read: Sequence[torch.Tensor] = ()) -> bool:
-    """No tensor that is written shares memory with another one (a weight under two names, a gradient given twice): the tensors of a
-    launch are worked on at the same time."""
+def apart(written: Sequence[tuple], read: Sequence[tuple] = ()) -> bool:
+    """Of (address, values) of fp32 tensors: none that is written shares memory with another one (a weight under two names, a gradient given
+    twice), since the tensors of a launch are worked on at the same time."""
+    spans = sorted([(a, a + 4 * n, True) for a, n in written] + [(a, a + 4 * n, False) for a, n in read])
+    if all(x[1] <= y[0] for x, y in zip(spans, spans[1:])):
+        return True
     any_end = written_end = 0
-    for start, end, w in sorted([(t.data_ptr(), t.data_ptr() + t.nbytes, True) for t in written] + [(t.data_ptr(), t.data_ptr() + t.nbytes, False) for t in read]):
+    for start, end, w in spans:
         if start < (any_end if w else written_end):
             return False
         any_end = max(any_end, end)
@@ -256,13 +265,16 @@ def apart(written: Sequence[torch.Tensor], read: Sequence[torch.Tensor] = ()) ->
 
 def adamw(items: List[tuple], lr: float, betas, eps: float) -> None:
     """``items``: (parameter, m, v, gradient, decay factor, 1 - b1^t, 1 - b2^t), tensors plain.  One after the other where some share memory."""
-    most = MAX_TENSORS if apart([t for it in items for t in it[:3]], [it[3] for it in items]) else 1
+    p, m, v, g, decay, c1, c2 = zip(*items)
+    n, at = [t.numel() for t in p], [_addresses(ts) for ts in (p, m, v, g)]
+    most = MAX_TENSORS if apart([x for a in at[:3] for x in zip(a, n)], list(zip(at[3], n))) else 1
     for i in range(0, len(items), most):
-        p, m, v, g, decay, c1, c2 = zip(*items[i:i + most])
-        N.check(N.lib().trl_train_adamw(_pointers(p), _pointers(m), _pointers(v), _pointers(g), _lengths(p), _floats(decay), _floats(c1), _floats(c2),
-                                        len(p), lr, betas[0], 1 - betas[0], betas[1], 1 - betas[1], eps, N.stream()), "train_adamw")
-        torch.autograd.graph.increment_version(p + m + v)         # written in place, as ``copy_`` says it
+        part = slice(i, i + most)
+        ptrs = [_pointers(a[part]) for a in at]
+        N.check(N.lib().trl_train_adamw(*ptrs, _lengths(n[part]), _floats(decay[part]), _floats(c1[part]), _floats(c2[part]),
+                                        len(n[part]), lr, betas[0], 1 - betas[0], betas[1], 1 - betas[1], eps, N.stream()), "train_adamw")
         N.count()
+    torch.autograd.graph.increment_version(p + m + v)             # written in place, as ``copy_`` says it
 
 
 def squares(grads: Dict[str, torch.Tensor]) -> Optional[torch.Tensor]:
@@ -271,11 +283,12 @@ def squares(grads: Dict[str, torch.Tensor]) -> Optional[torch.Tensor]:
     gs = list(grads.values())
     if not gs or not plain(*gs):
         return None
-    blocks = N.lib().trl_train_squares_blocks(max(g.numel() for g in gs))
+    n, at = [g.numel() for g in gs], _addresses(gs)
+    blocks = N.lib().trl_train_squares_blocks(max(n))
     part = torch.empty(len(gs), blocks, dtype=torch.float64, device=gs[0].device)
     for i in range(0, len(gs), MAX_TENSORS):
-        some = gs[i:i + MAX_TENSORS]
-        N.check(N.lib().trl_train_squares(_pointers(some), _lengths(some), len(some), blocks, part[i:].data_ptr(), N.stream()), "train_squares")
+        some = slice(i, i + MAX_TENSORS)
+        N.check(N.lib().trl_train_squares(_pointers(at[some]), _lengths(n[some]), len(n[some]), blocks, part[i:].data_ptr(), N.stream()), "train_squares")
         N.count()
     return part
 
@@ -283,9 +296,10 @@ def squares(grads: Dict[str, torch.Tensor]) -> Optional[torch.Tensor]:
 def scale(tensors: Sequence[torch.Tensor], c: float) -> None:
     """All of them times ``c``, in place (plain ones), one after the other where some share memory."""
     tensors = list(tensors)
-    most = MAX_TENSORS if apart(tensors) else 1
-    for i in range(0, len(tensors), most):
-        some = tensors[i:i + most]
-        N.check(N.lib().trl_train_scale(_pointers(some), _lengths(some), len(some), c, N.stream()), "train_scale")
-        torch.autograd.graph.increment_version(some)
+    n, at = [t.numel() for t in tensors], _addresses(tensors)
+    most = MAX_TENSORS if apart(list(zip(at, n))) else 1
+    for i in range(0, len(n), most):
+        some = slice(i, i + most)
+        N.check(N.lib().trl_train_scale(_pointers(at[some]), _lengths(n[some]), len(n[some]), c, N.stream()), "train_scale")
         N.count()
+    torch.autograd.graph.increment_version(tensors)

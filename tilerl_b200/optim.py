@@ -104,19 +104,18 @@ class AdamW:
         p.copy_(w.to(p.dtype))
 
     def step(self, grads: Dict[str, torch.Tensor], lr: Optional[float] = None) -> None:
+        from .ops import train_kernels
         items, rate, (b1, b2) = [], self.lr if lr is None else lr, self.betas
+        there = any(g.is_cuda for g in grads.values()) and train_kernels.there()
+        free = there and train_kernels.writable(*grads.values(), *self.m.values(), *self.v.values(), *(self.params[k] for k in grads if k in self.params))
         for k, g in grads.items():
             p = self.params[k]
-            if not (p.is_cuda and p.dtype == torch.float32):
-                self.step_param(k, g, lr)
-                continue
-            from .ops import train_kernels
-            if not train_kernels.there():
+            if not (there and p.is_cuda and p.dtype == torch.float32):
                 self.step_param(k, g, lr)
                 continue
             if k not in self.m:
                 self.m[k], self.v[k], self.t[k] = torch.zeros_like(p), torch.zeros_like(p), 0
-            if not train_kernels.plain(p, g, self.m[k], self.v[k]) or not train_kernels.writable(p, g, self.m[k], self.v[k]) or g.shape != p.shape:
+            if not train_kernels.plain(p, g, self.m[k], self.v[k]) or g.shape != p.shape or not (free or train_kernels.writable(p, g, self.m[k], self.v[k])):
                 self.step_param(k, g, lr)
                 continue
             self.t[k] += 1
